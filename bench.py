@@ -39,8 +39,7 @@ METRIC = "atom-steps/s (E+F+stress) & relaxed structures/s vs plain GPU path"
 UNIT = "atom-steps/s"
 WORKLOAD = "CuPdAg fcc 10x10x10 (4000 atoms), 282-10-10-1 FP64, Rc 6 A, NVT 600 K, dt 1 fs"
 SETTLE_STEPS = 20  # untimed NVT steps from the ideal lattice before the warm-up
-KERNEL_NAME = ("descriptor pass: k_legs (leg tables) + k_trip (triplet lists) + k_efs_leg (fused descriptors + "
-               "MLP + forces + virial), timed together")
+KERNEL_NAME = "descriptor pass: k_efs_tri (triplet lists + descriptors + MLP + forces + virial, factors in registers)"
 KERNEL_NAME_NOLEGS = "descriptor pass: k_efs (fused descriptors + MLP + forces + virial)"
 
 
@@ -212,8 +211,8 @@ def measured_peaks():
 
 
 def profile_traffic():
-    """DRAM bytes of one descriptor pass (k_legs + k_trip + k_efs_leg, one
-    ncu capture each) from the committed summary."""
+    """DRAM bytes of one descriptor pass (one ncu capture) from the committed
+    summary."""
     path = os.path.join(ROOT, "profiles", "descriptor_pass_md4000.md")
     try:
         for line in open(path):

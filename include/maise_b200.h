@@ -290,10 +290,10 @@ int mb_graphs(mb_potential *p, int enable);
  * `capacity` launches), and the kernel's pair/triplet counters are reset. */
 /* The autotuner's decisions so far: *count (at most cap) entries; entry k
  * holds the pass mode (0 descriptors, 1 energy, 2 E/F/S, 3 VJP), whether the
- * leg-table kernel ran (legs), the size bucket (N <= 2^bucket), the
- * neighbour capacity, the chosen shape (warps per atom, atoms per CTA) and
- * the leg kernel's reverse-pass layout (0 per-lane runs of list entries,
- * 1 consecutive entries per round). */
+ * fused triplet kernel of the reference bases ran (legs) or the general one,
+ * the size bucket (N <= 2^bucket), the neighbour capacity, the chosen shape
+ * (warps per atom, atoms per CTA) and the reverse pass's layout (0 per-lane
+ * runs of list entries, 1 consecutive entries per round). */
 int mb_tune_read(const mb_potential *pot, int cap, int *count, int *mode, int *legs, int *size_bucket, int *capacity,
                  int *wpa, int *apb, int *layout);
 int mb_profile(mb_potential *pot, int enable, int capacity);

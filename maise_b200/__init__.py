@@ -217,7 +217,8 @@ class Potential:
     def tune_table(self):
         """The autotuner's choices: list of dict(mode, legs, size_bucket,
         capacity, wpa, apb, layout), modes 'descriptors', 'energy', 'efs',
-        'vjp'; layout is the leg kernel's reverse pass ('runs' or 'rounds')."""
+        'vjp'; legs tells the fused triplet kernel (reference bases) from the
+        general one, layout its reverse pass ('rounds') from that one's ('runs')."""
         cap = 32
         cols = [np.zeros(cap, np.int32) for _ in range(7)]
         cnt = ctypes.c_int()

@@ -5,7 +5,10 @@
  *   k_nlist_brute   all (atom, image) pairs within Rc (LIST, src/cell.c:82-185)
  *   k_cell_*        integer cell-list build (bin, count, scan, fill) and
  *   k_nlist_cell    the same neighbour set from the 27 adjacent cells
- *   k_efs           one CTA per central atom: G2/G4 descriptors
+ *   k_efs_tri       the descriptor pass of the reference bases: per atom the
+ *                   triplet list, descriptors, MLP and reverse pass below with
+ *                   every factor of a triplet evaluated in registers
+ *   k_efs           one CTA per central atom, any basis: G2/G4 descriptors
  *                   (src/nprs.c:500-566), MLP forward and dE/dG
  *                   (src/nmlp.c:367-431), then the reverse pass that turns
  *                   dE_i/dG_i into forces on i and its neighbours and the
@@ -87,16 +90,9 @@ __device__ __forceinline__ double image_disp(const mb_cell &c, const double *xi,
     return r;
 }
 
-/* key of a list entry for the leg-table path: atom j and its integer image
- * (5 bits per axis, two's complement) */
-__device__ __forceinline__ unsigned entry_key(int j, int i0, int i1, int i2) {
-    return ((unsigned)j << 15) | (((unsigned)i0 & 31u) << 10) | (((unsigned)i1 & 31u) << 5) | ((unsigned)i2 & 31u);
-}
-
 /* one warp per atom; candidates in the reference's order (j, then images) */
 __global__ void k_nlist_brute(int N, int NM, int cap, const double *__restrict__ X, mb_cell c, double rc2,
-                              int *__restrict__ nn, int *__restrict__ nj, double4 *__restrict__ nd, int *status,
-                              unsigned *__restrict__ nk) {
+                              int *__restrict__ nn, int *__restrict__ nj, double4 *__restrict__ nd, int *status) {
     int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (warp >= N) return;
     int i = warp;
@@ -128,7 +124,6 @@ __global__ void k_nlist_brute(int N, int NM, int cap, const double *__restrict__
         if (ok && pos < cap) {
             nj[(size_t)i * cap + pos] = j;
             nd[(size_t)i * cap + pos] = make_double4(d[0], d[1], d[2], sqrt(r2));
-            if (nk) nk[(size_t)i * cap + pos] = entry_key(j, i0, i1, i2);
         }
         count += __popc(m);
     }
@@ -249,7 +244,7 @@ __global__ void k_cell_sort(int ncell, const int *start, int *atoms) {
 __global__ void k_nlist_cell(int N, int NM, int cap, const double *__restrict__ X, mb_cell c, double rc2,
                              const int *__restrict__ cell_of, const int *__restrict__ start,
                              const int *__restrict__ atoms, int *__restrict__ nn, int *__restrict__ nj,
-                             double4 *__restrict__ nd, int *status, unsigned *__restrict__ nk) {
+                             double4 *__restrict__ nd, int *status) {
     __shared__ int s_off[4][32], s_lo[4][32], s_img[4][32];
     const int w = (threadIdx.x >> 5) & 3;
     int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
@@ -321,7 +316,6 @@ __global__ void k_nlist_cell(int N, int NM, int cap, const double *__restrict__ 
         if (ok && pos < cap) {
             nj[(size_t)i * cap + pos] = j;
             nd[(size_t)i * cap + pos] = make_double4(d[0], d[1], d[2], sqrt(r2));
-            if (nk) nk[(size_t)i * cap + pos] = entry_key(j, img[0], img[1], img[2]);
         }
         count += __popc(m);
     }
@@ -543,6 +537,23 @@ __device__ __forceinline__ void warp_reduce64(double *v, int lane) {
             v[k] = keep + __shfl_xor_sync(FULL, send, off);
         }
     }
+}
+
+/* Sum of 16 per-lane values across a warp: lanes l and l ^ 1 end with the
+ * total of value l >> 1 (four halving steps and one exchange). */
+__device__ __forceinline__ double warp_reduce16(double *v, int lane) {
+#pragma unroll
+    for (int step = 0; step < 4; step++) {
+        const int off = 16 >> step, half = 8 >> step;
+        const bool upper = (lane & off) != 0;
+#pragma unroll
+        for (int k = 0; k < half; k++) {
+            const double send = upper ? v[k] : v[k + half];
+            const double keep = upper ? v[k + half] : v[k];
+            v[k] = keep + __shfl_xor_sync(FULL, send, off);
+        }
+    }
+    return v[0] + __shfl_xor_sync(FULL, v[0], 1);
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -1246,617 +1257,470 @@ __global__ void __launch_bounds__(WPA * 32 * APB, APB >= 4 ? 2 : 1) k_efs(EfsArg
 }
 
 /* ------------------------------------------------------------------ */
-/* leg-table path of the descriptor pass                                */
+/* fused triplet kernel (reference bases)                               */
 /* ------------------------------------------------------------------ */
 
-/* A triplet (i; j, k) of PRS_BP has three legs, i-j, i-k and j-k, and each
- * leg's factors -- exp(-eta_e r^2) for the G4 exponents and the cutoff fc(r)
- * (src/nprs.c:540-547) -- depend only on that pair.  The j-k leg is an entry
- * of j's own neighbour list, and each such entry serves every atom that has
- * both j and k as neighbours (about 29 triplets in a dense alloy).  k_legs
- * evaluates the factors once per list entry; k_efs_leg reads the j-k leg of
- * each triplet from j's row instead of evaluating it, and finds that row by
- * walking j's list and looking each entry up in a hash of i's own entries
- * keyed by (atom, image).  The walk enumerates exactly the triplets with
- * both r_ik < Rc (k is found in i's list) and r_jk < Rc (k is in j's list).
+/* k_efs_tri: the whole descriptor pass of an atom -- neighbour sort, G2,
+ * triplet list, forward grid, MLP, reverse pass -- with every factor of a
+ * triplet evaluated in registers.  It applies to bases whose forward and
+ * derivative functions share one cutoff and whose pair-mixed G4 exponents
+ * equal the species-0 ones (every reference model; src/nprs.c:222-252 mixes
+ * identical blocks), see mb_tri.
  *
- * The path applies to bases whose forward and derivative functions share one
- * cutoff and whose pair-mixed G4 exponents equal the species-0 ones (every
- * reference model; src/nprs.c:222-252 mixes identical blocks), so a leg's
- * factors serve the energy and the derivative terms alike. */
+ * What bounds it: instruction issue and the latency of dependent FP64
+ * operations at the 14 warps per SM that shared memory and 128 registers a
+ * thread allow (the 4000-atom ternary alloy, 2 warps per atom: issue slots 46%
+ * busy, FP64 pipe 33%, 1450 instructions per 32 triplets, of them 470 FP64).
+ * The j-k leg of a triplet is an entry of j's own list, and an earlier form of
+ * this pass looked its factors up there (leg tables and triplet lists in
+ * global memory, found through hashes, in three kernels): nine 16-byte loads a
+ * triplet from scattered 80-byte rows kept the L1 pipe 67% busy, and listing
+ * the triplets took a kernel of its own.  Here exp(-eta_e rho) and the cutoff
+ * are polynomials of the squared distances (mb_tri), about 100 FMAs in 7
+ * independent chains: no table, no square root, no trigonometry and no memory
+ * traffic per triplet.  The pass over that alloy went from 520 to 375 us, over
+ * the 20000-atom particle from 1.20 to 0.87 ms, over a 487-atom alloy from 140
+ * to 75 us. */
 
-#define LEG_PER_LANE (MB_LEG_MAX_CAP / 32)
-#define LEG_HASH 256 /* hash slots per atom: at least twice the neighbour capacity */
+#define TRI_ROW 10                        /* doubles of a neighbour's row; 80 bytes: 16-byte loads of
+                                           * consecutive rows fall in distinct banks */
+#define TRI_PER_LANE (MB_TRI_MAX_CAP / 32)
+#define TRI_NONE 0xffffu                  /* padding entry of a triplet list */
 
-
-__device__ __forceinline__ unsigned hash_slot(unsigned key) { return (key * 0x9E3779B1u) >> 24; }
-
-/* One warp per atom: sort the atom's entries stably by the neighbour's
- * species (in place: nj, nk, nd), record where each species starts
- * (nso[4i+s]; nso[4i+3] = count), write each entry's leg row with the
- * forward parameters of the pair (i, j): exp(-eta_e r^2) for e < ne (0
- * above), fc(r) and fc'(r)/r at the G4 cutoff, and put the entries' keys
- * (atom, image) with their sorted slots into the atom's hash
- * gh[i * LEG_HASH ..] (linear probing), where k_trip looks a neighbour's
- * neighbours up. */
-__global__ void k_legs(int N, int cap, const int *__restrict__ nn, int *__restrict__ nj, unsigned *__restrict__ nk,
-                       double4 *__restrict__ nd, const int *__restrict__ spc, const mb_params *__restrict__ Pg,
-                       double *__restrict__ leg, int *__restrict__ nso, uint2 *__restrict__ gh) {
-    /* the hash is built in shared memory, then copied out whole */
-    __shared__ uint2 hsh[4][LEG_HASH];
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= N) return;
-    const int i = warp, n = nn[i], s0 = spc[i], ne = Pg->ne;
-    const size_t row = (size_t)i * cap;
-    uint2 *hash = hsh[(threadIdx.x >> 5) & 3];
-    for (int t = lane; t < LEG_HASH; t += 32) hash[t] = make_uint2(0xffffffffu, 0u);
-    int jv[LEG_PER_LANE], spv[LEG_PER_LANE];
-    unsigned kv[LEG_PER_LANE];
-    double4 dv[LEG_PER_LANE];
-    int cnt[MB_MAXSPC] = {0, 0, 0};
-#pragma unroll
-    for (int q = 0; q < LEG_PER_LANE; q++) {
-        const int t = q * 32 + lane;
-        spv[q] = -1;
-        jv[q] = 0;
-        kv[q] = 0u;
-        dv[q] = make_double4(0.0, 0.0, 0.0, 1.0);
-        if (t < n) {
-            jv[q] = nj[row + t];
-            kv[q] = nk[row + t];
-            dv[q] = nd[row + t];
-            spv[q] = spc[jv[q]];
-        }
-#pragma unroll
-        for (int v = 0; v < MB_MAXSPC; v++) cnt[v] += __popc(__ballot_sync(FULL, spv[q] == v));
-    }
-    int off[MB_MAXSPC + 1];
-    off[0] = 0;
-#pragma unroll
-    for (int v = 0; v < MB_MAXSPC; v++) off[v + 1] = off[v] + cnt[v];
-    if (lane < 4) nso[4 * i + lane] = off[lane];
-    __syncwarp();
-    const unsigned below = (1u << lane) - 1u;
-    int run[MB_MAXSPC] = {0, 0, 0};
-#pragma unroll
-    for (int q = 0; q < LEG_PER_LANE; q++) {
-        int dst = 0;
-#pragma unroll
-        for (int v = 0; v < MB_MAXSPC; v++) {
-            const unsigned m = __ballot_sync(FULL, spv[q] == v);
-            if (spv[q] == v) dst = off[v] + run[v] + __popc(m & below);
-            run[v] += __popc(m);
-        }
-        if (spv[q] >= 0) {
-            nj[row + dst] = jv[q];
-            nk[row + dst] = kv[q];
-            nd[row + dst] = dv[q];
-            {
-                unsigned h = hash_slot(kv[q]);
-                for (int probe = 0; probe < LEG_HASH; probe++) {
-                    if (atomicCAS(&hash[h].x, 0xffffffffu, kv[q]) == 0xffffffffu) {
-                        hash[h].y = (unsigned)dst;
-                        break;
-                    }
-                    h = (h + 1u) & (LEG_HASH - 1u);
-                }
-            }
-            const int p = s0 * s0 + spv[q] * spv[q];
-            const double r = dv[q].w;
-            double f, df;
-            fcut_d(Pg->f_rc4[p], r, f, df);
-            double e[MB_LEG_STRIDE];
-#pragma unroll
-            for (int k = 0; k < 8; k++) e[k] = k < ne ? exp(-Pg->f_eta4[p][k] * r * r) : 0.0;
-            e[8] = f;
-            e[9] = df / r;
-            /* with at most 7 exponents slot 7 is free: fc again, so that the
-             * forward pass reads 4 of a row's 5 16-byte pieces */
-            if (ne <= 7) e[7] = f;
-            double2 *o = reinterpret_cast<double2 *>(leg + (row + dst) * MB_LEG_STRIDE);
-#pragma unroll
-            for (int k = 0; k < MB_LEG_STRIDE / 2; k++) o[k] = make_double2(e[2 * k], e[2 * k + 1]);
-        }
-    }
-    __syncwarp();
-    uint2 *out = gh + (size_t)i * LEG_HASH;
-    for (int t = lane; t < LEG_HASH; t += 32) out[t] = hash[t];
-}
-
-struct LegArgs {
-    int N, cap, mode;
+struct TriArgs {
+    int N, cap, mode, tlw; /* tlw: list entries of one warp */
     double urep;
-    const int *nn, *nj, *nso;
+    const int *nn, *nj;
     const double4 *nd;
-    const double *leg;
-    const uint2 *trip; /* triplet lists (k_trip) */
-    const int *tboff;
-    int tcap;
     const int *spc;
-    const mb_params *params;
-    const double *weights;
+    const double *weights, *w0; /* w0: first-layer weights by input (mb_tri) */
     double *EA, *EU, *G, *F, *vir;
     unsigned long long *counters;
     size_t smem_group;
     mb_params P; /* by value: read from the kernel-parameter space through the constant cache */
+    mb_tri T;
 };
 
-/* Row of one list entry in k_efs_leg's shared memory: x, y, z, 1/r as two
- * 16-byte loads, then r and a pad.  At 48 bytes a row, the 16-byte loads
- * of 8 consecutive entries (a quarter-warp) fall in distinct banks; rows of
- * 32 bytes (a double4) conflicted 2-way. */
-#define LEG_DROW 6
-__device__ __forceinline__ double4 leg_vec(const double *d, int u) {
-    const double2 *p = reinterpret_cast<const double2 *>(d + LEG_DROW * u);
-    const double2 a = p[0], b = p[1];
-    return make_double4(a.x, a.y, b.x, b.y);
-}
+#define TRI_STG 36 /* staging: [16 values][TRI_STG triplets]; both the lane-wise writes and the
+                    * mma operand reads touch 16 distinct banks a half-warp */
+#define TRI_TS 20  /* row stride of the reverse pass's 8 x 16 tiles (4 mod 16: operand reads of the
+                    * tile and of its transpose are conflict-free) */
 
-/* shared-memory carve-up of one atom group of k_efs_leg */
-struct LegSmem {
-    double *stage;                          /* tensor-core staging (forward) | */
-    double *Fnb, *grid, *red, *h;           /* reductions, MLP, reverse pass   */
-    double *d;                              /* per entry x, y, z, 1/r, r, 0    */
-    double *L, *G;
-    double *tmp;                            /* G2 terms (in the stage region) */
-    int *j, *sp, *seg;
+/* shared-memory carve-up of one atom group of k_efs_tri; regions whose
+ * lifetimes do not overlap share storage */
+struct TriSmem {
+    double *row;        /* [cap][TRI_ROW]: x, y, z, 1/r, r^2, f, h, r */
+    double *stage;      /* per warp TRI_STG x 16 (forward) | */
+    double *G, *h, *hp; /* descriptors or dE/dG, hidden layers and their partial sums | */
+    double *tile;       /* per warp 3 x 8 x TRI_TS (reverse) */
+    double *red;        /* [warp][block][64] forward sums | */
+    double *Fnb, *grid; /* neighbour forces per warp [cap][4], dE/dG by (eta, zeta, lambda) cell per block */
+    double *g2;         /* [warp][species][ng2] | */
+    double *fin;        /* [warp][9] */
+    unsigned short *tl; /* [warp][tlw] triplets a | b << 8 */
+    int *j;
+    int *bnd;           /* [warp][8] starts of the species blocks in the warp's list, and the end */
+    int *seg;           /* [0..3] counts, [4..7] offsets by relative species */
 };
 
-/* The G2 terms (tmp) are read before the forward triplets start, so they
- * share the region of the staging rows and the later reductions. */
-__host__ __device__ inline size_t leg_union_bytes(int cap, int ng2, int warps) {
-    const size_t u = efs_union_bytes(cap, 64, warps, 1), t = align16(sizeof(double) * cap * (ng2 > 1 ? ng2 : 1));
-    return u > t ? u : t;
+__host__ __device__ inline int tri_nblk(int ns) { return ns * (ns + 1) / 2; }
+
+/* list entries of one warp: it takes every warps-th group of 4 columns, and
+ * column b of the upper triangle holds b pairs; up to 3 padding entries per
+ * species block */
+__host__ __device__ inline int tri_list(int cap, int warps) {
+    int most = 0;
+    for (int w = 0; w < warps; w++) {
+        int sum = 0;
+        for (int b = 4 * w; b < cap; b += 4 * warps) sum += 4 * b + 6;
+        most = sum > most ? sum : most;
+    }
+    return (most + 4 * MB_MAX_BLOCKS + 7) & ~7;
 }
 
-__host__ __device__ inline size_t leg_smem_bytes(int cap, int D, int ng2, int warps) {
-    size_t b = leg_union_bytes(cap, ng2, warps);
-    b += sizeof(double) * cap * LEG_DROW;                      /* d */
-    b += sizeof(double) * cap * MB_LEG_STRIDE;                 /* L */
-    b += align16(sizeof(double) * D);                          /* G */
-    b += align16(sizeof(int) * cap) * 2;                       /* j, sp */
-    b += sizeof(int) * 8;                                      /* seg */
-    return align16(b);
+__host__ __device__ inline size_t tri_r1_bytes(int D, int warps) {
+    const size_t st = sizeof(double) * warps * 16 * TRI_STG;
+    const size_t mid = sizeof(double) * (D + (D & 1) + 4 * MB_MAXH + 16 * warps);
+    const size_t ti = sizeof(double) * warps * 24 * TRI_TS;
+    return align16(st > mid ? (st > ti ? st : ti) : (mid > ti ? mid : ti));
 }
 
-__device__ inline LegSmem leg_carve(char *base, int cap, int D, int ng2, int warps) {
-    LegSmem s;
-    char *p = base;
+__host__ __device__ inline size_t tri_r2_bytes(int cap, int ns, int warps) {
+    const size_t red = sizeof(double) * warps * tri_nblk(ns) * 64;
+    const size_t rev = sizeof(double) * (64 * tri_nblk(ns) + 4 * cap * warps);
+    return align16(red > rev ? red : rev);
+}
+
+__host__ __device__ inline size_t tri_small(int ns, int ng2, int warps) {
+    const int g2 = ns * ng2 > 9 ? ns * ng2 : 9;
+    return align16(sizeof(double) * warps * g2);
+}
+
+__host__ __device__ inline size_t tri_smem_bytes(int cap, int D, int ns, int ng2, int warps) {
+    return align16(sizeof(double) * cap * TRI_ROW + tri_r1_bytes(D, warps) + tri_r2_bytes(cap, ns, warps) +
+                   tri_small(ns, ng2, warps) + align16(sizeof(short) * tri_list(cap, warps) * warps) +
+                   align16(sizeof(int) * cap) + sizeof(int) * (8 * warps + 8));
+}
+
+__device__ inline TriSmem tri_carve(char *p, int cap, int D, int ns, int ng2, int warps, int tlw) {
+    TriSmem s;
+    s.row = (double *)p; p += sizeof(double) * cap * TRI_ROW;
     s.stage = (double *)p;
-    s.Fnb = (double *)p;
-    s.grid = s.Fnb + cap * 3;
-    s.red = s.grid + 64;
-    s.h = s.red + warps * 64;
-    s.tmp = (double *)p;
-    p += leg_union_bytes(cap, ng2, warps);
-    s.d = (double *)p; p += sizeof(double) * cap * LEG_DROW;
-    s.L = (double *)p; p += sizeof(double) * cap * MB_LEG_STRIDE;
-    s.G = (double *)p; p += align16(sizeof(double) * D);
+    s.tile = (double *)p;
+    s.G = (double *)p;
+    s.h = s.G + D + (D & 1);
+    s.hp = s.h + 4 * MB_MAXH;
+    p += tri_r1_bytes(D, warps);
+    s.red = (double *)p;
+    s.grid = (double *)p;
+    s.Fnb = s.grid + 64 * tri_nblk(ns);
+    p += tri_r2_bytes(cap, ns, warps);
+    s.g2 = (double *)p;
+    s.fin = (double *)p;
+    p += tri_small(ns, ng2, warps);
+    s.tl = (unsigned short *)p; p += align16(sizeof(short) * tlw * warps);
     s.j = (int *)p; p += align16(sizeof(int) * cap);
-    s.sp = (int *)p; p += align16(sizeof(int) * cap);
+    s.bnd = (int *)p; p += sizeof(int) * 8 * warps;
     s.seg = (int *)p;
     return s;
 }
 
-
-/* Triplet lists of the leg path: one warp per atom i, TRIP_WARPS atoms per
- * CTA.  PRS_BP takes the triplet (j, k) of i when NDX[i][j] and NDX[i][k]
- * are below the G4 cutoff and so is ndx[i][j][k] = |DX_j - DX_k|, both
- * displacements from i's list (src/nprs.c:528-537, src/cell.c:175-181).
- * The warp stages i's entries in relative-species order (position u, the
- * order k_efs_leg stages them in: relative species v holds absolute
- * species (s0 + v) % ns) and walks, per species block (alpha <= beta), the
- * pairs (a, b), b > a, 32 per round, with that test: the squared distance
- * summed without contraction as the reference forms it, compared with the
- * threshold for which sqrt(s) < Rc holds exactly.  An accepted pair's j-k
- * leg row is the entry of k (its atom at the image shift(b) - shift(a)) in
- * j's own list, found in j's hash (k_legs); a pair whose k is not in j's
- * list lies within rounding of the cutoff, where fc vanishes, and is left
- * out.  Entries {a | b << 8, j cap + c} are written in pair order (a, then
- * b), so every list is deterministic and at most cap (cap - 1) / 2 long;
- * tboff[8 i + blk] holds each block's start and tboff[8 i + nblk] the end.
- * counters[1] (if set) receives the number of triplets. */
-/* 4 atoms per CTA: the CTAs all fit in one wave either way, and with
- * smaller CTAs the SMs' shares of the 4000-atom alloy differ by 4 warps
- * instead of 8 (about 7 us faster a pass than 8 atoms per CTA; 2 per CTA
- * was no faster than 4) */
-#define TRIP_WARPS 4
-
-/* The 15-bit image field of an entry key (three 5-bit two's-complement
- * shifts) as three biased (x + 16) 7-bit fields, so that shifts add and
- * subtract as integers. */
-__device__ __forceinline__ unsigned spread_img(unsigned key) {
-    const unsigned f = (key & 0x7fffu) ^ 0x4210u; /* x + 16 per field */
-    return (f & 31u) | ((f & (31u << 5)) << 2) | ((f & (31u << 10)) << 4);
+/* exp(-eta_e rho) for e < NE: the chains run side by side over one
+ * coefficient at a time (two per 16-byte shared load) */
+template <int NE, int NSQ>
+__device__ __forceinline__ void tri_exp(const mb_tri_tab &tab, int nsq, double rho, double *E) {
+    const double2 *c = reinterpret_cast<const double2 *>(tab.ex), *kw = reinterpret_cast<const double2 *>(tab.kw);
+    double w[NE];
+#pragma unroll
+    for (int e = 0; e < NE; e += 2) {
+        const double2 k = kw[e / 2];
+        w[e] = fma(k.x, rho, -1.0);
+        if (e + 1 < NE) w[e + 1] = fma(k.y, rho, -1.0);
+    }
+#pragma unroll
+    for (int k = 0; k <= MB_TRI_DEG; k += 2) {
+        const double2 ck = c[k / 2];
+#pragma unroll
+        for (int e = 0; e < NE; e++) E[e] = k ? fma(E[e], w[e], ck.x) : ck.x;
+#pragma unroll
+        for (int e = 0; e < NE; e++) E[e] = fma(E[e], w[e], ck.y);
+    }
+    if constexpr (NSQ >= 0) {
+#pragma unroll
+        for (int q = 0; q < NSQ; q++)
+#pragma unroll
+            for (int e = 0; e < NE; e++) E[e] *= E[e];
+    } else {
+        for (int q = 0; q < nsq; q++)
+#pragma unroll
+            for (int e = 0; e < NE; e++) E[e] *= E[e];
+    }
 }
-#define IMG_48 (48u | (48u << 7) | (48u << 14))
-#define IMG_BIT5 ((1u << 5) | (1u << 12) | (1u << 19))
-#define IMG_BIT6 ((1u << 6) | (1u << 13) | (1u << 20))
 
-__global__ void __launch_bounds__(32 * TRIP_WARPS) k_trip(int N, int cap, int tcap, int ns, const int *__restrict__ nn,
-                                                          const int *__restrict__ nj, const unsigned *__restrict__ nk,
-                                                          const double4 *__restrict__ nd, const int *__restrict__ nso,
-                                                          const int *__restrict__ spc, const mb_params *__restrict__ Pg,
-                                                          const uint2 *__restrict__ gh, uint2 *__restrict__ trip,
-                                                          int *__restrict__ tboff, unsigned long long *counters) {
-    __shared__ double4 sd[TRIP_WARPS][MB_LEG_MAX_CAP];
-    __shared__ unsigned skey[TRIP_WARPS][MB_LEG_MAX_CAP];
-    __shared__ int sj[TRIP_WARPS][MB_LEG_MAX_CAP];
-    __shared__ int sseg[TRIP_WARPS][8];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int i = blockIdx.x * TRIP_WARPS + w;
-    if (i >= N) return; /* whole warps; nothing below synchronises the CTA */
-    double4 *d = sd[w];
-    unsigned *key = skey[w];
-    int *js = sj[w], *seg = sseg[w];
-    const int n = nn[i], s0 = spc[i];
-    const size_t row = (size_t)i * cap;
-    if (lane < 4) {
-        const int v = lane, sa = (s0 + v) % ns;
-        int c = 0, o = 0;
-        if (v < ns) c = nso[4 * i + sa + 1] - nso[4 * i + sa];
-        for (int u = 0; u < v; u++) {
-            const int su = (s0 + u) % ns;
-            o += nso[4 * i + su + 1] - nso[4 * i + su];
-        }
-        seg[v] = c;
-        seg[4 + v] = v < ns ? o : n;
+__device__ __forceinline__ double tri_f(const mb_tri_tab &tab, double v) {
+    const double2 *c = reinterpret_cast<const double2 *>(tab.f);
+    double p = fma(c[0].x, v, c[0].y);
+#pragma unroll
+    for (int k = 1; k <= MB_TRI_FDEG / 2; k++) p = fma(fma(p, v, c[k].x), v, c[k].y);
+    return p;
+}
+
+__device__ __forceinline__ double2 tri_fh(const mb_tri_tab &tab, double v) {
+    const double2 *c = reinterpret_cast<const double2 *>(tab.fh);
+    double2 p = c[0];
+#pragma unroll
+    for (int k = 1; k <= MB_TRI_FDEG; k++) {
+        const double2 ck = c[k];
+        p.x = fma(p.x, v, ck.x);
+        p.y = fma(p.y, v, ck.y);
     }
-    __syncwarp();
-    for (int u = lane; u < n; u += 32) {
-        int v = 0;
-        while (v + 1 < ns && u >= seg[4 + v + 1]) v++;
-        const int sa = (s0 + v) % ns;
-        const int t = nso[4 * i + sa] + (u - seg[4 + v]);
-        d[u] = nd[row + t];
-        key[u] = nk[row + t];
-        js[u] = nj[row + t];
-    }
-    __syncwarp();
-    uint2 *out = trip + (size_t)i * tcap;
-    int pos = 0, blkid = 0;
-    for (int al = 0; al < ns; al++)
-        for (int be = al; be < ns; be++, blkid++) {
-            if (lane == 0) tboff[8 * i + blkid] = pos;
-            const int sj_ = (s0 + al) % ns, sk_ = (s0 + be) % ns;
-            const int p01 = s0 * s0 + sj_ * sj_, p02 = s0 * s0 + sk_ * sk_, p12 = sj_ * sj_ + sk_ * sk_;
-            const double R01 = __ldg(&Pg->f_rc4[p01]), R02 = __ldg(&Pg->f_rc4[p02]);
-            const double thr = __ldg(&Pg->f_rc4thr[p12]);
-            const int na = seg[al], nb = seg[be], oa = seg[4 + al], ob = seg[4 + be];
-            const bool tri = al == be;
-            const int C = tri ? na * (na - 1) / 2 : na * nb;
-            /* the lane's candidates are c = lane, lane + 32, ...: candidate c
-             * is row r, position p of the block (row r of the strict upper
-             * triangle holds na - 1 - r pairs starting at column r + 1; a
-             * rectangular block's rows hold nb), and the cursor (r, p)
-             * moves on by 32 per candidate; it never passes the last row */
-            const int rmax = tri ? na - 2 : na - 1;
-            int r = 0, p = lane;
-            if (C > 0)
-                while (p >= (tri ? na - 1 - r : nb) && r < rmax) {
-                    p -= tri ? na - 1 - r : nb;
-                    r++;
-                }
-            /* two candidate pairs per lane and iteration (c and c + 32): both
-             * first hash probes are in flight together; entries are still
-             * written in candidate order */
-            for (int base = 0; base < C; base += 64) {
-                unsigned kk[2], h[2], ax[2], jx[2];
-                const uint2 *hj[2];
-                bool live[2];
+    return p;
+}
+
+/* (1 + lambda c)^zeta without its normalisation, and the derivative in c.
+ * STD: zeta = 1, 2, 4, 16 and lambda = -1, +1 (the reference bases), straight
+ * multiplications; otherwise any integer zeta. */
+template <bool STD>
+__device__ __forceinline__ void tri_angular(const mb_params &P, double c, double *lz, double *lzp) {
+    if constexpr (STD) {
 #pragma unroll
-                for (int q = 0; q < 2; q++) {
-                    const int c = base + 32 * q + lane;
-                    live[q] = false;
-                    kk[q] = 0u;
-                    h[q] = 0u;
-                    ax[q] = 0u;
-                    jx[q] = 0u;
-                    hj[q] = gh;
-                    if (c < C) {
-                        const int col = tri ? r + 1 + p : p;
-                        const int a = oa + r, b = ob + col;
-                        const double4 da = d[a], db = d[b];
-                        const double dx = xsub(da.x, db.x), dy = xsub(da.y, db.y), dz = xsub(da.z, db.z);
-                        const double s2 = xadd(xadd(xmul(dx, dx), xmul(dy, dy)), xmul(dz, dz));
-                        if (da.w < R01 && db.w < R02 && s2 < thr) {
-                            const unsigned ka = key[a], kb = key[b];
-                            const unsigned t = IMG_48 + spread_img(kb) - spread_img(ka);
-                            if ((t & IMG_BIT6) == 0u && (t & IMG_BIT5) == IMG_BIT5) {
-                                const unsigned f = (t & 31u) | ((t >> 2) & (31u << 5)) | ((t >> 4) & (31u << 10));
-                                kk[q] = (kb & ~0x7fffu) | (f ^ 0x4210u); /* k at its image relative to j */
-                                const int j = js[a];
-                                jx[q] = (unsigned)j;
-                                hj[q] = gh + (size_t)j * LEG_HASH;
-                                h[q] = hash_slot(kk[q]);
-                                ax[q] = (unsigned)a | ((unsigned)b << 8);
-                                live[q] = true;
-                            }
-                        }
-                    }
-                    p += 32;
-                    while (p >= (tri ? na - 1 - r : nb) && r < rmax) {
-                        p -= tri ? na - 1 - r : nb;
-                        r++;
-                    }
-                }
-                uint2 e[2];
-#pragma unroll
-                for (int q = 0; q < 2; q++) e[q] = live[q] ? __ldg(hj[q] + h[q]) : make_uint2(0xffffffffu, 0u);
-#pragma unroll
-                for (int q = 0; q < 2; q++) {
-                    bool ok = false;
-                    uint2 ent = make_uint2(0u, 0u);
-                    if (live[q]) {
-                        /* the first probe is in e[q]; at most LEG_HASH probes in all */
-                        uint2 x = e[q];
-                        unsigned hq = h[q];
-                        for (int probe = 0; probe < LEG_HASH; probe++) {
-                            if (x.x == kk[q]) {
-                                ok = true;
-                                ent = make_uint2(ax[q], jx[q] * (unsigned)cap + x.y);
-                                break;
-                            }
-                            if (x.x == 0xffffffffu) break;
-                            hq = (hq + 1u) & (LEG_HASH - 1u);
-                            x = __ldg(hj[q] + hq);
-                        }
-                    }
-                    const unsigned m = __ballot_sync(FULL, ok);
-                    if (ok) out[pos + __popc(m & ((1u << lane) - 1u))] = ent;
-                    pos += __popc(m);
-                }
+        for (int l = 0; l < 2; l++) {
+            const double lam = l ? 1.0 : -1.0, b1 = 1.0 + lam * c, b2 = b1 * b1, b4 = b2 * b2, b8 = b4 * b4;
+            lz[l] = b1;
+            lz[2 + l] = b2;
+            lz[4 + l] = b4;
+            lz[6 + l] = b8 * b8;
+            if (lzp) {
+                const double b3 = b1 * b2;
+                lzp[l] = lam;
+                lzp[2 + l] = 2.0 * lam * b1;
+                lzp[4 + l] = 4.0 * lam * b3;
+                lzp[6 + l] = 16.0 * lam * (b4 * b8) * b3;
             }
         }
-    if (lane == 0) {
-        tboff[8 * i + blkid] = pos;
-        if (counters) atomicAdd(&counters[1], (unsigned long long)pos);
-    }
-}
-
-/* body(ent) -> the entry's force on neighbour a, over list entries
- * [from, to): each lane takes a contiguous run of K entries (K odd);
- * consecutive entries mostly share a, so the a-side forces are summed in
- * registers and added to Fnb once per change of a. */
-template <class Body>
-__device__ __forceinline__ void leg_run_runs(const LegSmem &s, const uint2 *__restrict__ list, int from, int to,
-                                             int lane, Body body) {
-    int K = (to - from + 31) >> 5;
-    if (K > 0) K |= 1;
-    const int t0 = from + lane * K, t1 = min(to, t0 + K);
-    int ca = -1;
-    double sx = 0.0, sy = 0.0, sz = 0.0;
-    uint2 nxt = t0 < t1 ? __ldg(list + t0) : make_uint2(0u, 0u);
-    for (int t = t0; t < t1; t++) {
-        const uint2 ent = nxt;
-        if (t + 1 < t1) nxt = __ldg(list + t + 1); /* the next entry is in flight while this one is computed */
-        const int a = (int)(ent.x & 0xffu);
-        if (a != ca) {
-            if (ca >= 0) {
-                atomicAdd(&s.Fnb[3 * ca], -sx);
-                atomicAdd(&s.Fnb[3 * ca + 1], -sy);
-                atomicAdd(&s.Fnb[3 * ca + 2], -sz);
-            }
-            ca = a;
-            sx = sy = sz = 0.0;
-        }
-        const double3 g = body(ent);
-        sx += g.x;
-        sy += g.y;
-        sz += g.z;
-    }
-    if (ca >= 0) {
-        atomicAdd(&s.Fnb[3 * ca], -sx);
-        atomicAdd(&s.Fnb[3 * ca + 1], -sy);
-        atomicAdd(&s.Fnb[3 * ca + 2], -sz);
-    }
-}
-
-/* body(ent) -> the entry's force on neighbour a, over list entries
- * [from, to), 32 consecutive entries per round (the forward pass's
- * layout): a block's entries are ordered by a, so within a round the lanes
- * of one a are contiguous and their b slots all differ (few conflicting
- * b-side atomics); the a-side forces are summed per run of equal a by a
- * segmented warp sum and added by the run's first lane. */
-template <class Body>
-__device__ __forceinline__ void leg_run_conv(const LegSmem &s, const uint2 *__restrict__ list, int from, int to,
-                                             int lane, Body body) {
-    uint2 cur = from + lane < to ? __ldg(list + from + lane) : make_uint2(0u, 0u);
-    for (int base = from; base < to; base += 32) {
-        const int t = base + lane, tn = t + 32;
-        const uint2 nxt = tn < to ? __ldg(list + tn) : make_uint2(0u, 0u);
-        const bool valid = t < to;
-        const int a = valid ? (int)(cur.x & 0xffu) : 256 + lane; /* idle lanes: segments of their own */
-        double3 g = valid ? body(cur) : make_double3(0.0, 0.0, 0.0);
+    } else {
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const double x = __shfl_down_sync(FULL, g.x, o), y = __shfl_down_sync(FULL, g.y, o),
-                         z = __shfl_down_sync(FULL, g.z, o);
-            const int an = __shfl_down_sync(FULL, a, o);
-            if (lane + o < 32 && an == a) {
-                g.x += x;
-                g.y += y;
-                g.z += z;
-            }
+        for (int k = 0; k < 8; k++) {
+            lz[k] = 0.0;
+            if (lzp) lzp[k] = 0.0;
         }
-        const int ap = __shfl_up_sync(FULL, a, 1);
-        if (valid && (lane == 0 || ap != a)) {
-            atomicAdd(&s.Fnb[3 * a], -g.x);
-            atomicAdd(&s.Fnb[3 * a + 1], -g.y);
-            atomicAdd(&s.Fnb[3 * a + 2], -g.z);
-        }
-        cur = nxt;
+        angular<4, 2, false>(P, c, lz, lzp);
     }
 }
 
-/* The fused descriptor / MLP / force kernel on leg tables: the stages of
- * k_efs over the triplet lists of k_trip, with every triplet's leg factors
- * read from the rows k_legs wrote (i-j and i-k from i's own rows, staged;
- * j-k from j's row in global memory, L2-resident).  Reference bases: at
- * most 8 G4 exponents, zeta in {1, 2, 4, 16} or other integers, 2 lambdas. */
-/* Register budget per shape: the multi-warp shapes are compiled for 16
- * resident warps per SM (at most 128 registers a thread; a few bytes of
- * spills, measured 3-9% faster than 12 warps), the one-warp shapes for 12
- * (their shared memory allows no more at the alloy's neighbour counts).
- * RV selects the reverse pass's layout: 0 per-lane runs of entries (a-side
- * forces in registers), 1 consecutive entries per round (b-side atomics
- * without conflicts within a row). */
-template <int NE, int WPA, int APB, int RV>
-__global__ void __launch_bounds__(WPA * 32 * APB, (WPA >= 2 ? 512 : 384) / (WPA * 32 * APB))
-    k_efs_leg(const __grid_constant__ LegArgs A) {
-    constexpr int NZ = 4, NLAM = 2, NZL = 8;
-    static_assert(NE == 7 || NE == 8, "leg rows hold 8 exponents");
+/* absolute species of relative species v of an atom of species s0 */
+__device__ __forceinline__ int abs_species(int s0, int v, int ns) {
+    const int x = s0 + v;
+    return x >= ns ? x - ns : x;
+}
+
+/* NE: exponents evaluated (ne <= NE); WPA: warps per atom; APB: atoms per
+ * CTA; STD: the reference's function table (mb_tri), whose powers and
+ * squarings are straight-line code (the general form is 20% slower: the
+ * branches keep the compiler from interleaving the chains).  All shapes are
+ * compiled for 16 resident warps per SM (128 registers a thread). */
+template <int NE, int WPA, int APB, bool STD>
+__global__ void __launch_bounds__(WPA * 32 * APB, 512 / (WPA * 32 * APB)) k_efs_tri(const __grid_constant__ TriArgs A) {
+    constexpr int NZL = 8, NSQ = STD ? 2 : -1;
     extern __shared__ __align__(16) char smem_raw[];
+    __shared__ __align__(16) mb_tri_tab tab; /* polynomial coefficients: 16-byte broadcast loads */
     const mb_params &P = A.P;
-    /* G4 feature -> cell of the (eta, zeta-lambda) grid: the one table read
-     * at a different index by every thread, so it is kept in shared memory */
-    __shared__ unsigned char g4cell[MB_MAXG4];
-    for (int f = threadIdx.x; f < P.ng4; f += blockDim.x)
-        g4cell[f] = (unsigned char)(P.g4_e[f] * NZL + (P.g4_zl[f] / P.nlam) * NLAM + P.g4_zl[f] % P.nlam);
+    const mb_tri &T = A.T;
+    for (int k = threadIdx.x; k < (int)(sizeof(mb_tri_tab) / sizeof(double)); k += blockDim.x)
+        reinterpret_cast<double *>(&tab)[k] = reinterpret_cast<const double *>(&T.tab)[k];
     __syncthreads();
     const int NT = WPA * 32, group = threadIdx.x / NT;
     const int tid = threadIdx.x % NT, lane = threadIdx.x & 31, warp = tid >> 5;
     const int i = blockIdx.x * APB + group;
     if (i >= A.N) return; /* whole atom groups only: no barrier spans two groups */
-    const int D = P.D, ns = P.nspc, ng2 = P.ng2, ne = P.ne, cap = A.cap;
-    LegSmem s = leg_carve(smem_raw + (size_t)group * A.smem_group, cap, D, ng2, WPA);
-    const uint2 *tl = A.trip + (size_t)i * A.tcap;
-    const int *tb = A.tboff + 8 * (size_t)i;
-    const int n = A.nn[i];
-    const int s0 = A.spc[i];
+    const int D = P.D, ns = P.nspc, ng2 = P.ng2, ne = P.ne, cap = A.cap, nblk = tri_nblk(ns);
+    TriSmem s = tri_carve(smem_raw + (size_t)group * A.smem_group, cap, D, ns, ng2, WPA, A.tlw);
+    const int n = A.nn[i], s0 = A.spc[i];
     const double *net = A.weights + P.w_off[s0];
-    const size_t row = (size_t)i * cap;
 
-    /* ---- stage i's entries in relative-species order (k_legs sorted them by
-     * absolute species: relative species v is absolute (s0 + v) % ns) ---- */
-    if (tid < 4) {
-        const int v = tid, sa = (s0 + v) % ns;
-        int c = 0, o = 0;
-        if (v < ns) c = A.nso[4 * i + sa + 1] - A.nso[4 * i + sa];
-        for (int w = 0; w < v; w++) {
-            const int sw = (s0 + w) % ns;
-            o += A.nso[4 * i + sw + 1] - A.nso[4 * i + sw];
-        }
-        s.seg[v] = c;
-        s.seg[4 + v] = v < ns ? o : n;
-    }
-    for (int t = tid; t < D; t += NT) s.G[t] = 0.0;
-    group_sync<WPA>();
-    for (int u = tid; u < n; u += NT) {
-        int v = 0;
-        while (v + 1 < ns && u >= s.seg[4 + v + 1]) v++;
-        const int sa = (s0 + v) % ns;
-        const int t = A.nso[4 * i + sa] + (u - s.seg[4 + v]);
-        const int j = A.nj[row + t];
-        const double4 dv = A.nd[row + t];
-        s.j[u] = j;
-        s.sp[u] = sa;
-        double2 *dr = reinterpret_cast<double2 *>(s.d + LEG_DROW * u);
-        dr[0] = make_double2(dv.x, dv.y);
-        dr[1] = make_double2(dv.z, 1.0 / dv.w);
-        dr[2] = make_double2(dv.w, 0.0);
-        const double2 *src = reinterpret_cast<const double2 *>(A.leg + (row + t) * MB_LEG_STRIDE);
-        double2 *dst = reinterpret_cast<double2 *>(s.L + (size_t)u * MB_LEG_STRIDE);
+    /* ---- stage the neighbours, stably sorted by species relative to s0:
+     * every warp finds all the ranks (ballots) and writes its share of the rows ---- */
+    {
+        const size_t row = (size_t)i * cap;
+        int jv[TRI_PER_LANE], rv[TRI_PER_LANE], cnt[MB_MAXSPC] = {0, 0, 0};
+        constexpr int MINE = (TRI_PER_LANE + WPA - 1) / WPA; /* rows this warp writes, per lane */
+        double4 dv[MINE];
 #pragma unroll
-        for (int k = 0; k < MB_LEG_STRIDE / 2; k++) dst[k] = __ldg(src + k);
+        for (int q = 0; q < TRI_PER_LANE; q++) {
+            const int t = q * 32 + lane;
+            jv[q] = t < n ? A.nj[row + t] : -1;
+        }
+#pragma unroll
+        for (int k = 0; k < MINE; k++) {
+            const int t = (k * WPA + warp) * 32 + lane;
+            if (t < n) dv[k] = A.nd[row + t];
+        }
+#pragma unroll
+        for (int q = 0; q < TRI_PER_LANE; q++) {
+            rv[q] = -1;
+            if (jv[q] >= 0) {
+                const int d = A.spc[jv[q]] - s0;
+                rv[q] = d < 0 ? d + ns : d;
+            }
+        }
+        unsigned bal[TRI_PER_LANE][MB_MAXSPC];
+#pragma unroll
+        for (int q = 0; q < TRI_PER_LANE; q++)
+#pragma unroll
+            for (int v = 0; v < MB_MAXSPC; v++) {
+                bal[q][v] = v < ns && 32 * q < n ? __ballot_sync(FULL, rv[q] == v) : 0u;
+                cnt[v] += __popc(bal[q][v]);
+            }
+        if (warp == 0 && lane < 4) {
+            s.seg[lane] = lane == 0 ? cnt[0] : lane == 1 ? cnt[1] : lane == 2 ? cnt[2] : 0;
+            s.seg[4 + lane] = lane == 0 ? 0 : lane == 1 ? cnt[0] : lane == 2 ? cnt[0] + cnt[1] : n;
+        }
+        const unsigned below = (1u << lane) - 1u;
+        int run[MB_MAXSPC] = {0, cnt[0], cnt[0] + cnt[1]};
+#pragma unroll
+        for (int q = 0; q < TRI_PER_LANE; q++) {
+            if (q % WPA == warp && rv[q] >= 0) {
+                const int v = rv[q];
+                const int dst = (v == 0 ? run[0] + __popc(bal[q][0] & below)
+                                        : v == 1 ? run[1] + __popc(bal[q][1] & below) : run[2] + __popc(bal[q][2] & below));
+                const double4 d = dv[q / WPA];
+                const double r2 = d.x * d.x + d.y * d.y + d.z * d.z;
+                const double2 fh = tri_fh(tab, fma(r2, T.sv, -1.0));
+                double2 *o = reinterpret_cast<double2 *>(s.row + TRI_ROW * dst);
+                o[0] = make_double2(d.x, d.y);
+                o[1] = make_double2(d.z, 1.0 / d.w);
+                o[2] = make_double2(r2, fh.x);
+                o[3] = make_double2(fh.y, d.w);
+                s.j[dst] = jv[q];
+            }
+#pragma unroll
+            for (int v = 0; v < MB_MAXSPC; v++) run[v] += __popc(bal[q][v]);
+        }
     }
     group_sync<WPA>();
     if (tid == 0 && A.counters) atomicAdd(&A.counters[0], (unsigned long long)n);
+    const int o1 = s.seg[5], o2 = s.seg[6]; /* where relative species 1 and 2 begin */
 
     if (A.mode != MB_MODE_VJP) {
-        /* ---- forward pair terms: G2 (src/nprs.c:518-526) and repulsion ---- */
-        for (int t = tid; t < n; t += NT) {
-            const double r = s.d[LEG_DROW * t + 4];
-            const int p = s0 * s0 + s.sp[t] * s.sp[t];
-            const double fa = s.L[t * MB_LEG_STRIDE + 8]; /* one cutoff for all functions */
-            for (int f = 0; f < ng2; f++) {
-                const double x = r - P.f_rs[p][f];
-                s.tmp[t * ng2 + f] = fa * exp(-P.f_eta2[p][f] * (x * x));
+        /* ---- G2 (src/nprs.c:518-526): lane = (neighbour mod 4, function mod 8),
+         * fixed-order partial sums per warp ---- */
+        for (int f0 = 0; f0 < ng2; f0 += 8)
+            for (int v = 0; v < ns; v++) {
+                const int f = f0 + (lane & 7), sj = abs_species(s0, v, ns), p = s0 * s0 + sj * sj;
+                double acc = 0.0;
+                if (f < ng2) {
+                    const double rs = P.f_rs[p][f], eta = P.f_eta2[p][f];
+                    const int end = s.seg[4 + v] + s.seg[v];
+                    for (int t = s.seg[4 + v] + warp * 4 + (lane >> 3); t < end; t += 4 * WPA) {
+                        const double x = s.row[TRI_ROW * t + 7] - rs;
+                        acc += s.row[TRI_ROW * t + 5] * exp(-eta * (x * x));
+                    }
+                }
+                acc += __shfl_xor_sync(FULL, acc, 8);
+                acc += __shfl_xor_sync(FULL, acc, 16);
+                if (lane < 8 && f < ng2) s.g2[(warp * ns + v) * ng2 + f] = acc;
             }
-        }
-        group_sync<WPA>();
-        for (int w = tid; w < ns * ng2; w += NT) {
-            const int v = w / ng2, f = w % ng2;
-            double acc = 0.0;
-            for (int t = s.seg[4 + v]; t < s.seg[4 + v] + s.seg[v]; t++) acc += s.tmp[t * ng2 + f];
-            s.G[P.ind2[v] + f] = acc;
-        }
-        if (A.urep > 0.0 && tid == 0) {
+        if (A.urep > 0.0 && warp == 0) {
             double eu = 0.0;
-            for (int t = 0; t < n; t++) {
-                const double r = s.d[LEG_DROW * t + 4], R = P.rm[s0] + P.rm[s.sp[t]];
+            for (int t = lane; t < n; t += 32) {
+                const int v = (t >= o1) + (t >= o2);
+                const double r = s.row[TRI_ROW * t + 7], R = P.rm[s0] + P.rm[abs_species(s0, v, ns)];
                 if (r < R) eu += A.urep * fcut(R, r) * R / r;
             }
-            A.EU[i] = eu;
+            eu = warp_sum(eu);
+            if (lane == 0) A.EU[i] = eu;
         }
-        group_sync<WPA>(); /* the G2 terms in tmp are read; the triplet list reuses their space */
+    }
 
-        /* ---- forward triplet terms, block by block, on the FP64 tensor cores ---- */
+    /* ---- triplet list: per species block (al <= be) the pairs a < b of the
+     * atom's entries whose j-k distance is below the cutoff.  PRS_BP takes the
+     * triplet when |DX_j - DX_k| < Rc (src/nprs.c:528-537, src/cell.c:175-181):
+     * the squared distance summed without contraction as the reference forms
+     * it, against the threshold for which sqrt(s) < Rc holds exactly.  The
+     * block is walked in stripes of 8 rows (a >> 3) and groups of 4 columns
+     * (b >> 2), a candidate per lane, the atom's warps taking every WPA-th
+     * group; accepted pairs are appended column by column, so that a run of a
+     * list shares one stripe and few columns (the reverse pass sums such runs
+     * as 8 x 8 tiles).  A block's part is padded to a multiple of 4 entries, so
+     * that the tensor-core steps of the forward pass hold one block each. ---- */
+    unsigned short *tl = s.tl + warp * A.tlw;
+    int *bnd = s.bnd + 8 * warp;
+    int pos = 0;
+    {
         int blkid = 0;
+        const unsigned below = (1u << lane) - 1u;
         for (int al = 0; al < ns; al++)
             for (int be = al; be < ns; be++, blkid++) {
-                double c0 = 0.0, c1 = 0.0;
-                double *stw = s.stage + warp * 32 * EFS_STG;
-                auto body = [&](uint2 ent, bool valid) {
-                    double ex[8], lz[NZL];
-#pragma unroll
-                    for (int q = 0; q < 8; q++) ex[q] = 0.0;
-#pragma unroll
-                    for (int q = 0; q < NZL; q++) lz[q] = 0.0;
-                    if (valid) {
-                        const int a = (int)(ent.x & 0xffu), b = (int)((ent.x >> 8) & 0xffu);
-                        const double4 d1 = leg_vec(s.d, a), d2 = leg_vec(s.d, b);
-                        const double c = (d1.x * d2.x + d1.y * d2.y + d1.z * d2.z) * (d1.w * d2.w);
-                        const double2 *la = reinterpret_cast<const double2 *>(s.L + a * MB_LEG_STRIDE);
-                        const double2 *lb = reinterpret_cast<const double2 *>(s.L + b * MB_LEG_STRIDE);
-                        const double2 *lg = reinterpret_cast<const double2 *>(A.leg + (size_t)ent.y * MB_LEG_STRIDE);
-                        /* fc of the three legs: slot 7 when it is free (NE = 7), else slot 8 */
-                        const double A3 = NE == 7 ? 2.0 * la[3].y * lb[3].y * __ldg(lg + 3).y
-                                                  : 2.0 * la[4].x * lb[4].x * __ldg(lg + 4).x;
-                        angular<NZ, NLAM, false>(P, c, lz, nullptr);
-#pragma unroll
-                        for (int hh = 0; hh < (NE + 1) / 2; hh++) {
-                            const double2 x = la[hh], y = lb[hh], z = __ldg(lg + hh);
-                            ex[2 * hh] = A3 * (x.x * y.x) * z.x;
-                            if (2 * hh + 1 < NE) ex[2 * hh + 1] = A3 * (x.y * y.y) * z.y;
-                        }
-                    }
-#pragma unroll
-                    for (int q = 0; q < 8; q++) {
-                        stw[stg_slot(lane, q)] = ex[q];
-                        stw[stg_slot(lane, 8 + q)] = lz[q];
-                    }
-                    __syncwarp();
-#pragma unroll
-                    for (int st = 0; st < 8; st++) {
-                        const int t = 4 * st + (lane & 3);
-                        dmma884(c0, c1, stw[stg_slot(t, lane >> 2)], stw[stg_slot(t, 8 + (lane >> 2))]);
-                    }
-                    __syncwarp();
-                };
-                /* the block's list entries, 32 per round, the atom's warps taking every WPA-th round */
-                {
-                    const int to = tb[blkid + 1];
-                    int base = tb[blkid] + warp * 32;
-                    uint2 cur = base + lane < to ? __ldg(tl + base + lane) : make_uint2(0u, 0u);
-                    for (; base < to; base += 32 * WPA) {
-                        /* the next round's entry is in flight while this round is computed */
-                        const int tn = base + 32 * WPA + lane;
-                        const uint2 nxt = tn < to ? __ldg(tl + tn) : make_uint2(0u, 0u);
-                        body(cur, base + lane < to);
-                        cur = nxt;
+                if (lane == 0) bnd[blkid] = pos;
+                const int sj = abs_species(s0, al, ns), sk = abs_species(s0, be, ns);
+                const double thr = P.f_rc4thr[sj * sj + sk * sk];
+                const int oa = s.seg[4 + al], ea = oa + s.seg[al], ob = s.seg[4 + be], eb = ob + s.seg[be];
+                for (int st = oa >> 3; 8 * st < ea && ea > oa; st++) {
+                    const int a = 8 * st + (lane & 7);
+                    const double *pa = s.row + TRI_ROW * a;
+                    const double ax = pa[0], ay = pa[1], az = pa[2];
+                    /* the lane's columns: lo <= b < eb (none for rows outside the
+                     * block; what is read past the rows is discarded) */
+                    const int lo = a >= oa && a < ea ? max(ob, a + 1) : 0x7fffffff;
+                    /* groups g = warp (mod WPA) from the stripe's first column on */
+                    int g = max(ob, max(oa, 8 * st) + 1) >> 2;
+                    g += (warp - g) & (WPA - 1);
+                    const double *pb = s.row + TRI_ROW * (4 * g + (lane >> 3));
+                    unsigned ent = (unsigned)a | (unsigned)(4 * g + (lane >> 3)) << 8;
+#pragma unroll 1
+                    for (int b = 4 * g + (lane >> 3); b - (lane >> 3) < eb; b += 4 * WPA) {
+                        const double2 b01 = *reinterpret_cast<const double2 *>(pb);
+                        const double dx = xsub(ax, b01.x), dy = xsub(ay, b01.y), dz = xsub(az, pb[2]);
+                        const bool ok = xadd(xadd(xmul(dx, dx), xmul(dy, dy)), xmul(dz, dz)) < thr && b >= lo && b < eb;
+                        const unsigned m = __ballot_sync(FULL, ok);
+                        if (ok) tl[pos + __popc(m & below)] = (unsigned short)ent;
+                        pos += __popc(m);
+                        pb += 4 * WPA * TRI_ROW;
+                        ent += 4u * WPA << 8;
                     }
                 }
-                group_sync<WPA>();
-                group_store64<WPA>(c0, c1, s, warp, lane);
-                {
-                    const int base = P.ind4[al * al + be * be];
-                    /* the cells carry the zeta normalisation left out of the angular terms */
-                    for (int f = tid; f < P.ng4; f += NT)
-                        s.G[base + f] += s.red[g4cell[f]] * P.powz[(g4cell[f] & 7) >> 1];
-                }
-                group_sync<WPA>();
+                if (lane < (-pos & 3)) tl[pos + lane] = (unsigned short)TRI_NONE;
+                pos = (pos + 3) & ~3;
             }
+        if (lane == 0) bnd[blkid] = pos;
+    }
+    __syncwarp();
+
+    if (A.mode != MB_MODE_VJP) {
+        /* ---- forward: each lane forms a triplet's 8 exponential and 8 angular
+         * factors, staged through shared memory; the grid sum_t ex_t[e] lz_t[zl]
+         * of a block is an outer-product sum on the FP64 tensor cores, 4
+         * triplets a step, left in lane l as cells 2l, 2l+1 ---- */
+        double c0 = 0.0, c1 = 0.0;
+        double *stw = s.stage + warp * 16 * TRI_STG + lane;
+        const double *str = s.stage + warp * 16 * TRI_STG + (lane >> 2) * TRI_STG + (lane & 3);
+        double2 *red = reinterpret_cast<double2 *>(s.red + (size_t)warp * nblk * 64) + lane;
+        int blk = 0, nb = bnd[1], nacc = 0;
+        for (int base = 0; base < pos; base += 32) {
+            const unsigned ent = base + lane < pos ? tl[base + lane] : TRI_NONE;
+            const bool valid = ent != TRI_NONE;
+            nacc += __popc(__ballot_sync(FULL, valid));
+            /* padding lanes evaluate entry (0, 0) with weight 0 */
+            const unsigned ab = valid ? ent : 0u;
+            const double2 *pa = reinterpret_cast<const double2 *>(s.row + TRI_ROW * (ab & 0xffu));
+            const double2 *pb = reinterpret_cast<const double2 *>(s.row + TRI_ROW * (ab >> 8));
+            const double2 a0 = pa[0], a1 = pa[1], a2 = pa[2], b0 = pb[0], b1 = pb[1], b2 = pb[2];
+            const double wx = b0.x - a0.x, wy = b0.y - a0.y, wz = b1.x - a1.x;
+            const double s3 = wx * wx + wy * wy + wz * wz;
+            const double c = (a0.x * b0.x + a0.y * b0.y + a1.x * b1.x) * (a1.y * b1.y);
+            double A3 = 2.0 * a2.y * b2.y * tri_f(tab, fma(s3, T.sv, -1.0));
+            if (!valid) A3 = 0.0;
+            double ex[8], lz[NZL];
+            ex[7] = 0.0;
+            tri_exp<NE, NSQ>(tab, T.nsq, a2.x + b2.x + s3, ex);
+            tri_angular<STD>(P, c, lz, nullptr);
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                stw[q * TRI_STG] = q < NE ? A3 * ex[q] : 0.0;
+                stw[(8 + q) * TRI_STG] = lz[q];
+            }
+            __syncwarp();
+#pragma unroll
+            for (int st = 0; st < 8; st++) {
+                if (base + 4 * st >= nb && blk + 1 < nblk) {
+                    /* the next block begins (past the last one the values are zeros) */
+                    do {
+                        red[32 * blk] = make_double2(c0, c1);
+                        c0 = c1 = 0.0;
+                        blk++;
+                        nb = bnd[blk + 1];
+                    } while (base + 4 * st >= nb && blk + 1 < nblk);
+                }
+                dmma884(c0, c1, str[4 * st], str[4 * st + 8 * TRI_STG]);
+            }
+            __syncwarp();
+        }
+        for (; blk < nblk; blk++) {
+            red[32 * blk] = make_double2(c0, c1);
+            c0 = c1 = 0.0;
+        }
+        if (A.counters && lane == 0) atomicAdd(&A.counters[1], (unsigned long long)nacc);
+        group_sync<WPA>();
+        /* descriptors: the warps' sums in warp order; the cells carry the zeta
+         * normalisation left out of the angular terms (a power of two) */
+        for (int w = tid; w < ns * ng2; w += NT) {
+            const int v = w / ng2, f = w - v * ng2;
+            double g = 0.0;
+            for (int k = 0; k < WPA; k++) g += s.g2[(k * ns + v) * ng2 + f];
+            s.G[P.ind2[v] + f] = g;
+        }
+        for (int f = tid; f < P.ng4; f += NT) {
+            const int cell = T.fn_cell[f];
+            const double pz = P.powz[(cell & 7) >> 1];
+            int b = 0;
+            for (int al = 0; al < ns; al++)
+                for (int be = al; be < ns; be++, b++) {
+                    double g = 0.0;
+                    for (int k = 0; k < WPA; k++) g += s.red[(size_t)(k * nblk + b) * 64 + cell];
+                    s.G[P.ind4[al * al + be * be] + f] = g * pz;
+                }
+        }
+        group_sync<WPA>();
         if (A.mode == MB_MODE_DESCRIPTORS) {
             for (int t = tid; t < D; t += NT) A.G[(size_t)i * D + t] = s.G[t];
             return;
@@ -1865,42 +1729,93 @@ __global__ void __launch_bounds__(WPA * 32 * APB, (WPA >= 2 ? 512 : 384) / (WPA 
 
     /* ---- MLP: forward (src/nmlp.c:367-431) and dE/dG ---- */
     const int h1 = P.h1, h2 = P.h2;
-    const double *off = net, *W0 = off + D, *b0 = W0 + h1 * D, *W1 = b0 + h1, *b1 = W1 + h2 * h1, *W2 = b1 + h2,
+    const double *w0 = A.w0 + (size_t)s0 * D * T.wrow;
+    const double *b0 = net + D + h1 * D, *W1 = b0 + h1, *b1 = W1 + h2 * h1, *W2 = b1 + h2,
                  *b2 = W2 + h2;
-    double *H1 = s.h, *H2 = s.h + MB_MAXH, *Dl1 = s.h + 2 * MB_MAXH, *Dl2 = s.h + 3 * MB_MAXH;
+    double *H1 = s.h, *Dl1 = s.h + 2 * MB_MAXH, *Dl2 = s.h + 3 * MB_MAXH;
     if (A.mode != MB_MODE_VJP) {
-        for (int m = warp; m < h1; m += WPA) {
-            double acc = 0.0;
-            for (int l = lane; l < D; l += 32) acc += (s.G[l] - off[l]) * W0[m * D + l];
-            acc = warp_sum(acc);
-            if (lane == 0) H1[m] = tanh(b0[m] + acc);
+        if (h1 <= 16) {
+            /* an input a lane: its row of first-layer weights in 16-byte loads,
+             * every unit's partial sum in each lane, one halving reduction per
+             * warp, then the warps in order */
+            double acc[16];
+#pragma unroll
+            for (int m = 0; m < 16; m++) acc[m] = 0.0;
+#pragma unroll 2
+            for (int l = tid; l < D; l += NT) {
+                const double2 *w = reinterpret_cast<const double2 *>(w0 + (size_t)l * T.wrow);
+                double2 r[8];
+#pragma unroll
+                for (int m = 0; m < 8; m++)
+                    if (2 * m < h1) r[m] = w[m];
+                const double x = s.G[l] - w0[(size_t)l * T.wrow + h1];
+#pragma unroll
+                for (int m = 0; m < 8; m++)
+                    if (2 * m < h1) {
+                        acc[2 * m] = fma(x, r[m].x, acc[2 * m]);
+                        acc[2 * m + 1] = fma(x, r[m].y, acc[2 * m + 1]);
+                    }
+            }
+            const double tot = warp_reduce16(acc, lane);
+            if (!(lane & 1)) s.hp[16 * warp + (lane >> 1)] = tot;
+            group_sync<WPA>();
+            if (tid < h1) {
+                double v = b0[tid];
+                for (int w = 0; w < WPA; w++) v += s.hp[16 * w + tid];
+                H1[tid] = tanh(v);
+            }
+        } else {
+            for (int m = warp; m < h1; m += WPA) {
+                double acc = 0.0;
+                for (int l = lane; l < D; l += 32)
+                    acc += (s.G[l] - w0[(size_t)l * T.wrow + h1]) * w0[(size_t)l * T.wrow + m];
+                acc = warp_sum(acc);
+                if (lane == 0) H1[m] = tanh(b0[m] + acc);
+            }
         }
         group_sync<WPA>();
         if (warp == 0) {
-            double v = 0.0;
+            double v = 0.0, w2 = 0.0;
             if (lane < h2) {
                 v = b1[lane];
-                for (int k = 0; k < h1; k++) v += H1[k] * W1[lane * h1 + k];
+                w2 = W2[lane];
+#pragma unroll 8
+                for (int k = 0; k < h1; k++) v = fma(H1[k], W1[lane * h1 + k], v);
                 v = tanh(v);
-                H2[lane] = v;
             }
-            double e = lane < h2 ? v * W2[lane] : 0.0;
-            e = warp_sum(e);
+            const double e = warp_sum(w2 * v);
             if (lane == 0) A.EA[i] = b2[0] + e;
-            __syncwarp();
-            if (lane < h2) Dl2[lane] = W2[lane] * (1.0 - v * v);
+            if (lane < h2) Dl2[lane] = w2 * (1.0 - v * v);
             __syncwarp();
             if (lane < h1) {
                 double g = 0.0;
-                for (int m = 0; m < h2; m++) g += Dl2[m] * W1[m * h1 + lane];
+#pragma unroll 8
+                for (int m = 0; m < h2; m++) g = fma(Dl2[m], W1[m * h1 + lane], g);
                 Dl1[lane] = g * (1.0 - H1[lane] * H1[lane]);
+            } else if (lane == h1) {
+                Dl1[lane] = 0.0;
             }
         }
         group_sync<WPA>();
         if (A.mode == MB_MODE_ENERGY) return;
         for (int l = tid; l < D; l += NT) {
+            const double2 *w = reinterpret_cast<const double2 *>(w0 + (size_t)l * T.wrow);
             double g = 0.0;
-            for (int k = 0; k < h1; k++) g += Dl1[k] * W0[k * D + l];
+            if (h1 <= 16) {
+                double2 r[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++)
+                    if (2 * k < h1) r[k] = w[k];
+                /* an odd h1's last pair holds off[l], against Dl1[h1] = 0 */
+#pragma unroll
+                for (int k = 0; k < 8; k++)
+                    if (2 * k < h1) {
+                        const double2 d = reinterpret_cast<const double2 *>(Dl1)[k];
+                        g = fma(d.y, r[k].y, fma(d.x, r[k].x, g));
+                    }
+            } else {
+                for (int k = 0; k < h1; k++) g = fma(Dl1[k], w0[(size_t)l * T.wrow + k], g);
+            }
             s.G[l] = g;
         }
     } else {
@@ -1908,127 +1823,220 @@ __global__ void __launch_bounds__(WPA * 32 * APB, (WPA >= 2 ? 512 : 384) / (WPA 
     }
     group_sync<WPA>();
 
-    /* ---- reverse pair terms with the species-0 parameters ---- */
+    /* ---- dE/dG by grid cell, and the reverse pair terms with the species-0 parameters ---- */
+    for (int cell = tid; cell < 64; cell += NT) {
+        const int f0 = T.cell_fn[cell];
+        const int f1 = f0 >= 0 ? T.fn_next[f0] : -1;
+        const double pz = P.powz[(cell & 7) >> 1];
+        int b = 0;
+        for (int al = 0; al < ns; al++)
+            for (int be = al; be < ns; be++, b++) {
+                const double *g = s.G + P.ind4[al * al + be * be];
+                double v = f0 >= 0 ? g[f0] : 0.0;
+                for (int f = f1; f >= 0; f = T.fn_next[f]) v += g[f];
+                s.grid[64 * b + cell] = v * pz;
+            }
+    }
     double fi[3] = {0.0, 0.0, 0.0}, vr[6] = {0, 0, 0, 0, 0, 0};
-    for (int t = tid; t < n; t += NT) {
-        const double4 d = leg_vec(s.d, t);
-        const double r = s.d[LEG_DROW * t + 4], ir = d.w;
-        double f2, df2;
-        fcut_d(P.d_rc2, r, f2, df2);
-        const int ds1 = (s.sp[t] - s0 + ns) % ns;
-        const double *g = s.G + P.ind2[ds1];
+    /* lane = (neighbour mod 4, function mod 8) as in the forward sums */
+    for (int t0 = 4 * warp; t0 < n; t0 += 4 * WPA) {
+        const int t = min(t0 + (lane >> 3), n - 1);
+        const double *d = s.row + TRI_ROW * t;
+        const double r = d[7], f2 = d[5], df2 = d[6] * r;
+        const int v = (t >= o1) + (t >= o2);
+        const double *g = s.G + (v == 0 ? P.ind2[0] : v == 1 ? P.ind2[1] : P.ind2[2]);
         double cpair = 0.0;
-        for (int f = 0; f < ng2; f++) {
+        for (int f = lane & 7; f < ng2; f += 8) {
             const double x = r - P.d_rs[f], eta = P.d_eta2[f];
             cpair += g[f] * exp(-eta * x * x) * (-2.0 * eta * x * f2 + df2);
         }
-        const double cr = cpair * ir;
-        const double v0 = cr * d.x, v1 = cr * d.y, v2 = cr * d.z;
-        fi[0] += v0; fi[1] += v1; fi[2] += v2;
-        s.Fnb[3 * t] = -v0; s.Fnb[3 * t + 1] = -v1; s.Fnb[3 * t + 2] = -v2;
-        if (A.urep > 0.0) {
-            const double R = P.rm[s0] + P.rm[s.sp[t]];
+        cpair += __shfl_xor_sync(FULL, cpair, 1);
+        cpair += __shfl_xor_sync(FULL, cpair, 2);
+        cpair += __shfl_xor_sync(FULL, cpair, 4);
+        const int q = lane & 7;
+        if (t0 + (lane >> 3) < n && q < 4) {
+            s.Fnb[4 * t + q] = q < 3 ? -cpair * d[3] * d[q] : 0.0;
+            for (int w = 1; w < WPA; w++) s.Fnb[4 * (cap * w + t) + q] = 0.0;
+        }
+    }
+    if (A.urep > 0.0)
+        for (int t = tid; t < n; t += NT) {
+            const double *d = s.row + TRI_ROW * t;
+            const int v = (t >= o1) + (t >= o2);
+            const double r = d[7], R = P.rm[s0] + P.rm[abs_species(s0, v, ns)];
             if (r < R) {
                 /* CELL_UREP on the ordered pair (i, j): force on i only (src/cmod.c:100-112) */
                 double fu, dfu;
                 fcut_d(R, r, fu, dfu);
                 const double tu = -2.0 * A.urep * R / (r * r) * (-fu / r + dfu);
-                fi[0] -= tu * d.x; fi[1] -= tu * d.y; fi[2] -= tu * d.z;
-                vr[0] += 0.5 * tu * d.x * d.x; vr[1] += 0.5 * tu * d.y * d.y; vr[2] += 0.5 * tu * d.z * d.z;
-                vr[3] += 0.5 * tu * d.x * d.y; vr[4] += 0.5 * tu * d.y * d.z; vr[5] += 0.5 * tu * d.z * d.x;
+                fi[0] -= tu * d[0]; fi[1] -= tu * d[1]; fi[2] -= tu * d[2];
+                vr[0] += 0.5 * tu * d[0] * d[0]; vr[1] += 0.5 * tu * d[1] * d[1]; vr[2] += 0.5 * tu * d[2] * d[2];
+                vr[3] += 0.5 * tu * d[0] * d[1]; vr[4] += 0.5 * tu * d[1] * d[2]; vr[5] += 0.5 * tu * d[2] * d[0];
+            }
+        }
+    group_sync<WPA>();
+
+    /* ---- reverse triplet terms: 32 list entries a round, an entry a lane.
+     * The force on j is -(p1 d_j + sc d_k), on k -(p2 d_k + sc d_j), so a run
+     * of entries with one stripe of rows and 16 columns is three 8 x 16 tiles:
+     * sum_b sc_ab d_b, sum_a sc_ab d_a and the row and column sums of p1 and p2
+     * are products of the tiles with the displacements, done on the FP64 tensor
+     * cores and added to the warp's own Fnb with plain
+     * loads and stores.  (Shared FP64 atomics are compare-and-swap loops: six
+     * of them and a segmented warp sum per triplet were a third of the reverse
+     * pass.)  The force on i is minus the sum of its neighbours'. ---- */
+    {
+        double2 *Fw = reinterpret_cast<double2 *>(s.Fnb + 4 * cap * warp) + (lane & 1);
+        double *tile = s.tile + warp * 24 * TRI_TS;
+        double2 *ztile = reinterpret_cast<double2 *>(tile) + lane;
+        const double *tr = tile + TRI_TS * (lane >> 2) + (lane & 3), *tc = tile + TRI_TS * (lane & 3) + (lane >> 2);
+        const int m4 = lane >> 2, k4 = lane & 3;
+        const bool xyz = m4 < 3;                    /* mma columns 0-2: displacements */
+        const double one = m4 == 3 ? 1.0 : 0.0;     /* column 3: sums of p1 and p2 */
+        const double *rx = s.row + (xyz ? m4 : 0);
+        const double2 *rq = reinterpret_cast<const double2 *>(s.row) + (lane & 1);
+#pragma unroll
+        for (int q = 0; q < 8; q++)
+            if (q < 7 || lane < 16) ztile[q * 32] = make_double2(0.0, 0.0);
+        __syncwarp();
+        int eb[MB_MAX_BLOCKS - 1];
+#pragma unroll
+        for (int k = 0; k < MB_MAX_BLOCKS - 1; k++) eb[k] = k + 1 < nblk ? bnd[k + 1] : 0x7fffffff;
+        for (int base = 0; base < pos; base += 32) {
+            const int t = base + lane;
+            const unsigned ent = t < pos ? tl[t] : TRI_NONE;
+            const bool valid = ent != TRI_NONE;
+            const unsigned ab = valid ? ent : 0u; /* padding lanes evaluate entry (0, 0) and add nothing */
+            const int a = (int)(ab & 0xffu), b = (int)(ab >> 8);
+            int blk = 0;
+#pragma unroll
+            for (int k = 0; k < MB_MAX_BLOCKS - 1; k++) blk += t >= eb[k];
+            const double *grid = s.grid + 64 * min(blk, nblk - 1);
+            const double2 *pa = reinterpret_cast<const double2 *>(s.row + TRI_ROW * a);
+            const double2 *pb = reinterpret_cast<const double2 *>(s.row + TRI_ROW * b);
+            const double2 a0 = pa[0], a1 = pa[1], a2 = pa[2], q0 = pb[0], q1 = pb[1], q2 = pb[2];
+            const double ha = pa[3].x, hb = pb[3].x;
+            const double wx = q0.x - a0.x, wy = q0.y - a0.y, wz = q1.x - a1.x;
+            const double s3 = wx * wx + wy * wy + wz * wz;
+            const double ir12 = a1.y * q1.y;
+            const double c = (a0.x * q0.x + a0.y * q0.y + a1.x * q1.x) * ir12;
+            double E[8], lz[NZL], lzp[NZL];
+            tri_exp<NE, NSQ>(tab, T.nsq, a2.x + q2.x + s3, E);
+            tri_angular<STD>(P, c, lz, lzp);
+            double Q = 0.0, Qe = 0.0, Qc = 0.0, eta[8];
+#pragma unroll
+            for (int e = 0; e < NE; e += 2) {
+                const double2 x = reinterpret_cast<const double2 *>(tab.eta)[e / 2];
+                eta[e] = x.x;
+                eta[e + 1] = x.y;
+            }
+#pragma unroll
+            for (int e = 0; e < NE; e++) {
+                double u = 0.0, v = 0.0;
+#pragma unroll
+                for (int zl = 0; zl < NZL; zl += 2) {
+                    if (STD && e < MB_TRI_LOW && zl >= 4) break;
+                    const double2 cg = *reinterpret_cast<const double2 *>(grid + e * NZL + zl);
+                    u = fma(cg.y, lz[zl + 1], fma(cg.x, lz[zl], u));
+                    v = fma(cg.y, lzp[zl + 1], fma(cg.x, lzp[zl], v));
+                }
+                const double Eu = E[e] * u;
+                Q += Eu;
+                Qe = fma(eta[e], Eu, Qe);
+                Qc = fma(E[e], v, Qc);
+            }
+            /* legs: f = fc(r), h = fc'(r)/r (i-j: a, i-k: b, j-k: 3); with
+             * T = 2 f_a f_b f_3 sum: dT/dr / r of each leg, and dT/dcos */
+            const double2 fh = tri_fh(tab, fma(s3, T.sv, -1.0));
+            const double fab = 2.0 * a2.y * q2.y, Af = fab * fh.x, Y = 2.0 * Af * Qe, f3Q = 2.0 * fh.x * Q;
+            const double Tc = Af * Qc, tcc = Tc * c;
+            const double a3 = fab * fh.y * Q - Y;
+            const double p1 = ha * q2.y * f3Q - Y - tcc * a1.y * a1.y + a3;
+            const double p2 = a2.y * hb * f3Q - Y - tcc * q1.y * q1.y + a3;
+            const double sc = Tc * ir12 - a3;
+
+            /* column number among the warp's own columns */
+            const int col = (((b >> 2) / WPA) << 2) | (b & 3);
+            unsigned rem = __ballot_sync(FULL, valid);
+            while (rem) {
+                const int first = __shfl_sync(FULL, (a & ~7) | (col << 8), __ffs(rem) - 1);
+                const int a0r = first & 0xff, c0 = first >> 8;
+                const unsigned ra = (unsigned)(a - a0r), cc = (unsigned)(col - c0);
+                const bool mine = ((rem >> lane) & 1u) && ra < 8u && cc < 16u;
+                double *o = tile + TRI_TS * ra + cc;
+                if (mine) {
+                    o[0] = sc;
+                    o[8 * TRI_TS] = p1;
+                    o[16 * TRI_TS] = p2;
+                }
+                rem &= ~__ballot_sync(FULL, mine);
+                const bool wide = __any_sync(FULL, mine && cc >= 8u);
+                __syncwarp();
+                /* operands: the rows (a) and columns (b) of the tile; past the end
+                 * of the list the tile holds zeros and any row of the atom will do */
+                double da[2], ea0 = 0.0, ea1 = 0.0;
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+                    da[h] = xyz ? rx[TRI_ROW * min(a0r + 4 * h + k4, n - 1)] : 0.0;
+#pragma unroll
+                for (int ct = 0; ct < 2; ct++) {
+                    if (ct == 1 && !wide) break;
+                    double eb0 = 0.0, eb1 = 0.0;
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const int c = c0 + 8 * ct + 4 * h + k4, kb = (((c >> 2) * WPA + warp) << 2) | (c & 3);
+                        const double db = xyz ? rx[TRI_ROW * min(kb, n - 1)] : 0.0;
+                        dmma884(ea0, ea1, tr[8 * ct + 4 * h], db);
+                        dmma884(ea0, ea1, tr[8 * ct + 4 * h + 8 * TRI_TS], one);
+                        dmma884(eb0, eb1, tc[8 * ct + 4 * h * TRI_TS], da[h]);
+                        dmma884(eb0, eb1, tc[8 * ct + (4 * h + 16) * TRI_TS], one);
+                    }
+                    /* lane 4 m holds x, y of column m, lane 4 m + 1 z and the sum of p2
+                     * (its second value goes to the row's unused fourth word) */
+                    const double pb = __shfl_sync(FULL, eb1, lane | 1);
+                    const int c = c0 + 8 * ct + m4, br = (((c >> 2) * WPA + warp) << 2) | (c & 3);
+                    if (k4 < 2 && br < n) {
+                        const double2 d = rq[(TRI_ROW / 2) * br], f = Fw[2 * br];
+                        Fw[2 * br] = make_double2(f.x - fma(pb, d.x, eb0), f.y - fma(pb, d.y, eb1));
+                    }
+                    __syncwarp();
+                }
+                {
+                    const double pa = __shfl_sync(FULL, ea1, lane | 1);
+                    const int ar = a0r + m4;
+                    if (k4 < 2 && ar < n) {
+                        const double2 d = rq[(TRI_ROW / 2) * ar], f = Fw[2 * ar];
+                        Fw[2 * ar] = make_double2(f.x - fma(pa, d.x, ea0), f.y - fma(pa, d.y, ea1));
+                    }
+                    /* the tile is left as zeros */
+                    if (mine) o[0] = o[8 * TRI_TS] = o[16 * TRI_TS] = 0.0;
+                    __syncwarp();
+                }
             }
         }
     }
     group_sync<WPA>();
 
-    /* ---- reverse triplet terms over the same lists ---- */
-    {
-        int blkid = 0;
-        double eta[NE];
-#pragma unroll
-        for (int e = 0; e < NE; e++) eta[e] = e < ne ? P.d_eta4[e] : 0.0;
-        for (int al = 0; al < ns; al++)
-            for (int be = al; be < ns; be++, blkid++) {
-                const int base = P.ind4[al * al + be * be];
-                for (int t = tid; t < 64; t += NT) s.grid[t] = 0.0;
-                group_sync<WPA>();
-                for (int f = tid; f < P.ng4; f += NT)
-                    atomicAdd(&s.grid[g4cell[f]], s.G[base + f] * P.powz[(g4cell[f] & 7) >> 1]);
-                group_sync<WPA>();
-                auto body = [&](uint2 ent) -> double3 {
-                    const int a = (int)(ent.x & 0xffu), b = (int)((ent.x >> 8) & 0xffu);
-                    const double4 d1 = leg_vec(s.d, a), d2 = leg_vec(s.d, b);
-                    const double wx = d2.x - d1.x, wy = d2.y - d1.y, wz = d2.z - d1.z;
-                    const double ir1 = d1.w, ir2 = d2.w;
-                    const double c = (d1.x * d2.x + d1.y * d2.y + d1.z * d2.z) * (ir1 * ir2);
-                    const double2 *la = reinterpret_cast<const double2 *>(s.L + a * MB_LEG_STRIDE);
-                    const double2 *lb = reinterpret_cast<const double2 *>(s.L + b * MB_LEG_STRIDE);
-                    const double2 *lg = reinterpret_cast<const double2 *>(A.leg + (size_t)ent.y * MB_LEG_STRIDE);
-                    const double2 fa = la[4], fb = lb[4], fg = __ldg(lg + 4);
-                    double lz[NZL], lzp[NZL];
-#pragma unroll
-                    for (int k = 0; k < NZL; k++) { lz[k] = 0.0; lzp[k] = 0.0; }
-                    angular<NZ, NLAM, false>(P, c, lz, lzp);
-                    double Q = 0.0, Qe = 0.0, Qc = 0.0;
-#pragma unroll
-                    for (int hh = 0; hh < (NE + 1) / 2; hh++) {
-                        const double2 x = la[hh], y = lb[hh], z = __ldg(lg + hh);
-#pragma unroll
-                        for (int q = 0; q < 2; q++) {
-                            const int e = 2 * hh + q;
-                            if (e >= NE) break;
-                            const double E = q ? (x.y * y.y) * z.y : (x.x * y.x) * z.x;
-                            double u = 0.0, v = 0.0;
-#pragma unroll
-                            for (int zl = 0; zl < NZL; zl += 2) {
-                                const double2 cg = *reinterpret_cast<const double2 *>(s.grid + e * NZL + zl);
-                                u += cg.x * lz[zl] + cg.y * lz[zl + 1];
-                                v += cg.x * lzp[zl] + cg.y * lzp[zl + 1];
-                            }
-                            Q += E * u;
-                            Qe += eta[e] * E * u;
-                            Qc += E * v;
-                        }
-                    }
-                    /* legs: f = fc(r), h = fc'(r)/r (i-j: a, i-k: b, j-k: g) */
-                    const double Af = 2.0 * fa.x * fb.x * fg.x;
-                    const double T1 = 2.0 * fa.y * fb.x * fg.x * Q - 2.0 * Af * Qe; /* dT/dr1 / r1 */
-                    const double T2 = 2.0 * fa.x * fb.y * fg.x * Q - 2.0 * Af * Qe;
-                    const double T3 = 2.0 * fa.x * fb.x * fg.y * Q - 2.0 * Af * Qe;
-                    const double Tc = Af * Qc;
-                    const double a11 = T1 - Tc * c * ir1 * ir1, a22 = T2 - Tc * c * ir2 * ir2;
-                    const double a12 = Tc * ir1 * ir2, a3 = T3;
-                    const double g1x = a11 * d1.x + a12 * d2.x - a3 * wx;
-                    const double g1y = a11 * d1.y + a12 * d2.y - a3 * wy;
-                    const double g1z = a11 * d1.z + a12 * d2.z - a3 * wz;
-                    const double g2x = a22 * d2.x + a12 * d1.x + a3 * wx;
-                    const double g2y = a22 * d2.y + a12 * d1.y + a3 * wy;
-                    const double g2z = a22 * d2.z + a12 * d1.z + a3 * wz;
-                    fi[0] += g1x + g2x; fi[1] += g1y + g2y; fi[2] += g1z + g2z;
-                    atomicAdd(&s.Fnb[3 * b], -g2x);
-                    atomicAdd(&s.Fnb[3 * b + 1], -g2y);
-                    atomicAdd(&s.Fnb[3 * b + 2], -g2z);
-                    return make_double3(g1x, g1y, g1z);
-                };
-                {
-                    /* the block's entries in WPA contiguous parts, one per warp */
-                    const int from = tb[blkid], to = tb[blkid + 1], per = (to - from + WPA - 1) / WPA;
-                    const int lo = min(to, from + warp * per), hi = min(to, lo + per);
-                    if constexpr (RV == 0)
-                        leg_run_runs(s, tl, lo, hi, lane, body);
-                    else
-                        leg_run_conv(s, tl, lo, hi, lane, body);
-                }
-                group_sync<WPA>();
-            }
-    }
-
-    /* virial of atom i's energy: every neighbour force times its displacement */
+    /* neighbour forces out; the virial of atom i's energy is every neighbour
+     * force times its displacement */
+    const double2 *F4 = reinterpret_cast<const double2 *>(s.Fnb);
     for (int t = tid; t < n; t += NT) {
-        const double4 d = leg_vec(s.d, t);
-        const double fx = s.Fnb[3 * t], fy = s.Fnb[3 * t + 1], fz = s.Fnb[3 * t + 2];
-        vr[0] += fx * d.x; vr[1] += fy * d.y; vr[2] += fz * d.z;
-        vr[3] += fx * d.y; vr[4] += fy * d.z; vr[5] += fz * d.x;
+        const double *d = s.row + TRI_ROW * t;
+        double2 f0 = F4[2 * t], f1 = F4[2 * t + 1];
+        for (int w = 1; w < WPA; w++) {
+            const double2 g0 = F4[2 * (cap * w + t)], g1 = F4[2 * (cap * w + t) + 1];
+            f0.x += g0.x;
+            f0.y += g0.y;
+            f1.x += g1.x;
+        }
+        const double fx = f0.x, fy = f0.y, fz = f1.x;
+        const int j = s.j[t];
+        atomicAdd(&A.F[3 * j], fx);
+        atomicAdd(&A.F[3 * j + 1], fy);
+        atomicAdd(&A.F[3 * j + 2], fz);
+        fi[0] -= fx; fi[1] -= fy; fi[2] -= fz;
+        vr[0] += fx * d[0]; vr[1] += fy * d[1]; vr[2] += fz * d[2];
+        vr[3] += fx * d[1]; vr[4] += fy * d[2]; vr[5] += fz * d[0];
     }
     {
         /* the atom's force and virial: warp sums, then the warps in a fixed order */
@@ -2037,12 +2045,12 @@ __global__ void __launch_bounds__(WPA * 32 * APB, (WPA >= 2 ? 512 : 384) / (WPA 
         for (int k = 0; k < 9; k++) v[k] = warp_sum(v[k]);
         if (WPA > 1) {
             if (lane == 0)
-                for (int k = 0; k < 9; k++) s.red[warp * 9 + k] = v[k];
+                for (int k = 0; k < 9; k++) s.fin[warp * 9 + k] = v[k];
             group_sync<WPA>();
             if (tid == 0)
                 for (int k = 0; k < 9; k++) {
                     double t = 0.0;
-                    for (int w = 0; w < WPA; w++) t += s.red[w * 9 + k];
+                    for (int w = 0; w < WPA; w++) t += s.fin[w * 9 + k];
                     v[k] = t;
                 }
         }
@@ -2051,12 +2059,6 @@ __global__ void __launch_bounds__(WPA * 32 * APB, (WPA >= 2 ? 512 : 384) / (WPA 
             atomicAdd(&A.F[3 * i + 1], v[1]);
             atomicAdd(&A.F[3 * i + 2], v[2]);
             for (int k = 0; k < 6; k++) A.vir[(size_t)i * 6 + k] = v[3 + k];
-        }
-        for (int t = tid; t < n; t += NT) {
-            const int j = s.j[t];
-            atomicAdd(&A.F[3 * j], s.Fnb[3 * t]);
-            atomicAdd(&A.F[3 * j + 1], s.Fnb[3 * t + 1]);
-            atomicAdd(&A.F[3 * j + 2], s.Fnb[3 * t + 2]);
         }
     }
 }
@@ -2328,7 +2330,7 @@ struct EfsShape {
 };
 static const EfsShape kShapes[] = {{1, 4}, {4, 1}, {8, 1}};
 #define EFS_STATIC_SMEM (sizeof(mb_params) + 16) /* k_efs's __shared__ Ps, with alignment slack */
-#define LEG_STATIC_SMEM (MB_MAXG4 + 16)          /* k_efs_leg's __shared__ g4cell */
+#define TRI_STATIC_SMEM sizeof(mb_tri_tab)        /* k_efs_tri's __shared__ tab */
 #define MB_NSHAPES 3
 #define MB_MAX_DEVICES_K 64
 
@@ -2379,13 +2381,11 @@ extern "C" int mbk_nlist(mb_dev *d, int N, int NM, const mb_cell *c, double rc, 
         k_cell_sort<<<(ncell + 3) / 4, 128, 0, st>>>(ncell, d->cell_start, d->cell_atoms); /* a warp per cell */
         k_nlist_cell<<<blocks, warps_per_block * 32, 0, st>>>(N, NM, d->capNB, d->X, *c, rc2, d->cell_of,
                                                               d->cell_start, d->cell_atoms, d->nn, d->nj,
-                                                              (double4 *)d->nd, d->status,
-                                                              d->legs_on ? d->nk : nullptr);
+                                                              (double4 *)d->nd, d->status);
         *launches += 5;
     } else {
         k_nlist_brute<<<blocks, warps_per_block * 32, 0, st>>>(N, NM, d->capNB, d->X, *c, rc2, d->nn, d->nj,
-                                                               (double4 *)d->nd, d->status,
-                                                               d->legs_on ? d->nk : nullptr);
+                                                               (double4 *)d->nd, d->status);
         *launches += 1;
     }
     return (int)cudaGetLastError();
@@ -2432,59 +2432,32 @@ static int launch_any(const mb_model *m, int shape, EfsArgs a, cudaStream_t st, 
     }
 }
 
-/* ---- leg-table path ---- */
+/* ---- fused triplet kernel ---- */
 
-/* The leg-table path applies to the model: every forward and derivative
- * function shares the list cutoff, the pair-mixed G4 exponents equal the
- * species-0 ones to rounding (so one leg row serves the energy and the
- * derivative terms), and the basis has the reference's shape (<= 8 G4
- * exponents, <= 4 integer zeta, <= 2 lambda). */
-static bool leg_model_ok(const mb_model *m) {
-    const mb_params &P = m->P;
-    if (P.ng4 < 1 || P.ne > 8 || P.nz > 4 || P.nlam > 2 || !P.zeta_int) return false;
-    const double rc = m->rc_list;
-    if (P.d_rc2 != rc || P.d_rc4 != rc) return false;
-    for (int s = 0; s < P.nspc; s++)
-        for (int t = 0; t < P.nspc; t++) {
-            const int p = s * s + t * t;
-            if (P.f_rc2[p] != rc || P.f_rc4[p] != rc) return false;
-            for (int e = 0; e < P.ne; e++)
-                if (fabs(P.f_eta4[p][e] - P.d_eta4[e]) > 1e-12 * fabs(P.d_eta4[e])) return false;
-        }
-    return true;
+/* 1 when a pass can run on k_efs_tri: the basis qualifies (mb_tri) and the
+ * neighbour capacity is within what its lists and sort hold */
+extern "C" int mbk_tri_usable(const mb_dev *d, const mb_model *m) {
+    return m->T.ok && d->tri_w && d->capNB <= MB_TRI_MAX_CAP ? 1 : 0;
 }
 
-extern "C" int mbk_legs_model(const mb_model *m) { return leg_model_ok(m) ? 1 : 0; }
+/* One warp per atom for large structures, several where the atoms alone do
+ * not fill the SMs; the autotuner times them. */
+static const EfsShape kTriShapes[] = {{1, 4}, {1, 2}, {2, 1}, {4, 1}, {8, 1}};
+#define MB_NTRISHAPES 5
 
-/* 1 when a pass of N atoms in cell c can run on leg tables: the model
- * qualifies, the tables are allocated, and every entry key fits (atom
- * index in 17 bits, images within +-15, neighbour capacity <= 128) */
-extern "C" int mbk_legs_usable(const mb_dev *d, const mb_model *m, int N, const mb_cell *c) {
-    if (!d->nk || !d->leg || !d->nso || !d->trip || !d->tboff || !d->lhash) return 0;
-    if (N >= MB_LEG_MAX_ATOMS || d->capNB > MB_LEG_MAX_CAP) return 0;
-    for (int q = 0; q < 3; q++)
-        if (c->Nq[q] > MB_LEG_MAX_IMAGE) return 0;
-    return leg_model_ok(m) ? 1 : 0;
+static size_t tri_group_bytes(const mb_model *m, int capNB, int wpa) {
+    return tri_smem_bytes(capNB, m->P.D, m->P.nspc, m->P.ng2, wpa);
 }
 
-/* shapes 0-3 with the per-lane-run reverse layout, 4-7 the same shapes
- * with the consecutive-entry layout */
-static const EfsShape kLegShapes[] = {{1, 4}, {1, 2}, {2, 1}, {4, 1}, {1, 4}, {1, 2}, {2, 1}, {4, 1}};
-#define MB_NLEGSHAPES 8
-
-static size_t leg_group_bytes(const mb_model *m, int capNB, int wpa) {
-    return leg_smem_bytes(capNB, m->P.D, m->P.ng2, wpa);
-}
-
-template <int NE, int WPA, int APB, int RV>
-static int launch_leg(const LegArgs &a, cudaStream_t st) {
-    auto kern = k_efs_leg<NE, WPA, APB, RV>;
+template <int NE, int WPA, int APB, bool STD>
+static int launch_tri(const TriArgs &a, cudaStream_t st) {
+    auto kern = k_efs_tri<NE, WPA, APB, STD>;
     const size_t smem = a.smem_group * APB;
     static size_t configured[MB_MAX_DEVICES_K] = {0};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MB_MAX_DEVICES_K) return (int)cudaErrorInvalidDevice;
-    if (smem + LEG_STATIC_SMEM > 227 * 1024) return (int)cudaErrorInvalidConfiguration;
-    if (smem + LEG_STATIC_SMEM > 48 * 1024 && smem > configured[dev]) {
+    if (smem + TRI_STATIC_SMEM > 227 * 1024) return (int)cudaErrorInvalidConfiguration;
+    if (smem + TRI_STATIC_SMEM > 48 * 1024 && smem > configured[dev]) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         configured[dev] = smem;
@@ -2493,49 +2466,36 @@ static int launch_leg(const LegArgs &a, cudaStream_t st) {
     return (int)cudaGetLastError();
 }
 
-/* k_legs, k_trip, then k_efs_leg in shape `shape`; the events (if any) bracket the three */
-static int launch_leg_pass(const mb_dev *d, const mb_model *m, int shape, LegArgs a, cudaStream_t st, cudaEvent_t e0,
-                           cudaEvent_t e1) {
-    a.smem_group = leg_group_bytes(m, a.cap, kLegShapes[shape].wpa);
-    if (e0) mbk_record(e0, st);
-    k_legs<<<(a.N + 3) / 4, 128, 0, st>>>(a.N, a.cap, d->nn, d->nj, d->nk, (double4 *)d->nd, d->spc, d->params,
-                                         d->leg, d->nso, (uint2 *)d->lhash);
-    k_trip<<<(a.N + TRIP_WARPS - 1) / TRIP_WARPS, 32 * TRIP_WARPS, 0, st>>>(
-        a.N, a.cap, d->tcap, m->P.nspc, d->nn, d->nj, d->nk, (const double4 *)d->nd, d->nso, d->spc, d->params,
-        (const uint2 *)d->lhash, (uint2 *)d->trip, d->tboff, a.counters);
-    int rc;
-    if (m->P.ne <= 7) {
-        switch (shape) {
-            case 0: rc = launch_leg<7, 1, 4, 0>(a, st); break;
-            case 1: rc = launch_leg<7, 1, 2, 0>(a, st); break;
-            case 2: rc = launch_leg<7, 2, 1, 0>(a, st); break;
-            case 3: rc = launch_leg<7, 4, 1, 0>(a, st); break;
-            case 4: rc = launch_leg<7, 1, 4, 1>(a, st); break;
-            case 5: rc = launch_leg<7, 1, 2, 1>(a, st); break;
-            case 6: rc = launch_leg<7, 2, 1, 1>(a, st); break;
-            default: rc = launch_leg<7, 4, 1, 1>(a, st); break;
-        }
-    } else {
-        switch (shape) {
-            case 0: rc = launch_leg<8, 1, 4, 0>(a, st); break;
-            case 1: rc = launch_leg<8, 1, 2, 0>(a, st); break;
-            case 2: rc = launch_leg<8, 2, 1, 0>(a, st); break;
-            case 3: rc = launch_leg<8, 4, 1, 0>(a, st); break;
-            case 4: rc = launch_leg<8, 1, 4, 1>(a, st); break;
-            case 5: rc = launch_leg<8, 1, 2, 1>(a, st); break;
-            case 6: rc = launch_leg<8, 2, 1, 1>(a, st); break;
-            default: rc = launch_leg<8, 4, 1, 1>(a, st); break;
-        }
+template <int NE, bool STD>
+static int launch_tri_shape(int shape, const TriArgs &a, cudaStream_t st) {
+    switch (shape) {
+        case 0: return launch_tri<NE, 1, 4, STD>(a, st);
+        case 1: return launch_tri<NE, 1, 2, STD>(a, st);
+        case 2: return launch_tri<NE, 2, 1, STD>(a, st);
+        case 3: return launch_tri<NE, 4, 1, STD>(a, st);
+        default: return launch_tri<NE, 8, 1, STD>(a, st);
     }
+}
+
+/* k_efs_tri in shape `shape`; the events (if any) bracket it */
+static int launch_tri_pass(const mb_model *m, int shape, TriArgs &a, cudaStream_t st, cudaEvent_t e0, cudaEvent_t e1) {
+    a.smem_group = tri_group_bytes(m, a.cap, kTriShapes[shape].wpa);
+    a.tlw = tri_list(a.cap, kTriShapes[shape].wpa);
+    if (e0) mbk_record(e0, st);
+    int rc;
+    if (m->T.std)
+        rc = m->P.ne <= 7 ? launch_tri_shape<7, true>(shape, a, st) : launch_tri_shape<8, true>(shape, a, st);
+    else
+        rc = launch_tri_shape<8, false>(shape, a, st);
     if (e1) mbk_record(e1, st);
     return rc;
 }
 
-/* warps per atom and atoms per CTA of shape `shape` of the leg kernel
- * (legs != 0) or of k_efs */
-extern "C" int mbk_shape_dims(int legs, int shape, int *wpa, int *apb) {
-    if (shape < 0 || shape >= (legs ? MB_NLEGSHAPES : MB_NSHAPES)) return 1;
-    const EfsShape &e = legs ? kLegShapes[shape] : kShapes[shape];
+/* warps per atom and atoms per CTA of shape `shape` of k_efs_tri (tri != 0)
+ * or of k_efs */
+extern "C" int mbk_shape_dims(int tri, int shape, int *wpa, int *apb) {
+    if (shape < 0 || shape >= (tri ? MB_NTRISHAPES : MB_NSHAPES)) return 1;
+    const EfsShape &e = tri ? kTriShapes[shape] : kShapes[shape];
     *wpa = e.wpa;
     *apb = e.apb;
     return 0;
@@ -2547,25 +2507,23 @@ extern "C" int mbk_shape_dims(int legs, int shape, int *wpa, int *apb) {
 static int tune_key(const mb_dev *d, int N, int mode) {
     int bucket = 0;
     while ((1 << bucket) < N) bucket++;
-    return (mode << 28) | ((d->legs_on ? 1 : 0) << 26) | (bucket << 20) | (d->capNB & 0xfffff);
+    return (mode << 28) | ((d->tri_on ? 1 : 0) << 26) | (bucket << 20) | (d->capNB & 0xfffff);
 }
 
-/* Decision for a pass that may run on leg tables: the four leg shapes and
- * the shapes of k_efs are each timed once (after an untimed launch) and the
- * fastest kept, 16 + shape for the leg path, shape for k_efs.  Small
- * structures (a few dozen atoms: one CTA per atom, most SMs idle) can favour
- * k_efs's many-warp shapes; large ones the leg path. */
-static int tune_family(mb_dev *d, const mb_model *m, int N, int mode, const LegArgs &la, const EfsArgs &a,
+/* Decision for a pass that may run on k_efs_tri: its shapes and those of
+ * k_efs are each timed once (after an untimed launch) and the fastest kept,
+ * 16 + shape for k_efs_tri, shape for k_efs. */
+static int tune_family(mb_dev *d, const mb_model *m, int N, int mode, const TriArgs &la, const EfsArgs &a,
                        cudaStream_t st) {
     const int key = tune_key(d, N, mode);
     for (int k = 0; k < d->tune_n; k++)
         if (d->tune_key[k] == key) return d->tune_val[k];
     int best = 16;
     if (d->tune_fixed >= 0) {
-        /* a forced shape (of the leg path) is recorded as the decision for this key */
-        best = 16 + (d->tune_fixed < MB_NLEGSHAPES ? d->tune_fixed : 0);
+        /* a forced shape (of k_efs_tri) is recorded as the decision for this key */
+        best = 16 + (d->tune_fixed < MB_NTRISHAPES ? d->tune_fixed : 0);
     } else {
-        LegArgs tl = la;
+        TriArgs tl = la;
         EfsArgs te = a;
         tl.counters = nullptr;
         te.counters = nullptr;
@@ -2573,23 +2531,23 @@ static int tune_family(mb_dev *d, const mb_model *m, int N, int mode, const LegA
         cudaEventCreate(&e0);
         cudaEventCreate(&e1);
         float best_ms = 1e30f;
-        for (int c = 0; c < MB_NLEGSHAPES + MB_NSHAPES; c++) {
-            const bool leg = c < MB_NLEGSHAPES;
-            const int sh = leg ? c : c - MB_NLEGSHAPES;
-            const size_t need = leg ? leg_group_bytes(m, la.cap, kLegShapes[sh].wpa) * kLegShapes[sh].apb + LEG_STATIC_SMEM
+        for (int c = 0; c < MB_NTRISHAPES + MB_NSHAPES; c++) {
+            const bool tri = c < MB_NTRISHAPES;
+            const int sh = tri ? c : c - MB_NTRISHAPES;
+            const size_t need = tri ? tri_group_bytes(m, la.cap, kTriShapes[sh].wpa) * kTriShapes[sh].apb + TRI_STATIC_SMEM
                                     : group_bytes(m, a.cap, kShapes[sh].wpa) * kShapes[sh].apb + EFS_STATIC_SMEM;
             if (need > 227 * 1024) continue;
             float ms = 1e30f;
             int bad = 0;
             for (int rep = 0; rep < 2 && !bad; rep++) {
                 if (mode == MB_MODE_EFS || mode == MB_MODE_VJP) cudaMemsetAsync(d->F, 0, sizeof(double) * 3 * N, st);
-                bad = leg ? launch_leg_pass(d, m, sh, tl, st, rep ? e0 : nullptr, rep ? e1 : nullptr)
+                bad = tri ? launch_tri_pass(m, sh, tl, st, rep ? e0 : nullptr, rep ? e1 : nullptr)
                           : launch_any(m, sh, te, st, rep ? e0 : nullptr, rep ? e1 : nullptr);
             }
             if (!bad && cudaEventSynchronize(e1) == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
             if (ms < best_ms) {
                 best_ms = ms;
-                best = leg ? 16 + sh : sh;
+                best = tri ? 16 + sh : sh;
             }
         }
         cudaEventDestroy(e0);
@@ -2672,24 +2630,20 @@ extern "C" int mbk_descriptor_pass(mb_dev *d, const mb_model *m, int N, int mode
     a.counters = d->counters;
     a.smem_group = 0;
     cudaMemsetAsync(d->EU, 0, sizeof(double) * N, st);
-    int fam = -1; /* k_efs shape chosen against the leg path */
-    if (d->legs_on) {
-        LegArgs la;
+    int fam = -1; /* k_efs shape chosen against k_efs_tri */
+    if (d->tri_on) {
+        TriArgs la;
         la.N = N;
         la.cap = d->capNB;
         la.mode = mode;
+        la.tlw = 0;
         la.urep = urep;
         la.nn = d->nn;
         la.nj = d->nj;
-        la.nso = d->nso;
         la.nd = (const double4 *)d->nd;
-        la.trip = (const uint2 *)d->trip;
-        la.tboff = d->tboff;
-        la.tcap = d->tcap;
-        la.leg = d->leg;
         la.spc = d->spc;
-        la.params = d->params;
         la.weights = d->weights;
+        la.w0 = d->tri_w;
         la.EA = d->EA;
         la.EU = d->EU;
         la.G = d->G;
@@ -2698,6 +2652,7 @@ extern "C" int mbk_descriptor_pass(mb_dev *d, const mb_model *m, int N, int mode
         la.counters = d->counters;
         la.smem_group = 0;
         la.P = m->P;
+        la.T = m->T;
         const int v = tune_family(d, m, N, mode, la, a, st);
         if (v >= 16) {
             d->last_shape = v;
@@ -2708,8 +2663,8 @@ extern "C" int mbk_descriptor_pass(mb_dev *d, const mb_model *m, int N, int mode
                 d->ev_n++;
             }
             if (mode == MB_MODE_EFS || mode == MB_MODE_VJP) cudaMemsetAsync(d->F, 0, sizeof(double) * 3 * N, st);
-            const int rc = launch_leg_pass(d, m, v - 16, la, st, e0, e1);
-            (*launches) += 3;
+            const int rc = launch_tri_pass(m, v - 16, la, st, e0, e1);
+            (*launches)++;
             return rc;
         }
         fam = v;

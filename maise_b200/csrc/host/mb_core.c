@@ -26,7 +26,7 @@
  * of this is unchanged (buffers, sizes, step parameters, profiling state) */
 typedef struct {
     long gen;
-    int N, NM, chunk, st_on, ev_on, legs;
+    int N, NM, chunk, st_on, ev_on, tri;
     double urep, dt, tau, T;
     mb_cell c;
     void *flush, *trace, *st_pool, *ev_pool;
@@ -36,7 +36,7 @@ typedef struct {
 /* what a single-structure pass graph was captured for */
 typedef struct {
     long gen;
-    int N, NM, ND, mode, M[3], legs;
+    int N, NM, ND, mode, M[3], tri;
     double urep;
     void *h_res;
 } pass_key;
@@ -70,9 +70,9 @@ struct mb_potential {
     size_t h_buf_len;
     int *h_status;
     double *h_out;
-    /* leg tables for the descriptor pass: the model qualifies and they are
-     * not switched off (MAISE_B200_LEGS=0) */
-    int legs_enabled;
+    /* the fused triplet kernel: the model qualifies and it is not switched
+     * off (MAISE_B200_LEGS=0: the general kernel only) */
+    int tri_enabled;
     /* MD chunk graph */
     int use_graphs;
     cudaGraphExec_t md_exec;
@@ -147,7 +147,7 @@ int mb_open(const char *model_path, int device, mb_potential **out) {
     }
     {
         const char *lg = getenv("MAISE_B200_LEGS");
-        p->legs_enabled = mbk_legs_model(&p->m) && !(lg && lg[0] == '0');
+        p->tri_enabled = p->m.T.ok && !(lg && lg[0] == '0');
     }
     CK(cudaSetDevice(device), "cudaSetDevice");
     CK(cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking), "cudaStreamCreate");
@@ -159,6 +159,11 @@ int mb_open(const char *model_path, int device, mb_potential **out) {
     CK(cudaMemcpy(p->d.weights, p->m.weights, sizeof(double) * p->m.weights_len, cudaMemcpyHostToDevice), "upload weights");
     CK(cudaMemcpy(p->d.weights + p->m.weights_len, p->m.mass, sizeof(double) * MB_MAXSPC, cudaMemcpyHostToDevice),
        "upload masses");
+    if (p->m.tri_weights) {
+        wbytes = sizeof(double) * (size_t)p->m.nspc * p->m.P.D * p->m.T.wrow;
+        CK(cudaMalloc((void **)&p->d.tri_w, wbytes), "cudaMalloc weights by input");
+        CK(cudaMemcpy(p->d.tri_w, p->m.tri_weights, wbytes, cudaMemcpyHostToDevice), "upload weights by input");
+    }
     CK(cudaMalloc((void **)&p->d.out, sizeof(double) * 16), "cudaMalloc out");
     CK(cudaMemset(p->d.out, 0, sizeof(double) * 16), "memset out");
     CK(cudaMalloc((void **)&p->d.part, sizeof(double) * 2 * MB_RED_MAXB * 8), "cudaMalloc part");
@@ -175,7 +180,6 @@ int mb_open(const char *model_path, int device, mb_potential **out) {
 }
 
 static void dev_free(mb_dev *d) {
-    cudaFree(d->nk); cudaFree(d->leg); cudaFree(d->nso); cudaFree(d->trip); cudaFree(d->tboff); cudaFree(d->lhash);
     cudaFree(d->X); cudaFree(d->V); cudaFree(d->spc); cudaFree(d->nn); cudaFree(d->nj); cudaFree(d->nd);
     cudaFree(d->F); cudaFree(d->EA); cudaFree(d->EU); cudaFree(d->vir); cudaFree(d->G);
     cudaFree(d->cell_of); cudaFree(d->cell_cnt); cudaFree(d->cell_start); cudaFree(d->cell_atoms);
@@ -198,6 +202,7 @@ int mb_close(mb_potential *p) {
     dev_free(&p->d);
     cudaFree(p->d.params);
     cudaFree(p->d.weights);
+    cudaFree(p->d.tri_w);
     cudaFree(p->d.out);
     cudaFree(p->d.part);
     cudaFree(p->d.ticket);
@@ -263,7 +268,7 @@ int mb_tune_read(const mb_potential *p, int cap, int *count, int *mode, int *leg
     n = p->d.tune_n < cap ? p->d.tune_n : cap;
     *count = n;
     for (k = 0; k < n; k++) {
-        /* a key with the leg path usable holds 16 + shape when the leg kernel
+        /* a key with the fused triplet kernel usable holds 16 + shape when it
          * won and a k_efs shape otherwise */
         const int key = p->d.tune_key[k], v = p->d.tune_val[k], lg = ((key >> 26) & 1) && v >= 16;
         mode[k] = key >> 28;
@@ -271,7 +276,7 @@ int mb_tune_read(const mb_potential *p, int cap, int *count, int *mode, int *leg
         size_bucket[k] = (key >> 20) & 0x3f;
         capacity[k] = key & 0xfffff;
         if (mbk_shape_dims(lg, lg ? v - 16 : v, &wpa[k], &apb[k])) wpa[k] = apb[k] = 0;
-        layout[k] = lg && v - 16 >= 4; /* leg shapes 4-7: reverse pass over consecutive entries */
+        layout[k] = lg; /* the triplet kernel's reverse pass runs over consecutive entries */
     }
     return MB_OK;
 }
@@ -409,30 +414,16 @@ static int ensure(mb_potential *p, int N, int nb, int ncell) {
         CK(cudaMalloc((void **)&d->cell_atoms, sizeof(int) * cap), "alloc cell_atoms");
         d->capN = cap;
         p->gen++;
-        cudaFree(d->nj); cudaFree(d->nd); cudaFree(d->nk); cudaFree(d->leg); cudaFree(d->nso);
-        cudaFree(d->trip); cudaFree(d->tboff); cudaFree(d->lhash);
-        d->nj = NULL; d->nd = NULL; d->nk = NULL; d->leg = NULL; d->nso = NULL; d->trip = NULL; d->tboff = NULL;
-        d->lhash = NULL;
+        cudaFree(d->nj); cudaFree(d->nd);
+        d->nj = NULL; d->nd = NULL;
         d->capNB = 0;
     }
     if (nb > d->capNB || !d->nj) {
         int cap = nb > d->capNB ? nb : d->capNB;
         cap = (cap + 7) & ~7;
-        cudaFree(d->nj); cudaFree(d->nd); cudaFree(d->nk); cudaFree(d->leg); cudaFree(d->nso);
-        cudaFree(d->trip); cudaFree(d->tboff); cudaFree(d->lhash);
-        d->nk = NULL; d->leg = NULL; d->nso = NULL; d->trip = NULL; d->tboff = NULL; d->lhash = NULL;
+        cudaFree(d->nj); cudaFree(d->nd);
         CK(cudaMalloc((void **)&d->nj, sizeof(int) * (size_t)cap * d->capN), "alloc nj");
         CK(cudaMalloc((void **)&d->nd, sizeof(double) * 4 * (size_t)cap * d->capN), "alloc nd");
-        if (p->legs_enabled && cap <= MB_LEG_MAX_CAP) {
-            /* leg tables of the descriptor pass (the model qualifies for them) */
-            CK(cudaMalloc((void **)&d->nk, sizeof(unsigned) * (size_t)cap * d->capN), "alloc nk");
-            CK(cudaMalloc((void **)&d->leg, sizeof(double) * MB_LEG_STRIDE * (size_t)cap * d->capN), "alloc legs");
-            CK(cudaMalloc((void **)&d->nso, sizeof(int) * 4 * (size_t)d->capN), "alloc nso");
-            d->tcap = cap * (cap - 1) / 2;
-            CK(cudaMalloc((void **)&d->trip, 2 * sizeof(unsigned) * (size_t)d->tcap * d->capN), "alloc trip");
-            CK(cudaMalloc((void **)&d->tboff, sizeof(int) * 8 * (size_t)d->capN), "alloc tboff");
-            CK(cudaMalloc((void **)&d->lhash, 2 * sizeof(unsigned) * 256 * (size_t)d->capN), "alloc list hash");
-        }
         d->capNB = cap;
         p->gen++;
     }
@@ -634,7 +625,7 @@ static int graph_pass(mb_potential *p, int N, int NM, int ND, const mb_cell *c, 
     k.M[2] = c->M[2];
     k.urep = urep;
     k.h_res = p->h_res;
-    k.legs = p->d.legs_on;
+    k.tri = p->d.tri_on;
     if (!q->x || memcmp(&k, &q->k, sizeof(k))) {
         cudaGraph_t g = NULL;
         if (!q->seen_valid || memcmp(&k, &q->seen, sizeof(k))) {
@@ -695,7 +686,7 @@ static int run_pass(mb_potential *p, int N, int NM, int ND, const double *lat9, 
     if (ND == 3) pV = p_gpa / MB_EV2GPA * cell_volume(lat9);
     ncell = c.M[0] ? c.M[0] * c.M[1] * c.M[2] : 1;
     if ((r = ensure(p, N, p->d.capNB ? p->d.capNB : (NM < 64 ? NM : 64), ncell))) return r;
-    p->d.legs_on = mbk_legs_usable(&p->d, &p->m, N, &c);
+    p->d.tri_on = p->tri_enabled && mbk_tri_usable(&p->d, &p->m);
     p->res_staged = 0;
     r = MB_FALLBACK;
     if (p->use_graphs && !p->pbroken && !p->d.ev_on && mbk_shape_ready(&p->d, N, mode)) {
@@ -807,7 +798,6 @@ int mb_neighbours(mb_potential *p, int N, int NM, int ND, int XT, const int *atm
     if (path == 2 && !c.M[0]) return fail(MB_ERR_ARG, "the cell cannot be binned (a periodic direction is under 3 Rc wide)");
     ncell = c.M[0] ? c.M[0] * c.M[1] * c.M[2] : 1;
     if ((r = ensure(p, N, p->d.capNB ? p->d.capNB : (NM < 64 ? NM : 64), ncell))) return r;
-    p->d.legs_on = 0;
     for (tries = 0; tries < 3; tries++) {
         if ((r = upload(p, N, XT, atmn, lat9, x))) return r;
         CK(cudaMemsetAsync(p->d.status, 0, sizeof(int) * 4, p->stream), "memset status");
@@ -874,7 +864,6 @@ int mb_descriptor_jvp(mb_potential *p, int N, int NM, int ND, int XT, const int 
     setup_cell(p, lat9, ND, N, &c);
     ncell = c.M[0] ? c.M[0] * c.M[1] * c.M[2] : 1;
     if ((r = ensure(p, N, p->d.capNB ? p->d.capNB : (NM < 64 ? NM : 64), ncell))) return r;
-    p->d.legs_on = 0;
     for (tries = 0; tries < 3; tries++) {
         if ((r = upload(p, N, XT, atmn, lat9, x))) return r;
         CK(cudaMemsetAsync(p->d.status, 0, sizeof(int) * 4, p->stream), "memset status");
@@ -1199,7 +1188,7 @@ static int md_chunk(mb_potential *p, int N, int NM, const mb_cell *c, double ure
                     int step, int chunk, int *graphed) {
     int r, s;
     *graphed = 0;
-    p->d.legs_on = mbk_legs_usable(&p->d, &p->m, N, c);
+    p->d.tri_on = p->tri_enabled && mbk_tri_usable(&p->d, &p->m);
     CK(cudaMemsetAsync(p->d.status, 0, sizeof(int) * 4, p->stream), "memset status");
     if ((r = mbk_set_out(&p->d, 10, (double)step, p->stream))) return cuda_fail((cudaError_t)r, "set step");
     if (p->use_graphs && mbk_shape_ready(&p->d, N, MB_MODE_EFS)) {
@@ -1221,7 +1210,7 @@ static int md_chunk(mb_potential *p, int N, int NM, const mb_cell *c, double ure
         k.trace = p->d.trace;
         k.st_pool = p->d.st_pool;
         k.ev_pool = p->d.ev_pool;
-        k.legs = p->d.legs_on;
+        k.tri = p->d.tri_on;
         if (!p->md_exec || memcmp(&k, &p->md_k, sizeof(k))) {
             cudaGraph_t g = NULL;
             cudaError_t e;

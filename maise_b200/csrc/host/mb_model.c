@@ -318,8 +318,124 @@ static int parse_basis(const mb_lines *L, mb_model *m, char *err, size_t el) {
     return 0;
 }
 
+/* Chebyshev interpolation of fn on [-1, 1] at deg + 1 nodes, as monomial
+ * coefficients, highest degree first (the functions below are smooth enough
+ * that the conversion loses nothing). */
+static void poly_fit(long double (*fn)(long double, const long double *), const long double *arg, int deg, double *out) {
+    const long double pi = acosl(-1.0L);
+    long double c[16], t0[16] = {0}, t1[16] = {0}, m[16] = {0};
+    int j, k;
+    for (j = 0; j <= deg; j++) {
+        long double s = 0.0L;
+        for (k = 0; k <= deg; k++) {
+            const long double th = pi * (2 * k + 1) / (2 * (deg + 1));
+            s += fn(cosl(th), arg) * cosl(j * th);
+        }
+        c[j] = s * (j ? 2.0L : 1.0L) / (deg + 1);
+    }
+    t0[0] = 1.0L;
+    t1[1] = 1.0L;
+    for (k = 0; k <= deg; k++) m[k] = c[0] * t0[k] + c[1] * t1[k];
+    for (j = 2; j <= deg; j++) {
+        long double t2[16];
+        for (k = 0; k <= deg; k++) t2[k] = (k ? 2.0L * t1[k - 1] : 0.0L) - t0[k];
+        for (k = 0; k <= deg; k++) {
+            m[k] += c[j] * t2[k];
+            t0[k] = t1[k];
+            t1[k] = t2[k];
+        }
+    }
+    for (k = 0; k <= deg; k++) out[k] = (double)m[deg - k];
+}
+
+static long double fn_exp(long double u, const long double *a) { return expl(-a[0] * (u + 1.0L)); }
+static long double fn_fc(long double v, const long double *a) {
+    return 0.5L * (1.0L + cosl(acosl(-1.0L) * sqrtl(0.5L * (v + 1.0L))));
+}
+/* f'(r) / r = -pi^2 / (2 Rc^2) sin(x) / x, x = pi r / Rc */
+static long double fn_h(long double v, const long double *a) {
+    const long double pi = acosl(-1.0L), x = pi * sqrtl(0.5L * (v + 1.0L));
+    return -pi * pi / (2.0L * a[0] * a[0]) * (x > 1e-10L ? sinl(x) / x : 1.0L);
+}
+
+/* The fused triplet kernel applies when every forward and derivative
+ * function shares the list cutoff, the pair-mixed G4 exponents equal the
+ * species-0 ones to rounding (so that one factor serves the energy and the
+ * derivative terms), the basis has the reference's shape (<= 8 G4 exponents,
+ * <= 4 integer zeta, <= 2 lambda) and no exponent is so large that the
+ * polynomial would need more than MB_TRI_MAXSQ squarings. */
+static void tri_tables(mb_model *m) {
+    const mb_params *P = &m->P;
+    mb_tri *T = &m->T;
+    const long double rc = m->rc_list;
+    long double top = 0.0L;
+    double h[MB_TRI_FDEG + 1];
+    int s, t, e, f, last[64];
+    memset(T, 0, sizeof(*T));
+    if (P->ng4 < 1 || P->ne > MB_TRI_MAXE || P->nz > 4 || P->nlam > 2 || !P->zeta_int) return;
+    if (P->d_rc2 != m->rc_list || P->d_rc4 != m->rc_list) return;
+    for (s = 0; s < P->nspc; s++)
+        for (t = 0; t < P->nspc; t++) {
+            const int p = s * s + t * t;
+            if (P->f_rc2[p] != m->rc_list || P->f_rc4[p] != m->rc_list) return;
+            for (e = 0; e < P->ne; e++)
+                if (fabs(P->f_eta4[p][e] - P->d_eta4[e]) > 1e-12 * fabs(P->d_eta4[e])) return;
+        }
+    for (e = 0; e < P->ne; e++) {
+        if (!(P->d_eta4[e] >= 0.0)) return;
+        if (P->d_eta4[e] > top) top = P->d_eta4[e];
+    }
+    top *= 1.5L * rc * rc; /* the largest eta rho at the middle of rho's range */
+    if (!(top <= 0.42L * (1 << MB_TRI_MAXSQ))) return;
+    /* two squarings always (the kernel's straight-line form), more where needed */
+    top *= 0.25L;
+    T->nsq = 2;
+    while (top > 0.42L) {
+        top *= 0.5L;
+        T->nsq++;
+    }
+    if (!(top > 1e-6L)) top = 1e-6L;
+    poly_fit(fn_exp, &top, MB_TRI_DEG, T->tab.ex);
+    for (e = 0; e < P->ne; e++) {
+        T->tab.kw[e] = (double)(P->d_eta4[e] / (top * (1 << T->nsq)));
+        T->tab.eta[e] = P->d_eta4[e];
+    }
+    poly_fit(fn_fc, &rc, MB_TRI_FDEG, T->tab.f);
+    poly_fit(fn_h, &rc, MB_TRI_FDEG, h);
+    for (e = 0; e <= MB_TRI_FDEG; e++) {
+        T->tab.fh[e][0] = T->tab.f[e];
+        T->tab.fh[e][1] = h[e];
+    }
+    T->sv = (double)(2.0L / (rc * rc));
+    for (e = 0; e < 64; e++) T->cell_fn[e] = -1, last[e] = -1;
+    for (f = 0; f < P->ng4; f++) {
+        const int c = P->g4_e[f] * 8 + (P->g4_zl[f] / P->nlam) * 2 + P->g4_zl[f] % P->nlam;
+        T->fn_next[f] = -1;
+        T->fn_cell[f] = (short)c;
+        if (last[c] < 0) T->cell_fn[c] = (short)f;
+        else T->fn_next[last[c]] = (short)f;
+        last[c] = f;
+    }
+    T->wrow = (P->h1 + 2) & ~1;
+    m->tri_weights = (double *)calloc((size_t)m->nspc * P->D * T->wrow, sizeof(double));
+    for (s = 0; s < m->nspc; s++) {
+        const double *off = m->weights + P->w_off[s], *W0 = off + P->D;
+        for (t = 0; t < P->D; t++) {
+            double *r = m->tri_weights + ((size_t)s * P->D + t) * T->wrow;
+            for (e = 0; e < P->h1; e++) r[e] = W0[(size_t)e * P->D + t];
+            r[P->h1] = off[t];
+        }
+    }
+    T->std = T->nsq == 2 && P->zeta_std && P->nlam == 2 && P->lam[0] == -1.0 && P->lam[1] == 1.0;
+    for (e = 0; e < MB_TRI_LOW && e < MB_TRI_MAXE; e++)
+        for (s = 4; s < 8; s++)
+            if (T->cell_fn[8 * e + s] >= 0) T->std = 0;
+    T->ok = 1;
+}
+
 void mb_model_free(mb_model *m) {
     free(m->weights);
+    free(m->tri_weights);
     memset(m, 0, sizeof(*m));
 }
 
@@ -401,6 +517,7 @@ int mb_model_load(const char *path, mb_model *m, char *err, size_t el) {
         m->P.rm[s] = mb_min_dist[z];
         m->mass[s] = mb_mass_of_z(z);
     }
+    tri_tables(m);
     free(V);
     lines_free(&L);
     return 0;

@@ -63,12 +63,48 @@ typedef struct {
  */
 #define MB_NET_SIZE(D, h1, h2) ((D) + (h1) * (D) + (h1) + (h2) * (h1) + (h2) + (h2) + 1)
 
+/* Tables of the fused triplet kernel (k_efs_tri).  The sum of a triplet's
+ * squared legs is rho = r_ij^2 + r_ik^2 + r_jk^2 < 3 Rc^2, so the factor
+ * exp(-eta_e rho) of G4 is a smooth function on a known interval: one
+ * polynomial of exp(-z) serves every exponent, at z = eta_e rho / 2^nsq, and
+ * the result is squared nsq times.  The cutoff f = (1 + cos(pi r / Rc)) / 2
+ * and h = f'(r) / r are entire functions of r^2: polynomials in
+ * 2 r^2 / Rc^2 - 1.  Coefficients are stored highest degree first. */
+#define MB_TRI_MAXE 8
+#define MB_TRI_DEG 11  /* exp: truncation below 2e-17 for z within +-0.42 of its middle */
+#define MB_TRI_FDEG 11 /* f and h: truncation below 1e-18 */
+#define MB_TRI_MAXSQ 4
+#define MB_TRI_LOW 3
+typedef struct {
+    double ex[MB_TRI_DEG + 1];    /* exp(-z), z = zmid (1 + w) */
+    double kw[MB_TRI_MAXE];       /* w = kw[e] rho - 1 */
+    double f[MB_TRI_FDEG + 1];
+    double fh[MB_TRI_FDEG + 1][2]; /* f and h side by side (reverse pass) */
+    double eta[MB_TRI_MAXE];
+} mb_tri_tab;
+typedef struct {
+    mb_tri_tab tab;
+    int ok, nsq;                  /* the basis qualifies for k_efs_tri; squarings (at least 2) */
+    /* the reference's function table: zeta = 1, 2, 4, 16, lambda = -1, 1,
+     * nsq = 2, and the first MB_TRI_LOW exponents used with zeta = 1, 2 only */
+    int std;
+    double sv;                    /* 2 / Rc^2 */
+    /* (eta, zeta, lambda) cell -> its first G4 function (-1: none), and the
+     * next function of the same cell (-1: none); the cell of each function */
+    short cell_fn[64], fn_next[MB_MAXG4], fn_cell[MB_MAXG4];
+    /* first-layer weights by input: per species and input l a row of wrow
+     * doubles (even: 16-byte loads) holding W0[0..h1-1][l] and off[l] */
+    int wrow;
+} mb_tri;
+
 /* Host copy of a parsed model. */
 typedef struct {
     int nspc, spcz[MB_MAXSPC];
     int nl, nu[4], nw;
     mb_params P;
+    mb_tri T;
     double rc_list;          /* neighbour-list cutoff */
+    double *tri_weights;     /* [nspc][D][T.wrow], see mb_tri */
     double *weights;         /* host copy of the weight buffer */
     size_t weights_len;
     double mass[MB_MAXSPC];  /* amu * 103.6427 (src/cmod.c:1130) */
@@ -86,12 +122,7 @@ typedef struct {
     int M[3];      /* cell-list bins per direction (0: brute force) */
 } mb_cell;
 
-/* leg-table path of the descriptor pass: one row per neighbour-list entry,
- * exp(-eta_e r^2) for e < 8, fc(r), fc'(r)/r */
-#define MB_LEG_STRIDE 10
-#define MB_LEG_MAX_ATOMS (1 << 17) /* atom index in 17 bits of an entry key */
-#define MB_LEG_MAX_IMAGE 15        /* |image| per axis in 5 bits of an entry key */
-#define MB_LEG_MAX_CAP 128         /* neighbour capacity the leg kernels handle */
+#define MB_TRI_MAX_CAP 128 /* neighbour capacity the fused triplet kernel handles */
 
 /* status bits written by kernels */
 #define MB_ST_NBR_OVERFLOW 1   /* an atom reached NM neighbours */
@@ -134,22 +165,8 @@ typedef struct {
     unsigned long long *counters; /* [2]: pairs and triplets seen by the descriptor kernel */
     mb_params *params;
     double *weights;
-    /* leg tables (see mb_kernels.cu, k_legs): with legs_on the list kernels
-     * also write each entry's key (atom << 15 | image, 5 bits per axis),
-     * k_legs sorts every atom's list by species (nso[4N]: species starts
-     * and the count) and fills leg[N*capNB*MB_LEG_STRIDE] with each entry's
-     * exp(-eta_e r^2), fc(r) and fc'(r)/r; NULL where not allocated */
-    unsigned *nk;
-    double *leg;
-    int *nso;
-    /* triplet lists of the leg path (k_trip): trip[N*tcap] entries
-     * {a | b << 8, j-k leg row} per atom, tboff[8N] the species blocks'
-     * starts and the end; tcap = capNB (capNB - 1) / 2 bounds any list */
-    void *trip;
-    int *tboff;
-    int tcap;
-    void *lhash;      /* [N*256] uint2 (key, slot) per atom: the hash of its list (k_legs) */
-    int legs_on;
+    double *tri_w;    /* first-layer weights by input (mb_tri); owned by the handle */
+    int tri_on;       /* the next descriptor pass may run on k_efs_tri */
     /* optional CUDA-event timing of the descriptor kernel */
     int ev_on, ev_n, ev_cap;
     void *ev_pool;    /* cudaEvent_t[2*ev_cap] */
@@ -179,9 +196,8 @@ int mbk_nvt_update(mb_dev *d, const mb_model *m, int N, double dt, double tau, d
 int mbk_set_out(mb_dev *d, int idx, double v, void *stream);
 void mbk_record(void *event, void *stream);
 int mbk_shape_ready(const mb_dev *d, int N, int mode);
-int mbk_legs_model(const mb_model *m);
-int mbk_legs_usable(const mb_dev *d, const mb_model *m, int N, const mb_cell *c);
-int mbk_shape_dims(int legs, int shape, int *wpa, int *apb);
+int mbk_tri_usable(const mb_dev *d, const mb_model *m);
+int mbk_shape_dims(int tri, int shape, int *wpa, int *apb);
 int mbk_graph_cell_nodes(void *graph, void **nodes, int *rows, int cap);
 int mbk_graph_set_cell(void *exec, void *const *nodes, const int *rows, int count, const mb_cell *c, double pV);
 size_t mbk_efs_smem(const mb_model *m, int capNB, int shape);
