@@ -38,8 +38,8 @@
  *   k_tr_frc     one warp per marked atom: f_i, dfq and the force loss term
  *   k_tr_fown    one CTA per block owner: the force-gradient terms of the
  *                owner's network, summed over its blocks in block order
- *   k_tr_grad    one thread per parameter: the sum over the atoms of its
- *                species in atom order, / S, + 2 LREG V
+ *   k_tr_gpart   partial sums of the gradient over chunks of one species'
+ *                atoms; k_tr_gsum adds the chunks in order, / S, + 2 LREG V
  */
 #include <cuda_runtime.h>
 #include <math.h>
@@ -65,33 +65,62 @@ __host__ __device__ inline int off_W0(const TrainDims &t) { return t.h1 + t.h2 +
 __host__ __device__ inline int off_W1(const TrainDims &t) { return off_W0(t) + t.h1 * t.D; }
 __host__ __device__ inline int off_W2(const TrainDims &t) { return off_W1(t) + t.h2 * t.h1; }
 
-__global__ void k_tr_fwd(TrainDims t, const double *__restrict__ X, const int *__restrict__ spc,
-                         const double *__restrict__ V, double *__restrict__ H1, double *__restrict__ H2,
-                         double *__restrict__ Eat) {
+/* Sum of 16 per-lane values across a warp: lanes l and l ^ 1 end with the
+ * total of value l >> 1 (four halving steps and one exchange). */
+__device__ __forceinline__ double reduce16(double *v, int lane) {
+#pragma unroll
+    for (int step = 0; step < 4; step++) {
+        const int off = 16 >> step, half = 8 >> step;
+        const bool upper = (lane & off) != 0;
+#pragma unroll
+        for (int k = 0; k < half; k++) {
+            const double send = upper ? v[k] : v[k + half];
+            const double keep = upper ? v[k + half] : v[k];
+            v[k] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+        }
+    }
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+/* one warp per atom: 16 first-layer units at a time in the lanes' partial
+ * sums (each input read once), then a unit a lane */
+__global__ void __launch_bounds__(128) k_tr_fwd(TrainDims t, const double *__restrict__ X, const int *__restrict__ spc,
+                                                const double *__restrict__ V, double *__restrict__ H1,
+                                                double *__restrict__ H2, double *__restrict__ Eat) {
     const int a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (a >= t.Na) return;
     const double *v = V + (size_t)spc[a] * t.P, *x = X + (size_t)a * t.D;
     const double *W0 = v + off_W0(t), *b0 = v;
-    double h1[MB_TRAIN_MAXH];
-    for (int k = 0; k < t.h1; k++) {
-        double acc = 0.0;
-        for (int n = lane; n < t.D; n += 32) acc += W0[(size_t)k * t.D + n] * x[n];
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        h1[k] = tanh(b0[k] + acc);
-    }
-    if (lane == 0) {
-        const double *W1 = v + off_W1(t), *b1 = v + off_b1(t), *W2 = v + off_W2(t), *b2 = v + off_b2(t);
-        double e = b2[0];
-        for (int m = 0; m < t.h2; m++) {
-            double s = b1[m];
-            for (int k = 0; k < t.h1; k++) s += W1[m * t.h1 + k] * h1[k];
-            const double h = tanh(s);
-            H2[(size_t)a * t.h2 + m] = h;
-            e += W2[m] * h;
+    double h = 0.0; /* lane k: activation k of the first layer */
+    for (int u = 0; u < t.h1; u += 16) {
+        double acc[16];
+#pragma unroll
+        for (int k = 0; k < 16; k++) acc[k] = 0.0;
+        for (int n = lane; n < t.D; n += 32) {
+            const double xn = x[n], *w = W0 + (size_t)u * t.D + n;
+#pragma unroll
+            for (int k = 0; k < 16; k++)
+                if (u + k < t.h1) acc[k] = fma(w[(size_t)k * t.D], xn, acc[k]);
         }
-        for (int k = 0; k < t.h1; k++) H1[(size_t)a * t.h1 + k] = h1[k];
-        Eat[a] = e;
+        const double tot = reduce16(acc, lane);
+        const double mine = __shfl_sync(0xffffffffu, tot, 2 * (lane & 15)); /* unit u + (lane & 15) */
+        if ((lane & 16) == (u & 16) && lane < t.h1) h = tanh(b0[lane] + mine);
     }
+    const double *W1 = v + off_W1(t), *b1 = v + off_b1(t), *W2 = v + off_W2(t), *b2 = v + off_b2(t);
+    double s = lane < t.h2 ? b1[lane] : 0.0;
+    for (int k = 0; k < t.h1; k++) {
+        const double hk = __shfl_sync(0xffffffffu, h, k);
+        if (lane < t.h2) s = fma(W1[lane * t.h1 + k], hk, s);
+    }
+    double e = 0.0;
+    if (lane < t.h2) {
+        const double g = tanh(s);
+        H2[(size_t)a * t.h2 + lane] = g;
+        e = W2[lane] * g;
+    }
+    for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+    if (lane < t.h1) H1[(size_t)a * t.h1 + lane] = h;
+    if (lane == 0) Eat[a] = b2[0] + e;
 }
 
 __global__ void k_tr_struct(TrainDims t, const int *__restrict__ soff, const double *__restrict__ Eat,
@@ -233,7 +262,7 @@ __global__ void k_tr_frc(TrainDims t, int NF, const int *__restrict__ fatom, con
  * with e, d = 1 - e^2, c = 2 e (e^2 - 1) of o's activations (GP, GPp, GPc,
  * src/nmlp.c:8-27) and alpha[n] = sum_m W2[m] d2[m] W1[m][n].  Phi and Gam
  * receive sum_b phi and sum_b gamma; the first-layer terms
- * -(ad1 (x) phi + gamma (x) x_o) and b0 -= gamma are formed in k_tr_grad. */
+ * -(ad1 (x) phi + gamma (x) x_o) and b0 -= gamma are formed in k_tr_gpart. */
 __global__ void __launch_bounds__(128) k_tr_fown(TrainDims t, const int *__restrict__ owners,
                                                  const int *__restrict__ ooff, const int *__restrict__ olist,
                                                  const int *__restrict__ bmk, const int *__restrict__ spc,
@@ -325,61 +354,112 @@ struct ForceTerms {
     const double *AD1, *Phi, *Gam, *fB1, *fW1, *fW2;
 };
 
-/* one thread per parameter of one species: the sum over that species'
- * atoms (in atom order) of the parameter's back-propagated terms, energy
- * and (with force training) force */
-__global__ void k_tr_grad(TrainDims t, const int *__restrict__ satoms, const int *__restrict__ soffs,
-                          const double *__restrict__ X, const double *__restrict__ H1, const double *__restrict__ H2,
-                          const double *__restrict__ d0, const double *__restrict__ d1, const double *__restrict__ ca,
-                          ForceTerms ft, const double *__restrict__ V, double *__restrict__ grad) {
+/* The gradient is a sum over a species' atoms of outer products (W0: h1 x D
+ * a species from a few thousand atoms).  One thread per parameter walking its
+ * species' atoms was a serial chain of dependent loads on 9000 threads
+ * (4.2 ms for 12800 atoms); here the atoms are cut into chunks of at most
+ * GR_CHUNK atoms of one species, a CTA forms a chunk's partial sums for
+ * GR_N inputs of W0 (or for all the other parameters), and k_tr_gsum adds
+ * the chunks in order: 500 CTAs, X read once from L2, and the same sums on
+ * every run.  Chunks of atoms that own force blocks hold the force terms. */
+#define GR_CHUNK 128
+#define GR_N 64
+struct GradChunk {
+    int lo, n, force; /* atoms list[lo .. lo + n) of the species list or of the owner list */
+    int spc;
+};
+
+__global__ void __launch_bounds__(256) k_tr_gpart(TrainDims t, const GradChunk *__restrict__ chunks,
+                                                  const int *__restrict__ satoms, const int *__restrict__ sowners,
+                                                  const double *__restrict__ X, const double *__restrict__ H1,
+                                                  const double *__restrict__ H2, const double *__restrict__ d0,
+                                                  const double *__restrict__ d1, const double *__restrict__ ca,
+                                                  ForceTerms ft, double *__restrict__ part) {
+    __shared__ int at[GR_CHUNK];
+    __shared__ double cf[GR_CHUNK * MB_TRAIN_MAXH];
+    const GradChunk c = chunks[blockIdx.x];
+    const int tid = threadIdx.x, h1 = t.h1, h2 = t.h2, D = t.D;
+    double *out = part + (size_t)blockIdx.x * t.P;
+    const int *list = c.force ? sowners : satoms;
+    for (int q = tid; q < c.n; q += 256) at[q] = list[c.lo + q];
+    __syncthreads();
+    if (blockIdx.y < gridDim.y - 1) {
+        /* W0[k][n] of GR_N inputs n: 4 threads an input, each the units k = kg, kg + 4, ... */
+        const double *cx = c.force ? ft.Gam : d0;
+        for (int e = tid; e < c.n * h1; e += 256) {
+            const double v = cx[(size_t)at[e / h1] * h1 + e % h1];
+            cf[e] = c.force ? -v : v;
+        }
+        __syncthreads();
+        const int n = blockIdx.y * GR_N + (tid & (GR_N - 1)), kg = tid / GR_N;
+        double acc[MB_TRAIN_MAXH / 4];
+#pragma unroll
+        for (int j = 0; j < MB_TRAIN_MAXH / 4; j++) acc[j] = 0.0;
+        if (n < D) {
+#pragma unroll 4
+            for (int q = 0; q < c.n; q++) {
+                const double x = X[(size_t)at[q] * D + n];
+#pragma unroll
+                for (int j = 0; j < MB_TRAIN_MAXH / 4; j++)
+                    if (kg + 4 * j < h1) acc[j] = fma(cf[q * h1 + kg + 4 * j], x, acc[j]);
+            }
+            if (c.force)
+                for (int q = 0; q < c.n; q++) {
+                    const double x = ft.Phi[(size_t)at[q] * D + n];
+#pragma unroll
+                    for (int j = 0; j < MB_TRAIN_MAXH / 4; j++)
+                        if (kg + 4 * j < h1) acc[j] = fma(-ft.AD1[(size_t)at[q] * h1 + kg + 4 * j], x, acc[j]);
+                }
+#pragma unroll
+            for (int j = 0; j < MB_TRAIN_MAXH / 4; j++)
+                if (kg + 4 * j < h1) out[off_W0(t) + (size_t)(kg + 4 * j) * D + n] = acc[j];
+        }
+        return;
+    }
+    /* the other parameters, one a thread */
+    const int rest = t.P - h1 * D;
+    for (int r = tid; r < rest; r += 256) {
+        const int p = r < off_W0(t) ? r : r + h1 * D;
+        double acc = 0.0;
+        if (p < off_b1(t)) {
+            if (c.force)
+                for (int q = 0; q < c.n; q++) acc -= ft.Gam[(size_t)at[q] * h1 + p];
+            else
+                for (int q = 0; q < c.n; q++) acc += d0[(size_t)at[q] * h1 + p];
+        } else if (p < off_b2(t)) {
+            const double *v = (c.force ? ft.fB1 : d1) + p - off_b1(t);
+            for (int q = 0; q < c.n; q++) acc += v[(size_t)at[q] * h2];
+        } else if (p < off_W0(t)) {
+            if (!c.force)
+                for (int q = 0; q < c.n; q++) acc += ca[at[q]];
+        } else if (p < off_W2(t)) {
+            const int m = (p - off_W1(t)) / h1, k = (p - off_W1(t)) % h1;
+            if (c.force)
+                for (int q = 0; q < c.n; q++) acc += ft.fW1[((size_t)at[q] * h2 + m) * h1 + k];
+            else
+#pragma unroll 4
+                for (int q = 0; q < c.n; q++)
+                    acc = fma(d1[(size_t)at[q] * h2 + m], H1[(size_t)at[q] * h1 + k], acc);
+        } else {
+            const int m = p - off_W2(t);
+            if (c.force)
+                for (int q = 0; q < c.n; q++) acc += ft.fW2[(size_t)at[q] * h2 + m];
+            else
+                for (int q = 0; q < c.n; q++) acc = fma(ca[at[q]], H2[(size_t)at[q] * h2 + m], acc);
+        }
+        out[p] = acc;
+    }
+}
+
+/* one thread per parameter: its species' chunks in order, / S, + 2 LREG V */
+__global__ void k_tr_gsum(TrainDims t, const int *__restrict__ coff, const double *__restrict__ part,
+                          const double *__restrict__ V, double *__restrict__ grad) {
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= t.nspc * t.P) return;
     const int s = idx / t.P, p = idx % t.P;
-    const int lo = soffs[s], hi = soffs[s + 1];
-    const bool F = ft.Gam != nullptr;
     double acc = 0.0;
-    if (p < off_b1(t)) {
-        const int k = p;
-        for (int q = lo; q < hi; q++) {
-            const int a = satoms[q];
-            acc += d0[(size_t)a * t.h1 + k];
-            if (F) acc -= ft.Gam[(size_t)a * t.h1 + k];
-        }
-    } else if (p < off_b2(t)) {
-        const int m = p - off_b1(t);
-        for (int q = lo; q < hi; q++) {
-            const int a = satoms[q];
-            acc += d1[(size_t)a * t.h2 + m];
-            if (F) acc += ft.fB1[(size_t)a * t.h2 + m];
-        }
-    } else if (p < off_W0(t)) {
-        for (int q = lo; q < hi; q++) acc += ca[satoms[q]];
-    } else if (p < off_W1(t)) {
-        const int k = (p - off_W0(t)) / t.D, n = (p - off_W0(t)) % t.D;
-        for (int q = lo; q < hi; q++) {
-            const int a = satoms[q];
-            double dk = d0[(size_t)a * t.h1 + k];
-            if (F) {
-                dk -= ft.Gam[(size_t)a * t.h1 + k];
-                acc -= ft.AD1[(size_t)a * t.h1 + k] * ft.Phi[(size_t)a * t.D + n];
-            }
-            acc += dk * X[(size_t)a * t.D + n];
-        }
-    } else if (p < off_W2(t)) {
-        const int m = (p - off_W1(t)) / t.h1, k = (p - off_W1(t)) % t.h1;
-        for (int q = lo; q < hi; q++) {
-            const int a = satoms[q];
-            acc += d1[(size_t)a * t.h2 + m] * H1[(size_t)a * t.h1 + k];
-            if (F) acc += ft.fW1[((size_t)a * t.h2 + m) * t.h1 + k];
-        }
-    } else {
-        const int m = p - off_W2(t);
-        for (int q = lo; q < hi; q++) {
-            const int a = satoms[q];
-            acc += ca[a] * H2[(size_t)a * t.h2 + m];
-            if (F) acc += ft.fW2[(size_t)a * t.h2 + m];
-        }
-    }
+#pragma unroll 4
+    for (int c = coff[s]; c < coff[s + 1]; c++) acc += part[(size_t)c * t.P + p];
     grad[idx] = acc / (double)t.S + 2.0 * t.LREG * V[idx];
 }
 
@@ -391,7 +471,11 @@ struct mb_train {
     TrainDims t;
     int NW;
     double *X, *Eref, *wt, *V, *H1, *H2, *Eat, *Es, *cs, *ls, *d0, *d1, *ca, *grad;
-    int *spc, *sat, *soff, *satoms, *soffs;
+    int *spc, *sat, *soff, *satoms;
+    /* chunks of the gradient sums (tr_chunks): coff[s] the first of species s */
+    GradChunk *chunks;
+    int nchunk, *coff, *sowners, hsoffs[4];
+    double *part;
     double *h_ls;
     long evals;
     /* force training (mb_train_set_forces): NF marked atoms, NB blocks,
@@ -416,7 +500,8 @@ extern "C" int mb_train_close(mb_train *tr) {
     cudaFree(tr->X); cudaFree(tr->Eref); cudaFree(tr->wt); cudaFree(tr->V); cudaFree(tr->grad);
     cudaFree(tr->H1); cudaFree(tr->H2); cudaFree(tr->d0); cudaFree(tr->d1); cudaFree(tr->Eat); cudaFree(tr->ca);
     cudaFree(tr->Es); cudaFree(tr->cs); cudaFree(tr->ls); cudaFree(tr->spc); cudaFree(tr->sat); cudaFree(tr->soff);
-    cudaFree(tr->satoms); cudaFree(tr->soffs);
+    cudaFree(tr->satoms);
+    cudaFree(tr->chunks); cudaFree(tr->coff); cudaFree(tr->sowners); cudaFree(tr->part);
     cudaFree(tr->fatom); cudaFree(tr->boff); cudaFree(tr->bown); cudaFree(tr->bmk); cudaFree(tr->owners);
     cudaFree(tr->ooff); cudaFree(tr->olist); cudaFree(tr->Fref); cudaFree(tr->Fn); cudaFree(tr->Pj);
     cudaFree(tr->AD1); cudaFree(tr->fpred); cudaFree(tr->dfq); cudaFree(tr->lf); cudaFree(tr->Phi);
@@ -426,6 +511,44 @@ extern "C" int mb_train_close(mb_train *tr) {
     if (tr->st) cudaStreamDestroy(tr->st);
     free(tr);
     return MB_OK;
+}
+
+/* Lay out the gradient's chunks: per species its atoms, then the atoms that
+ * own force blocks (hfoffs[s] .. hfoffs[s + 1] of sowners; NULL without
+ * force data), and the buffer of their partial sums. */
+static int tr_chunks(mb_train *tr, const int *hfoffs) {
+    const TrainDims &t = tr->t;
+    int n = 0, coff[4] = {0, 0, 0, 0}, rc;
+    for (int s = 0; s < t.nspc; s++) {
+        n += (tr->hsoffs[s + 1] - tr->hsoffs[s] + GR_CHUNK - 1) / GR_CHUNK;
+        if (hfoffs) n += (hfoffs[s + 1] - hfoffs[s] + GR_CHUNK - 1) / GR_CHUNK;
+    }
+    GradChunk *h = (GradChunk *)malloc(sizeof(GradChunk) * (n ? n : 1));
+    if (!h) return mb_handle_fail(MB_ERR_ARG, "out of memory");
+    n = 0;
+    for (int s = 0; s < t.nspc; s++) {
+        coff[s] = n;
+        for (int f = 0; f < (hfoffs ? 2 : 1); f++) {
+            const int *o = f ? hfoffs : tr->hsoffs;
+            for (int lo = o[s]; lo < o[s + 1]; lo += GR_CHUNK)
+                h[n++] = {lo, o[s + 1] - lo < GR_CHUNK ? o[s + 1] - lo : GR_CHUNK, f, s};
+        }
+    }
+    for (int s = t.nspc; s < 4; s++) coff[s] = n;
+    cudaFree(tr->chunks);
+    cudaFree(tr->coff);
+    cudaFree(tr->part);
+    tr->chunks = nullptr;
+    tr->coff = nullptr;
+    tr->part = nullptr;
+    tr->nchunk = n;
+    rc = tr_cuda(cudaMalloc((void **)&tr->chunks, sizeof(GradChunk) * (n ? n : 1)), "cudaMalloc chunks");
+    if (!rc) rc = tr_cuda(cudaMalloc((void **)&tr->coff, sizeof(coff)), "cudaMalloc coff");
+    if (!rc) rc = tr_cuda(cudaMalloc((void **)&tr->part, sizeof(double) * (size_t)(n ? n : 1) * t.P), "cudaMalloc part");
+    if (!rc) rc = tr_cuda(cudaMemcpy(tr->chunks, h, sizeof(GradChunk) * n, cudaMemcpyHostToDevice), "H2D chunks");
+    if (!rc) rc = tr_cuda(cudaMemcpy(tr->coff, coff, sizeof(coff), cudaMemcpyHostToDevice), "H2D coff");
+    free(h);
+    return rc;
 }
 
 extern "C" int mb_train_open(int device, int S, const int *nat, const int *atmn, int nspc, int D, int h1, int h2,
@@ -501,7 +624,6 @@ extern "C" int mb_train_open(int device, int S, const int *nat, const int *atmn,
     TA(sat, Na);
     TA(soff, S + 1);
     TA(satoms, Na);
-    TA(soffs, 4);
 #undef TA
     if (!rc) rc = tr_cuda(cudaMemcpy(tr->X, hX, sizeof(double) * (size_t)Na * D, cudaMemcpyHostToDevice), "H2D");
     if (!rc) rc = tr_cuda(cudaMemcpy(tr->Eref, E_ref, sizeof(double) * S, cudaMemcpyHostToDevice), "H2D");
@@ -510,7 +632,8 @@ extern "C" int mb_train_open(int device, int S, const int *nat, const int *atmn,
     if (!rc) rc = tr_cuda(cudaMemcpy(tr->sat, hsat, sizeof(int) * Na, cudaMemcpyHostToDevice), "H2D");
     if (!rc) rc = tr_cuda(cudaMemcpy(tr->soff, hsoff, sizeof(int) * (S + 1), cudaMemcpyHostToDevice), "H2D");
     if (!rc) rc = tr_cuda(cudaMemcpy(tr->satoms, hsatoms, sizeof(int) * Na, cudaMemcpyHostToDevice), "H2D");
-    if (!rc) rc = tr_cuda(cudaMemcpy(tr->soffs, hsoffs, sizeof(int) * 4, cudaMemcpyHostToDevice), "H2D");
+    memcpy(tr->hsoffs, hsoffs, sizeof(hsoffs));
+    if (!rc) rc = tr_chunks(tr, nullptr);
     if (!rc) rc = tr_cuda(cudaMallocHost((void **)&tr->h_ls, sizeof(double) * S), "cudaMallocHost");
     free(hX);
     free(hsat);
@@ -544,7 +667,7 @@ extern "C" int mb_train_set_forces(mb_train *tr, int NF, const int *f_atom, cons
     /* atom -> structure, to check that every block belongs to its marked atom's structure */
     int *sat = (int *)malloc(sizeof(int) * t.Na), *atmn = (int *)malloc(sizeof(int) * t.Na);
     int *cnt = (int *)calloc((size_t)t.Na + 1, sizeof(int)), *bmk = (int *)malloc(sizeof(int) * NB);
-    int *ooff = nullptr, *olist = nullptr, *owners = nullptr;
+    int *ooff = nullptr, *olist = nullptr, *owners = nullptr, *sown = nullptr, hfoffs[4] = {0, 0, 0, 0};
     double *hFn = nullptr;
     int rc = MB_OK;
     if (!sat || !atmn || !cnt || !bmk) { rc = mb_handle_fail(MB_ERR_ARG, "out of memory"); goto out; }
@@ -570,8 +693,9 @@ extern "C" int mb_train_set_forces(mb_train *tr, int NF, const int *f_atom, cons
     ooff = (int *)malloc(sizeof(int) * ((size_t)t.Na + 1));
     olist = (int *)malloc(sizeof(int) * NB);
     owners = (int *)malloc(sizeof(int) * t.Na);
+    sown = (int *)malloc(sizeof(int) * t.Na);
     hFn = (double *)malloc(sizeof(double) * (size_t)NB * t.D * 3);
-    if (!ooff || !olist || !owners || !hFn) { rc = mb_handle_fail(MB_ERR_ARG, "out of memory"); goto out; }
+    if (!ooff || !olist || !owners || !sown || !hFn) { rc = mb_handle_fail(MB_ERR_ARG, "out of memory"); goto out; }
     {
         int nown = 0, k = 0;
         int *cur = (int *)malloc(sizeof(int) * t.Na);
@@ -588,6 +712,14 @@ extern "C" int mb_train_set_forces(mb_train *tr, int NF, const int *f_atom, cons
         for (int b = 0; b < NB; b++) olist[cur[blk_atom[b]]++] = b;
         free(cur);
         tr->Nown = nown;
+        /* the owners by species, for the gradient's chunks */
+        k = 0;
+        for (int sp = 0; sp < 3; sp++) {
+            hfoffs[sp] = k;
+            for (int q = 0; q < nown; q++)
+                if (atmn[owners[q]] == sp) sown[k++] = owners[q];
+        }
+        hfoffs[3] = k;
     }
     /* blocks on the network's input scale: Fn_b[l] DR[s_o][l] (ADJT_LNK, src/nmod.c:244-259) */
     for (int b = 0; b < NB; b++) {
@@ -609,10 +741,11 @@ extern "C" int mb_train_set_forces(mb_train *tr, int NF, const int *f_atom, cons
     TA(olist, NB); TA(Fref, 3 * NF); TA(Fn, (size_t)NB * t.D * 3); TA(Pj, (size_t)NB * t.h1 * 3);
     TA(AD1, (size_t)t.Na * t.h1); TA(fpred, 3 * NF); TA(dfq, 3 * NF); TA(lf, NF); TA(Phi, (size_t)t.Na * t.D);
     TA(Gam, (size_t)t.Na * t.h1); TA(fB1, (size_t)t.Na * t.h2); TA(fW1, (size_t)t.Na * t.h2 * t.h1);
-    TA(fW2, (size_t)t.Na * t.h2);
+    TA(fW2, (size_t)t.Na * t.h2); TA(sowners, tr->Nown);
     TC(fatom, f_atom, NF); TC(boff, blk_off, NF + 1); TC(bown, blk_atom, NB); TC(bmk, bmk, NB);
     TC(owners, owners, tr->Nown); TC(ooff, ooff, tr->Nown + 1); TC(olist, olist, NB); TC(Fref, F_ref, 3 * NF);
-    TC(Fn, hFn, (size_t)NB * t.D * 3);
+    TC(Fn, hFn, (size_t)NB * t.D * 3); TC(sowners, sown, tr->Nown);
+    if (!rc) rc = tr_chunks(tr, hfoffs);
 #undef TA
 #undef TC
     /* atoms that own no block keep zero force terms */
@@ -623,7 +756,7 @@ extern "C" int mb_train_set_forces(mb_train *tr, int NF, const int *f_atom, cons
     if (!rc) rc = tr_cuda(cudaMemset(tr->fW2, 0, sizeof(double) * (size_t)t.Na * t.h2), "memset");
     if (!rc) rc = tr_cuda(cudaMallocHost((void **)&tr->h_lf, sizeof(double) * NF), "cudaMallocHost");
 out:
-    free(sat); free(atmn); free(cnt); free(bmk); free(ooff); free(olist); free(owners); free(hFn);
+    free(sat); free(atmn); free(cnt); free(bmk); free(ooff); free(olist); free(owners); free(sown); free(hFn);
     return rc;
 }
 
@@ -654,8 +787,9 @@ static int tr_run(mb_train *tr, const double *V, double *grad) {
                                                                    tr->fW2);
             ft = {tr->AD1, tr->Phi, tr->Gam, tr->fB1, tr->fW1, tr->fW2};
         }
-        k_tr_grad<<<(tr->NW + 127) / 128, 128, 0, st>>>(t, tr->satoms, tr->soffs, tr->X, tr->H1, tr->H2, tr->d0,
-                                                        tr->d1, tr->ca, ft, tr->V, tr->grad);
+        k_tr_gpart<<<dim3(tr->nchunk, (t.D + GR_N - 1) / GR_N + 1), 256, 0, st>>>(
+            t, tr->chunks, tr->satoms, tr->sowners, tr->X, tr->H1, tr->H2, tr->d0, tr->d1, tr->ca, ft, tr->part);
+        k_tr_gsum<<<(tr->NW + 127) / 128, 128, 0, st>>>(t, tr->coff, tr->part, tr->V, tr->grad);
     }
     rc = tr_cuda(cudaGetLastError(), "training kernels");
     if (!rc) rc = tr_cuda(cudaMemcpyAsync(tr->h_ls, tr->ls, sizeof(double) * t.S, cudaMemcpyDeviceToHost, st), "D2H");
