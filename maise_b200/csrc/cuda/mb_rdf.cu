@@ -5,14 +5,17 @@
  * src/cell.c:419-430) that COMP_CL (src/eutl.c:394-413) combines and
  * RANK_TR (src/emod.c:351-368) compares against its cutoff.
  *
- *   k_rdf_ref   one CTA per structure: every (atom, image) pair within Rmax
- *               with species(j) >= species(i) spreads a Gaussian of width
- *               sigma over the bins within 3 sigma of r, tapered by
- *               cos(pi/2 (x - Rmin)/(Rmax - Rmin)) above Rmin; same-species
- *               blocks halved; optionally scaled to unit length.  The
- *               histogram lives in shared memory (FP64) and is written once.
+ *   k_rdf_ref   one CTA per structure, a warp per (i, j) pair of atoms with
+ *               its lanes over the periodic images: every image within Rmax of
+ *               a pair with species(j) >= species(i) spreads a Gaussian of
+ *               width sigma over the bins within 3 sigma of r, a bin a lane,
+ *               tapered by cos(pi/2 (x - Rmin)/(Rmax - Rmin)) above Rmin;
+ *               same-species blocks halved; optionally scaled to unit length.
+ *               The histogram lives in shared memory (FP64) and is written once.
  *   k_gram      the overlap matrix C = R R^T of the S histograms (a dense
- *               FP64 product of S x S outputs over nbins x npair terms).
+ *               FP64 product of S x S outputs over nbins x npair terms) on the
+ *               FP64 tensor cores, the terms split over enough CTAs to fill the
+ *               GPU; k_gram_sum adds the splits in order.
  */
 #include <cuda_runtime.h>
 #include <math_constants.h>
@@ -23,23 +26,30 @@
 
 namespace {
 
-constexpr int RDF_THREADS = 256;
+constexpr int RDF_THREADS = 512;
+constexpr int RDF_SHIFTS = 128; /* image shifts kept in shared memory (more are formed again per pair) */
 
-/* Cartesian displacement of j's image (i0,i1,i2) from i, in LIST's
- * operation order (src/cell.c:115-121) */
-__device__ __forceinline__ double rdf_disp2(const double *L, const double *xi, const double *xj, int i0, int i1,
-                                            int i2) {
+/* squared distance of j's image from i in LIST's operation order
+ * (src/cell.c:115-121): the image's shift is the same sum of i0 L0, i1 L1,
+ * i2 L2 for every pair and is formed once per structure */
+__device__ __forceinline__ double rdf_disp2(const double *sh, const double *dij) {
     double r = 0.0;
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+        const double x = __dadd_rn(sh[q], dij[q]);
+        r = __dadd_rn(r, __dmul_rn(x, x));
+    }
+    return r;
+}
+
+__device__ __forceinline__ void rdf_shift(const double *L, int i0, int i1, int i2, double *sh) {
 #pragma unroll
     for (int q = 0; q < 3; q++) {
         double x = 0.0;
         x = __dadd_rn(x, __dmul_rn((double)i0, L[q]));
         x = __dadd_rn(x, __dmul_rn((double)i1, L[3 + q]));
-        x = __dadd_rn(x, __dmul_rn((double)i2, L[6 + q]));
-        x = __dadd_rn(x, __dsub_rn(xj[q], xi[q]));
-        r = __dadd_rn(r, __dmul_rn(x, x));
+        sh[q] = __dadd_rn(x, __dmul_rn((double)i2, L[6 + q]));
     }
-    return r;
 }
 
 struct RdfArgs {
@@ -50,11 +60,17 @@ struct RdfArgs {
     double *out; /* [S][npair][nbins] */
 };
 
+/* Bound by the Gaussians: a pair within Rmax spreads over 25 of 3000 bins,
+ * one exponential and one shared FP64 addition each.  With a thread per
+ * (i, j, image) candidate the few accepted lanes of a warp walked their 25
+ * bins alone (and every bin its cosine); with the warp on one pair at a time,
+ * a bin a lane, 150 structures of 8 to 64 atoms take 202 us instead of
+ * 5826. */
 __global__ void __launch_bounds__(RDF_THREADS) k_rdf_ref(RdfArgs A) {
     extern __shared__ __align__(16) double hist[]; /* [npair][nbins] */
-    __shared__ double L[9], R[9], red[RDF_THREADS / 32];
+    __shared__ double L[9], R[9], red[RDF_THREADS / 32], sh[RDF_SHIFTS][3];
     __shared__ int nq[3];
-    const int s = blockIdx.x, tid = threadIdx.x;
+    const int s = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int o = A.off[s], N = A.off[s + 1] - o, ns = A.nspc, nb = A.nbins;
     const int npair = ns * (ns + 1) / 2;
     for (int k = tid; k < npair * nb; k += blockDim.x) hist[k] = 0.0;
@@ -82,27 +98,45 @@ __global__ void __launch_bounds__(RDF_THREADS) k_rdf_ref(RdfArgs A) {
     const int Do = (int)(3.0 * A.sigma / dr);
     const double DRi = 0.5 / (A.sigma * A.sigma);
     const int w0 = 2 * nq[0] + 1, w1 = 2 * nq[1] + 1, w2 = 2 * nq[2] + 1, nimg = w0 * w1 * w2;
-    const long long total = (long long)N * N * nimg;
-    for (long long c = tid; c < total; c += blockDim.x) {
-        const int im = (int)(c % nimg);
-        const long long ij = c / nimg;
-        const int j = (int)(ij % N), i = (int)(ij / N);
+    const int zero = (nq[0] * w1 + nq[1]) * w2 + nq[2]; /* the unshifted image */
+    for (int im = tid; im < nimg && im < RDF_SHIFTS; im += blockDim.x) {
+        const int t = im / w2;
+        rdf_shift(L, t / w1 - nq[0], t % w1 - nq[1], im % w2 - nq[2], sh[im]);
+    }
+    __syncthreads();
+    for (long long ij = warp; ij < (long long)N * N; ij += RDF_THREADS / 32) {
+        const int i = (int)(ij / N), j = (int)(ij - (long long)i * N);
         const int si = A.spc[o + i], sj = A.spc[o + j];
         if (sj < si) continue;
-        const int i2 = im % w2 - nq[2], t = im / w2, i1 = t % w1 - nq[1], i0 = t / w1 - nq[0];
-        if (i == j && i0 == 0 && i1 == 0 && i2 == 0) continue;
         const double *xi = A.x + 3 * (size_t)(o + i), *xj = A.x + 3 * (size_t)(o + j);
-        const double r2 = rdf_disp2(L, xi, xj, i0, i1, i2);
-        if (!(r2 < rc2)) continue;
-        const double r = sqrt(r2);
-        const int ob = (int)(r / dr);
+        const double dij[3] = {__dsub_rn(xj[0], xi[0]), __dsub_rn(xj[1], xi[1]), __dsub_rn(xj[2], xi[2])};
         const int pair = si * ns - si * (si - 1) / 2 + (sj - si); /* (si, sj), si <= sj, row-major */
         double *h = hist + (size_t)pair * nb;
-        for (int k = ob - Do; k <= ob + Do; k++) {
-            if (k < 0 || k >= nb) continue;
-            const double xk = (double)k * dr;
-            const double f = xk < A.rmin ? 1.0 : cos(0.5 * CUDART_PI * (xk - A.rmin) / (A.rmax - A.rmin));
-            atomicAdd(h + k, f * exp(-(r - xk) * (r - xk) * DRi));
+        for (int base = 0; base < nimg; base += 32) {
+            const int im = base + lane;
+            double r2 = rc2;
+            if (im < nimg && !(i == j && im == zero)) {
+                if (im < RDF_SHIFTS) {
+                    r2 = rdf_disp2(sh[im], dij);
+                } else {
+                    double t3[3];
+                    const int t = im / w2;
+                    rdf_shift(L, t / w1 - nq[0], t % w1 - nq[1], im % w2 - nq[2], t3);
+                    r2 = rdf_disp2(t3, dij);
+                }
+            }
+            const double rl = sqrt(r2);
+            for (unsigned m = __ballot_sync(0xffffffffu, r2 < rc2); m; m &= m - 1) {
+                const double r = __shfl_sync(0xffffffffu, rl, __ffs(m) - 1);
+                const int ob = (int)(r / dr);
+                for (int k = ob - Do + lane; k <= ob + Do; k += 32) {
+                    if (k < 0 || k >= nb) continue;
+                    const double xk = (double)k * dr;
+                    double f = exp(-(r - xk) * (r - xk) * DRi);
+                    if (xk >= A.rmin) f *= cos(0.5 * CUDART_PI * (xk - A.rmin) / (A.rmax - A.rmin));
+                    atomicAdd(h + k, f);
+                }
+            }
         }
     }
     __syncthreads();
@@ -127,44 +161,97 @@ __global__ void __launch_bounds__(RDF_THREADS) k_rdf_ref(RdfArgs A) {
     for (int k = tid; k < npair * nb; k += blockDim.x) out[k] = hist[k] * scale;
 }
 
-/* C[p][q] = sum_t A[p][t] A[q][t], p, q < S, t < T: 64 x 64 tiles, each
- * thread a 4 x 4 block, the operands staged through shared memory in
- * chunks of 16 terms */
-__global__ void __launch_bounds__(256) k_gram(int S, int T, const double *__restrict__ A, double *__restrict__ C) {
-    __shared__ double a[16][64 + 1], b[16][64 + 1];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const int p0 = blockIdx.y * 64, q0 = blockIdx.x * 64;
-    double acc[4][4] = {};
-    for (int t0 = 0; t0 < T; t0 += 16) {
-        for (int e = threadIdx.x; e < 16 * 64; e += 256) {
-            const int r = e / 16, k = e % 16;
-            const int p = p0 + r, q = q0 + r, t = t0 + k;
-            a[k][r] = (p < S && t < T) ? A[(size_t)p * T + t] : 0.0;
-            b[k][r] = (q < S && t < T) ? A[(size_t)q * T + t] : 0.0;
+/* Partial sums of C[p][q] = sum_t A[p][t] A[q][t] over the terms of split
+ * blockIdx.y, for the 64 x 64 tile blockIdx.x of the upper triangle of tiles
+ * (C is symmetric): 4 warps of 32 x 32, operands staged 32 terms at a time in
+ * rows of 36 (the mma operand reads, 4 rows x 4 terms a half-warp, touch 16
+ * distinct banks).  With one CTA per tile and no split, 150 histograms of
+ * 9000 terms ran on 9 SMs for 2707 us; split over 47 CTAs a tile they take
+ * 73 us with the final sum. */
+#define GRAM_T 64
+#define GRAM_K 32
+#define GRAM_LD 36
+__device__ __forceinline__ void gram_tile(int tile, int nt, int &ti, int &tj) {
+    ti = 0;
+    while (tile >= nt - ti) {
+        tile -= nt - ti;
+        ti++;
+    }
+    tj = ti + tile;
+}
+
+__global__ void __launch_bounds__(128) k_gram(int S, int T, int nt, int per, const double *__restrict__ A,
+                                              double *__restrict__ part, double *__restrict__ C) {
+    __shared__ double a[GRAM_T * GRAM_LD], b[GRAM_T * GRAM_LD];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int ti, tj;
+    gram_tile(blockIdx.x, nt, ti, tj);
+    const int p0 = ti * GRAM_T, q0 = tj * GRAM_T;
+    const int t_lo = blockIdx.y * per, t_hi = min(T, t_lo + per);
+    const int wr = (warp >> 1) * 32, wc = (warp & 1) * 32, fr = (lane >> 2) * GRAM_LD + (lane & 3);
+    double c[4][4][2] = {};
+    for (int t0 = t_lo; t0 < t_hi; t0 += GRAM_K) {
+#pragma unroll 4
+        for (int e = tid; e < GRAM_T * GRAM_K; e += 128) {
+            const int r = e / GRAM_K, k = e % GRAM_K, t = t0 + k;
+            a[r * GRAM_LD + k] = (p0 + r < S && t < t_hi) ? A[(size_t)(p0 + r) * T + t] : 0.0;
+            b[r * GRAM_LD + k] = (q0 + r < S && t < t_hi) ? A[(size_t)(q0 + r) * T + t] : 0.0;
         }
         __syncthreads();
 #pragma unroll
-        for (int k = 0; k < 16; k++) {
+        for (int k = 0; k < GRAM_K; k += 4) {
             double av[4], bv[4];
 #pragma unroll
             for (int u = 0; u < 4; u++) {
-                av[u] = a[k][ty * 4 + u];
-                bv[u] = b[k][tx * 4 + u];
+                av[u] = a[(wr + 8 * u) * GRAM_LD + fr + k];
+                bv[u] = b[(wc + 8 * u) * GRAM_LD + fr + k];
             }
 #pragma unroll
             for (int u = 0; u < 4; u++)
 #pragma unroll
-                for (int v = 0; v < 4; v++) acc[u][v] += av[u] * bv[v];
+                for (int v = 0; v < 4; v++)
+                    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+                                 : "+d"(c[u][v][0]), "+d"(c[u][v][1])
+                                 : "d"(av[u]), "d"(bv[v]));
         }
         __syncthreads();
     }
+    if (C) { /* no split: straight to both triangles */
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+#pragma unroll
+            for (int v = 0; v < 4; v++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int p = p0 + wr + 8 * u + (lane >> 2), q = q0 + wc + 8 * v + 2 * (lane & 3) + h;
+                    if (p < S && q < S) {
+                        C[(size_t)p * S + q] = c[u][v][h];
+                        if (ti != tj) C[(size_t)q * S + p] = c[u][v][h];
+                    }
+                }
+        return;
+    }
+    double *o = part + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * GRAM_T * GRAM_T;
 #pragma unroll
     for (int u = 0; u < 4; u++)
 #pragma unroll
-        for (int v = 0; v < 4; v++) {
-            const int p = p0 + ty * 4 + u, q = q0 + tx * 4 + v;
-            if (p < S && q < S) C[(size_t)p * S + q] = acc[u][v];
-        }
+        for (int v = 0; v < 4; v++)
+            *reinterpret_cast<double2 *>(o + (wr + 8 * u + (lane >> 2)) * GRAM_T + wc + 8 * v + 2 * (lane & 3)) =
+                make_double2(c[u][v][0], c[u][v][1]);
+}
+
+/* one thread per output of a tile: its splits in order, to both triangles */
+__global__ void __launch_bounds__(256) k_gram_sum(int S, int nt, int nsplit, const double *__restrict__ part,
+                                                  double *__restrict__ C) {
+    int ti, tj;
+    gram_tile(blockIdx.x, nt, ti, tj);
+    const int e = blockIdx.y * 256 + threadIdx.x, p = ti * GRAM_T + e / GRAM_T, q = tj * GRAM_T + e % GRAM_T;
+    if (p >= S || q >= S) return;
+    double acc = 0.0;
+#pragma unroll 4
+    for (int k = 0; k < nsplit; k++) acc += part[((size_t)k * gridDim.x + blockIdx.x) * GRAM_T * GRAM_T + e];
+    C[(size_t)p * S + q] = acc;
+    if (ti != tj) C[(size_t)q * S + p] = acc;
 }
 
 }  // namespace
@@ -213,7 +300,7 @@ extern "C" int mb_rdf(int device, int S, const int *nat, const int *atmn, const 
     if (!rc) rc = rdf_cuda(cudaMemcpy(d_spc, atmn, sizeof(int) * off[S], cudaMemcpyHostToDevice), "H2D");
     if (!rc) rc = rdf_cuda(cudaMemcpy(d_lat, lat, sizeof(double) * 9 * S, cudaMemcpyHostToDevice), "H2D");
     if (!rc) rc = rdf_cuda(cudaMemcpy(d_x, x, sizeof(double) * 3 * off[S], cudaMemcpyHostToDevice), "H2D");
-    if (!rc && smem > 48 * 1024)
+    if (!rc && smem + 4096 > 48 * 1024) /* (k_rdf_ref's static arrays count too) */
         rc = rdf_cuda(cudaFuncSetAttribute(k_rdf_ref, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                       "shared-memory opt-in");
     if (!rc) {
@@ -233,16 +320,31 @@ extern "C" int mb_rdf(int device, int S, const int *nat, const int *atmn, const 
 extern "C" int mb_rdf_overlap(int device, int S, int len, const double *rdf, double *cxc) {
     if (S < 1 || len < 1 || !rdf || !cxc) return mb_handle_fail(MB_ERR_ARG, "bad arguments");
     int rc = rdf_cuda(cudaSetDevice(device), "cudaSetDevice");
-    double *d_a = nullptr, *d_c = nullptr;
+    double *d_a = nullptr, *d_c = nullptr, *d_part = nullptr;
+    /* tiles of the upper triangle, and as many splits of the terms as give
+     * about two CTAs an SM without going below two stages of GRAM_K terms */
+    const int nt = (S + GRAM_T - 1) / GRAM_T;
+    const long long tiles = (long long)nt * (nt + 1) / 2;
+    int sms = 148, nsplit, per;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    nsplit = (int)((2LL * sms + tiles - 1) / tiles);
+    if (nsplit > len / (2 * GRAM_K)) nsplit = len / (2 * GRAM_K);
+    if (nsplit < 1) nsplit = 1;
+    per = ((len + nsplit - 1) / nsplit + GRAM_K - 1) / GRAM_K * GRAM_K;
+    nsplit = (len + per - 1) / per;
+    const size_t npart = (size_t)nsplit * tiles * GRAM_T * GRAM_T;
     if (!rc) rc = rdf_cuda(cudaMalloc(&d_a, sizeof(double) * (size_t)S * len), "cudaMalloc");
     if (!rc) rc = rdf_cuda(cudaMalloc(&d_c, sizeof(double) * (size_t)S * S), "cudaMalloc");
+    if (!rc && nsplit > 1) rc = rdf_cuda(cudaMalloc(&d_part, sizeof(double) * npart), "cudaMalloc");
     if (!rc) rc = rdf_cuda(cudaMemcpy(d_a, rdf, sizeof(double) * (size_t)S * len, cudaMemcpyHostToDevice), "H2D");
     if (!rc) {
-        k_gram<<<dim3((S + 63) / 64, (S + 63) / 64), 256>>>(S, len, d_a, d_c);
+        k_gram<<<dim3((unsigned)tiles, nsplit), 128>>>(S, len, nt, per, d_a, d_part, nsplit > 1 ? nullptr : d_c);
+        if (nsplit > 1) k_gram_sum<<<dim3((unsigned)tiles, GRAM_T * GRAM_T / 256), 256>>>(S, nt, nsplit, d_part, d_c);
         rc = rdf_cuda(cudaGetLastError(), "k_gram");
     }
     if (!rc) rc = rdf_cuda(cudaMemcpy(cxc, d_c, sizeof(double) * (size_t)S * S, cudaMemcpyDeviceToHost), "D2H");
     cudaFree(d_a);
     cudaFree(d_c);
+    cudaFree(d_part);
     return rc;
 }
