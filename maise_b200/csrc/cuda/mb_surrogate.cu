@@ -10,11 +10,12 @@
  * relaxes every offspring.
  *
  * Kernels:
- *   k_rdf       one CTA per structure: fractional coordinates in shared
- *               memory, every (i, j, image) within rmax deposits a tapered
- *               Gaussian into a shared histogram (FP64 distances and
+ *   k_rdf       one CTA per structure, a warp per (i, j) pair of atoms with its
+ *               lanes over the images that can lie within rmax; distances
+ *               within rmax are queued per warp and spread as tapered Gaussians
+ *               8 bins at a time into a shared histogram (FP64 distances and
  *               weights, FP32 shared atomics); writes the histogram / N.
- *   k_gemm      64x64x16 register-tiled FP32 GEMM, C = op(A) op(B), with
+ *   k_gemm      register-tiled FP32 GEMM (tiles of 64x64 or 32x32), C = op(A) op(B), with
  *               fused epilogues: bias + SiLU (keeping the pre-activation),
  *               bias only, plain store, and product with SiLU'(Z) for the
  *               backward pass.  The layers are at most 4096 x 768 x 128,
@@ -33,17 +34,44 @@
 
 /* ------------------------------------------------------------ histogram */
 
+/* Images kept per structure: those whose shift can bring a minimum-image
+ * displacement (at most the cell's half diagonal long) within rmax.  The
+ * (2 n + 1)^3 images of the plane spacings hold 5 to 10 times as many. */
+#define RDF_IMGS 512
+#define RDF_QUEUE 64 /* distances a warp holds before spreading them */
+
+/* Spread the queued distances: 8 lanes an entry, 4 entries a step. */
+__device__ __forceinline__ void rdf_spread(const double *qr, const int *qp, int n, int lane, int nbins, int Do,
+                                           double dr, double DR, const double *taper, float *hist) {
+    for (int e = lane >> 3; e < n; e += 4) {
+        const double r = qr[e];
+        const int o = (int)(r / dr);
+        float *h = hist + qp[e] * nbins;
+        for (int k = o - Do + (lane & 7); k <= o + Do; k += 8) {
+            if (k < 0 || k >= nbins) continue;
+            const double xk = k * dr;
+            atomicAdd(h + k, (float)(taper[k] * exp(-(r - xk) * (r - xk) * DR)));
+        }
+    }
+}
+
+/* Bound by the candidate distances and the Gaussians (7 bins a pair at the
+ * default width).  A thread per (i, j) pair walking all images alone, a cosine
+ * and an exponential per bin, took 3689 us for 2048 structures of 16 to 48
+ * atoms; with the images pruned once per structure and the bins spread over
+ * lanes it takes 500 us. */
 __global__ void __launch_bounds__(256) k_rdf(int S, const int *__restrict__ off, const int *__restrict__ spc,
                                             const double *__restrict__ lat, const double *__restrict__ x, int nspc,
                                             int nbins, double rmax, double sigma, float *__restrict__ feat,
                                             int *__restrict__ status) {
-    extern __shared__ float hist[];
-    __shared__ double L[9], Li[9];
-    __shared__ double fr[3 * SUR_MAX_ATOMS];
-    __shared__ int sp[SUR_MAX_ATOMS];
-    __shared__ int nimg[3];
+    extern __shared__ __align__(16) double taper[]; /* [nbins], then the histogram */
+    float *hist = reinterpret_cast<float *>(taper + nbins);
+    __shared__ double L[9], Li[9], half2;
+    __shared__ double fr[3 * SUR_MAX_ATOMS], sh[3 * RDF_IMGS], qr[8][RDF_QUEUE];
+    __shared__ int sp[SUR_MAX_ATOMS], qp[8][RDF_QUEUE];
+    __shared__ int nimg[3], nsh;
     __shared__ int bad;
-    const int s = blockIdx.x, tid = threadIdx.x, bd = blockDim.x;
+    const int s = blockIdx.x, tid = threadIdx.x, bd = blockDim.x, lane = tid & 31, warp = tid >> 5;
     if (s >= S) return;
     const int a0 = off[s], N = off[s + 1] - a0;
     const int P = nspc * (nspc + 1) / 2;
@@ -76,6 +104,17 @@ __global__ void __launch_bounds__(256) k_rdf(int S, const int *__restrict__ off,
             if (!(n <= SUR_MAX_IMG)) bad = 1;
             nimg[a] = bad ? 0 : (int)n;
         }
+        /* the longest half diagonal bounds a minimum-image displacement */
+        half2 = 0.0;
+        for (int q = 0; q < 4; q++) {
+            double d2 = 0.0;
+            for (int c = 0; c < 3; c++) {
+                const double v = 0.5 * (L[c] + ((q & 1) ? -L[3 + c] : L[3 + c]) + ((q & 2) ? -L[6 + c] : L[6 + c]));
+                d2 += v * v;
+            }
+            half2 = fmax(half2, d2);
+        }
+        nsh = 0;
     }
     __syncthreads();
     if (bad) {
@@ -88,13 +127,30 @@ __global__ void __launch_bounds__(256) k_rdf(int S, const int *__restrict__ off,
         for (int c = 0; c < 3; c++) fr[3 * i + c] = xi[0] * Li[c] + xi[1] * Li[3 + c] + xi[2] * Li[6 + c];
         sp[i] = spc[a0 + i];
     }
+    for (int k = tid; k < nbins; k += bd) taper[k] = cos(0.5 * M_PI * (k * (rmax / nbins)) / rmax);
+    const int n0 = nimg[0], n1 = nimg[1], n2 = nimg[2], w1 = 2 * n1 + 1, w2 = 2 * n2 + 1;
+    const double reach = (rmax + sqrt(half2)) * (1.0 + 1e-9), rc2 = rmax * rmax;
+    for (int im = tid; im < (2 * n0 + 1) * w1 * w2; im += bd) {
+        const double ta = im / (w1 * w2) - n0, tb = (im / w2) % w1 - n1, tc = im % w2 - n2;
+        const double vx = ta * L[0] + tb * L[3] + tc * L[6], vy = ta * L[1] + tb * L[4] + tc * L[7],
+                     vz = ta * L[2] + tb * L[5] + tc * L[8];
+        if (vx * vx + vy * vy + vz * vz <= reach * reach) {
+            const int e = atomicAdd(&nsh, 1);
+            if (e < RDF_IMGS) {
+                sh[3 * e] = ta;
+                sh[3 * e + 1] = tb;
+                sh[3 * e + 2] = tc;
+            }
+        }
+    }
     __syncthreads();
+    /* (a cell so skewed that the list overflows walks every image) */
+    const int every = nsh > RDF_IMGS, count = every ? (2 * n0 + 1) * w1 * w2 : nsh;
     const double dr = rmax / nbins;
     const int Do = (int)(3.0 * sigma / dr);
     const double DR = 0.5 / (sigma * sigma);
-    const double rc2 = rmax * rmax;
-    const int n0 = nimg[0], n1 = nimg[1], n2 = nimg[2];
-    for (int w = tid; w < N * N; w += bd) {
+    int nq = 0;
+    for (int w = warp; w < N * N; w += 8) {
         const int i = w / N, j = w - i * N;
         const int si = sp[i], sj = sp[j];
         if (sj < si) continue;
@@ -104,25 +160,36 @@ __global__ void __launch_bounds__(256) k_rdf(int S, const int *__restrict__ off,
             const double t = fr[3 * j + c] - fr[3 * i + c];
             d[c] = t - rint(t);
         }
-        for (int ta = -n0; ta <= n0; ta++)
-            for (int tb = -n1; tb <= n1; tb++)
-                for (int tc = -n2; tc <= n2; tc++) {
-                    const double u0 = d[0] + ta, u1 = d[1] + tb, u2 = d[2] + tc;
-                    const double vx = u0 * L[0] + u1 * L[3] + u2 * L[6];
-                    const double vy = u0 * L[1] + u1 * L[4] + u2 * L[7];
-                    const double vz = u0 * L[2] + u1 * L[5] + u2 * L[8];
-                    const double r2 = vx * vx + vy * vy + vz * vz;
-                    if (!(r2 < rc2) || r2 == 0.0) continue;
-                    const double r = sqrt(r2);
-                    const int o = (int)(r / dr);
-                    for (int k = o - Do; k <= o + Do; k++) {
-                        if (k < 0 || k >= nbins) continue;
-                        const double xk = k * dr;
-                        const double f = cos(0.5 * M_PI * xk / rmax) * exp(-(r - xk) * (r - xk) * DR);
-                        atomicAdd(&hist[p * nbins + k], (float)f);
-                    }
-                }
+        for (int base = 0; base < count; base += 32) {
+            const int im = base + lane;
+            double r2 = rc2;
+            if (im < count) {
+                const double u0 = d[0] + (every ? (double)(im / (w1 * w2) - n0) : sh[3 * im]);
+                const double u1 = d[1] + (every ? (double)((im / w2) % w1 - n1) : sh[3 * im + 1]);
+                const double u2 = d[2] + (every ? (double)(im % w2 - n2) : sh[3 * im + 2]);
+                const double vx = u0 * L[0] + u1 * L[3] + u2 * L[6];
+                const double vy = u0 * L[1] + u1 * L[4] + u2 * L[7];
+                const double vz = u0 * L[2] + u1 * L[5] + u2 * L[8];
+                r2 = vx * vx + vy * vy + vz * vz;
+            }
+            const bool in = r2 < rc2 && r2 != 0.0;
+            const unsigned m = __ballot_sync(0xffffffffu, in);
+            if (in) {
+                const int e = nq + __popc(m & ((1u << lane) - 1u));
+                qr[warp][e] = sqrt(r2);
+                qp[warp][e] = p;
+            }
+            nq += __popc(m);
+            if (nq > RDF_QUEUE - 32) {
+                __syncwarp();
+                rdf_spread(qr[warp], qp[warp], nq, lane, nbins, Do, dr, DR, taper, hist);
+                __syncwarp();
+                nq = 0;
+            }
+        }
     }
+    __syncwarp();
+    rdf_spread(qr[warp], qp[warp], nq, lane, nbins, Do, dr, DR, taper, hist);
     __syncthreads();
     const float invN = 1.0f / (float)N;
     for (int k = tid; k < P * nbins; k += bd) {
@@ -135,8 +202,6 @@ __global__ void __launch_bounds__(256) k_rdf(int S, const int *__restrict__ off,
 
 /* ----------------------------------------------------------------- GEMM */
 
-#define GB_M 64
-#define GB_N 64
 #define GB_K 16
 
 __device__ __forceinline__ float silu_f(float z) { return z / (1.0f + expf(-z)); }
@@ -148,75 +213,70 @@ __device__ __forceinline__ float dsilu_f(float z) {
 /* C[m, n] = sum_k A(m, k) B(k, n), A(m, k) = TA ? A[k lda + m] : A[m lda + k],
  * B(k, n) = TB ? B[n ldb + k] : B[k ldb + n]; row-major C with leading
  * dimension ldc; EP selects the epilogue (SUR_EP_*). */
-template <bool TA, bool TB, int EP>
+/* Tiles of GB x GB outputs, 256 threads of R x R each (R = GB / 16); the next
+ * GB_K terms are loaded into registers while the current ones are multiplied.
+ * GB is 64 where such tiles give at least one CTA an SM, 32 below: the first
+ * layer of 2048 rows (128 outputs, 768 terms) is 64 tiles of 64, each a chain
+ * of 48 load-multiply stages (86 us), and 256 tiles of 32 (35 us).  Every output
+ * sums its terms in ascending order in either. */
+template <bool TA, bool TB, int EP, int GB>
 __global__ void __launch_bounds__(256) k_gemm(int M, int N, int K, const float *__restrict__ A, int lda,
                                              const float *__restrict__ B, int ldb, float *__restrict__ C, int ldc,
                                              const float *__restrict__ bias, float *__restrict__ Z,
                                              const float *__restrict__ Zp) {
-    __shared__ float As[GB_K][GB_M + 4];
-    __shared__ float Bs[GB_K][GB_N + 4];
+    constexpr int R = GB / 16, LOADS = GB * GB_K / 256;
+    __shared__ __align__(16) float As[GB_K][GB + 4];
+    __shared__ __align__(16) float Bs[GB_K][GB + 4];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int m0 = blockIdx.y * GB_M, n0 = blockIdx.x * GB_N;
-    float acc[4][4];
+    const int m0 = blockIdx.y * GB, n0 = blockIdx.x * GB;
+    float acc[R][R];
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < R; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = 0.0f;
+        for (int j = 0; j < R; j++) acc[i][j] = 0.0f;
+    float ra[LOADS], rb[LOADS];
+    auto load = [&](int k0) {
+#pragma unroll
+        for (int r = 0; r < LOADS; r++) {
+            const int e = tid + 256 * r;
+            const int m = TA ? e % GB : e / GB_K, ka = TA ? e / GB : e % GB_K;
+            const int n = TB ? e / GB_K : e % GB, kb = TB ? e % GB_K : e / GB;
+            const int gm = m0 + m, gn = n0 + n;
+            ra[r] = gm < M && k0 + ka < K ? (TA ? A[(size_t)(k0 + ka) * lda + gm] : A[(size_t)gm * lda + k0 + ka]) : 0.0f;
+            rb[r] = gn < N && k0 + kb < K ? (TB ? B[(size_t)gn * ldb + k0 + kb] : B[(size_t)(k0 + kb) * ldb + gn]) : 0.0f;
+        }
+    };
+    load(0);
     for (int k0 = 0; k0 < K; k0 += GB_K) {
 #pragma unroll
-        for (int r = 0; r < 4; r++) {
+        for (int r = 0; r < LOADS; r++) {
             const int e = tid + 256 * r;
-            int m, k;
-            if (TA) {
-                m = e % GB_M;
-                k = e / GB_M;
-            } else {
-                k = e % GB_K;
-                m = e / GB_K;
-            }
-            const int gm = m0 + m, gk = k0 + k;
-            float v = 0.0f;
-            if (gm < M && gk < K) v = TA ? A[(size_t)gk * lda + gm] : A[(size_t)gm * lda + gk];
-            As[k][m] = v;
-        }
-#pragma unroll
-        for (int r = 0; r < 4; r++) {
-            const int e = tid + 256 * r;
-            int n, k;
-            if (TB) {
-                k = e % GB_K;
-                n = e / GB_K;
-            } else {
-                n = e % GB_N;
-                k = e / GB_N;
-            }
-            const int gn = n0 + n, gk = k0 + k;
-            float v = 0.0f;
-            if (gn < N && gk < K) v = TB ? B[(size_t)gn * ldb + gk] : B[(size_t)gk * ldb + gn];
-            Bs[k][n] = v;
+            As[TA ? e / GB : e % GB_K][TA ? e % GB : e / GB_K] = ra[r];
+            Bs[TB ? e % GB_K : e / GB][TB ? e / GB_K : e % GB] = rb[r];
         }
         __syncthreads();
+        if (k0 + GB_K < K) load(k0 + GB_K);
 #pragma unroll
         for (int kk = 0; kk < GB_K; kk++) {
-            float a[4], b[4];
+            float a[R], b[R];
 #pragma unroll
-            for (int i = 0; i < 4; i++) a[i] = As[kk][ty * 4 + i];
+            for (int i = 0; i < R; i++) a[i] = As[kk][ty * R + i];
 #pragma unroll
-            for (int j = 0; j < 4; j++) b[j] = Bs[kk][tx * 4 + j];
+            for (int j = 0; j < R; j++) b[j] = Bs[kk][tx * R + j];
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < R; i++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                for (int j = 0; j < R; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
         }
         __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int gm = m0 + ty * 4 + i;
+    for (int i = 0; i < R; i++) {
+        const int gm = m0 + ty * R + i;
         if (gm >= M) continue;
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int gn = n0 + tx * 4 + j;
+        for (int j = 0; j < R; j++) {
+            const int gn = n0 + tx * R + j;
             if (gn >= N) continue;
             const size_t o = (size_t)gm * ldc + gn;
             float v = acc[i][j];
@@ -237,9 +297,17 @@ __global__ void __launch_bounds__(256) k_gemm(int M, int N, int K, const float *
 
 extern "C" int surk_gemm(int ta, int tb, int ep, int M, int N, int K, const float *A, int lda, const float *B, int ldb,
                          float *C, int ldc, const float *bias, float *Z, const float *Zp, void *stream) {
-    dim3 grid((N + GB_N - 1) / GB_N, (M + GB_M - 1) / GB_M);
+    const bool small = (long)((N + 63) / 64) * ((M + 63) / 64) < 148;
+    const int gb = small ? 32 : 64;
+    dim3 grid((N + gb - 1) / gb, (M + gb - 1) / gb);
     cudaStream_t st = (cudaStream_t)stream;
-#define SUR_GEMM(TA_, TB_, EP_) k_gemm<TA_, TB_, EP_><<<grid, 256, 0, st>>>(M, N, K, A, lda, B, ldb, C, ldc, bias, Z, Zp)
+#define SUR_GEMM(TA_, TB_, EP_)                                                                             \
+    do {                                                                                                    \
+        if (small)                                                                                          \
+            k_gemm<TA_, TB_, EP_, 32><<<grid, 256, 0, st>>>(M, N, K, A, lda, B, ldb, C, ldc, bias, Z, Zp);  \
+        else                                                                                                \
+            k_gemm<TA_, TB_, EP_, 64><<<grid, 256, 0, st>>>(M, N, K, A, lda, B, ldb, C, ldc, bias, Z, Zp);  \
+    } while (0)
     if (!ta && tb && ep == SUR_EP_BIAS_SILU) SUR_GEMM(false, true, SUR_EP_BIAS_SILU);
     else if (!ta && tb && ep == SUR_EP_BIAS) SUR_GEMM(false, true, SUR_EP_BIAS);
     else if (!ta && !tb && ep == SUR_EP_DSILU) SUR_GEMM(false, false, SUR_EP_DSILU);
@@ -322,8 +390,12 @@ __global__ void k_colstats(int S, int F, const float *__restrict__ X, float *__r
 extern "C" int surk_rdf(int S, const int *off, const int *spc, const double *lat, const double *x, int nspc, int nbins,
                         double rmax, double sigma, float *feat, int *status, void *stream) {
     const int P = nspc * (nspc + 1) / 2;
-    const size_t smem = sizeof(float) * P * nbins;
-    if (nspc < 1 || nspc > SUR_MAX_SPC || nbins < 1 || smem > 48 * 1024) return (int)cudaErrorInvalidValue;
+    const size_t hist = sizeof(float) * P * nbins, smem = hist + sizeof(double) * nbins;
+    if (nspc < 1 || nspc > SUR_MAX_SPC || nbins < 1 || hist > 48 * 1024) return (int)cudaErrorInvalidValue;
+    if (smem > 16 * 1024) { /* with the static arrays (26 KB) past the default limit */
+        const cudaError_t e = cudaFuncSetAttribute(k_rdf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+    }
     k_rdf<<<S, 256, smem, (cudaStream_t)stream>>>(S, off, spc, lat, x, nspc, nbins, rmax, sigma, feat, status);
     return (int)cudaGetLastError();
 }
