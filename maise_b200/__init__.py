@@ -109,6 +109,27 @@ def _i32(a):
     return np.ascontiguousarray(np.asarray(a, dtype=np.int32).reshape(-1))
 
 
+def pack(structures):
+    """(nat[S], atmn, LAT[S,3,3], X) of a list of dict(X, LAT, atmn): atom
+    counts, species and Cartesian positions end to end, lattices stacked.
+    Arrays of the usual shapes are concatenated as they are, anything else
+    is converted structure by structure."""
+    at, xs, ls = ([s[k] for s in structures] for k in ("atmn", "X", "LAT"))
+    nat = np.fromiter(map(len, at), np.int32, len(at))
+    if all(type(x) is np.ndarray and x.ndim == 2 and x.shape[1] == 3 for x in xs) and all(
+            type(v) is np.ndarray and v.shape == (3, 3) for v in ls):
+        X, LAT = np.concatenate(xs), np.concatenate(ls).reshape(-1, 3, 3)
+    else:
+        X = np.concatenate([np.asarray(x, float).reshape(-1, 3) for x in xs])
+        LAT = np.stack([np.asarray(v, float).reshape(3, 3) for v in ls])
+    if all(type(a) is np.ndarray and a.ndim == 1 for a in at):
+        atmn = np.concatenate(at).astype(np.int32, copy=False)
+    else:
+        atmn = np.concatenate([np.asarray(a, np.int32) for a in at])
+    return (nat, np.ascontiguousarray(atmn), np.ascontiguousarray(LAT, dtype=np.float64),
+            np.ascontiguousarray(X, dtype=np.float64))
+
+
 def maxwell(amu, T, seed=1):
     """Maxwell velocities (A/fs) drawn as src/cmod.c:224-280 does; no GPU needed."""
     lib = load_library()
@@ -364,10 +385,7 @@ class Potential:
     def relax_batch(self, structures, p_gpa=0.0, urep=0.0, rlxt=3, mitr=500, fmax=0.01):
         """Relax a list of dict(X, LAT, atmn) in one persistent launch.
         Returns dict(H[S], X list, LAT[S,3,3], iters[S], status[S], evals, ms)."""
-        nat = np.array([len(s["atmn"]) for s in structures], np.int32)
-        atmn = np.ascontiguousarray(np.concatenate([np.asarray(s["atmn"], np.int32) for s in structures]))
-        X = np.ascontiguousarray(np.concatenate([np.asarray(s["X"], float).reshape(-1, 3) for s in structures]))
-        LAT = np.ascontiguousarray(np.stack([np.asarray(s["LAT"], float).reshape(3, 3) for s in structures]))
+        nat, atmn, LAT, X = pack(structures)
         S = len(structures)
         H = np.zeros(S)
         iters = np.zeros(S, np.int32)
@@ -387,10 +405,7 @@ class Potential:
     def efs_batch(self, structures, p_gpa=0.0, urep=0.0):
         """FP32 batched E/F/S of a list of dict(X, LAT, atmn), no relaxation.
         Returns dict(H[S], F list of [N,3], U[S,6])."""
-        nat = np.array([len(s["atmn"]) for s in structures], np.int32)
-        atmn = np.ascontiguousarray(np.concatenate([np.asarray(s["atmn"], np.int32) for s in structures]))
-        X = np.ascontiguousarray(np.concatenate([np.asarray(s["X"], float).reshape(-1, 3) for s in structures]))
-        LAT = np.ascontiguousarray(np.stack([np.asarray(s["LAT"], float).reshape(3, 3) for s in structures]))
+        nat, atmn, LAT, X = pack(structures)
         S = len(structures)
         H = np.zeros(S)
         F = np.zeros_like(X)

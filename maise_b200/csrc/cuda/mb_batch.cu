@@ -25,6 +25,7 @@
 
 #include "../../../include/maise_b200.h"
 #include "../mb_internal.h"
+#include "../host/mb_batch.h"
 
 #define FULLM 0xffffffffu
 
@@ -1102,7 +1103,7 @@ __global__ void __launch_bounds__(W * 32) k_relax_batch(BArgs A) {
             q[0] = sh.L[0]; q[1] = sh.L[4]; q[2] = sh.L[8]; q[3] = sh.L[1]; q[4] = sh.L[5];
             q[5] = sh.L[6]; q[6] = sh.L[3]; q[7] = sh.L[7]; q[8] = sh.L[2];
         }
-        for (int k = tid; k < n * n; k += blockDim.x) H[k] = (k / n == k % n) ? 1.0 : 0.0;
+        int ident = 1; /* H is the identity and not written out */
         __syncthreads();
         double f = evaluate<W, C>(A, sh, sh.x, sh.g), fprev = f;
         double maxf = sh.scal[1], maxu = sh.scal[2];
@@ -1116,7 +1117,9 @@ __global__ void __launch_bounds__(W * 32) k_relax_batch(BArgs A) {
              * elements */
             for (int r = tid; r < n; r += blockDim.x) {
                 double t = 0.0;
-                for (int c = 0; c < n; c++) t += H[c * n + r] * sh.g[c];
+                if (ident) t = sh.g[r];
+                else
+                    for (int c = 0; c < n; c++) t += H[c * n + r] * sh.g[c];
                 sh.p[r] = -t;
             }
             __syncthreads();
@@ -1124,7 +1127,7 @@ __global__ void __launch_bounds__(W * 32) k_relax_batch(BArgs A) {
             for (int k = tid; k < n; k += blockDim.x) { dphi0 += sh.g[k] * sh.p[k]; }
             dphi0 = cta_sum(sh, dphi0);
             if (!(dphi0 < 0.0)) {
-                for (int k = tid; k < n * n; k += blockDim.x) H[k] = (k / n == k % n) ? 1.0 : 0.0;
+                ident = 1;
                 for (int k = tid; k < n; k += blockDim.x) sh.p[k] = -sh.g[k];
                 __syncthreads();
                 first = 1;
@@ -1221,7 +1224,7 @@ __global__ void __launch_bounds__(W * 32) k_relax_batch(BArgs A) {
                 } else if (!first) {
                     /* no acceptable step along the quasi-Newton direction:
                      * restart once from steepest descent before giving up */
-                    for (int k = tid; k < n * n; k += blockDim.x) H[k] = (k / n == k % n) ? 1.0 : 0.0;
+                    ident = 1;
                     first = 1;
                     __syncthreads();
                     continue;
@@ -1241,13 +1244,15 @@ __global__ void __launch_bounds__(W * 32) k_relax_batch(BArgs A) {
             sy = cta_sum(sh, sy);
             yy = cta_sum(sh, yy);
             if (sy > 0.0) {
-                if (first)
-                    for (int k = tid; k < n * n; k += blockDim.x) H[k] = (k / n == k % n) ? sy / yy : 0.0;
-                __syncthreads();
+                /* before an update H is a multiple of the identity (6.20 at the
+                 * first): its elements are written by the update, not before */
+                const double diag = first ? sy / yy : 1.0;
                 /* Hy into g (g is replaced below) */
                 for (int r = tid; r < n; r += blockDim.x) {
                     double t = 0.0;
-                    for (int c = 0; c < n; c++) t += H[c * n + r] * sh.hy[c];
+                    if (ident) t = diag * sh.hy[r];
+                    else
+                        for (int c = 0; c < n; c++) t += H[c * n + r] * sh.hy[c];
                     sh.g[r] = t;
                 }
                 __syncthreads();
@@ -1263,8 +1268,10 @@ __global__ void __launch_bounds__(W * 32) k_relax_batch(BArgs A) {
                     int r = k / n, c = k % n;
                     const double pp = __dmul_rn(sh.p[r], sh.p[c]);
                     const double gp = __dadd_rn(__dmul_rn(sh.g[r], sh.p[c]), __dmul_rn(sh.p[r], sh.g[c]));
-                    H[k] += c1 * pp - gp / sy;
+                    const double old = !ident ? H[k] : r == c ? diag : 0.0;
+                    H[k] = old + (c1 * pp - gp / sy);
                 }
+                ident = 0;
             }
             __syncthreads();
             vcopy(sh.x, sh.xt, n);
@@ -1314,7 +1321,7 @@ __global__ void __launch_bounds__(W * 32) k_relax_batch(BArgs A) {
 
 /* ---------------- host launcher ---------------- */
 
-static int build_bparams(const mb_model *m, BParams *B, float **w_out, size_t *wlen) {
+static int build_bparams(const mb_model *m, BParams *B, float *w) {
     const mb_params &P = m->P;
     memset(B, 0, sizeof(*B));
     if (P.ne > BNE || P.nz > BNZ || P.nlam > BNLAM || P.D > BMAXD || P.ng2 > 16) return -1;
@@ -1353,10 +1360,7 @@ static int build_bparams(const mb_model *m, BParams *B, float **w_out, size_t *w
         B->w_off[s] = P.w_off[s];
     }
     B->rc = m->rc_list;
-    *wlen = m->weights_len;
-    float *w = (float *)malloc(sizeof(float) * m->weights_len);
     for (size_t k = 0; k < m->weights_len; k++) w[k] = (float)m->weights[k];
-    *w_out = w;
     return 0;
 }
 
@@ -1421,26 +1425,77 @@ static double batch_sigma() {
     return 0.5;
 }
 
-extern "C" int mbk_relax_batch(const mb_model *m, int S, const int *d_nat, const int *d_off, const int *d_spc,
-                               const int *d_order, double *d_lat, double *d_x, double p_ev, double urep, int rlxt, int mitr, double fmax,
-                               double *d_H, int *d_iters, int *d_status, double *d_frc, double *d_str,
-                               void *stream, long long *evals_out, float *ms_out) {
-    /* evals_out[4]: evaluations, atom evaluations, pairs, triplets */
+/* CTAs (SMs) per structure.  A launch lasts as long as its total work on all
+ * units or as its longest BFGS chain on one, whichever is more; an evaluation
+ * on a cluster of 2 or 4 CTAs takes 0.62 or 0.44 of one CTA's time (536, 330 and
+ * 235 us for 64 atoms).  Structures stop after about 200 iterations on
+ * average, the longest run to mitr.  256 Mg-Ca structures, one CTA, pairs and
+ * clusters of 4: 6 iterations 6.4, 6.5 and 9.4 ms; 100 iterations 110, 131
+ * and 188 ms; 1000 iterations 1.60, 0.93 and 0.88 s.  40 structures, 6
+ * iterations: 4.6, 2.8 and 2.0 ms. */
+static int batch_clusters(int S, int mitr, int sms) {
+    const double t[3] = {1.0, 0.62, 0.44};
+    const double it = mitr + 1.0, mean = it < 200.0 ? it : 200.0;
+    int best = 1;
+    double tb = 0.0;
+    for (int k = 0; k < 3; k++) {
+        const int c = 1 << k, units = sms / c;
+        const double work = 0.7 * t[k] * mean * S / units; /* the mean structure costs 0.7 of the largest */
+        const double chain = t[k] * it;
+        const double d = work > chain ? work : chain;
+        if (k == 0 || d < tb) {
+            tb = d;
+            best = c;
+        }
+    }
+    return best;
+}
+
+/* The model's FP32 parameters and weights on the device, uploaded on a
+ * handle's first batched call. */
+static cudaError_t batch_model(const mb_model *m, mb_batch_ws *ws, cudaStream_t st) {
+    if (ws->model) return cudaSuccess;
+    const size_t wb = sizeof(float) * m->weights_len, bytes = sizeof(BParams) + wb;
+    char *h = (char *)malloc(bytes);
+    if (!h) return cudaErrorMemoryAllocation;
+    cudaError_t e = build_bparams(m, (BParams *)h, (float *)(h + sizeof(BParams))) ? cudaErrorInvalidValue : cudaSuccess;
+    void *d = nullptr;
+    if (!e) e = cudaMalloc(&d, bytes);
+    if (!e) e = cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, st);
+    if (!e) e = cudaStreamSynchronize(st);
+    free(h);
+    if (e) {
+        cudaFree(d);
+        return e;
+    }
+    ws->model = d;
+    return cudaSuccess;
+}
+
+extern "C" void mbk_batch_free(mb_batch_ws *ws) {
+    cudaFree(ws->model);
+    mb_ws_free(&ws->io);
+    mb_ws_free(&ws->scratch);
+    if (ws->e0) cudaEventDestroy((cudaEvent_t)ws->e0);
+    if (ws->e1) cudaEventDestroy((cudaEvent_t)ws->e1);
+    memset(ws, 0, sizeof(*ws));
+}
+
+/* d_evals[4] (zeroed by the caller): evaluations, atom evaluations, pairs, triplets */
+extern "C" int mbk_relax_batch(const mb_model *m, mb_batch_ws *ws, int S, const int *d_nat, const int *d_off,
+                               const int *d_spc, const int *d_order, double *d_lat, double *d_x, double p_ev,
+                               double urep, int rlxt, int mitr, double fmax, double *d_H, int *d_iters, int *d_status,
+                               double *d_frc, double *d_str, long long *d_evals, void *stream) {
     cudaStream_t st = (cudaStream_t)stream;
-    BParams hp;
-    float *hw = nullptr;
-    size_t wlen = 0;
-    if (build_bparams(m, &hp, &hw, &wlen)) return (int)cudaErrorInvalidValue;
     int dev = 0, sms = 0, units = 0;
+    cudaError_t e = batch_model(m, ws, st);
+    if (e != cudaSuccess) return (int)e;
+    if (!ws->e0) e = cudaEventCreate((cudaEvent_t *)&ws->e0);
+    if (!e && !ws->e1) e = cudaEventCreate((cudaEvent_t *)&ws->e1);
+    if (e != cudaSuccess) return (int)e;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    /* A population that fits the SMs in about two rounds is bound by its
-     * slowest BFGS chains: clusters of 4 CTAs (4 SMs) evaluate each structure,
-     * cutting a chain's latency about threefold (256 Mg-Ca structures: 0.88 s
-     * against 1.60 s).  Larger populations keep one CTA per structure, which
-     * has the higher throughput (4096 Cu-Pd-Ag offspring: 2.10 s against
-     * 2.48 s with pairs). */
-    int wide = 1, csize = S <= 2 * sms ? 4 : 1;
+    int wide = 1, csize = batch_clusters(S, mitr, sms);
     {
         /* MAISE_B200_BATCH_WARPS=4 selects the narrow CTA and
          * MAISE_B200_BATCH_CLUSTER=1|2|4 the CTAs per structure (A/B timing) */
@@ -1449,10 +1504,10 @@ extern "C" int mbk_relax_batch(const mb_model *m, int S, const int *d_nat, const
         if (fc) csize = atoi(fc) == 4 ? 4 : atoi(fc) == 2 ? 2 : 1;
         if (!wide) csize = 1;
     }
-    cudaError_t e = !wide        ? batch_config<4, 1>(sms, &units)
-                    : csize == 4 ? batch_config<BWARPS_WIDE, 4>(sms, &units)
-                    : csize == 2 ? batch_config<BWARPS_WIDE, 2>(sms, &units)
-                                 : batch_config<BWARPS_WIDE, 1>(sms, &units);
+    e = !wide        ? batch_config<4, 1>(sms, &units)
+        : csize == 4 ? batch_config<BWARPS_WIDE, 4>(sms, &units)
+        : csize == 2 ? batch_config<BWARPS_WIDE, 2>(sms, &units)
+                     : batch_config<BWARPS_WIDE, 1>(sms, &units);
     if (csize > 1 && (e != cudaSuccess || units < 1)) {
         /* clusters of this size cannot be placed (e.g. on a partitioned
          * GPU): one CTA per structure */
@@ -1460,53 +1515,38 @@ extern "C" int mbk_relax_batch(const mb_model *m, int S, const int *d_nat, const
         csize = 1;
         e = batch_config<BWARPS_WIDE, 1>(sms, &units);
     }
-    if (e != cudaSuccess) { free(hw); return (int)e; }
-    if (units < 1) { free(hw); return (int)cudaErrorInvalidConfiguration; }
+    if (e != cudaSuccess) return (int)e;
+    if (units < 1) return (int)cudaErrorInvalidConfiguration;
     const int gunits = units < S ? units : S; /* CTAs, or clusters of csize CTAs */
     const int grid = gunits * csize;
-    BParams *dp = nullptr;
-    float *dw = nullptr;
-    double *hm = nullptr;
-    float4 *nbd = nullptr;
-    int *nbj = nullptr, *queue = nullptr;
-    long long *evals = nullptr;
-    cudaEvent_t e0, e1;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
-    e = cudaMalloc(&dp, sizeof(BParams));
-    if (!e) e = cudaMalloc(&dw, sizeof(float) * wlen);
-    if (!e) e = cudaMalloc(&hm, sizeof(double) * (size_t)grid * BMAXDOF * BMAXDOF);
-    if (!e) e = cudaMalloc(&nbd, sizeof(float4) * (size_t)grid * BMAXN * BMAXNB);
-    if (!e) e = cudaMalloc(&nbj, sizeof(int) * (size_t)grid * BMAXN * BMAXNB);
-    if (!e) e = cudaMalloc(&queue, sizeof(int));
-    if (!e) e = cudaMalloc(&evals, 4 * sizeof(long long));
-    if (!e) e = cudaMemcpyAsync(dp, &hp, sizeof(BParams), cudaMemcpyHostToDevice, st);
-    if (!e) e = cudaMemcpyAsync(dw, hw, sizeof(float) * wlen, cudaMemcpyHostToDevice, st);
-    if (!e) e = cudaMemsetAsync(queue, 0, sizeof(int), st);
-    if (!e) e = cudaMemsetAsync(evals, 0, 4 * sizeof(long long), st);
-    if (!e) {
-        BArgs a;
-        a.S = S; a.rlxt = rlxt; a.mitr = mitr;
-        a.p_ev = p_ev; a.urep = urep; a.fmax = fmax; a.sigma = batch_sigma();
-        a.nat = d_nat; a.off = d_off; a.spc = d_spc; a.order = d_order;
-        a.lat = d_lat; a.x = d_x; a.H = d_H; a.iters = d_iters; a.status = d_status;
-        a.fout = d_frc; a.uout = d_str;
-        a.P = dp; a.W = dw; a.queue = queue; a.hmat = hm; a.nbd = nbd; a.nbj = nbj; a.evals = evals;
-        a.work = (unsigned long long *)(evals + 1);
-        cudaEventRecord(e0, st);
-        e = !wide        ? batch_launch<4, 1>(gunits, st, a)
-            : csize == 4 ? batch_launch<BWARPS_WIDE, 4>(gunits, st, a)
-            : csize == 2 ? batch_launch<BWARPS_WIDE, 2>(gunits, st, a)
-                         : batch_launch<BWARPS_WIDE, 1>(gunits, st, a);
-        cudaEventRecord(e1, st);
-        if (!e) e = cudaGetLastError();
-    }
-    if (!e) e = cudaStreamSynchronize(st);
-    if (!e && evals_out) e = cudaMemcpy(evals_out, evals, 4 * sizeof(long long), cudaMemcpyDeviceToHost);
-    if (!e && ms_out) cudaEventElapsedTime(ms_out, e0, e1);
-    cudaFree(dp); cudaFree(dw); cudaFree(hm); cudaFree(nbd); cudaFree(nbj); cudaFree(queue); cudaFree(evals);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    free(hw);
+    /* scratch per CTA: neighbour lists, and the inverse Hessian (no iterations need none) */
+    const size_t b_nbd = sizeof(float4) * (size_t)grid * BMAXN * BMAXNB, b_nbj = sizeof(int) * (size_t)grid * BMAXN * BMAXNB,
+                 b_hm = mitr > 0 ? sizeof(double) * (size_t)grid * BMAXDOF * BMAXDOF : 0;
+    e = (cudaError_t)mb_ws_grow(&ws->scratch, b_nbd + b_nbj + b_hm + 16, 0);
+    if (e != cudaSuccess) return (int)e;
+    char *q = (char *)ws->scratch.dev;
+    BArgs a;
+    a.S = S; a.rlxt = rlxt; a.mitr = mitr;
+    a.p_ev = p_ev; a.urep = urep; a.fmax = fmax; a.sigma = batch_sigma();
+    a.nat = d_nat; a.off = d_off; a.spc = d_spc; a.order = d_order;
+    a.lat = d_lat; a.x = d_x; a.H = d_H; a.iters = d_iters; a.status = d_status;
+    a.fout = d_frc; a.uout = d_str;
+    a.P = (const BParams *)ws->model;
+    a.W = (const float *)((char *)ws->model + sizeof(BParams));
+    a.queue = (int *)q;
+    a.nbd = (float4 *)(q + 16);
+    a.nbj = (int *)(q + 16 + b_nbd);
+    a.hmat = (double *)(q + 16 + b_nbd + b_nbj);
+    a.evals = d_evals;
+    a.work = (unsigned long long *)(d_evals + 1);
+    e = cudaMemsetAsync(a.queue, 0, sizeof(int), st);
+    if (e != cudaSuccess) return (int)e;
+    cudaEventRecord((cudaEvent_t)ws->e0, st);
+    e = !wide        ? batch_launch<4, 1>(gunits, st, a)
+        : csize == 4 ? batch_launch<BWARPS_WIDE, 4>(gunits, st, a)
+        : csize == 2 ? batch_launch<BWARPS_WIDE, 2>(gunits, st, a)
+                     : batch_launch<BWARPS_WIDE, 1>(gunits, st, a);
+    cudaEventRecord((cudaEvent_t)ws->e1, st);
+    if (!e) e = cudaGetLastError();
     return (int)e;
 }

@@ -288,14 +288,15 @@ extern "C" int mb_rdf(int device, int S, const int *nat, const int *atmn, const 
             return mb_handle_fail(MB_ERR_ARG, "species index out of range");
         }
     int rc = rdf_cuda(cudaSetDevice(device), "cudaSetDevice");
-    int *d_off = nullptr, *d_spc = nullptr;
-    double *d_lat = nullptr, *d_x = nullptr, *d_out = nullptr;
+    /* one allocation: offsets, species, lattices, positions, results */
     const size_t nout = (size_t)S * npair * nbins;
-    if (!rc) rc = rdf_cuda(cudaMalloc(&d_off, sizeof(int) * (S + 1)), "cudaMalloc");
-    if (!rc) rc = rdf_cuda(cudaMalloc(&d_spc, sizeof(int) * off[S]), "cudaMalloc");
-    if (!rc) rc = rdf_cuda(cudaMalloc(&d_lat, sizeof(double) * 9 * S), "cudaMalloc");
-    if (!rc) rc = rdf_cuda(cudaMalloc(&d_x, sizeof(double) * 3 * off[S]), "cudaMalloc");
-    if (!rc) rc = rdf_cuda(cudaMalloc(&d_out, sizeof(double) * nout), "cudaMalloc");
+    const size_t b_spc = (sizeof(int) * (S + 1) + 15) & ~(size_t)15;
+    const size_t b_lat = b_spc + ((sizeof(int) * (size_t)off[S] + 15) & ~(size_t)15);
+    const size_t b_x = b_lat + ((sizeof(double) * 9 * S + 15) & ~(size_t)15), b_out = b_x + ((sizeof(double) * 3 * (size_t)off[S] + 15) & ~(size_t)15);
+    char *d = nullptr;
+    if (!rc) rc = rdf_cuda(cudaMalloc(&d, b_out + sizeof(double) * nout), "cudaMalloc");
+    int *d_off = (int *)d, *d_spc = (int *)(d + b_spc);
+    double *d_lat = (double *)(d + b_lat), *d_x = (double *)(d + b_x), *d_out = (double *)(d + b_out);
     if (!rc) rc = rdf_cuda(cudaMemcpy(d_off, off, sizeof(int) * (S + 1), cudaMemcpyHostToDevice), "H2D");
     if (!rc) rc = rdf_cuda(cudaMemcpy(d_spc, atmn, sizeof(int) * off[S], cudaMemcpyHostToDevice), "H2D");
     if (!rc) rc = rdf_cuda(cudaMemcpy(d_lat, lat, sizeof(double) * 9 * S, cudaMemcpyHostToDevice), "H2D");
@@ -312,7 +313,7 @@ extern "C" int mb_rdf(int device, int S, const int *nat, const int *atmn, const 
         rc = rdf_cuda(cudaGetLastError(), "k_rdf_ref");
     }
     if (!rc) rc = rdf_cuda(cudaMemcpy(rdf, d_out, sizeof(double) * nout, cudaMemcpyDeviceToHost), "D2H");
-    cudaFree(d_off); cudaFree(d_spc); cudaFree(d_lat); cudaFree(d_x); cudaFree(d_out);
+    cudaFree(d);
     free(off);
     return rc;
 }

@@ -18,6 +18,7 @@ const mb_model *mb_handle_model(const mb_potential *p);
 void *mb_handle_stream(mb_potential *p);
 int mb_handle_device(const mb_potential *p);
 int mb_handle_fail(int code, const char *msg);
+mb_batch_ws *mb_handle_batch(mb_potential *p);
 void mb_handle_set_batch_stats(mb_potential *p, const long long *evals, float ms);
 
 /* The population relax and the batched E/F/S share this: with frc/str set
@@ -26,95 +27,92 @@ void mb_handle_set_batch_stats(mb_potential *p, const long long *evals, float ms
 static int batch_run(mb_potential *pot, int S, const int *nat, const int *atmn, double *lat, double *x, double p_gpa,
                      double urep, int rlxt, int mitr, double fmax, double *H, int *iters, int *status, double *frc,
                      double *str, int keep_xyz) {
-    int *off, *order, total = 0, s, rc = MB_OK;
-    int *d_nat = NULL, *d_off = NULL, *d_spc = NULL, *d_iters = NULL, *d_status = NULL, *d_order = NULL;
-    double *d_lat = NULL, *d_x = NULL, *d_H = NULL, *d_frc = NULL, *d_str = NULL;
-    long long evals[4] = {0, 0, 0, 0}; /* evaluations, atom evaluations, pairs, triplets */
+    int *off, *order, total = 0, s;
+    size_t at = 0, up, b_nat, b_off, b_order, b_spc, b_lat, b_x, b_H, b_iters, b_status, b_frc, b_str, b_ev, down;
+    char *h, *d;
     float ms = 0.0f;
     const mb_model *m;
-    void *st;
+    mb_batch_ws *ws;
+    cudaStream_t st;
     cudaError_t e;
     if (!pot || S < 1 || !nat || !atmn || !lat || !x || !H || !iters || !status || !(fmax > 0) || mitr < 0)
         return mb_handle_fail(MB_ERR_ARG, "bad arguments");
     if (!(rlxt == 2 || rlxt == 3)) return mb_handle_fail(MB_ERR_ARG, "batched relax supports RLXT 2 and 3");
     m = mb_handle_model(pot);
-    off = (int *)malloc(sizeof(int) * (S + 1));
     for (s = 0; s < S; s++) {
-        if (nat[s] < 1 || nat[s] > 64) {
-            free(off);
-            return mb_handle_fail(MB_ERR_ARG, "batched relax takes 1..64 atoms per structure");
-        }
-        off[s] = total;
+        if (nat[s] < 1 || nat[s] > 64) return mb_handle_fail(MB_ERR_ARG, "batched relax takes 1..64 atoms per structure");
         total += nat[s];
     }
-    off[S] = total;
     for (s = 0; s < total; s++)
-        if (atmn[s] < 0 || atmn[s] >= m->nspc) {
-            free(off);
-            return mb_handle_fail(MB_ERR_ARG, "species index out of range");
-        }
+        if (atmn[s] < 0 || atmn[s] >= m->nspc) return mb_handle_fail(MB_ERR_ARG, "species index out of range");
+    /* one block for the call's data, the same offsets on the device and in
+     * pinned memory: inputs first, what is both in the middle, results last */
+#define PUT(name, bytes) (name = at, at += ((size_t)(bytes) + 15) & ~(size_t)15)
+    PUT(b_nat, sizeof(int) * S);
+    PUT(b_off, sizeof(int) * (S + 1));
+    PUT(b_order, sizeof(int) * S);
+    PUT(b_spc, sizeof(int) * total);
+    PUT(b_lat, sizeof(double) * 9 * S);
+    PUT(b_x, sizeof(double) * 3 * total);
+    up = at;
+    PUT(b_ev, 4 * sizeof(long long)); /* evaluations, atom evaluations, pairs, triplets */
+    PUT(b_H, sizeof(double) * S);
+    PUT(b_iters, sizeof(int) * S);
+    PUT(b_status, sizeof(int) * S);
+    PUT(b_frc, frc ? sizeof(double) * 3 * total : 0);
+    PUT(b_str, frc ? sizeof(double) * 6 * S : 0);
+#undef PUT
+    cudaSetDevice(mb_handle_device(pot));
+    st = (cudaStream_t)mb_handle_stream(pot);
+    ws = mb_handle_batch(pot);
+    e = (cudaError_t)mb_ws_grow(&ws->io, at, at);
+    if (e) return mb_handle_fail(MB_ERR_CUDA, cudaGetErrorString(e));
+    h = (char *)ws->io.host;
+    d = (char *)ws->io.dev;
+    off = (int *)(h + b_off);
+    order = (int *)(h + b_order);
+    memcpy(h + b_nat, nat, sizeof(int) * S);
+    for (s = 0, off[0] = 0; s < S; s++) off[s + 1] = off[s] + nat[s];
     /* the persistent CTAs take structures largest first, so that the last
      * ones to start are small and the population finishes evenly */
-    order = (int *)malloc(sizeof(int) * S);
     {
-        int n, k = 0;
-        for (n = 64; n >= 1; n--)
-            for (s = 0; s < S; s++)
-                if (nat[s] == n) order[k++] = s;
+        int first[66] = {0}, n;
+        for (s = 0; s < S; s++) first[64 - nat[s] + 1]++;
+        for (n = 1; n < 66; n++) first[n] += first[n - 1];
+        for (s = 0; s < S; s++) order[first[64 - nat[s]]++] = s;
     }
-    cudaSetDevice(mb_handle_device(pot));
-    st = mb_handle_stream(pot);
-    e = cudaMalloc((void **)&d_nat, sizeof(int) * S);
-    if (!e) e = cudaMalloc((void **)&d_off, sizeof(int) * (S + 1));
-    if (!e) e = cudaMalloc((void **)&d_spc, sizeof(int) * total);
-    if (!e) e = cudaMalloc((void **)&d_iters, sizeof(int) * S);
-    if (!e) e = cudaMalloc((void **)&d_status, sizeof(int) * S);
-    if (!e) e = cudaMalloc((void **)&d_lat, sizeof(double) * 9 * S);
-    if (!e) e = cudaMalloc((void **)&d_x, sizeof(double) * 3 * total);
-    if (!e) e = cudaMalloc((void **)&d_H, sizeof(double) * S);
-    if (!e) e = cudaMalloc((void **)&d_order, sizeof(int) * S);
-    if (!e && frc) e = cudaMalloc((void **)&d_frc, sizeof(double) * 3 * total);
-    if (!e && str) e = cudaMalloc((void **)&d_str, sizeof(double) * 6 * S);
-    if (!e) e = cudaMemcpyAsync(d_order, order, sizeof(int) * S, cudaMemcpyHostToDevice, (cudaStream_t)st);
-    if (!e) e = cudaMemcpyAsync(d_nat, nat, sizeof(int) * S, cudaMemcpyHostToDevice, (cudaStream_t)st);
-    if (!e) e = cudaMemcpyAsync(d_off, off, sizeof(int) * (S + 1), cudaMemcpyHostToDevice, (cudaStream_t)st);
-    if (!e) e = cudaMemcpyAsync(d_spc, atmn, sizeof(int) * total, cudaMemcpyHostToDevice, (cudaStream_t)st);
-    if (!e) e = cudaMemcpyAsync(d_lat, lat, sizeof(double) * 9 * S, cudaMemcpyHostToDevice, (cudaStream_t)st);
-    if (!e) e = cudaMemcpyAsync(d_x, x, sizeof(double) * 3 * total, cudaMemcpyHostToDevice, (cudaStream_t)st);
-    if (e) {
-        rc = mb_handle_fail(MB_ERR_CUDA, cudaGetErrorString(e));
-        goto out;
-    }
-    e = (cudaError_t)mbk_relax_batch(m, S, d_nat, d_off, d_spc, d_order, d_lat, d_x, p_gpa / MB_EV2GPA, urep > 0 ? urep : 0.0,
-                                     rlxt, mitr, fmax, d_H, d_iters, d_status, frc ? d_frc : NULL,
-                                     frc ? d_str : NULL, st, evals, &ms);
-    if (e == cudaErrorInvalidValue) {
-        rc = mb_handle_fail(MB_ERR_MODEL, "batched relax needs a basis with <= 7 G4 exponents, zeta in {integers}, "
-                                          "2 lambdas, <= 16 G2 functions and D <= 288");
-        goto out;
-    }
-    if (e) {
-        rc = mb_handle_fail(MB_ERR_CUDA, cudaGetErrorString(e));
-        goto out;
-    }
-    e = cudaSuccess;
+    memcpy(h + b_spc, atmn, sizeof(int) * total);
+    memcpy(h + b_lat, lat, sizeof(double) * 9 * S);
+    memcpy(h + b_x, x, sizeof(double) * 3 * total);
+    memset(h + b_ev, 0, 4 * sizeof(long long));
+    e = cudaMemcpyAsync(d, h, b_ev + 4 * sizeof(long long), cudaMemcpyHostToDevice, st);
+    if (!e)
+        e = (cudaError_t)mbk_relax_batch(m, ws, S, (int *)(d + b_nat), (int *)(d + b_off), (int *)(d + b_spc),
+                                         (int *)(d + b_order), (double *)(d + b_lat), (double *)(d + b_x),
+                                         p_gpa / MB_EV2GPA, urep > 0 ? urep : 0.0, rlxt, mitr, fmax,
+                                         (double *)(d + b_H), (int *)(d + b_iters), (int *)(d + b_status),
+                                         frc ? (double *)(d + b_frc) : NULL, frc ? (double *)(d + b_str) : NULL,
+                                         (long long *)(d + b_ev), st);
+    if (e == cudaErrorInvalidValue)
+        return mb_handle_fail(MB_ERR_MODEL, "batched relax needs a basis with <= 7 G4 exponents, zeta in {integers}, "
+                                            "2 lambdas, <= 16 G2 functions and D <= 288");
+    /* results: from the lattices on when they are wanted back, else past the inputs */
+    down = keep_xyz ? b_lat : up;
+    if (!e) e = cudaMemcpyAsync(h + down, d + down, at - down, cudaMemcpyDeviceToHost, st);
+    if (!e) e = cudaStreamSynchronize(st);
+    if (e) return mb_handle_fail(MB_ERR_CUDA, cudaGetErrorString(e));
     if (keep_xyz) {
-        e = cudaMemcpy(lat, d_lat, sizeof(double) * 9 * S, cudaMemcpyDeviceToHost);
-        if (!e) e = cudaMemcpy(x, d_x, sizeof(double) * 3 * total, cudaMemcpyDeviceToHost);
+        memcpy(lat, h + b_lat, sizeof(double) * 9 * S);
+        memcpy(x, h + b_x, sizeof(double) * 3 * total);
     }
-    if (!e && frc) e = cudaMemcpy(frc, d_frc, sizeof(double) * 3 * total, cudaMemcpyDeviceToHost);
-    if (!e && frc && str) e = cudaMemcpy(str, d_str, sizeof(double) * 6 * S, cudaMemcpyDeviceToHost);
-    if (!e) e = cudaMemcpy(H, d_H, sizeof(double) * S, cudaMemcpyDeviceToHost);
-    if (!e) e = cudaMemcpy(iters, d_iters, sizeof(int) * S, cudaMemcpyDeviceToHost);
-    if (!e) e = cudaMemcpy(status, d_status, sizeof(int) * S, cudaMemcpyDeviceToHost);
-    if (e) rc = mb_handle_fail(MB_ERR_CUDA, cudaGetErrorString(e));
-    mb_handle_set_batch_stats(pot, evals, ms);
-out:
-    cudaFree(d_nat); cudaFree(d_off); cudaFree(d_spc); cudaFree(d_iters); cudaFree(d_status);
-    cudaFree(d_lat); cudaFree(d_x); cudaFree(d_H); cudaFree(d_order); cudaFree(d_frc); cudaFree(d_str);
-    free(off);
-    free(order);
-    return rc;
+    if (frc) memcpy(frc, h + b_frc, sizeof(double) * 3 * total);
+    if (frc && str) memcpy(str, h + b_str, sizeof(double) * 6 * S);
+    memcpy(H, h + b_H, sizeof(double) * S);
+    memcpy(iters, h + b_iters, sizeof(int) * S);
+    memcpy(status, h + b_status, sizeof(int) * S);
+    cudaEventElapsedTime(&ms, (cudaEvent_t)ws->e0, (cudaEvent_t)ws->e1);
+    mb_handle_set_batch_stats(pot, (long long *)(h + b_ev), ms);
+    return MB_OK;
 }
 
 int mb_relax_batch(mb_potential *pot, int S, const int *nat, const int *atmn, double *lat, double *x, double p_gpa,

@@ -16,6 +16,7 @@
 
 #include "../../../include/maise_b200.h"
 #include "../mb_internal.h"
+#include "mb_batch.h"
 #include "mb_bfgs.h"
 
 #define MB_EV2GPA 160.2176565       /* src/util.c:8 */
@@ -61,6 +62,7 @@ struct mb_potential {
     int device;
     long long batch_evals, batch_work[3];
     float batch_ms;
+    mb_batch_ws batch; /* kept between batched calls */
     cudaStream_t stream;
     mb_dev d;
     long launches;
@@ -113,6 +115,31 @@ static int cuda_fail(cudaError_t e, const char *what) {
         cudaError_t e_ = (call);                    \
         if (e_ != cudaSuccess) return cuda_fail(e_, what); \
     } while (0)
+
+int mb_ws_grow(mb_ws *w, size_t dev_bytes, size_t host_bytes) {
+    cudaError_t e = cudaSuccess;
+    if (dev_bytes > w->dev_len) {
+        cudaFree(w->dev);
+        w->dev = NULL;
+        w->dev_len = 0;
+        e = cudaMalloc(&w->dev, dev_bytes);
+        if (!e) w->dev_len = dev_bytes;
+    }
+    if (!e && host_bytes > w->host_len) {
+        cudaFreeHost(w->host);
+        w->host = NULL;
+        w->host_len = 0;
+        e = cudaMallocHost(&w->host, host_bytes);
+        if (!e) w->host_len = host_bytes;
+    }
+    return (int)e;
+}
+
+void mb_ws_free(mb_ws *w) {
+    cudaFree(w->dev);
+    cudaFreeHost(w->host);
+    memset(w, 0, sizeof(*w));
+}
 
 /* ------------------------------------------------------------------ */
 /* handle lifecycle                                                    */
@@ -199,6 +226,7 @@ int mb_close(mb_potential *p) {
         }
     }
     cudaFreeHost(p->h_res);
+    mbk_batch_free(&p->batch);
     dev_free(&p->d);
     cudaFree(p->d.params);
     cudaFree(p->d.weights);
@@ -245,6 +273,7 @@ void *mb_stream(mb_potential *p) { return p ? (void *)p->stream : NULL; }
 const mb_model *mb_handle_model(const mb_potential *p) { return &p->m; }
 void *mb_handle_stream(mb_potential *p) { return (void *)p->stream; }
 int mb_handle_device(const mb_potential *p) { return p->device; }
+mb_batch_ws *mb_handle_batch(mb_potential *p) { return &p->batch; }
 int mb_handle_fail(int code, const char *msg) { return fail(code, "%s", msg); }
 void mb_handle_set_batch_stats(mb_potential *p, const long long *evals, float ms) {
     p->batch_evals = evals[0];

@@ -10,6 +10,7 @@
 #include <string.h>
 
 #include "../../../include/maise_surrogate.h"
+#include "../mb_internal.h"
 #include "mb_surrogate_k.h"
 
 int mb_handle_fail(int code, const char *msg);
@@ -32,6 +33,8 @@ struct mb_surrogate {
     int *idx;
     double *loss;
     int loss_cap;
+    mb_ws io;   /* structures of a call, staged through pinned memory */
+    mb_ws feat; /* their features; pinned side: predictions */
 };
 
 #define CK(call)                                                                   \
@@ -191,6 +194,8 @@ void mb_sur_close(mb_surrogate *s) {
     cudaFree(s->mean);
     cudaFree(s->istd);
     cudaFree(s->loss);
+    mb_ws_free(&s->io);
+    mb_ws_free(&s->feat);
     if (s->st) cudaStreamDestroy(s->st);
     free(s);
 }
@@ -254,61 +259,55 @@ typedef struct {
     int total;
 } dev_structs;
 
-static void free_structs(dev_structs *d) {
-    cudaFree(d->off);
-    cudaFree(d->spc);
-    cudaFree(d->lat);
-    cudaFree(d->x);
-    cudaFree(d->status);
-    memset(d, 0, sizeof(*d));
-}
-
+/* The structures' arrays in one block at the same offsets in pinned and in
+ * device memory (both kept by the handle), copied at once. */
 static int upload_structs(mb_surrogate *s, int S, const int *nat, const int *atmn, const double *lat, const double *x,
                           dev_structs *d) {
     int *off, k, total = 0;
-    cudaError_t e;
-    memset(d, 0, sizeof(*d));
-    off = (int *)malloc(sizeof(int) * (S + 1));
+    size_t at = 16, b_off, b_spc, b_lat, b_x;
+    char *h, *g;
     for (k = 0; k < S; k++) {
-        if (nat[k] < 1 || nat[k] > SUR_MAX_ATOMS) {
-            free(off);
+        if (nat[k] < 1 || nat[k] > SUR_MAX_ATOMS)
             return mb_handle_fail(MB_ERR_ARG, "the surrogate takes 1..256 atoms per structure");
-        }
-        off[k] = total;
         total += nat[k];
     }
-    off[S] = total;
     for (k = 0; k < total; k++)
-        if (atmn[k] < 0 || atmn[k] >= s->nspc) {
-            free(off);
-            return mb_handle_fail(MB_ERR_ARG, "species index out of range");
-        }
+        if (atmn[k] < 0 || atmn[k] >= s->nspc) return mb_handle_fail(MB_ERR_ARG, "species index out of range");
+#define PUT(name, bytes) (name = at, at += ((size_t)(bytes) + 15) & ~(size_t)15)
+    PUT(b_off, sizeof(int) * (S + 1));
+    PUT(b_spc, sizeof(int) * total);
+    PUT(b_lat, sizeof(double) * 9 * S);
+    PUT(b_x, sizeof(double) * 3 * total);
+#undef PUT
+    CK((cudaError_t)mb_ws_grow(&s->io, at, at));
+    h = (char *)s->io.host;
+    g = (char *)s->io.dev;
+    off = (int *)(h + b_off);
+    for (k = 0, off[0] = 0; k < S; k++) off[k + 1] = off[k] + nat[k];
+    memset(h, 0, 16); /* the status word */
+    memcpy(h + b_spc, atmn, sizeof(int) * total);
+    memcpy(h + b_lat, lat, sizeof(double) * 9 * S);
+    memcpy(h + b_x, x, sizeof(double) * 3 * total);
+    CK(cudaMemcpyAsync(g, h, at, cudaMemcpyHostToDevice, s->st));
+    d->status = (int *)g;
+    d->off = (int *)(g + b_off);
+    d->spc = (int *)(g + b_spc);
+    d->lat = (double *)(g + b_lat);
+    d->x = (double *)(g + b_x);
     d->total = total;
-    e = cudaMalloc((void **)&d->off, sizeof(int) * (S + 1));
-    if (!e) e = cudaMalloc((void **)&d->spc, sizeof(int) * total);
-    if (!e) e = cudaMalloc((void **)&d->lat, sizeof(double) * 9 * S);
-    if (!e) e = cudaMalloc((void **)&d->x, sizeof(double) * 3 * total);
-    if (!e) e = cudaMalloc((void **)&d->status, sizeof(int));
-    if (!e) e = cudaMemcpyAsync(d->off, off, sizeof(int) * (S + 1), cudaMemcpyHostToDevice, s->st);
-    if (!e) e = cudaMemcpyAsync(d->spc, atmn, sizeof(int) * total, cudaMemcpyHostToDevice, s->st);
-    if (!e) e = cudaMemcpyAsync(d->lat, lat, sizeof(double) * 9 * S, cudaMemcpyHostToDevice, s->st);
-    if (!e) e = cudaMemcpyAsync(d->x, x, sizeof(double) * 3 * total, cudaMemcpyHostToDevice, s->st);
-    if (!e) e = cudaMemsetAsync(d->status, 0, sizeof(int), s->st);
-    if (!e) e = cudaStreamSynchronize(s->st); /* `off` is pageable and freed next */
-    free(off);
-    if (e) {
-        free_structs(d);
-        return mb_handle_fail(MB_ERR_CUDA, cudaGetErrorString(e));
-    }
     return MB_OK;
 }
 
+/* queue the histogram; its status word lands in the pinned block */
 static int run_rdf(mb_surrogate *s, int S, dev_structs *d, float *d_feat) {
-    int status = 0;
     KK(surk_rdf(S, d->off, d->spc, d->lat, d->x, s->nspc, s->nbins, s->rmax, s->sigma, d_feat, d->status, s->st));
-    CK(cudaMemcpyAsync(&status, d->status, sizeof(int), cudaMemcpyDeviceToHost, s->st));
-    CK(cudaStreamSynchronize(s->st));
-    if (status)
+    CK(cudaMemcpyAsync(s->io.host, d->status, sizeof(int), cudaMemcpyDeviceToHost, s->st));
+    return MB_OK;
+}
+
+/* after the stream has been waited for */
+static int rdf_status(const mb_surrogate *s) {
+    if (*(const int *)s->io.host)
         return mb_handle_fail(MB_ERR_ARG, "a cell is degenerate or too thin for the histogram range (more than 6 "
                                           "periodic images per direction)");
     return MB_OK;
@@ -317,87 +316,67 @@ static int run_rdf(mb_surrogate *s, int S, dev_structs *d, float *d_feat) {
 int mb_sur_features(mb_surrogate *s, int S, const int *nat, const int *atmn, const double *lat, const double *x,
                     float *feat) {
     dev_structs d;
-    float *d_feat = NULL;
     int rc;
     if (!s || S < 1 || !nat || !atmn || !lat || !x || !feat) return mb_handle_fail(MB_ERR_ARG, "bad arguments");
     CK(cudaSetDevice(s->device));
     if ((rc = upload_structs(s, S, nat, atmn, lat, x, &d))) return rc;
-    if (cudaMalloc((void **)&d_feat, sizeof(float) * (size_t)S * s->nin) != cudaSuccess) {
-        free_structs(&d);
-        return mb_handle_fail(MB_ERR_CUDA, "cudaMalloc features");
-    }
-    rc = run_rdf(s, S, &d, d_feat);
-    if (!rc && cudaMemcpy(feat, d_feat, sizeof(float) * (size_t)S * s->nin, cudaMemcpyDeviceToHost) != cudaSuccess)
-        rc = mb_handle_fail(MB_ERR_CUDA, "feature download");
-    cudaFree(d_feat);
-    free_structs(&d);
-    return rc;
+    CK((cudaError_t)mb_ws_grow(&s->feat, sizeof(float) * (size_t)S * s->nin, 0));
+    if ((rc = run_rdf(s, S, &d, (float *)s->feat.dev))) return rc;
+    CK(cudaStreamSynchronize(s->st));
+    if ((rc = rdf_status(s))) return rc;
+    CK(cudaMemcpy(feat, s->feat.dev, sizeof(float) * (size_t)S * s->nin, cudaMemcpyDeviceToHost));
+    return MB_OK;
 }
 
 /* ---------------------------------------------------------- prediction */
 
 #define PRED_CHUNK 4096
 
+/* queue the network on the features in chunks of rows; the outputs land in
+ * the pinned side of s->feat */
 static int predict_dev(mb_surrogate *s, int S, const float *d_feat, double *pred) {
     float *y;
     int c0, k, rc;
-    if ((rc = ensure_rows(s, PRED_CHUNK))) return rc;
-    y = (float *)malloc(sizeof(float) * PRED_CHUNK);
+    if ((rc = ensure_rows(s, S < PRED_CHUNK ? S : PRED_CHUNK))) return rc;
+    CK((cudaError_t)mb_ws_grow(&s->feat, 0, sizeof(float) * (size_t)S));
+    y = (float *)s->feat.host;
     for (c0 = 0; c0 < S; c0 += PRED_CHUNK) {
         const int B = S - c0 < PRED_CHUNK ? S - c0 : PRED_CHUNK;
-        int e = surk_gather(B, s->nin, NULL, d_feat + (size_t)c0 * s->nin, s->mean, s->istd, s->x, NULL, 0.0f, 1.0f,
-                            NULL, s->st);
-        if (e) {
-            free(y);
-            return mb_handle_fail(MB_ERR_CUDA, cudaGetErrorString((cudaError_t)e));
-        }
-        if ((rc = forward(s, B, s->x))) {
-            free(y);
-            return rc;
-        }
-        if (cudaMemcpyAsync(y, s->z[NL - 1], sizeof(float) * B, cudaMemcpyDeviceToHost, s->st) != cudaSuccess ||
-            cudaStreamSynchronize(s->st) != cudaSuccess) {
-            free(y);
-            return mb_handle_fail(MB_ERR_CUDA, "prediction download");
-        }
-        for (k = 0; k < B; k++) pred[c0 + k] = (double)y[k] * s->tstd + s->tmean;
+        KK(surk_gather(B, s->nin, NULL, d_feat + (size_t)c0 * s->nin, s->mean, s->istd, s->x, NULL, 0.0f, 1.0f, NULL,
+                       s->st));
+        if ((rc = forward(s, B, s->x))) return rc;
+        CK(cudaMemcpyAsync(y + c0, s->z[NL - 1], sizeof(float) * B, cudaMemcpyDeviceToHost, s->st));
     }
-    free(y);
+    CK(cudaStreamSynchronize(s->st));
+    for (k = 0; k < S; k++) pred[k] = (double)y[k] * s->tstd + s->tmean;
     return MB_OK;
 }
 
 int mb_sur_predict(mb_surrogate *s, int S, const float *feat, double *pred) {
-    float *d_feat = NULL;
-    int rc;
     if (!s || S < 1 || !feat || !pred) return mb_handle_fail(MB_ERR_ARG, "bad arguments");
     CK(cudaSetDevice(s->device));
-    CK(cudaMalloc((void **)&d_feat, sizeof(float) * (size_t)S * s->nin));
-    if (cudaMemcpyAsync(d_feat, feat, sizeof(float) * (size_t)S * s->nin, cudaMemcpyHostToDevice, s->st) !=
-        cudaSuccess) {
-        cudaFree(d_feat);
-        return mb_handle_fail(MB_ERR_CUDA, "feature upload");
-    }
-    rc = predict_dev(s, S, d_feat, pred);
-    cudaFree(d_feat);
-    return rc;
+    CK((cudaError_t)mb_ws_grow(&s->feat, sizeof(float) * (size_t)S * s->nin, 0));
+    CK(cudaMemcpyAsync(s->feat.dev, feat, sizeof(float) * (size_t)S * s->nin, cudaMemcpyHostToDevice, s->st));
+    return predict_dev(s, S, (const float *)s->feat.dev, pred);
 }
 
 int mb_sur_screen(mb_surrogate *s, int S, const int *nat, const int *atmn, const double *lat, const double *x,
                   double *pred) {
     dev_structs d;
-    float *d_feat = NULL;
+    double *tmp;
     int rc;
     if (!s || S < 1 || !nat || !atmn || !lat || !x || !pred) return mb_handle_fail(MB_ERR_ARG, "bad arguments");
     CK(cudaSetDevice(s->device));
     if ((rc = upload_structs(s, S, nat, atmn, lat, x, &d))) return rc;
-    if (cudaMalloc((void **)&d_feat, sizeof(float) * (size_t)S * s->nin) != cudaSuccess) {
-        free_structs(&d);
-        return mb_handle_fail(MB_ERR_CUDA, "cudaMalloc features");
-    }
-    rc = run_rdf(s, S, &d, d_feat);
-    if (!rc) rc = predict_dev(s, S, d_feat, pred);
-    cudaFree(d_feat);
-    free_structs(&d);
+    CK((cudaError_t)mb_ws_grow(&s->feat, sizeof(float) * (size_t)S * s->nin, 0));
+    if ((rc = run_rdf(s, S, &d, (float *)s->feat.dev))) return rc;
+    /* nothing is written to pred when a cell was refused */
+    tmp = (double *)malloc(sizeof(double) * S);
+    if (!tmp) return mb_handle_fail(MB_ERR_ARG, "out of memory");
+    rc = predict_dev(s, S, (const float *)s->feat.dev, tmp);
+    if (!rc) rc = rdf_status(s);
+    if (!rc) memcpy(pred, tmp, sizeof(double) * S);
+    free(tmp);
     return rc;
 }
 

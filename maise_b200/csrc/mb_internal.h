@@ -181,6 +181,15 @@ typedef struct {
     int tune_key[MB_TUNE_SLOTS], tune_val[MB_TUNE_SLOTS];
 } mb_dev;
 
+/* Device memory with a pinned host mirror that a handle keeps between calls:
+ * grown on demand, freed with the handle. */
+typedef struct {
+    void *dev, *host;
+    size_t dev_len, host_len;
+} mb_ws;
+int mb_ws_grow(mb_ws *w, size_t dev_bytes, size_t host_bytes); /* 0 or a CUDA error; contents are lost on growth */
+void mb_ws_free(mb_ws *w);
+
 /* Launchers (mb_kernels.cu).  All enqueue on `stream`; return 0 or a CUDA
  * error code.  Counts of launched kernels are added to *launches. */
 int mbk_wrap(mb_dev *d, int N, const mb_cell *c, void *stream, long *launches);

@@ -22,7 +22,7 @@ import os
 
 import numpy as np
 
-from . import _D, _I, _dp, load_library
+from . import _D, _I, _dp, load_library, pack
 
 __all__ = ["relax_generation", "write_member", "rank", "rdf", "overlaps", "duplicates"]
 
@@ -48,10 +48,7 @@ def relax_generation(pot, evos_dir, gen, offspring, first_member, p_gpa=0.0, ure
 
         idx = np.sort(keep_best(surrogate.screen(offspring), keep))
     chosen = [offspring[k] for k in idx]
-    nat = np.array([len(s["atmn"]) for s in chosen], np.int32)
-    atmn = np.ascontiguousarray(np.concatenate([np.asarray(s["atmn"], np.int32) for s in chosen]))
-    X = np.ascontiguousarray(np.concatenate([np.asarray(s["X"], float).reshape(-1, 3) for s in chosen]))
-    LAT = np.ascontiguousarray(np.stack([np.asarray(s["LAT"], float).reshape(3, 3) for s in chosen]))
+    nat, atmn, LAT, X = pack(chosen)
     S = len(chosen)
     H = np.zeros(S)
     iters = np.zeros(S, np.int32)
@@ -93,12 +90,9 @@ def rdf(structures, nspc, nbins=3000, rmin=5.8, rmax=6.0, sigma=0.008, normalise
     """RANK_TR's per-species-pair RDF of every structure, on the GPU:
     [S, nspc (nspc + 1) / 2, nbins] (the reference's defaults)."""
     lib = load_library()
-    nat = np.array([len(s["atmn"]) for s in structures], np.int32)
-    atmn = np.ascontiguousarray(np.concatenate([np.asarray(s["atmn"], np.int32) for s in structures]))
-    X = np.ascontiguousarray(np.concatenate([np.asarray(s["X"], float).reshape(-1, 3) for s in structures]))
-    LAT = np.ascontiguousarray(np.stack([np.asarray(s["LAT"], float).reshape(3, 3) for s in structures]))
+    nat, atmn, LAT, X = pack(structures)
     npair = nspc * (nspc + 1) // 2
-    out = np.zeros((len(nat), npair, nbins))
+    out = np.empty((len(nat), npair, nbins))
     _check(lib, lib.mb_rdf(device, len(nat), nat.ctypes.data_as(_I), atmn.ctypes.data_as(_I), _dp(LAT), _dp(X), ND,
                            nspc, nbins, rmin, rmax, sigma, int(normalise), _dp(out)))
     return out
@@ -108,7 +102,7 @@ def overlaps(R, device=0):
     """CxC of every pair of members: [S, S] from RDFs R[S, ...]."""
     lib = load_library()
     R = np.ascontiguousarray(np.asarray(R, float).reshape(len(R), -1))
-    out = np.zeros((len(R), len(R)))
+    out = np.empty((len(R), len(R)))
     _check(lib, lib.mb_rdf_overlap(device, len(R), R.shape[1], _dp(R), _dp(out)))
     return out
 

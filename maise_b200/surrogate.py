@@ -15,7 +15,7 @@ import ctypes
 
 import numpy as np
 
-from . import MaiseError, load_library
+from . import MaiseError, load_library, pack
 
 _F = ctypes.POINTER(ctypes.c_float)
 _D = ctypes.POINTER(ctypes.c_double)
@@ -54,15 +54,6 @@ def _f32(a, n=None):
     if n is not None and a.size != n:
         raise ValueError(f"expected {n} values, got {a.size}")
     return a
-
-
-def pack(structures):
-    """(nat, atmn, lat, x) arrays of a list of dict(X, LAT, atmn)."""
-    nat = np.array([len(s["atmn"]) for s in structures], np.int32)
-    atmn = np.ascontiguousarray(np.concatenate([np.asarray(s["atmn"], np.int32) for s in structures]))
-    lat = np.ascontiguousarray(np.stack([np.asarray(s["LAT"], float).reshape(9) for s in structures]))
-    x = np.ascontiguousarray(np.concatenate([np.asarray(s["X"], float).reshape(-1) for s in structures]))
-    return nat, atmn, lat, x
 
 
 class Surrogate:
