@@ -62,10 +62,29 @@ __device__ __forceinline__ void wrap_atom(int i, double *__restrict__ X, const m
     }
 }
 
-__global__ void k_wrap(int N, double *__restrict__ X, mb_cell c, int *status) {
+/* JAR on every atom; F (if set) is cleared for the pass that follows */
+__global__ void k_wrap(int N, double *__restrict__ X, mb_cell c, int *status, double *__restrict__ F) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
     wrap_atom(i, X, c, status);
+    if (F) F[3 * i] = F[3 * i + 1] = F[3 * i + 2] = 0.0;
+}
+
+/* Start of a pass on host arrays: positions and species read from pinned host
+ * memory, JAR (periodic cells), forces cleared.  One launch in the place of two
+ * copies, a clear and k_wrap, which for a small structure each cost more than
+ * they move (with the results stored by k_finalize, and the list kernel below,
+ * a 32-atom E/F/S call went from 120 to 77 us). */
+__global__ void k_intake(int N, const double *__restrict__ hx, mb_cell c, const int *__restrict__ hspc,
+                         double *__restrict__ X, int *__restrict__ spc, int *status, double *__restrict__ F) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= N) return;
+    X[3 * i] = hx[3 * i];
+    X[3 * i + 1] = hx[3 * i + 1];
+    X[3 * i + 2] = hx[3 * i + 2];
+    spc[i] = hspc[i];
+    if (c.ND > 0) wrap_atom(i, X, c, status);
+    if (F) F[3 * i] = F[3 * i + 1] = F[3 * i + 2] = 0.0;
 }
 
 /* ------------------------------------------------------------------ */
@@ -90,42 +109,97 @@ __device__ __forceinline__ double image_disp(const mb_cell &c, const double *xi,
     return r;
 }
 
-/* one warp per atom; candidates in the reference's order (j, then images) */
+/* append the accepted candidates of a round to atom i's list, in lane order */
+__device__ __forceinline__ void list_append(bool ok, int j, const double *d, double r2, size_t row, int cap, int lane,
+                                            int &count, int *__restrict__ nj, double4 *__restrict__ nd) {
+    const unsigned m = __ballot_sync(FULL, ok);
+    const int pos = count + __popc(m & ((1u << lane) - 1u));
+    if (ok && pos < cap) {
+        nj[row + pos] = j;
+        nd[row + pos] = make_double4(d[0], d[1], d[2], sqrt(r2));
+    }
+    count += __popc(m);
+}
+
+/* One warp per atom; candidates in the reference's order (j, then images).
+ * Cells with 16 to 128 images: the lanes hold the images' shifts (formed in
+ * image_disp's order, so the sums round as there) and walk the atoms j
+ * together.  Otherwise (clusters above all) the lanes walk the flat candidate
+ * index; with that for every cell, its two divisions a candidate took 16 us
+ * for 32 atoms of 27 images and 22 us for 47 of 125 (now 8 and 11). */
+#define BRUTE_IMG 4
 __global__ void k_nlist_brute(int N, int NM, int cap, const double *__restrict__ X, mb_cell c, double rc2,
                               int *__restrict__ nn, int *__restrict__ nj, double4 *__restrict__ nd, int *status) {
     int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (warp >= N) return;
     int i = warp;
+    const size_t row = (size_t)i * cap;
     int w0 = 2 * c.Nq[0] + 1, w1 = 2 * c.Nq[1] + 1, w2 = 2 * c.Nq[2] + 1;
     int nimg = w0 * w1 * w2;
-    long long total = (long long)N * nimg;
     double xi[3] = {X[3 * i], X[3 * i + 1], X[3 * i + 2]};
     int count = 0;
-    for (long long base = 0; base < total; base += 32) {
-        long long cidx = base + lane;
-        bool ok = false;
-        int j = 0, i0 = 0, i1 = 0, i2 = 0;
-        double d[3] = {0, 0, 0}, r2 = 0.0;
-        if (cidx < total) {
-            j = (int)(cidx / nimg);
-            int im = (int)(cidx % nimg);
-            i2 = im % w2 - c.Nq[2];
-            int t = im / w2;
-            i1 = t % w1 - c.Nq[1];
-            i0 = t / w1 - c.Nq[0];
-            if (!(j == i && i0 == 0 && i1 == 0 && i2 == 0)) {
-                double xj[3] = {X[3 * j], X[3 * j + 1], X[3 * j + 2]};
-                r2 = image_disp(c, xi, xj, i0, i1, i2, d);
-                ok = r2 < rc2;
+    if (nimg >= 16 && nimg <= 32 * BRUTE_IMG) {
+        double sh[BRUTE_IMG][3];
+        const int zero = (c.Nq[0] * w1 + c.Nq[1]) * w2 + c.Nq[2]; /* the unshifted image */
+#pragma unroll
+        for (int t = 0; t < BRUTE_IMG; t++) {
+            const int im = 32 * t + lane, i2 = im % w2 - c.Nq[2], u = im / w2, i1 = u % w1 - c.Nq[1], i0 = u / w1 - c.Nq[0];
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                double x = 0.0;
+                x = xadd(x, xmul((double)i0, c.L[q]));
+                x = xadd(x, xmul((double)i1, c.L[3 + q]));
+                sh[t][q] = xadd(x, xmul((double)i2, c.L[6 + q]));
             }
         }
-        unsigned m = __ballot_sync(FULL, ok);
-        int pos = count + __popc(m & ((1u << lane) - 1u));
-        if (ok && pos < cap) {
-            nj[(size_t)i * cap + pos] = j;
-            nd[(size_t)i * cap + pos] = make_double4(d[0], d[1], d[2], sqrt(r2));
+        /* four rounds' distances side by side (their FP64 chains overlap), then
+         * four appends: images 0-31 of atoms j..j+3, or all images of atom j */
+        const int T = nimg > 32 ? BRUTE_IMG : 1;
+        for (int j0 = 0; j0 < N; j0 += BRUTE_IMG / T) {
+            double d[BRUTE_IMG][3], r2[BRUTE_IMG];
+            bool ok[BRUTE_IMG];
+            int jj[BRUTE_IMG];
+#pragma unroll
+            for (int u = 0; u < BRUTE_IMG; u++) {
+                const int j = T == 1 ? min(j0 + u, N - 1) : j0, im = (T == 1 ? 0 : 32 * u) + lane;
+                jj[u] = j;
+                r2[u] = 0.0;
+#pragma unroll
+                for (int q = 0; q < 3; q++) {
+                    d[u][q] = xadd(T == 1 ? sh[0][q] : sh[u][q], xsub(X[3 * j + q], xi[q]));
+                    r2[u] = xadd(r2[u], xmul(d[u][q], d[u][q]));
+                }
+                ok[u] = im < nimg && r2[u] < rc2 && !(j == i && im == zero) && (T > 1 || j0 + u < N);
+            }
+#pragma unroll
+            for (int u = 0; u < BRUTE_IMG; u++) list_append(ok[u], jj[u], d[u], r2[u], row, cap, lane, count, nj, nd);
         }
-        count += __popc(m);
+    } else {
+        long long total = (long long)N * nimg;
+        for (long long base = 0; base < total; base += 32) {
+            long long cidx = base + lane;
+            bool ok = false;
+            int j = 0, i0 = 0, i1 = 0, i2 = 0;
+            double d[3] = {0, 0, 0}, r2 = 0.0;
+            if (cidx < total) {
+                if (nimg == 1) {
+                    j = (int)cidx;
+                } else {
+                    j = (int)(cidx / nimg);
+                    int im = (int)(cidx % nimg);
+                    i2 = im % w2 - c.Nq[2];
+                    int t = im / w2;
+                    i1 = t % w1 - c.Nq[1];
+                    i0 = t / w1 - c.Nq[0];
+                }
+                if (!(j == i && i0 == 0 && i1 == 0 && i2 == 0)) {
+                    double xj[3] = {X[3 * j], X[3 * j + 1], X[3 * j + 2]};
+                    r2 = image_disp(c, xi, xj, i0, i1, i2, d);
+                    ok = r2 < rc2;
+                }
+            }
+            list_append(ok, j, d, r2, row, cap, lane, count, nj, nd);
+        }
     }
     if (lane == 0) {
         nn[i] = count < cap ? count : cap;
@@ -1589,6 +1663,8 @@ __global__ void __launch_bounds__(WPA * 32 * APB, 512 / (WPA * 32 * APB)) k_efs_
             }
             eu = warp_sum(eu);
             if (lane == 0) A.EU[i] = eu;
+        } else if (tid == 0) {
+            A.EU[i] = 0.0;
         }
     }
 
@@ -2188,77 +2264,106 @@ __host__ __device__ inline int red_chunk(int N, int nparts) {
     return c > 512 ? c : 512;
 }
 
-/* Sum of acc[0..K-1] over the CTA's 256 threads (fixed tree) into red[k][0]. */
+/* Sum of acc[0..K-1] over the CTA's 256 threads into red[k][0] (warp trees,
+ * then the 8 warps in order). */
 template <int K>
-__device__ __forceinline__ void block_tree(double (*red)[256], const double *acc, int t) {
-    for (int k = 0; k < K; k++) red[k][t] = acc[k];
-    __syncthreads();
-    for (int h = 128; h > 0; h >>= 1) {
-        if (t < h)
-            for (int k = 0; k < K; k++) red[k][t] += red[k][t + h];
-        __syncthreads();
+__device__ __forceinline__ void block_tree(double (*red)[8], const double *acc, int t) {
+    const int lane = t & 31, warp = t >> 5;
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        const double v = warp_sum(acc[k]);
+        if (lane == 0) red[k][warp] = v;
     }
+    __syncthreads();
+    if (t < K) {
+        double s = 0.0;
+        for (int w = 0; w < 8; w++) s += red[t][w];
+        red[t][0] = s;
+    }
+    __syncthreads();
 }
 
 /* After block_tree: CTA partials go to part[cta][0..K-1]; returns true in
- * thread 0 of the CTA that finished last, which then holds the sums of the
- * partials in CTA order in tot[] (and has reset the ticket). */
+ * the threads of warp 0 of the CTA that finished last, all of which then hold
+ * the sums of the partials in tot[] (lanes over CTAs, then a tree: a fixed
+ * order), and the ticket is reset. */
 template <int K>
-__device__ __forceinline__ bool last_cta(double (*red)[256], double *part, unsigned *ticket, double *tot, int t) {
+__device__ __forceinline__ bool last_cta(double (*red)[8], double *part, unsigned *ticket, double *tot, int t) {
     __shared__ bool is_last;
     const int nb = gridDim.x;
     if (nb == 1) {
-        if (t == 0)
-            for (int k = 0; k < K; k++) tot[k] = red[k][0];
-        return t == 0;
+        for (int k = 0; k < K; k++) tot[k] = red[k][0];
+        return t < 32;
     }
+    if (t < K) part[blockIdx.x * 8 + t] = red[t][0];
+    __syncwarp();
     if (t == 0) {
-        for (int k = 0; k < K; k++) part[blockIdx.x * 8 + k] = red[k][0];
         __threadfence();
         is_last = atomicAdd(ticket, 1u) == (unsigned)(nb - 1);
     }
     __syncthreads();
-    if (!is_last || t != 0) return false;
+    if (!is_last || t >= 32) return false;
     __threadfence();
     const volatile double *vp = part;
     for (int k = 0; k < K; k++) {
         double s = 0.0;
-        for (int c = 0; c < nb; c++) s += vp[c * 8 + k];
-        tot[k] = s;
+        for (int c = t; c < nb; c += 32) s += vp[c * 8 + k];
+        tot[k] = warp_sum(s);
     }
-    *ticket = 0u;
+    if (t == 0) *ticket = 0u;
     return true;
 }
 
+/* where a pass's results go on the host (pinned memory; any may be NULL) */
+struct HostOut {
+    double *out;       /* [16], as the device's */
+    int *status;       /* [4] */
+    double *F, *X, *EA;
+};
+
 /* out[0]=E, out[1]=H, out[2..7]=U: every CTA reduces a fixed chunk of atoms
  * (threads strided, then a tree) and zeroes the chunk's force components
- * below 1e-8 (src/cmod.c:177-184); the last CTA adds the partials in CTA
- * order.  Every sum has a fixed order, so results are reproducible. */
+ * below 1e-8 (src/cmod.c:177-184); the last CTA adds the partials.  For a pass
+ * on host arrays it also stores the results into pinned host memory (forces,
+ * wrapped positions, atom energies, totals, status): one launch in the place
+ * of five copies.  Every sum has a fixed order, so results are reproducible. */
 __global__ void __launch_bounds__(256) k_finalize(int N, int mode, double pV, const double *EA, const double *EU,
                                                   const double *vir, double *F, double *out, double *part,
-                                                  unsigned *ticket) {
-    __shared__ double red[7][256];
+                                                  unsigned *ticket, const double *X, const int *status, HostOut ho) {
+    __shared__ double red[7][8];
     const int t = threadIdx.x, chunk = red_chunk(N, part ? 1 : 0);
     const int lo = blockIdx.x * chunk, hi = min(N, lo + chunk);
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
     for (int i = lo + t; i < hi; i += 256) {
-        acc[0] += EA[i] + EU[i];
+        const double ea = EA[i];
+        acc[0] += ea + EU[i];
+        if (ho.EA) ho.EA[i] = ea;
         if (mode != MB_MODE_ENERGY)
             for (int k = 0; k < 6; k++) acc[1 + k] += vir[(size_t)i * 6 + k];
     }
-    if (mode == MB_MODE_EFS)
-        for (int i = 3 * lo + t; i < 3 * hi; i += 256)
-            if (fabs(F[i]) < 1e-8) F[i] = 0.0;
+    if (mode == MB_MODE_EFS || (mode == MB_MODE_VJP && ho.F))
+        for (int i = 3 * lo + t; i < 3 * hi; i += 256) {
+            double f = F[i];
+            if (mode == MB_MODE_EFS && fabs(f) < 1e-8) F[i] = f = 0.0;
+            if (ho.F) ho.F[i] = f;
+        }
+    if (ho.X)
+        for (int i = 3 * lo + t; i < 3 * hi; i += 256) ho.X[i] = X[i];
     block_tree<7>(red, acc, t);
     double tot[7];
-    if (last_cta<7>(red, part, ticket, tot, t)) {
-        out[0] = tot[0];
-        out[1] = tot[0] + pV;
-        for (int k = 0; k < 6; k++) {
-            double u = tot[1 + k];
-            if (mode == MB_MODE_EFS && fabs(u) < 1e-8) u = 0.0;
-            out[2 + k] = u;
+    if (last_cta<7>(red, part, ticket, tot, t) && t < 8) {
+        /* E, H = E + pV, U (lane 0, 1, 2..7) */
+        double v = tot[0];
+        for (int k = 1; k < 7; k++)
+            if (t == k + 1) v = tot[k];
+        if (t == 1) v = tot[0] + pV;
+        if (t >= 2 && mode == MB_MODE_EFS && fabs(v) < 1e-8) v = 0.0;
+        out[t] = v;
+        if (ho.out) {
+            ho.out[t] = v;
+            ho.out[8 + t] = out[8 + t];
         }
+        if (ho.status && t < 4) ho.status[t] = status[t];
     }
 }
 
@@ -2274,7 +2379,7 @@ __global__ void __launch_bounds__(256) k_finalize(int N, int mode, double pV, co
 __global__ void __launch_bounds__(256) k_nvt_thermostat(int N, const double *V, const int *spc, const double *mass,
                                                         double dt, double tau, double T, double *out, double *trace,
                                                         int capTrace, double *part, unsigned *ticket) {
-    __shared__ double red[1][256];
+    __shared__ double red[1][8];
     const int t = threadIdx.x, chunk = red_chunk(N, part ? 1 : 0);
     const int lo = blockIdx.x * chunk, hi = min(N, lo + chunk);
     double k[1] = {0.0};
@@ -2284,7 +2389,7 @@ __global__ void __launch_bounds__(256) k_nvt_thermostat(int N, const double *V, 
     }
     block_tree<1>(red, k, t);
     double tot[1];
-    if (last_cta<1>(red, part, ticket, tot, t)) {
+    if (last_cta<1>(red, part, ticket, tot, t) && t == 0) {
         double K = 0.5 * tot[0];
         double fs = 1.0 / (tau * tau) * (2.0 * K / ((3.0 * (double)N) * T) - 1.0);
         const int step = (int)out[10];
@@ -2360,8 +2465,18 @@ extern "C" size_t mbk_efs_smem(const mb_model *m, int capNB, int shape) {
 }
 
 extern "C" int mbk_wrap(mb_dev *d, int N, const mb_cell *c, void *stream, long *launches) {
+    d->f_clear = 0;
     if (c->ND <= 0 || N <= 0) return 0;
-    k_wrap<<<(N + 127) / 128, 128, 0, (cudaStream_t)stream>>>(N, d->X, *c, d->status);
+    k_wrap<<<(N + 127) / 128, 128, 0, (cudaStream_t)stream>>>(N, d->X, *c, d->status, d->F);
+    d->f_clear = 1;
+    (*launches)++;
+    return (int)cudaGetLastError();
+}
+
+extern "C" int mbk_intake(mb_dev *d, int N, const mb_cell *c, const double *hx, const int *hspc, void *stream,
+                          long *launches) {
+    k_intake<<<(N + 127) / 128, 128, 0, (cudaStream_t)stream>>>(N, hx, *c, hspc, d->X, d->spc, d->status, d->F);
+    d->f_clear = 1;
     (*launches)++;
     return (int)cudaGetLastError();
 }
@@ -2384,7 +2499,8 @@ extern "C" int mbk_nlist(mb_dev *d, int N, int NM, const mb_cell *c, double rc, 
                                                               (double4 *)d->nd, d->status);
         *launches += 5;
     } else {
-        k_nlist_brute<<<blocks, warps_per_block * 32, 0, st>>>(N, NM, d->capNB, d->X, *c, rc2, d->nn, d->nj,
+        /* a warp a CTA: few atoms, as many SMs as there are */
+        k_nlist_brute<<<N, 32, 0, st>>>(N, NM, d->capNB, d->X, *c, rc2, d->nn, d->nj,
                                                                (double4 *)d->nd, d->status);
         *launches += 1;
     }
@@ -2510,9 +2626,10 @@ static int tune_key(const mb_dev *d, int N, int mode) {
     return (mode << 28) | ((d->tri_on ? 1 : 0) << 26) | (bucket << 20) | (d->capNB & 0xfffff);
 }
 
-/* Decision for a pass that may run on k_efs_tri: its shapes and those of
- * k_efs are each timed once (after an untimed launch) and the fastest kept,
- * 16 + shape for k_efs_tri, shape for k_efs. */
+/* Decision for a pass that may run on k_efs_tri: its shapes are each timed
+ * once (after an untimed launch) and the fastest kept, as 16 + shape.  k_efs,
+ * slower at every size measured (32 atoms: 73 us against 40; 487: 199 against
+ * 64; 4000: 890 against 375), stands by for shapes that do not fit. */
 static int tune_family(mb_dev *d, const mb_model *m, int N, int mode, const TriArgs &la, const EfsArgs &a,
                        cudaStream_t st) {
     const int key = tune_key(d, N, mode);
@@ -2533,6 +2650,7 @@ static int tune_family(mb_dev *d, const mb_model *m, int N, int mode, const TriA
         float best_ms = 1e30f;
         for (int c = 0; c < MB_NTRISHAPES + MB_NSHAPES; c++) {
             const bool tri = c < MB_NTRISHAPES;
+            if (!tri && best_ms < 1e30f) break;
             const int sh = tri ? c : c - MB_NTRISHAPES;
             const size_t need = tri ? tri_group_bytes(m, la.cap, kTriShapes[sh].wpa) * kTriShapes[sh].apb + TRI_STATIC_SMEM
                                     : group_bytes(m, a.cap, kShapes[sh].wpa) * kShapes[sh].apb + EFS_STATIC_SMEM;
@@ -2629,7 +2747,6 @@ extern "C" int mbk_descriptor_pass(mb_dev *d, const mb_model *m, int N, int mode
     a.vir = d->vir;
     a.counters = d->counters;
     a.smem_group = 0;
-    cudaMemsetAsync(d->EU, 0, sizeof(double) * N, st);
     int fam = -1; /* k_efs shape chosen against k_efs_tri */
     if (d->tri_on) {
         TriArgs la;
@@ -2653,7 +2770,8 @@ extern "C" int mbk_descriptor_pass(mb_dev *d, const mb_model *m, int N, int mode
         la.smem_group = 0;
         la.P = m->P;
         la.T = m->T;
-        const int v = tune_family(d, m, N, mode, la, a, st);
+        const int tuned = d->tune_n, v = tune_family(d, m, N, mode, la, a, st);
+        if (d->tune_n != tuned) d->f_clear = 0; /* trial launches added to F */
         if (v >= 16) {
             d->last_shape = v;
             cudaEvent_t e0 = 0, e1 = 0;
@@ -2662,13 +2780,17 @@ extern "C" int mbk_descriptor_pass(mb_dev *d, const mb_model *m, int N, int mode
                 e1 = ((cudaEvent_t *)d->ev_pool)[2 * d->ev_n + 1];
                 d->ev_n++;
             }
-            if (mode == MB_MODE_EFS || mode == MB_MODE_VJP) cudaMemsetAsync(d->F, 0, sizeof(double) * 3 * N, st);
+            if ((mode == MB_MODE_EFS || mode == MB_MODE_VJP) && !d->f_clear)
+                cudaMemsetAsync(d->F, 0, sizeof(double) * 3 * N, st);
+            d->f_clear = 0;
             const int rc = launch_tri_pass(m, v - 16, la, st, e0, e1);
             (*launches)++;
             return rc;
         }
         fam = v;
     }
+    d->f_clear = 0;
+    cudaMemsetAsync(d->EU, 0, sizeof(double) * N, st);
     int shape = fam >= 0 ? fam : tune_shape(d, m, N, mode, a, st);
     d->last_shape = shape;
     cudaEvent_t e0 = 0, e1 = 0;
@@ -2711,10 +2833,13 @@ extern "C" int mbk_jvp(mb_dev *d, const mb_model *m, int N, const double *dx, co
     return (int)cudaGetLastError();
 }
 
-extern "C" int mbk_finalize(mb_dev *d, int N, int mode, double pV, void *stream, long *launches) {
+extern "C" int mbk_finalize(mb_dev *d, int N, int mode, double pV, const mb_host_out *host, void *stream,
+                            long *launches) {
     const int chunk = red_chunk(N, d->part ? 1 : 0), nb = (N + chunk - 1) / chunk;
+    HostOut ho = {nullptr, nullptr, nullptr, nullptr, nullptr};
+    if (host) ho = {host->out, host->status, mode == MB_MODE_ENERGY ? nullptr : host->F, host->X, host->EA};
     k_finalize<<<nb > 0 ? nb : 1, 256, 0, (cudaStream_t)stream>>>(N, mode, pV, d->EA, d->EU, d->vir, d->F, d->out,
-                                                                   d->part, d->ticket);
+                                                                   d->part, d->ticket, d->X, d->status, ho);
     (*launches)++;
     return (int)cudaGetLastError();
 }
@@ -2779,6 +2904,7 @@ struct CellArg {
 
 static const CellArg kCellArgs[] = {
     {(const void *)k_wrap, karity(k_wrap), 2},
+    {(const void *)k_intake, karity(k_intake), 2},
     {(const void *)k_cell_bin, karity(k_cell_bin), 2},
     {(const void *)k_nlist_cell, karity(k_nlist_cell), 4},
     {(const void *)k_nlist_brute, karity(k_nlist_brute), 4},

@@ -129,7 +129,7 @@ extern "C" int mb_efs_noalloc(mb_potential *pot, int N, int NM, int ND, const do
         !(r = mbk_nlist(&d, N, NM, &c, m->rc_list, st, &launches)) && (stage = "descriptor kernel") &&
         !(r = mbk_descriptor_pass(&d, m, N, MB_MODE_EFS, urep > 0.0 ? urep : 0.0, 0, 0, st, &launches)) &&
         (stage = "finalize"))
-        r = mbk_finalize(&d, N, MB_MODE_EFS, pV, st, &launches);
+        r = mbk_finalize(&d, N, MB_MODE_EFS, pV, nullptr, st, &launches);
     if (r) {
         static char msg[160];
         snprintf(msg, sizeof(msg), "%s: %s", stage, cudaGetErrorString((cudaError_t)r));

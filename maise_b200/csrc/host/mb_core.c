@@ -39,7 +39,8 @@ typedef struct {
     long gen;
     int N, NM, ND, mode, M[3], tri;
     double urep;
-    void *h_res;
+    void *h_res, *h_buf;
+    int intake;
 } pass_key;
 
 #define MB_PASS_NODES 8
@@ -86,9 +87,9 @@ struct mb_potential {
      * at each call's cell; results staged in pinned h_res */
     pass_graph pgs[4];
     int pbroken;
-    double *h_res; /* F[3N] then X[3N] of the last graphed pass */
+    double *h_res; /* F[3N], X[3N], EA[N] of the last pass on host arrays, stored by its last kernel */
     size_t h_res_len;
-    int res_staged;
+    int intake; /* positions and species wait in h_buf for the pass's first kernel */
     /* timings moved out of the event pools (graph replays reuse the events) */
     double st_acc_ms, ev_acc_ms;
     int st_acc_n, ev_acc_n;
@@ -477,6 +478,7 @@ static int host_buf(mb_potential *p, size_t n) {
     if (n <= p->h_buf_len) return MB_OK;
     cudaFreeHost(p->h_buf);
     p->h_buf = NULL;
+    p->h_buf_len = 0;
     CK(cudaMallocHost((void **)&p->h_buf, sizeof(double) * n), "cudaMallocHost");
     p->h_buf_len = n;
     return MB_OK;
@@ -571,7 +573,8 @@ static void frac_to_cart(int N, const double *xf, const double *L, double *x) {
 /* the E / E+F+S sequence                                              */
 /* ------------------------------------------------------------------ */
 
-static int upload(mb_potential *p, int N, int XT, const int *atmn, const double *lat9, const double *x) {
+/* check the species and lay positions (Cartesian) and species out in pinned h_buf */
+static int stage(mb_potential *p, int N, int XT, const int *atmn, const double *lat9, const double *x) {
     int r, s;
     double *hx;
     for (s = 0; s < N; s++)
@@ -583,6 +586,15 @@ static int upload(mb_potential *p, int N, int XT, const int *atmn, const double 
     else
         memcpy(hx, x, sizeof(double) * 3 * N);
     memcpy((int *)(hx + 3 * N), atmn, sizeof(int) * N);
+    return MB_OK;
+}
+
+/* stage() and the copies to the device */
+static int upload(mb_potential *p, int N, int XT, const int *atmn, const double *lat9, const double *x) {
+    const double *hx;
+    int r;
+    if ((r = stage(p, N, XT, atmn, lat9, x))) return r;
+    hx = p->h_buf;
     CK(cudaMemcpyAsync(p->d.X, hx, sizeof(double) * 3 * N, cudaMemcpyHostToDevice, p->stream), "H2D positions");
     CK(cudaMemcpyAsync(p->d.spc, hx + 3 * N, sizeof(int) * N, cudaMemcpyHostToDevice, p->stream), "H2D species");
     return MB_OK;
@@ -594,27 +606,27 @@ static int upload(mb_potential *p, int N, int XT, const int *atmn, const double 
  * grow: the positions were already wrapped in place, so the caller
  * re-uploads them and calls again. */
 #define MB_RETRY 1000
-/* the device part of one pass, queued on the handle's stream: wrap, list,
- * descriptor pass, finalize, then the status word and E, H, U to the host
- * (and, with stage set, F and the wrapped X into the pinned h_res) */
-static int enqueue_pass(mb_potential *p, int N, int NM, const mb_cell *c, double pV, int mode, double urep,
-                        int stage) {
+/* the device part of one pass, queued on the handle's stream: intake (host
+ * arrays) or wrap, list, descriptor pass and finalize, which leaves the status
+ * word, E, H, U, F, the wrapped X and the atom energies in pinned memory */
+static int enqueue_pass(mb_potential *p, int N, int NM, const mb_cell *c, double pV, int mode, double urep) {
+    const mb_host_out ho = {p->h_out, p->h_status, p->h_res, p->h_res + 3 * N, p->h_res + 6 * N};
     int r;
     CK(cudaMemsetAsync(p->d.status, 0, sizeof(int) * 4, p->stream), "memset status");
-    if ((r = mbk_wrap(&p->d, N, c, p->stream, &p->launches))) return cuda_fail((cudaError_t)r, "wrap");
+    if (p->intake)
+        r = mbk_intake(&p->d, N, c, p->h_buf, (const int *)(p->h_buf + 3 * N), p->stream, &p->launches);
+    else
+        r = mbk_wrap(&p->d, N, c, p->stream, &p->launches);
+    if (r) return cuda_fail((cudaError_t)r, "wrap");
     if ((r = mbk_nlist(&p->d, N, NM, c, p->m.rc_list, p->stream, &p->launches)))
         return cuda_fail((cudaError_t)r, "neighbour list");
     if ((r = mbk_descriptor_pass(&p->d, &p->m, N, mode, urep, 0, 0, p->stream, &p->launches)))
         return cuda_fail((cudaError_t)r, "descriptor kernel");
-    if (mode != MB_MODE_DESCRIPTORS)
-        if ((r = mbk_finalize(&p->d, N, mode, pV, p->stream, &p->launches))) return cuda_fail((cudaError_t)r, "finalize");
-    CK(cudaMemcpyAsync(p->h_status, p->d.status, sizeof(int) * 4, cudaMemcpyDeviceToHost, p->stream), "D2H status");
-    CK(cudaMemcpyAsync(p->h_out, p->d.out, sizeof(double) * 16, cudaMemcpyDeviceToHost, p->stream), "D2H out");
-    if (stage) {
-        if (mode == MB_MODE_EFS || mode == MB_MODE_VJP)
-            CK(cudaMemcpyAsync(p->h_res, p->d.F, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, p->stream), "D2H F");
-        CK(cudaMemcpyAsync(p->h_res + 3 * N, p->d.X, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, p->stream),
-           "D2H X");
+    if (mode != MB_MODE_DESCRIPTORS) {
+        if ((r = mbk_finalize(&p->d, N, mode, pV, &ho, p->stream, &p->launches)))
+            return cuda_fail((cudaError_t)r, "finalize");
+    } else {
+        CK(cudaMemcpyAsync(p->h_status, p->d.status, sizeof(int) * 4, cudaMemcpyDeviceToHost, p->stream), "D2H status");
     }
     return MB_OK;
 }
@@ -634,15 +646,7 @@ static void drop_pass_graph(pass_graph *q) {
 static int graph_pass(mb_potential *p, int N, int NM, int ND, const mb_cell *c, double pV, int mode, double urep) {
     pass_key k;
     pass_graph *q = &p->pgs[mode & 3];
-    int r, m;
-    if (6 * (size_t)N > p->h_res_len) {
-        for (m = 0; m < 4; m++) drop_pass_graph(&p->pgs[m]);
-        cudaFreeHost(p->h_res);
-        p->h_res = NULL;
-        p->h_res_len = 0;
-        CK(cudaMallocHost((void **)&p->h_res, sizeof(double) * 6 * N), "cudaMallocHost");
-        p->h_res_len = 6 * (size_t)N;
-    }
+    int r;
     memset(&k, 0, sizeof(k));
     k.gen = p->gen;
     k.N = N;
@@ -654,6 +658,8 @@ static int graph_pass(mb_potential *p, int N, int NM, int ND, const mb_cell *c, 
     k.M[2] = c->M[2];
     k.urep = urep;
     k.h_res = p->h_res;
+    k.h_buf = p->h_buf;
+    k.intake = p->intake;
     k.tri = p->d.tri_on;
     if (!q->x || memcmp(&k, &q->k, sizeof(k))) {
         cudaGraph_t g = NULL;
@@ -666,10 +672,10 @@ static int graph_pass(mb_potential *p, int N, int NM, int ND, const mb_cell *c, 
         }
         cudaError_t e;
         const long l0 = p->launches;
-        const int expect = (ND > 0) + (c->M[0] > 0 ? 2 : 1) + (mode != MB_MODE_DESCRIPTORS);
+        const int expect = (p->intake || ND > 0) + (c->M[0] > 0 ? 2 : 1) + (mode != MB_MODE_DESCRIPTORS);
         drop_pass_graph(q);
         CK(cudaStreamBeginCapture(p->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
-        r = enqueue_pass(p, N, NM, c, pV, mode, urep, 1);
+        r = enqueue_pass(p, N, NM, c, pV, mode, urep);
         e = cudaStreamEndCapture(p->stream, &g);
         if (r) {
             if (g) cudaGraphDestroy(g);
@@ -703,7 +709,6 @@ static int graph_pass(mb_potential *p, int N, int NM, int ND, const mb_cell *c, 
     }
     CK(cudaGraphLaunch(q->x, p->stream), "graph launch");
     p->launches += q->launches;
-    p->res_staged = 1;
     return MB_OK;
 }
 
@@ -716,13 +721,20 @@ static int run_pass(mb_potential *p, int N, int NM, int ND, const double *lat9, 
     ncell = c.M[0] ? c.M[0] * c.M[1] * c.M[2] : 1;
     if ((r = ensure(p, N, p->d.capNB ? p->d.capNB : (NM < 64 ? NM : 64), ncell))) return r;
     p->d.tri_on = p->tri_enabled && mbk_tri_usable(&p->d, &p->m);
-    p->res_staged = 0;
+    if (7 * (size_t)N > p->h_res_len) {
+        cudaFreeHost(p->h_res);
+        p->h_res = NULL;
+        p->h_res_len = 0;
+        CK(cudaMallocHost((void **)&p->h_res, sizeof(double) * 7 * N), "cudaMallocHost");
+        p->h_res_len = 7 * (size_t)N;
+    }
     r = MB_FALLBACK;
     if (p->use_graphs && !p->pbroken && !p->d.ev_on && mbk_shape_ready(&p->d, N, mode)) {
         r = graph_pass(p, N, NM, ND, &c, pV, mode, urep);
         if (r != MB_OK && r != MB_FALLBACK) return r;
     }
-    if (r == MB_FALLBACK && (r = enqueue_pass(p, N, NM, &c, pV, mode, urep, 0))) return r;
+    if (r == MB_FALLBACK && (r = enqueue_pass(p, N, NM, &c, pV, mode, urep))) return r;
+    p->intake = 0;
     CK(cudaStreamSynchronize(p->stream), "synchronize");
     if (p->h_status[0] & MB_ST_WRAP) return fail(MB_ERR_STATE, "non-finite or runaway positions");
     if (p->h_status[0] & MB_ST_NBR_OVERFLOW)
@@ -743,9 +755,13 @@ static int host_pass(mb_potential *p, int N, int NM, int ND, int XT, const int *
     CK(cudaSetDevice(p->device), "cudaSetDevice");
     if ((r = ensure(p, N, p->d.capNB ? p->d.capNB : (NM < 64 ? NM : 64), 1))) return r;
     for (tries = 0; tries < 3; tries++) {
-        if ((r = upload(p, N, XT, atmn, lat9, x))) return r;
+        if ((r = stage(p, N, XT, atmn, lat9, x))) return r;
+        p->intake = 1;
         r = run_pass(p, N, NM, ND, lat9, mode, urep, p_gpa);
-        if (r != MB_RETRY) return r;
+        if (r != MB_RETRY) {
+            p->intake = 0;
+            return r;
+        }
     }
     return fail(MB_ERR_CAPACITY, "neighbour capacity could not be established");
 }
@@ -758,18 +774,10 @@ int mb_efs(mb_potential *p, int N, int NM, int ND, int XT, const int *atmn, cons
     if (E) *E = p->h_out[0];
     if (str)
         for (k = 0; k < 6; k++) str[k] = p->h_out[2 + k];
-    if (p->res_staged) {
-        /* the replayed pass left F and the wrapped X in pinned staging */
-        if (frc) memcpy(frc, p->h_res, sizeof(double) * 3 * N);
-        if (x_wrapped) memcpy(x_wrapped, p->h_res + 3 * N, sizeof(double) * 3 * N);
-        if (!ea) return MB_OK;
-    } else {
-        if (frc) CK(cudaMemcpyAsync(frc, p->d.F, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, p->stream), "D2H forces");
-        if (x_wrapped)
-            CK(cudaMemcpyAsync(x_wrapped, p->d.X, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, p->stream), "D2H X");
-    }
-    if (ea) CK(cudaMemcpyAsync(ea, p->d.EA, sizeof(double) * N, cudaMemcpyDeviceToHost, p->stream), "D2H EA");
-    CK(cudaStreamSynchronize(p->stream), "synchronize");
+    /* the pass left F, the wrapped X and the atom energies in pinned memory */
+    if (frc) memcpy(frc, p->h_res, sizeof(double) * 3 * N);
+    if (x_wrapped) memcpy(x_wrapped, p->h_res + 3 * N, sizeof(double) * 3 * N);
+    if (ea) memcpy(ea, p->h_res + 6 * N, sizeof(double) * N);
     return MB_OK;
 }
 
@@ -779,10 +787,7 @@ int mb_energy(mb_potential *p, int N, int NM, int ND, int XT, const int *atmn, c
     if (r) return r;
     if (H) *H = p->h_out[1];
     if (E) *E = p->h_out[0];
-    if (ea) {
-        CK(cudaMemcpyAsync(ea, p->d.EA, sizeof(double) * N, cudaMemcpyDeviceToHost, p->stream), "D2H EA");
-        CK(cudaStreamSynchronize(p->stream), "synchronize");
-    }
+    if (ea) memcpy(ea, p->h_res + 6 * N, sizeof(double) * N);
     return MB_OK;
 }
 
@@ -808,8 +813,7 @@ int mb_descriptor_vjp(mb_potential *p, int N, int NM, int ND, int XT, const int 
     if (r) return r;
     if (str)
         for (k = 0; k < 6; k++) str[k] = p->h_out[2 + k];
-    if (frc) CK(cudaMemcpyAsync(frc, p->d.F, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, p->stream), "D2H forces");
-    CK(cudaStreamSynchronize(p->stream), "synchronize");
+    if (frc) memcpy(frc, p->h_res, sizeof(double) * 3 * N);
     return MB_OK;
 }
 
@@ -989,10 +993,7 @@ static double relax_eval(relax_ctx *r, double *x, double *g) {
     if (!g) {
         rc = mb_energy(r->p, r->N, r->NM, r->ND, 1, r->atmn, r->L, r->xc, r->p_gpa, r->urep, &r->H, NULL, NULL);
         r->ne++;
-        if (!rc && r->p->res_staged)
-            memcpy(r->xc, r->p->h_res + 3 * r->N, sizeof(double) * 3 * r->N);
-        else if (!rc && cudaMemcpy(r->xc, r->p->d.X, sizeof(double) * 3 * r->N, cudaMemcpyDeviceToHost) != cudaSuccess)
-            rc = fail(MB_ERR_CUDA, "D2H positions");
+        if (!rc) memcpy(r->xc, r->p->h_res + 3 * r->N, sizeof(double) * 3 * r->N);
         if (rc) { r->err = rc; return NAN; }
     } else {
         double U[6], R[9], V = cell_volume(r->L);
@@ -1201,7 +1202,7 @@ static int md_step(mb_potential *p, int N, int NM, const mb_cell *c, double urep
         return cuda_fail((cudaError_t)r, "neighbour list");
     if ((r = mbk_descriptor_pass(&p->d, &p->m, N, MB_MODE_EFS, urep, 0, 0, p->stream, &p->launches)))
         return cuda_fail((cudaError_t)r, "descriptor kernel");
-    if ((r = mbk_finalize(&p->d, N, MB_MODE_EFS, 0.0, p->stream, &p->launches)))
+    if ((r = mbk_finalize(&p->d, N, MB_MODE_EFS, 0.0, NULL, p->stream, &p->launches)))
         return cuda_fail((cudaError_t)r, "finalize");
     if ((r = mbk_nvt_update(&p->d, &p->m, N, dt, tau, T / MB_KB_INV, c, p->stream, &p->launches)))
         return cuda_fail((cudaError_t)r, "integrator");

@@ -167,6 +167,7 @@ typedef struct {
     double *weights;
     double *tri_w;    /* first-layer weights by input (mb_tri); owned by the handle */
     int tri_on;       /* the next descriptor pass may run on k_efs_tri */
+    int f_clear;      /* F was cleared by the pass's first kernel */
     /* optional CUDA-event timing of the descriptor kernel */
     int ev_on, ev_n, ev_cap;
     void *ev_pool;    /* cudaEvent_t[2*ev_cap] */
@@ -196,7 +197,15 @@ int mbk_wrap(mb_dev *d, int N, const mb_cell *c, void *stream, long *launches);
 int mbk_nlist(mb_dev *d, int N, int NM, const mb_cell *c, double rc, void *stream, long *launches);
 int mbk_descriptor_pass(mb_dev *d, const mb_model *m, int N, int mode, double urep, int need_nb_max, int nb_max,
                         void *stream, long *launches);
-int mbk_finalize(mb_dev *d, int N, int mode, double pV, void *stream, long *launches);
+/* pinned host memory that receives a pass's results (any may be NULL): out[16], status[4], F[3N], X[3N], EA[N] */
+typedef struct {
+    double *out;
+    int *status;
+    double *F, *X, *EA;
+} mb_host_out;
+int mbk_finalize(mb_dev *d, int N, int mode, double pV, const mb_host_out *host, void *stream, long *launches);
+/* positions and species from pinned host memory, JAR, F cleared */
+int mbk_intake(mb_dev *d, int N, const mb_cell *c, const double *hx, const int *hspc, void *stream, long *launches);
 int mbk_jvp(mb_dev *d, const mb_model *m, int N, const double *dx, const double *eps, double *dG, void *stream,
             long *launches);
 /* thermostat and integrator, then JAR on the moved atoms (cell c; none when c->ND <= 0) */
