@@ -15,7 +15,8 @@ import ctypes
 
 import numpy as np
 
-from . import MaiseError, load_library, pack
+from . import MaiseError, load_library
+from . import pack as _pack
 
 _F = ctypes.POINTER(ctypes.c_float)
 _D = ctypes.POINTER(ctypes.c_double)
@@ -54,6 +55,13 @@ def _f32(a, n=None):
     if n is not None and a.size != n:
         raise ValueError(f"expected {n} values, got {a.size}")
     return a
+
+
+def pack(structures):
+    """(nat, atmn, lat, x) arrays of a list of dict(X, LAT, atmn): lat [S, 9],
+    x flat."""
+    nat, atmn, lat, x = _pack(structures)
+    return nat, atmn, lat.reshape(-1, 9), x.reshape(-1)
 
 
 class Surrogate:
