@@ -20,6 +20,7 @@
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdlib.h>
+#include <math.h>
 #include <math_constants.h>
 #include <stdint.h>
 
@@ -36,6 +37,9 @@ constexpr int BMAXNB = 96;
 constexpr int BMAXDOF = 3 * BMAXN + 9;
 constexpr int BMAXD = 288;
 constexpr int BTL = 1024;
+constexpr int BTL16 = 2 * BTL; /* entries of the same room as 16-bit pairs (atom_pass_tri) */
+constexpr int BTS = 20;        /* row stride of atom_pass_tri's 8 x 16 tiles */
+constexpr int BLOW = MB_TRI_LOW;
 /* warps per structure: 12 (one structure per SM) by default, 4 (three
  * structures per SM) on request.  Both hold the 12 warps per SM that 168
  * registers a thread allow; the wide CTA finishes each structure in about a
@@ -64,6 +68,14 @@ struct BParams {
     int w_off[MB_MAXSPC];
 };
 
+/* What atom_pass_tri reads per triplet, from the kernel-parameter space. */
+struct BTri {
+    float ke[8], eta[8]; /* exp(-eta rho) = 2^(ke rho) */
+    float iw, mh;        /* 1 / Rc^2 and -2 / Rc^2 */
+    float rc2;           /* triplet gate on the squared j-k distance */
+    float powz[4];       /* 2^(1 - zeta) */
+};
+
 struct BArgs {
     int S, rlxt, mitr;
     double p_ev, urep, fmax, sigma;
@@ -74,7 +86,6 @@ struct BArgs {
     /* optional: forces [3 * atoms] and virial U [6 * S] at each structure's
      * final state (FP32 evaluation, FP64 reductions); NULL to skip */
     double *fout, *uout;
-    const BParams *P;
     const float *W;
     int *queue;
     double *hmat;  /* per CTA: BMAXDOF^2 */
@@ -84,13 +95,23 @@ struct BArgs {
     /* work done (for the roofline): atom evaluations, neighbour pairs and
      * triplets of the forward pass; per-warp counts added at kernel exit */
     unsigned long long *work;
+    BTri T;
+    BParams P; /* by value: the triplet loops read it through the constant cache */
 };
 
 struct WarpWS {
     float4 d[BMAXNB];
     float ir[BMAXNB], fa[BMAXNB], fb[BMAXNB];
-    alignas(16) float P[BMAXNB * 8]; /* exp(-eta r^2) per neighbour, BNE used of 8 */
-    float Fnb[BMAXNB * 3];
+    union {
+        struct { /* atom_pass */
+            alignas(16) float P[BMAXNB * 8]; /* exp(-eta r^2) per neighbour, BNE used of 8 */
+            float Fnb[BMAXNB * 3];
+        };
+        struct { /* atom_pass_tri */
+            float4 F4[BMAXNB];
+            float tile[3 * 8 * BTS];
+        };
+    };
     alignas(16) float grid[BCELLS];
     float G[BMAXD];
     float h[4 * MB_MAXH];
@@ -279,12 +300,70 @@ __device__ __forceinline__ bool tgate(const BParams &P, const WarpWS &ws, int s0
     return fwd || rev;
 }
 
+/* MLP forward and dE/dG of atom i (src/nmlp.c:367-431): descriptors ws.G in,
+ * dE/dG out in their place */
+__device__ __forceinline__ void mlp_pass(const BArgs &A, const BParams &P, double *ea, WarpWS &ws, int i, int s0,
+                                         int lane) {
+    const int D = P.D;
+    const int h1 = P.h1, h2 = P.h2;
+    const float *net = A.W + P.w_off[s0];
+    const float *off = net, *W0 = off + D, *b0 = W0 + h1 * D, *W1 = b0 + h1, *b1 = W1 + h2 * h1, *W2 = b1 + h2,
+                *b2 = W2 + h2;
+    float *H1 = ws.h, *Dl1 = ws.h + 2 * MB_MAXH;
+    if (h1 <= 16) {
+        /* every hidden unit's partial sum in each lane, then one reduction */
+        float acc[16];
+#pragma unroll
+        for (int m = 0; m < 16; m++) acc[m] = 0.0f;
+        for (int l = lane; l < D; l += 32) {
+            const float x = ws.G[l] - off[l];
+#pragma unroll
+            for (int m = 0; m < 16; m++)
+                if (m < h1) acc[m] += x * W0[m * D + l];
+        }
+        const float tot = warp_reduce16f(acc, lane);
+        const int cell = (lane >> 1) & 15;
+        if (!(lane & 1) && cell < h1) H1[cell] = tanhf(b0[cell] + tot);
+    } else {
+        for (int m = 0; m < h1; m++) {
+            float acc = 0.0f;
+            for (int l = lane; l < D; l += 32) acc += (ws.G[l] - off[l]) * W0[m * D + l];
+            acc = bsumf(acc);
+            if (lane == 0) H1[m] = tanhf(b0[m] + acc);
+        }
+    }
+    __syncwarp();
+    float v = 0.0f;
+    if (lane < h2) {
+        v = b1[lane];
+        for (int k = 0; k < h1; k++) v += H1[k] * W1[lane * h1 + k];
+        v = tanhf(v);
+    }
+    float e = lane < h2 ? v * W2[lane] : 0.0f;
+    e = bsumf(e);
+    if (lane == 0) ea[i] = (double)b2[0] + (double)e;
+    float dl2 = lane < h2 ? W2[lane] * (1.0f - v * v) : 0.0f;
+    float dl1 = 0.0f;
+    for (int m = 0; m < h2; m++) {
+        float t = __shfl_sync(FULLM, dl2, m);
+        if (lane < h1) dl1 += t * W1[m * h1 + lane];
+    }
+    if (lane < h1) Dl1[lane] = dl1 * (1.0f - H1[lane] * H1[lane]);
+    __syncwarp();
+    for (int l = lane; l < D; l += 32) {
+        float g = 0.0f;
+        for (int k = 0; k < h1; k++) g += Dl1[k] * W0[k * D + l];
+        ws.G[l] = g;
+    }
+    __syncwarp();
+}
+
 /* ---------------- one atom: descriptors, MLP, reverse pass (FP32) ---------------- */
 
 template <int W>
 __device__ void atom_pass(const BArgs &A, BShared<W> &sh, WarpWS &ws, int i, const float4 *nbd, const int *nbj,
-                          double *virw) {
-    const BParams &P = *A.P;
+                          double *vr) {
+    const BParams &P = A.P;
     const int lane = threadIdx.x & 31;
     const int n = sh.nn[i], s0 = sh.spc[i], ns = P.nspc, D = P.D, ng2 = P.ng2;
     if (lane == 0) {
@@ -486,58 +565,7 @@ __device__ void atom_pass(const BArgs &A, BShared<W> &sh, WarpWS &ws, int i, con
             __syncwarp();
         }
 
-    /* MLP forward and dE/dG (src/nmlp.c:367-431) */
-    const int h1 = P.h1, h2 = P.h2;
-    const float *net = A.W + P.w_off[s0];
-    const float *off = net, *W0 = off + D, *b0 = W0 + h1 * D, *W1 = b0 + h1, *b1 = W1 + h2 * h1, *W2 = b1 + h2,
-                *b2 = W2 + h2;
-    float *H1 = ws.h, *Dl1 = ws.h + 2 * MB_MAXH;
-    if (h1 <= 16) {
-        /* every hidden unit's partial sum in each lane, then one reduction */
-        float acc[16];
-#pragma unroll
-        for (int m = 0; m < 16; m++) acc[m] = 0.0f;
-        for (int l = lane; l < D; l += 32) {
-            const float x = ws.G[l] - off[l];
-#pragma unroll
-            for (int m = 0; m < 16; m++)
-                if (m < h1) acc[m] += x * W0[m * D + l];
-        }
-        const float tot = warp_reduce16f(acc, lane);
-        const int cell = (lane >> 1) & 15;
-        if (!(lane & 1) && cell < h1) H1[cell] = tanhf(b0[cell] + tot);
-    } else {
-        for (int m = 0; m < h1; m++) {
-            float acc = 0.0f;
-            for (int l = lane; l < D; l += 32) acc += (ws.G[l] - off[l]) * W0[m * D + l];
-            acc = bsumf(acc);
-            if (lane == 0) H1[m] = tanhf(b0[m] + acc);
-        }
-    }
-    __syncwarp();
-    float v = 0.0f;
-    if (lane < h2) {
-        v = b1[lane];
-        for (int k = 0; k < h1; k++) v += H1[k] * W1[lane * h1 + k];
-        v = tanhf(v);
-    }
-    float e = lane < h2 ? v * W2[lane] : 0.0f;
-    e = bsumf(e);
-    if (lane == 0) sh.ea[i] = (double)b2[0] + (double)e;
-    float dl2 = lane < h2 ? W2[lane] * (1.0f - v * v) : 0.0f;
-    float dl1 = 0.0f;
-    for (int m = 0; m < h2; m++) {
-        float t = __shfl_sync(FULLM, dl2, m);
-        if (lane < h1) dl1 += t * W1[m * h1 + lane];
-    }
-    if (lane < h1) Dl1[lane] = dl1 * (1.0f - H1[lane] * H1[lane]);
-    __syncwarp();
-    for (int l = lane; l < D; l += 32) {
-        float g = 0.0f;
-        for (int k = 0; k < h1; k++) g += Dl1[k] * W0[k * D + l];
-        ws.G[l] = g;
-    }
-    __syncwarp();
+    mlp_pass(A, P, sh.ea, ws, i, s0, lane);
 
     /* reverse pairs (species-0 derivative parameters) */
     float fi0 = 0.0f, fi1 = 0.0f, fi2 = 0.0f;
@@ -545,7 +573,6 @@ __device__ void atom_pass(const BArgs &A, BShared<W> &sh, WarpWS &ws, int i, con
      * force array: at short distances it is the largest term (hundreds of
      * eV/A) and an FP32 sum of it would carry most of the rounding */
     double fu0 = 0.0, fu1 = 0.0, fu2 = 0.0;
-    double vr[6] = {0, 0, 0, 0, 0, 0};
     for (int t = lane; t < n; t += 32) {
         float4 d = ws.d[t];
         float r = d.w, ir = ws.ir[t];
@@ -732,8 +759,433 @@ __device__ void atom_pass(const BArgs &A, BShared<W> &sh, WarpWS &ws, int i, con
         atomicAdd(&sh.F[3 * j + 1], (double)ws.Fnb[3 * t + 1]);
         atomicAdd(&sh.F[3 * j + 2], (double)ws.Fnb[3 * t + 2]);
     }
+    __syncwarp();
+}
+
+/* ---------------- the same for the reference bases ---------------- */
+
+/* (1 + lambda c)^zeta for zeta = 1, 2, 4, 16 and lambda = -1, +1 (index
+ * 2 z + l) without the 2^(1 - zeta), and the derivatives in c */
+__device__ __forceinline__ void angular_std(float c, float *lz, float *lzp) {
 #pragma unroll
-    for (int k = 0; k < 6; k++) virw[k] += bsum(vr[k]);
+    for (int l = 0; l < 2; l++) {
+        const float lam = l ? 1.0f : -1.0f, b1 = 1.0f + lam * c, b2 = b1 * b1, b4 = b2 * b2, b8 = b4 * b4;
+        lz[l] = b1;
+        lz[2 + l] = b2;
+        lz[4 + l] = b4;
+        lz[6 + l] = b8 * b8;
+        if (lzp) {
+            const float b3 = b1 * b2;
+            lzp[l] = lam;
+            lzp[2 + l] = 2.0f * lam * b1;
+            lzp[4 + l] = 4.0f * lam * b3;
+            lzp[6 + l] = 16.0f * lam * (b4 * b8) * b3;
+        }
+    }
+}
+
+__device__ __forceinline__ float ex2f(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+/* The cutoff in w = 1 - r^2 / Rc^2: f = cos^2(pi r / 2 Rc) has a double zero
+ * at w = 0, so f = w^2 q(w) and f'(r) / r = -(2 / Rc^2) w g(w) with q and g
+ * smooth and positive on [0, 1]: interpolated at 6 Chebyshev nodes, relative
+ * errors 1.4e-9 and 5.7e-9.  No square root, division or trigonometry, and
+ * accurate relative to f up to the cutoff. */
+__device__ __forceinline__ float cut_f(float w) {
+    float q = 4.25195744e-05f;
+    q = fmaf(q, w, 6.47454464e-04f);
+    q = fmaf(q, w, 8.10431821e-03f);
+    q = fmaf(q, w, 6.59302329e-02f);
+    q = fmaf(q, w, 3.08425200e-01f);
+    q = fmaf(q, w, 6.16850274e-01f);
+    return w * w * q;
+}
+__device__ __forceinline__ float cut_g(float w) {
+    float g = 3.03081031e-04f;
+    g = fmaf(g, w, 3.87248896e-03f);
+    g = fmaf(g, w, 4.05310985e-02f);
+    g = fmaf(g, w, 2.63717965e-01f);
+    g = fmaf(g, w, 9.25275916e-01f);
+    g = fmaf(g, w, 1.23370054e+00f);
+    return w * g;
+}
+
+/* Append the pairs a < b of species block (al, be) whose j-k distance is in
+ * reach to the warp's list, as a | b << 8: stripes of 8 rows (a >> 3) and
+ * groups of 4 columns (b >> 2), a candidate per lane, accepted pairs column by
+ * column.  (st, g) is where to go on (g < 0: at the stripe's first group);
+ * returns false when the list is full before the block's end. */
+__device__ __forceinline__ bool fill_stripes(WarpWS &ws, float rc2, int oa, int ea, int ob, int eb, int &st, int &g,
+                                             int &pos, int lane) {
+    unsigned short *tl = reinterpret_cast<unsigned short *>(ws.tl);
+    const unsigned below = (1u << lane) - 1u;
+    if (ea <= oa) return true;
+    for (; 8 * st < ea; st++, g = -1) {
+        const int a = 8 * st + (lane & 7); /* below BMAXNB, a multiple of 8, as b is */
+        const float4 da = ws.d[a];
+        const int lo = a >= oa && a < ea ? max(ob, a + 1) : 0x7fffffff;
+        if (g < 0) g = max(ob, max(oa, 8 * st) + 1) >> 2;
+        for (; 4 * g < eb; g++) {
+            if (pos + 32 > BTL16) return false;
+            const int b = 4 * g + (lane >> 3);
+            const float4 db = ws.d[b];
+            const float dx = da.x - db.x, dy = da.y - db.y, dz = da.z - db.z;
+            const bool ok = dx * dx + dy * dy + dz * dz < rc2 && b >= lo && b < eb;
+            const unsigned m = __ballot_sync(FULLM, ok);
+            if (ok) tl[pos + __popc(m & below)] = (unsigned short)(a | b << 8);
+            pos += __popc(m);
+        }
+    }
+    return true;
+}
+
+/* atom_pass for the bases that k_efs_tri takes in its straight-line form
+ * (one cutoff, one set of G4 exponents, zeta 1, 2, 4, 16, lambda -1, +1; see
+ * mb_tri), where a triplet needs no table: all exponentials are 2^(ke rho) of
+ * rho = r_ij^2 + r_ik^2 + r_jk^2 and the cutoff is a polynomial in r^2.
+ *
+ * What bounds it: instruction issue and latency at 12 warps per SM.  Against
+ * atom_pass the triplet loops lose the square root, divisions, cosines, range
+ * reductions and table reads; the list needs no index inversion; and the
+ * reverse pass sums runs of entries as 8 x 16 tiles instead of a segmented
+ * warp sum and six shared FP32 atomics (compare-and-swap loops) per triplet.
+ * E/F/S of 256 Mg-Ca structures of 8 to 64 atoms: a call 1.08 -> 0.82 ms, error
+ * against 64 bits unchanged (3.1e-7). */
+template <int W>
+__device__ void atom_pass_tri(const BArgs &A, BShared<W> &sh, WarpWS &ws, int i, const float4 *nbd, const int *nbj,
+                              double *vr) {
+    const BParams &P = A.P;
+    const int lane = threadIdx.x & 31;
+    const int n = sh.nn[i], s0 = sh.spc[i], ns = P.nspc, D = P.D, ng2 = P.ng2;
+    const unsigned below = (1u << lane) - 1u;
+    if (lane == 0) {
+        ws.work[0] += 1ull;
+        ws.work[1] += (unsigned long long)n;
+    }
+    /* ---- neighbours stably sorted by relative species ---- */
+    int cnt[3] = {0, 0, 0};
+    int rv[BMAXNB / 32], jv[BMAXNB / 32];
+#pragma unroll
+    for (int q = 0; q < BMAXNB / 32; q++) {
+        const int t = 32 * q + lane;
+        jv[q] = t < n ? nbj[i * BMAXNB + t] : 0;
+        int d = t < n ? sh.spc[jv[q]] - s0 : -64;
+        rv[q] = d < 0 ? d + ns : d; /* negative past the end */
+#pragma unroll
+        for (int v = 0; v < 3; v++) cnt[v] += __popc(__ballot_sync(FULLM, rv[q] == v));
+    }
+    for (int t = lane; t < D; t += 32) ws.G[t] = 0.0f;
+    const int o1 = cnt[0], o2 = cnt[0] + cnt[1]; /* where relative species 1 and 2 begin */
+    {
+        int run[3] = {0, o1, o2};
+#pragma unroll
+        for (int q = 0; q < BMAXNB / 32; q++) {
+            const int t = 32 * q + lane;
+            int dst = 0;
+#pragma unroll
+            for (int v = 0; v < 3; v++) {
+                const unsigned m = __ballot_sync(FULLM, rv[q] == v);
+                if (rv[q] == v) dst = run[v] + __popc(m & below);
+                run[v] += __popc(m);
+            }
+            if (t < n) {
+                const float4 dv = nbd[i * BMAXNB + t];
+                const float w = fmaf(-dv.w * dv.w, A.T.iw, 1.0f);
+                ws.d[dst] = dv;
+                ws.ir[dst] = 1.0f / dv.w;
+                ws.fa[dst] = cut_f(w);
+                ws.fb[dst] = A.T.mh * cut_g(w);
+                ws.j[dst] = jv[q];
+            }
+        }
+    }
+    __syncwarp();
+    auto seg = [&](int v) { return v == 0 ? 0 : v == 1 ? o1 : v == 2 ? o2 : n; };
+    auto species = [&](int v) { return s0 + v >= ns ? s0 + v - ns : s0 + v; };
+
+    /* ---- G2: lane = (neighbour mod 4, function mod 8) ---- */
+    for (int f0 = 0; f0 < ng2; f0 += 8)
+        for (int v = 0; v < ns; v++) {
+            const int f = f0 + (lane & 7), sj = species(v), p = s0 * s0 + sj * sj;
+            float acc = 0.0f;
+            if (f < ng2) {
+                const float rs = P.f_rs[p][f], eta = P.f_eta2[p][f];
+                for (int t = seg(v) + (lane >> 3); t < seg(v + 1); t += 4) {
+                    const float x = ws.d[t].w - rs;
+                    acc += ws.fa[t] * expf(-eta * (x * x));
+                }
+            }
+            acc += __shfl_xor_sync(FULLM, acc, 8);
+            acc += __shfl_xor_sync(FULLM, acc, 16);
+            if (lane < 8 && f < ng2) ws.G[P.ind2[v] + f] = acc;
+        }
+    double eu = 0.0;
+    if (A.urep > 0.0) {
+        for (int t = lane; t < n; t += 32) {
+            const double R = P.rm[s0] + P.rm[species((t >= o1) + (t >= o2))], rd = (double)ws.d[t].w;
+            if (rd < R) eu += A.urep * 0.5 * (1.0 + cospi(rd / R)) * R / rd;
+        }
+        eu = bsum(eu);
+    }
+    if (lane == 0) sh.eu[i] = eu;
+    __syncwarp();
+
+    /* ---- triplet list and forward sums, a species block at a time ---- */
+    const unsigned short *tl = reinterpret_cast<const unsigned short *>(ws.tl);
+    int pos = 0, whole = 1, blkid = 0, ntrip = 0;
+    for (int al = 0; al < ns; al++)
+        for (int be = al; be < ns; be++, blkid++) {
+            const int oa = seg(al), ea = seg(al + 1), ob = seg(be), eb = seg(be + 1);
+            float acc[BCELLS];
+#pragma unroll
+            for (int k = 0; k < BCELLS; k++) acc[k] = 0.0f;
+            int start = pos, st = oa >> 3, g = -1;
+            for (;;) {
+                const int from = pos;
+                const bool done = fill_stripes(ws, A.T.rc2, oa, ea, ob, eb, st, g, pos, lane);
+                __syncwarp();
+                ntrip += pos - from;
+                for (int t = from + lane; t < pos; t += 32) {
+                    const unsigned ab = tl[t];
+                    const int a = ab & 0xffu, b = ab >> 8;
+                    const float4 d1 = ws.d[a], d2 = ws.d[b];
+                    const float dx = d1.x - d2.x, dy = d1.y - d2.y, dz = d1.z - d2.z;
+                    const float s3 = dx * dx + dy * dy + dz * dz;
+                    const float c = (d1.x * d2.x + d1.y * d2.y + d1.z * d2.z) * (ws.ir[a] * ws.ir[b]);
+                    const float A3 = 2.0f * ws.fa[a] * ws.fa[b] * cut_f(fmaf(-s3, A.T.iw, 1.0f));
+                    const float rho = fmaf(d1.w, d1.w, fmaf(d2.w, d2.w, s3));
+                    float lz[BNZL];
+                    angular_std(c, lz, nullptr);
+#pragma unroll
+                    for (int e = 0; e < BNE; e++) {
+                        const float ex = A3 * ex2f(A.T.ke[e] * rho);
+                        const float2 ex2 = make_float2(ex, ex);
+#pragma unroll
+                        for (int zl = 0; zl < BNZL; zl += 2) {
+                            if (e < BLOW && zl >= 4) break;
+                            const float2 r = __ffma2_rn(ex2, make_float2(lz[zl], lz[zl + 1]),
+                                                        make_float2(acc[e * BNZL + zl], acc[e * BNZL + zl + 1]));
+                            acc[e * BNZL + zl] = r.x;
+                            acc[e * BNZL + zl + 1] = r.y;
+                        }
+                    }
+                }
+                __syncwarp();
+                if (done) break;
+                whole = 0;
+                start = pos = 0;
+            }
+            ws.blk[blkid][0] = start;
+            ws.blk[blkid][1] = pos;
+            warp_reduce64f(acc, lane);
+            ws.red[2 * lane] = acc[0];
+            ws.red[2 * lane + 1] = acc[1];
+            __syncwarp();
+            {
+                const int base = P.ind4[al * al + be * be];
+                for (int f = lane; f < P.ng4; f += 32) {
+                    const int cell = P.g4_cell[f];
+                    ws.G[base + f] += ws.red[cell] * A.T.powz[(cell & 7) >> 1];
+                }
+            }
+            __syncwarp();
+        }
+    if (lane == 0) ws.work[2] += (unsigned long long)ntrip;
+
+    mlp_pass(A, P, sh.ea, ws, i, s0, lane);
+
+    /* ---- reverse pairs ---- */
+    double fu0 = 0.0, fu1 = 0.0, fu2 = 0.0; /* the force on atom i */
+    for (int t = lane; t < n; t += 32) {
+        const float4 d = ws.d[t];
+        const float r = d.w, f2 = ws.fa[t], df2 = ws.fb[t] * r;
+        const int v = (t >= o1) + (t >= o2);
+        const float *gg = ws.G + P.ind2[v];
+        float cp = 0.0f;
+        for (int f = 0; f < ng2; f++) {
+            const float x = r - P.d_rs[f], eta = P.d_eta2[f];
+            cp += gg[f] * expf(-eta * x * x) * (-2.0f * eta * x * f2 + df2);
+        }
+        const float cr = cp * ws.ir[t];
+        ws.F4[t] = make_float4(-cr * d.x, -cr * d.y, -cr * d.z, 0.0f);
+        if (A.urep > 0.0) {
+            const double R = P.rm[s0] + P.rm[species(v)], rd = (double)r;
+            if (rd < R) {
+                double sn, cs;
+                sincospi(rd / R, &sn, &cs);
+                const double fu = 0.5 * (1.0 + cs), dfu = -0.5 * CUDART_PI / R * sn;
+                const double tu = -2.0 * A.urep * R / (rd * rd) * (-fu / rd + dfu);
+                fu0 -= tu * d.x; fu1 -= tu * d.y; fu2 -= tu * d.z;
+                vr[0] += 0.5 * tu * d.x * d.x; vr[1] += 0.5 * tu * d.y * d.y; vr[2] += 0.5 * tu * d.z * d.z;
+                vr[3] += 0.5 * tu * d.x * d.y; vr[4] += 0.5 * tu * d.y * d.z; vr[5] += 0.5 * tu * d.z * d.x;
+            }
+        }
+    }
+    for (int k = lane; k < 3 * 8 * BTS; k += 32) ws.tile[k] = 0.0f;
+    __syncwarp();
+
+    /* ---- reverse triplets: the force on j is -(p1 d_j + sc d_k), on k
+     * -(p2 d_k + sc d_j); a run of entries of one stripe of 8 rows and 16
+     * columns is laid out as 8 x 16 tiles of sc, p1 and p2, whose columns and
+     * rows are summed against the displacements without atomics.  The row
+     * stride puts the 32 reads of either sum in distinct banks. ---- */
+    blkid = 0;
+    const int cr_r = lane >> 4, cr_c = lane & 15; /* column sums: rows 4 cr_r + k of column cr_c */
+    const int rr_r = lane & 7, rr_q = lane >> 3;  /* row sums: columns rr_q + 4 k of row rr_r */
+    const float *tcol = ws.tile + 4 * cr_r * BTS + cr_c, *trow = ws.tile + rr_r * BTS + rr_q;
+    for (int al = 0; al < ns; al++)
+        for (int be = al; be < ns; be++, blkid++) {
+            const int base4 = P.ind4[al * al + be * be];
+            const int oa = seg(al), ea = seg(al + 1), ob = seg(be), eb = seg(be + 1);
+            for (int t = lane; t < BCELLS; t += 32) ws.grid[t] = 0.0f;
+            __syncwarp();
+            for (int f = lane; f < P.ng4; f += 32) {
+                const int cell = P.g4_cell[f];
+                atomicAdd(&ws.grid[cell], ws.G[base4 + f] * A.T.powz[(cell & 7) >> 1]);
+            }
+            __syncwarp();
+            int st = oa >> 3, g = -1, lo = ws.blk[blkid][0], hi = ws.blk[blkid][1];
+            const float4 *g4 = reinterpret_cast<const float4 *>(ws.grid);
+            for (;;) {
+                bool done = true;
+                if (!whole) {
+                    lo = hi = 0;
+                    done = fill_stripes(ws, A.T.rc2, oa, ea, ob, eb, st, g, hi, lane);
+                    __syncwarp();
+                }
+                for (int base = lo; base < hi; base += 32) {
+                    const bool valid = base + lane < hi;
+                    const unsigned ab = tl[min(base + lane, hi - 1)];
+                    const int a = ab & 0xffu, b = ab >> 8;
+                    const float4 d1 = ws.d[a], d2 = ws.d[b];
+                    const float ir1 = ws.ir[a], ir2 = ws.ir[b], f1 = ws.fa[a], f2 = ws.fa[b];
+                    const float wx = d2.x - d1.x, wy = d2.y - d1.y, wz = d2.z - d1.z;
+                    const float s3 = wx * wx + wy * wy + wz * wz;
+                    const float ir12 = ir1 * ir2;
+                    const float c = (d1.x * d2.x + d1.y * d2.y + d1.z * d2.z) * ir12;
+                    const float rho = fmaf(d1.w, d1.w, fmaf(d2.w, d2.w, s3));
+                    float lz[BNZL], lzp[BNZL];
+                    angular_std(c, lz, lzp);
+                    float Q = 0.0f, Qe = 0.0f, Qc = 0.0f;
+#pragma unroll
+                    for (int e = 0; e < BNE; e++) {
+                        const float E = ex2f(A.T.ke[e] * rho);
+                        const float4 ga = g4[2 * e];
+                        float2 u = __ffma2_rn(make_float2(ga.x, ga.y), make_float2(lz[0], lz[1]), make_float2(0.0f, 0.0f));
+                        float2 v = __ffma2_rn(make_float2(ga.x, ga.y), make_float2(lzp[0], lzp[1]), make_float2(0.0f, 0.0f));
+                        u = __ffma2_rn(make_float2(ga.z, ga.w), make_float2(lz[2], lz[3]), u);
+                        v = __ffma2_rn(make_float2(ga.z, ga.w), make_float2(lzp[2], lzp[3]), v);
+                        if (e >= BLOW) {
+                            const float4 gb = g4[2 * e + 1];
+                            u = __ffma2_rn(make_float2(gb.x, gb.y), make_float2(lz[4], lz[5]), u);
+                            v = __ffma2_rn(make_float2(gb.x, gb.y), make_float2(lzp[4], lzp[5]), v);
+                            u = __ffma2_rn(make_float2(gb.z, gb.w), make_float2(lz[6], lz[7]), u);
+                            v = __ffma2_rn(make_float2(gb.z, gb.w), make_float2(lzp[6], lzp[7]), v);
+                        }
+                        const float Eu = E * (u.x + u.y);
+                        Q += Eu;
+                        Qe = fmaf(A.T.eta[e], Eu, Qe);
+                        Qc = fmaf(E, v.x + v.y, Qc);
+                    }
+                    const float w3 = fmaf(-s3, A.T.iw, 1.0f), f3 = cut_f(w3), h3 = A.T.mh * cut_g(w3);
+                    const float fab = 2.0f * f1 * f2, Af = fab * f3, Y = 2.0f * Af * Qe, f3Q = 2.0f * f3 * Q;
+                    const float Tc = Af * Qc, tcc = Tc * c;
+                    const float a3 = fab * h3 * Q - Y;
+                    const float p1 = ws.fb[a] * f2 * f3Q - Y - tcc * ir1 * ir1 + a3;
+                    const float p2 = f1 * ws.fb[b] * f3Q - Y - tcc * ir2 * ir2 + a3;
+                    const float sc = Tc * ir12 - a3;
+
+                    unsigned rem = __ballot_sync(FULLM, valid);
+                    while (rem) {
+                        const int first = __shfl_sync(FULLM, (a & ~7) | (b << 8), __ffs(rem) - 1);
+                        const int a0 = first & 0xff, c0 = first >> 8;
+                        const unsigned ra = (unsigned)(a - a0), cc = (unsigned)(b - c0);
+                        const bool mine = ((rem >> lane) & 1u) && ra < 8u && cc < 16u;
+                        float *o = ws.tile + BTS * ra + cc;
+                        if (mine) {
+                            o[0] = sc;
+                            o[8 * BTS] = p1;
+                            o[16 * BTS] = p2;
+                        }
+                        rem &= ~__ballot_sync(FULLM, mine);
+                        __syncwarp();
+                        /* past the list's end the tile holds zeros and any entry of the atom will do */
+                        float px = 0.0f, py = 0.0f, pz = 0.0f, ps = 0.0f;
+#pragma unroll
+                        for (int k = 0; k < 4; k++) {
+                            const float4 d = ws.d[min(a0 + 4 * cr_r + k, n - 1)];
+                            const float s = tcol[k * BTS];
+                            px = fmaf(s, d.x, px);
+                            py = fmaf(s, d.y, py);
+                            pz = fmaf(s, d.z, pz);
+                            ps += tcol[(16 + k) * BTS];
+                        }
+                        float qx = 0.0f, qy = 0.0f, qz = 0.0f, qs = 0.0f;
+#pragma unroll
+                        for (int k = 0; k < 4; k++) {
+                            const float4 d = ws.d[min(c0 + rr_q + 4 * k, n - 1)];
+                            const float s = trow[4 * k];
+                            qx = fmaf(s, d.x, qx);
+                            qy = fmaf(s, d.y, qy);
+                            qz = fmaf(s, d.z, qz);
+                            qs += trow[8 * BTS + 4 * k];
+                        }
+                        px += __shfl_xor_sync(FULLM, px, 16);
+                        py += __shfl_xor_sync(FULLM, py, 16);
+                        pz += __shfl_xor_sync(FULLM, pz, 16);
+                        ps += __shfl_xor_sync(FULLM, ps, 16);
+#pragma unroll
+                        for (int h = 8; h < 32; h <<= 1) {
+                            qx += __shfl_xor_sync(FULLM, qx, h);
+                            qy += __shfl_xor_sync(FULLM, qy, h);
+                            qz += __shfl_xor_sync(FULLM, qz, h);
+                            qs += __shfl_xor_sync(FULLM, qs, h);
+                        }
+                        const int tb = c0 + cr_c, ta = a0 + rr_r;
+                        if (lane < 16 && tb < n) {
+                            const float4 d = ws.d[tb], f = ws.F4[tb];
+                            ws.F4[tb] = make_float4(f.x - fmaf(ps, d.x, px), f.y - fmaf(ps, d.y, py),
+                                                    f.z - fmaf(ps, d.z, pz), 0.0f);
+                        }
+                        __syncwarp(); /* rows and columns may be the same neighbour */
+                        if (lane < 8 && ta < n) {
+                            const float4 d = ws.d[ta], f = ws.F4[ta];
+                            ws.F4[ta] = make_float4(f.x - fmaf(qs, d.x, qx), f.y - fmaf(qs, d.y, qy),
+                                                    f.z - fmaf(qs, d.z, qz), 0.0f);
+                        }
+                        if (mine) o[0] = o[8 * BTS] = o[16 * BTS] = 0.0f;
+                        __syncwarp();
+                    }
+                }
+                __syncwarp();
+                if (done) break;
+            }
+        }
+    /* neighbour forces out; atom i's is minus their sum, the virial of its
+     * energy every neighbour force times its displacement, in FP64 */
+    for (int t = lane; t < n; t += 32) {
+        const float4 d = ws.d[t], f = ws.F4[t];
+        const double fx = f.x, fy = f.y, fz = f.z;
+        const int j = ws.j[t];
+        vr[0] += fx * d.x; vr[1] += fy * d.y; vr[2] += fz * d.z;
+        vr[3] += fx * d.y; vr[4] += fy * d.z; vr[5] += fz * d.x;
+        fu0 -= fx; fu1 -= fy; fu2 -= fz;
+        atomicAdd(&sh.F[3 * j], fx);
+        atomicAdd(&sh.F[3 * j + 1], fy);
+        atomicAdd(&sh.F[3 * j + 2], fz);
+    }
+    {
+        const double s0x = bsum(fu0), s0y = bsum(fu1), s0z = bsum(fu2);
+        if (lane == 0) {
+            atomicAdd(&sh.F[3 * i], s0x);
+            atomicAdd(&sh.F[3 * i + 1], s0y);
+            atomicAdd(&sh.F[3 * i + 2], s0z);
+        }
+    }
     __syncwarp();
 }
 
@@ -744,9 +1196,9 @@ __device__ void atom_pass(const BArgs &A, BShared<W> &sh, WarpWS &ws, int i, con
  * rank W + w (mod C W), i.e. warp w of cluster rank `rank`.  Leaves
  * partial forces in sh.F (all atoms), ea/eu of its own atoms, the per-warp
  * virials in sh.vir and any overflow in sh.flag. */
-template <int W, int C>
+template <int W, int C, bool T>
 __device__ void eval_part(const BArgs &A, BShared<W> &sh, const double *dof, int rank) {
-    const BParams &P = *A.P;
+    const BParams &P = A.P;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, N = sh.N, rlxt = A.rlxt;
     const int first_atom = rank * W + w, stride = C * W;
     float4 *nbd = A.nbd + (size_t)blockIdx.x * BMAXN * BMAXNB;
@@ -853,7 +1305,20 @@ __device__ void eval_part(const BArgs &A, BShared<W> &sh, const double *dof, int
     __syncthreads();
     /* descriptors, MLP and forces, one warp per atom */
     double virw[6] = {0, 0, 0, 0, 0, 0};
-    for (int i = first_atom; i < N; i += stride) atom_pass(A, sh, sh.ws[w], i, nbd, nbj, virw);
+    for (int i = first_atom; i < N; i += stride) {
+        if constexpr (T) {
+            atom_pass_tri(A, sh, sh.ws[w], i, nbd, nbj, virw); /* a lane's share, summed below */
+        } else {
+            double vr[6] = {0, 0, 0, 0, 0, 0};
+            atom_pass(A, sh, sh.ws[w], i, nbd, nbj, vr);
+#pragma unroll
+            for (int k = 0; k < 6; k++) virw[k] += bsum(vr[k]);
+        }
+    }
+    if constexpr (T) {
+#pragma unroll
+        for (int k = 0; k < 6; k++) virw[k] = bsum(virw[k]);
+    }
     if (lane == 0)
         for (int k = 0; k < 6; k++) sh.vir[w][k] = virw[k];
     __syncthreads();
@@ -960,13 +1425,13 @@ __device__ double eval_finish(const BArgs &A, BShared<W> &sh, double *gout) {
  * ranks (cluster barrier), every rank evaluates its atoms, and a second
  * barrier precedes the combination: two barriers per evaluation, matched
  * one for one by the other ranks' command loop. */
-template <int W, int C>
+template <int W, int C, bool T>
 __device__ double evaluate(const BArgs &A, BShared<W> &sh, const double *dof, double *gout) {
     if constexpr (C > 1) {
         if (threadIdx.x == 0) sh.cmd_dof = dof == sh.x ? 0 : 1;
         cooperative_groups::this_cluster().sync();
     }
-    eval_part<W, C>(A, sh, dof, 0);
+    eval_part<W, C, T>(A, sh, dof, 0);
     if constexpr (C > 1) {
         cooperative_groups::this_cluster().sync();
         eval_combine<W, C>(sh);
@@ -978,7 +1443,7 @@ __device__ double evaluate(const BArgs &A, BShared<W> &sh, const double *dof, do
  * vector, evaluate their atoms, and meet rank 0 at the second barrier.
  * Rank 0 posts structure -1 when the queue is empty; one last barrier
  * keeps every rank's shared memory alive until all have read it. */
-template <int W, int C>
+template <int W, int C, bool T>
 __device__ void cluster_worker(const BArgs &A, BShared<W> &sh, int rank) {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
@@ -1004,7 +1469,7 @@ __device__ void cluster_worker(const BArgs &A, BShared<W> &sh, int rank) {
         const double *src = which ? r0->xt : r0->x;
         for (int k = tid; k < n; k += blockDim.x) sh.x[k] = src[k];
         __syncthreads();
-        eval_part<W, C>(A, sh, sh.x, rank);
+        eval_part<W, C, T>(A, sh, sh.x, rank);
         cl.sync();
     }
     cl.sync();
@@ -1056,8 +1521,8 @@ __device__ void vcopy(double *dst, const double *src, int n) {
     for (int k = threadIdx.x; k < n; k += blockDim.x) dst[k] = src[k];
 }
 
-template <int W, int C>
-__global__ void __launch_bounds__(W * 32) k_relax_batch(BArgs A) {
+template <int W, int C, bool T>
+__global__ void __launch_bounds__(W * 32) k_relax_batch(const __grid_constant__ BArgs A) {
     extern __shared__ __align__(16) char smem_raw[];
     BShared<W> &sh = *reinterpret_cast<BShared<W> *>(smem_raw);
     const int tid = threadIdx.x;
@@ -1067,7 +1532,7 @@ __global__ void __launch_bounds__(W * 32) k_relax_batch(BArgs A) {
     if constexpr (C > 1) {
         const int rank = (int)cooperative_groups::this_cluster().block_rank();
         if (rank != 0) {
-            cluster_worker<W, C>(A, sh, rank);
+            cluster_worker<W, C, T>(A, sh, rank);
             flush_work(A, sh);
             return;
         }
@@ -1105,7 +1570,7 @@ __global__ void __launch_bounds__(W * 32) k_relax_batch(BArgs A) {
         }
         int ident = 1; /* H is the identity and not written out */
         __syncthreads();
-        double f = evaluate<W, C>(A, sh, sh.x, sh.g), fprev = f;
+        double f = evaluate<W, C, T>(A, sh, sh.x, sh.g), fprev = f;
         double maxf = sh.scal[1], maxu = sh.scal[2];
         int first = 1, iter = 0, status = 1;
         if (sh.flag) status = 2;
@@ -1153,7 +1618,7 @@ __global__ void __launch_bounds__(W * 32) k_relax_batch(BArgs A) {
             for (trial = 0; trial < 60 && !done; trial++) {
                 for (int k = tid; k < n; k += blockDim.x) sh.xt[k] = sh.x[k] + alpha * sh.p[k];
                 __syncthreads();
-                ft = evaluate<W, C>(A, sh, sh.xt, sh.gt);
+                ft = evaluate<W, C, T>(A, sh, sh.xt, sh.gt);
                 double t = 0.0;
                 for (int k = tid; k < n; k += blockDim.x) t += sh.gt[k] * sh.p[k];
                 dt = cta_sum(sh, t);
@@ -1285,7 +1750,7 @@ __global__ void __launch_bounds__(W * 32) k_relax_batch(BArgs A) {
         /* forces and virial of the final state, on request: the last
          * evaluation was at the final DOF vector only if no step was taken */
         if (A.fout) {
-            if (iter > 0) f = evaluate<W, C>(A, sh, sh.x, sh.g);
+            if (iter > 0) f = evaluate<W, C, T>(A, sh, sh.x, sh.g);
             for (int k = tid; k < 3 * N; k += blockDim.x) A.fout[3 * (size_t)o + k] = sh.F[k];
             if (A.uout && tid < 6) A.uout[6 * (size_t)s + tid] = sh.uvir[tid] + (tid < 3 ? sh.scal[4] : 0.0);
             __syncthreads();
@@ -1364,7 +1829,7 @@ static int build_bparams(const mb_model *m, BParams *B, float *w) {
     return 0;
 }
 
-/* launch geometry of k_relax_batch<W, C> on this device: how many CTAs
+/* launch geometry of k_relax_batch<W, C, T> on this device: how many CTAs
  * (C = 1) or clusters of C CTAs can be resident at once */
 static void cluster_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute *at, int units, int W, int C, size_t smem,
                            cudaStream_t st) {
@@ -1381,34 +1846,59 @@ static void cluster_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute *at, int
     cfg->numAttrs = 1;
 }
 
-template <int W, int C>
+template <int W, int C, bool T>
 static cudaError_t batch_config(int sms, int *units) {
     const size_t smem = sizeof(BShared<W>);
-    cudaError_t e = cudaFuncSetAttribute(k_relax_batch<W, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k_relax_batch<W, C, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     if (C == 1) {
         int per = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_relax_batch<W, C>, W * 32, smem);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_relax_batch<W, C, T>, W * 32, smem);
         *units = per * sms;
         return e;
     }
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at;
     cluster_config(&cfg, &at, 1, W, C, smem, 0);
-    return cudaOccupancyMaxActiveClusters(units, k_relax_batch<W, C>, &cfg);
+    return cudaOccupancyMaxActiveClusters(units, k_relax_batch<W, C, T>, &cfg);
 }
 
-template <int W, int C>
+template <int W, int C, bool T>
 static cudaError_t batch_launch(int units, cudaStream_t st, const BArgs &a) {
     if (C == 1) {
-        k_relax_batch<W, C><<<units, W * 32, sizeof(BShared<W>), st>>>(a);
+        k_relax_batch<W, C, T><<<units, W * 32, sizeof(BShared<W>), st>>>(a);
         return cudaGetLastError();
     }
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at;
     cluster_config(&cfg, &at, units, W, C, sizeof(BShared<W>), st);
-    return cudaLaunchKernelEx(&cfg, k_relax_batch<W, C>, a);
+    return cudaLaunchKernelEx(&cfg, k_relax_batch<W, C, T>, a);
 }
+
+template <bool T>
+static cudaError_t batch_geometry(int wide, int csize, int sms, int *units) {
+    return !wide        ? batch_config<4, 1, T>(sms, units)
+           : csize == 4 ? batch_config<BWARPS_WIDE, 4, T>(sms, units)
+           : csize == 2 ? batch_config<BWARPS_WIDE, 2, T>(sms, units)
+                        : batch_config<BWARPS_WIDE, 1, T>(sms, units);
+}
+
+template <bool T>
+static cudaError_t batch_run(int wide, int csize, int units, cudaStream_t st, const BArgs &a) {
+    return !wide        ? batch_launch<4, 1, T>(units, st, a)
+           : csize == 4 ? batch_launch<BWARPS_WIDE, 4, T>(units, st, a)
+           : csize == 2 ? batch_launch<BWARPS_WIDE, 2, T>(units, st, a)
+                        : batch_launch<BWARPS_WIDE, 1, T>(units, st, a);
+}
+
+/* Single evaluations of models whose basis is the reference's function table
+ * (mb_tri), with at most the 7 exponents the batched kernel holds, take
+ * atom_pass_tri.  Other bases keep atom_pass, which reads its functions from
+ * tables, and so do relaxations: the two differ by FP32 rounding, and over a
+ * line search that turns a step differently here and there (up to 6
+ * iterations of a population: 1.6% of the iteration counts and status words
+ * changed, positions by up to 0.05 A), where results are expected to repeat. */
+static bool batch_tri(const mb_model *m, int mitr) { return mitr == 0 && m->T.ok && m->T.std && m->P.ne <= BNE; }
 
 /* Curvature constant of the line search's strong Wolfe test.  The
  * reference's minimiser uses its tolerance, 0.1, which on the EA population
@@ -1451,29 +1941,32 @@ static int batch_clusters(int S, int mitr, int sms) {
     return best;
 }
 
-/* The model's FP32 parameters and weights on the device, uploaded on a
+/* The model's FP32 parameters (host) and weights (device), formed on a
  * handle's first batched call. */
 static cudaError_t batch_model(const mb_model *m, mb_batch_ws *ws, cudaStream_t st) {
     if (ws->model) return cudaSuccess;
-    const size_t wb = sizeof(float) * m->weights_len, bytes = sizeof(BParams) + wb;
-    char *h = (char *)malloc(bytes);
-    if (!h) return cudaErrorMemoryAllocation;
-    cudaError_t e = build_bparams(m, (BParams *)h, (float *)(h + sizeof(BParams))) ? cudaErrorInvalidValue : cudaSuccess;
+    const size_t bytes = sizeof(float) * m->weights_len;
+    BParams *B = (BParams *)malloc(sizeof(BParams));
+    float *w = (float *)malloc(bytes);
     void *d = nullptr;
+    cudaError_t e = !B || !w ? cudaErrorMemoryAllocation : build_bparams(m, B, w) ? cudaErrorInvalidValue : cudaSuccess;
     if (!e) e = cudaMalloc(&d, bytes);
-    if (!e) e = cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, st);
+    if (!e) e = cudaMemcpyAsync(d, w, bytes, cudaMemcpyHostToDevice, st);
     if (!e) e = cudaStreamSynchronize(st);
-    free(h);
+    free(w);
     if (e) {
         cudaFree(d);
+        free(B);
         return e;
     }
     ws->model = d;
+    ws->params = B;
     return cudaSuccess;
 }
 
 extern "C" void mbk_batch_free(mb_batch_ws *ws) {
     cudaFree(ws->model);
+    free(ws->params);
     mb_ws_free(&ws->io);
     mb_ws_free(&ws->scratch);
     if (ws->e0) cudaEventDestroy((cudaEvent_t)ws->e0);
@@ -1504,16 +1997,15 @@ extern "C" int mbk_relax_batch(const mb_model *m, mb_batch_ws *ws, int S, const 
         if (fc) csize = atoi(fc) == 4 ? 4 : atoi(fc) == 2 ? 2 : 1;
         if (!wide) csize = 1;
     }
-    e = !wide        ? batch_config<4, 1>(sms, &units)
-        : csize == 4 ? batch_config<BWARPS_WIDE, 4>(sms, &units)
-        : csize == 2 ? batch_config<BWARPS_WIDE, 2>(sms, &units)
-                     : batch_config<BWARPS_WIDE, 1>(sms, &units);
+    const bool tri = batch_tri(m, mitr);
+    auto config = [&](int c) { return tri ? batch_geometry<true>(wide, c, sms, &units) : batch_geometry<false>(wide, c, sms, &units); };
+    e = config(csize);
     if (csize > 1 && (e != cudaSuccess || units < 1)) {
         /* clusters of this size cannot be placed (e.g. on a partitioned
          * GPU): one CTA per structure */
         cudaGetLastError();
         csize = 1;
-        e = batch_config<BWARPS_WIDE, 1>(sms, &units);
+        e = config(1);
     }
     if (e != cudaSuccess) return (int)e;
     if (units < 1) return (int)cudaErrorInvalidConfiguration;
@@ -1531,21 +2023,27 @@ extern "C" int mbk_relax_batch(const mb_model *m, mb_batch_ws *ws, int S, const 
     a.nat = d_nat; a.off = d_off; a.spc = d_spc; a.order = d_order;
     a.lat = d_lat; a.x = d_x; a.H = d_H; a.iters = d_iters; a.status = d_status;
     a.fout = d_frc; a.uout = d_str;
-    a.P = (const BParams *)ws->model;
-    a.W = (const float *)((char *)ws->model + sizeof(BParams));
+    a.P = *(const BParams *)ws->params;
+    a.W = (const float *)ws->model;
     a.queue = (int *)q;
     a.nbd = (float4 *)(q + 16);
     a.nbj = (int *)(q + 16 + b_nbd);
     a.hmat = (double *)(q + 16 + b_nbd + b_nbj);
     a.evals = d_evals;
     a.work = (unsigned long long *)(d_evals + 1);
+    memset(&a.T, 0, sizeof(a.T));
+    for (int k = 0; k < m->P.ne && k < BNE; k++) {
+        a.T.eta[k] = (float)m->P.d_eta4[k];
+        a.T.ke[k] = (float)(-m->P.d_eta4[k] / log(2.0));
+    }
+    a.T.iw = (float)(1.0 / (m->rc_list * m->rc_list));
+    a.T.mh = (float)(-2.0 / (m->rc_list * m->rc_list));
+    a.T.rc2 = (float)m->P.d_rc4sq;
+    for (int k = 0; k < 4; k++) a.T.powz[k] = (float)m->P.powz[k];
     e = cudaMemsetAsync(a.queue, 0, sizeof(int), st);
     if (e != cudaSuccess) return (int)e;
     cudaEventRecord((cudaEvent_t)ws->e0, st);
-    e = !wide        ? batch_launch<4, 1>(gunits, st, a)
-        : csize == 4 ? batch_launch<BWARPS_WIDE, 4>(gunits, st, a)
-        : csize == 2 ? batch_launch<BWARPS_WIDE, 2>(gunits, st, a)
-                     : batch_launch<BWARPS_WIDE, 1>(gunits, st, a);
+    e = tri ? batch_run<true>(wide, csize, gunits, st, a) : batch_run<false>(wide, csize, gunits, st, a);
     cudaEventRecord((cudaEvent_t)ws->e1, st);
     if (!e) e = cudaGetLastError();
     return (int)e;

@@ -7,7 +7,8 @@ extern "C" {
 #endif
 /* What a handle keeps for its batched calls. */
 typedef struct {
-    void *model; /* FP32 parameters and weights on the device (uploaded once) */
+    void *model; /* FP32 weights on the device (uploaded once) */
+    void *params; /* FP32 parameters, passed to the kernel by value */
     mb_ws io;    /* inputs and results of a call, staged through pinned memory */
     mb_ws scratch; /* per-CTA inverse Hessians and neighbour lists */
     void *e0, *e1; /* events around the launch */
