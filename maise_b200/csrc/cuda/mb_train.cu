@@ -30,10 +30,9 @@
  * W0[h1][D], W1[h2][h1], W2[h2].  Hidden layers tanh, output linear.
  *
  * Kernels (FP64; every sum in a fixed order, so results are reproducible):
- *   k_tr_fwd     one warp per atom: hidden activations and the atom energy
+ *   k_tr_fwd     one warp per 8 atoms of a species: hidden activations, the
+ *                atom energies and dE/d(layer-1 pre-activation)
  *   k_tr_struct  one thread per structure: E(s), c_s and the loss term
- *   k_tr_delta   one thread per atom: back-propagated deltas
- *   k_tr_ad1     one thread per atom: dE/d(layer-1 pre-activation)
  *   k_tr_fproj   one CTA per block: W0 Fn_b (h1 x 3)
  *   k_tr_frc     one warp per marked atom: f_i, dfq and the force loss term
  *   k_tr_fown    one CTA per block owner: the force-gradient terms of the
@@ -65,62 +64,90 @@ __host__ __device__ inline int off_W0(const TrainDims &t) { return t.h1 + t.h2 +
 __host__ __device__ inline int off_W1(const TrainDims &t) { return off_W0(t) + t.h1 * t.D; }
 __host__ __device__ inline int off_W2(const TrainDims &t) { return off_W1(t) + t.h2 * t.h1; }
 
-/* Sum of 16 per-lane values across a warp: lanes l and l ^ 1 end with the
- * total of value l >> 1 (four halving steps and one exchange). */
-__device__ __forceinline__ double reduce16(double *v, int lane) {
-#pragma unroll
-    for (int step = 0; step < 4; step++) {
-        const int off = 16 >> step, half = 8 >> step;
-        const bool upper = (lane & off) != 0;
-#pragma unroll
-        for (int k = 0; k < half; k++) {
-            const double send = upper ? v[k] : v[k + half];
-            const double keep = upper ? v[k + half] : v[k];
-            v[k] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-        }
-    }
-    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+/* D(8x8) += A(8x4) B(4x8) in FP64 on the tensor cores: lane l holds A[l/4][l%4],
+ * B[l%4][l/4] and D[l/4][2(l%4) + {0, 1}]. */
+__device__ __forceinline__ void dmma(double &c0, double &c1, double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+                 : "+d"(c0), "+d"(c1)
+                 : "d"(a), "d"(b));
 }
 
-/* one warp per atom: 16 first-layer units at a time in the lanes' partial
- * sums (each input read once), then a unit a lane */
-__global__ void __launch_bounds__(128) k_tr_fwd(TrainDims t, const double *__restrict__ X, const int *__restrict__ spc,
-                                                const double *__restrict__ V, double *__restrict__ H1,
-                                                double *__restrict__ H2, double *__restrict__ Eat) {
-    const int a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (a >= t.Na) return;
-    const double *v = V + (size_t)spc[a] * t.P, *x = X + (size_t)a * t.D;
-    const double *W0 = v + off_W0(t), *b0 = v;
-    double h = 0.0; /* lane k: activation k of the first layer */
-    for (int u = 0; u < t.h1; u += 16) {
-        double acc[16];
-#pragma unroll
-        for (int k = 0; k < 16; k++) acc[k] = 0.0;
-        for (int n = lane; n < t.D; n += 32) {
-            const double xn = x[n], *w = W0 + (size_t)u * t.D + n;
-#pragma unroll
-            for (int k = 0; k < 16; k++)
-                if (u + k < t.h1) acc[k] = fma(w[(size_t)k * t.D], xn, acc[k]);
+struct SpeciesOff { int o[4]; }; /* atoms o[s] .. o[s + 1] of the species list are of species s */
+
+/* One warp per 8 atoms of one species: the first layer as an 8 x 16 x D product
+ * on the FP64 tensor cores (16 units at a time), then the small layers with an
+ * (atom, unit) a lane.  With a warp per atom every atom read its species'
+ * first-layer weights (22 kB) again, 290 MB from L1 and L2 for 12800 atoms of
+ * 282 inputs, and the kernels that formed the deltas and
+ * AD1[n] = dE/d(pre-activation n of the first layer)
+ *        = (sum_m W2[m] (1 - e2[m]^2) W1[m][n]) (1 - e1[n]^2)
+ * a thread per atom had 100 CTAs: 67 + 14 + 9 us for 12800 atoms, now 35, bound
+ * by the latency of the input loads at 11 warps per SM. */
+#define FW_WARPS 4
+__global__ void __launch_bounds__(FW_WARPS * 32) k_tr_fwd(TrainDims t, SpeciesOff so, const int *__restrict__ satoms,
+                                                          const double *__restrict__ X, const double *__restrict__ V,
+                                                          double *__restrict__ H1, double *__restrict__ H2,
+                                                          double *__restrict__ Eat, double *__restrict__ AD1) {
+    __shared__ double sh1[FW_WARPS][8 * MB_TRAIN_MAXH], sh2[FW_WARPS][8 * MB_TRAIN_MAXH];
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, r = lane >> 2, q = lane & 3;
+    int w = blockIdx.x * FW_WARPS + wp, sp = 0;
+    for (; sp < t.nspc; sp++) {
+        const int tiles = (so.o[sp + 1] - so.o[sp] + 7) >> 3;
+        if (w < tiles) break;
+        w -= tiles;
+    }
+    if (sp == t.nspc) return;
+    const int lo = so.o[sp] + 8 * w, n = min(8, so.o[sp + 1] - lo), h1 = t.h1, h2 = t.h2, D = t.D;
+    const double *v = V + (size_t)sp * t.P, *x = X + (size_t)satoms[lo + min(r, n - 1)] * D;
+    const double *b0 = v, *W0 = v + off_W0(t), *W1 = v + off_W1(t), *b1 = v + off_b1(t), *W2 = v + off_W2(t),
+                 *b2 = v + off_b2(t);
+    double *e1 = sh1[wp], *e2 = sh2[wp];
+    for (int u0 = 0; u0 < h1; u0 += 16) {
+        const bool ua = u0 + r < h1, ub = u0 + 8 + r < h1;
+        const double *wa = W0 + (size_t)(ua ? u0 + r : 0) * D, *wb = W0 + (size_t)(ub ? u0 + 8 + r : 0) * D;
+        double c0 = 0.0, c1 = 0.0, d0 = 0.0, d1 = 0.0;
+#pragma unroll 8
+        for (int k = q; k < D + q; k += 4) { /* uniform trip count: the tail's lanes carry zeros */
+            const bool in = k < D;
+            const double xa = in ? x[k] : 0.0, fa = in && ua ? wa[k] : 0.0, fb = in && ub ? wb[k] : 0.0;
+            dmma(c0, c1, xa, fa);
+            dmma(d0, d1, xa, fb);
         }
-        const double tot = reduce16(acc, lane);
-        const double mine = __shfl_sync(0xffffffffu, tot, 2 * (lane & 15)); /* unit u + (lane & 15) */
-        if ((lane & 16) == (u & 16) && lane < t.h1) h = tanh(b0[lane] + mine);
+        const int u = u0 + 2 * q;
+        if (u < h1) e1[r * h1 + u] = c0;
+        if (u + 1 < h1) e1[r * h1 + u + 1] = c1;
+        if (u + 8 < h1) e1[r * h1 + u + 8] = d0;
+        if (u + 9 < h1) e1[r * h1 + u + 9] = d1;
     }
-    const double *W1 = v + off_W1(t), *b1 = v + off_b1(t), *W2 = v + off_W2(t), *b2 = v + off_b2(t);
-    double s = lane < t.h2 ? b1[lane] : 0.0;
-    for (int k = 0; k < t.h1; k++) {
-        const double hk = __shfl_sync(0xffffffffu, h, k);
-        if (lane < t.h2) s = fma(W1[lane * t.h1 + k], hk, s);
+    __syncwarp();
+    for (int k = lane; k < 8 * h1; k += 32) e1[k] = tanh(b0[k % h1] + e1[k]);
+    __syncwarp();
+    for (int k = lane; k < 8 * h2; k += 32) {
+        const int a = k / h2, m = k - a * h2;
+        double g = b1[m];
+        for (int j = 0; j < h1; j++) g = fma(W1[m * h1 + j], e1[a * h1 + j], g);
+        e2[k] = tanh(g);
     }
-    double e = 0.0;
-    if (lane < t.h2) {
-        const double g = tanh(s);
-        H2[(size_t)a * t.h2 + lane] = g;
-        e = W2[lane] * g;
+    __syncwarp();
+    for (int k = lane; k < 8 * h1; k += 32) {
+        const int a = k / h1, j = k - a * h1;
+        if (a >= n) break;
+        const size_t o = (size_t)satoms[lo + a] * h1 + j;
+        const double e = e1[k];
+        double al = 0.0;
+        for (int m = 0; m < h2; m++) {
+            const double g = e2[a * h2 + m];
+            al = fma(W2[m] * (1.0 - g * g), W1[m * h1 + j], al);
+        }
+        H1[o] = e;
+        AD1[o] = al * (1.0 - e * e);
     }
-    for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
-    if (lane < t.h1) H1[(size_t)a * t.h1 + lane] = h;
-    if (lane == 0) Eat[a] = b2[0] + e;
+    for (int k = lane; k < n * h2; k += 32) H2[(size_t)satoms[lo + k / h2] * h2 + k % h2] = e2[k];
+    if (lane < n) {
+        double e = 0.0;
+        for (int m = 0; m < h2; m++) e = fma(W2[m], e2[lane * h2 + m], e);
+        Eat[satoms[lo + lane]] = b2[0] + e;
+    }
 }
 
 __global__ void k_tr_struct(TrainDims t, const int *__restrict__ soff, const double *__restrict__ Eat,
@@ -137,48 +164,7 @@ __global__ void k_tr_struct(TrainDims t, const int *__restrict__ soff, const dou
     ls[s] = r * r * wt[s];
 }
 
-__global__ void k_tr_delta(TrainDims t, const int *__restrict__ spc, const int *__restrict__ sat,
-                           const double *__restrict__ V, const double *__restrict__ H1, const double *__restrict__ H2,
-                           const double *__restrict__ cs, double *__restrict__ d0, double *__restrict__ d1,
-                           double *__restrict__ ca) {
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= t.Na) return;
-    const double *v = V + (size_t)spc[a] * t.P, *W1 = v + off_W1(t), *W2 = v + off_W2(t);
-    const double c = cs[sat[a]];
-    ca[a] = c;
-    double dl1[MB_TRAIN_MAXH];
-    for (int m = 0; m < t.h2; m++) {
-        const double h = H2[(size_t)a * t.h2 + m];
-        dl1[m] = c * W2[m] * (1.0 - h * h);
-        d1[(size_t)a * t.h2 + m] = dl1[m];
-    }
-    for (int k = 0; k < t.h1; k++) {
-        double g = 0.0;
-        for (int m = 0; m < t.h2; m++) g += dl1[m] * W1[m * t.h1 + k];
-        const double h = H1[(size_t)a * t.h1 + k];
-        d0[(size_t)a * t.h1 + k] = g * (1.0 - h * h);
-    }
-}
-
 /* ---- force training ---- */
-
-/* per atom: ad1[n] = dE/d(pre-activation n of the first hidden layer)
- * = (sum_m W2[m] (1 - e2[m]^2) W1[m][n]) (1 - e1[n]^2) */
-__global__ void k_tr_ad1(TrainDims t, const int *__restrict__ spc, const double *__restrict__ V,
-                         const double *__restrict__ H1, const double *__restrict__ H2, double *__restrict__ AD1) {
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= t.Na) return;
-    const double *v = V + (size_t)spc[a] * t.P, *W1 = v + off_W1(t), *W2 = v + off_W2(t);
-    for (int n = 0; n < t.h1; n++) {
-        double al = 0.0;
-        for (int m = 0; m < t.h2; m++) {
-            const double h = H2[(size_t)a * t.h2 + m];
-            al += W2[m] * (1.0 - h * h) * W1[m * t.h1 + n];
-        }
-        const double e = H1[(size_t)a * t.h1 + n];
-        AD1[(size_t)a * t.h1 + n] = al * (1.0 - e * e);
-    }
-}
 
 /* one CTA per block b: Pj[b][n][q] = sum_l W0[n][l] Fn_b[l][q] with the
  * first-layer weights of the block owner's species */
@@ -351,7 +337,7 @@ __global__ void __launch_bounds__(128) k_tr_fown(TrainDims t, const int *__restr
 
 /* force-gradient accumulators per atom (all NULL without force training) */
 struct ForceTerms {
-    const double *AD1, *Phi, *Gam, *fB1, *fW1, *fW2;
+    const double *Phi, *Gam, *fB1, *fW1, *fW2;
 };
 
 /* The gradient is a sum over a species' atoms of outer products (W0: h1 x D
@@ -369,83 +355,120 @@ struct GradChunk {
     int spc;
 };
 
+/* acc += cf^T Y for 8 inputs of Y (rows at[0 .. m), m a multiple of 4) and the
+ * 16 units from u0: atoms are the contraction index, 4 a tensor-core step */
+__device__ __forceinline__ void gr_product(const double *cf, const int *at, int m, int h1, int u0, int D, int n0,
+                                           const double *__restrict__ Y, int lane, double *acc) {
+    const int r = lane >> 2, q = lane & 3;
+    const bool in = n0 + r < D, ua = u0 + r < h1, ub = u0 + 8 + r < h1;
+    const double *y = Y + (in ? n0 + r : 0), *ca = cf + (ua ? u0 + r : 0), *cb = cf + (ub ? u0 + 8 + r : 0);
+#pragma unroll 8
+    for (int k = q; k < m; k += 4) {
+        const double b = in ? y[(size_t)at[k] * D] : 0.0, a0 = ua ? ca[k * h1] : 0.0, a1 = ub ? cb[k * h1] : 0.0;
+        dmma(acc[0], acc[1], a0, b);
+        dmma(acc[2], acc[3], a1, b);
+    }
+}
+
+/* The energy part's coefficients are c_s AD1 for the first layer (c_s of the
+ * atom's structure) and c_s W2 (1 - e2^2) for the second: formed here as they
+ * are staged.  The outer products run on the FP64 tensor cores, 8 inputs and 16
+ * units a warp, so that an input is read once and 8 loads are in flight
+ * (GPART_NOTE). */
 __global__ void __launch_bounds__(256) k_tr_gpart(TrainDims t, const GradChunk *__restrict__ chunks,
                                                   const int *__restrict__ satoms, const int *__restrict__ sowners,
-                                                  const double *__restrict__ X, const double *__restrict__ H1,
-                                                  const double *__restrict__ H2, const double *__restrict__ d0,
-                                                  const double *__restrict__ d1, const double *__restrict__ ca,
-                                                  ForceTerms ft, double *__restrict__ part) {
+                                                  const int *__restrict__ sat, const double *__restrict__ cs,
+                                                  const double *__restrict__ V, const double *__restrict__ X,
+                                                  const double *__restrict__ H1, const double *__restrict__ H2,
+                                                  const double *__restrict__ AD1, ForceTerms ft,
+                                                  double *__restrict__ part) {
     __shared__ int at[GR_CHUNK];
+    __shared__ double cc[GR_CHUNK];
     __shared__ double cf[GR_CHUNK * MB_TRAIN_MAXH];
     const GradChunk c = chunks[blockIdx.x];
-    const int tid = threadIdx.x, h1 = t.h1, h2 = t.h2, D = t.D;
+    const int tid = threadIdx.x, h1 = t.h1, h2 = t.h2, D = t.D, m4 = (c.n + 3) & ~3;
     double *out = part + (size_t)blockIdx.x * t.P;
     const int *list = c.force ? sowners : satoms;
-    for (int q = tid; q < c.n; q += 256) at[q] = list[c.lo + q];
+    for (int q = tid; q < m4; q += 256) {
+        at[q] = list[c.lo + min(q, c.n - 1)]; /* padding rows get coefficients of 0 */
+        cc[q] = q < c.n && !c.force ? cs[sat[at[q]]] : 0.0;
+    }
     __syncthreads();
     if (blockIdx.y < gridDim.y - 1) {
-        /* W0[k][n] of GR_N inputs n: 4 threads an input, each the units k = kg, kg + 4, ... */
-        const double *cx = c.force ? ft.Gam : d0;
-        for (int e = tid; e < c.n * h1; e += 256) {
-            const double v = cx[(size_t)at[e / h1] * h1 + e % h1];
-            cf[e] = c.force ? -v : v;
-        }
-        __syncthreads();
-        const int n = blockIdx.y * GR_N + (tid & (GR_N - 1)), kg = tid / GR_N;
-        double acc[MB_TRAIN_MAXH / 4];
-#pragma unroll
-        for (int j = 0; j < MB_TRAIN_MAXH / 4; j++) acc[j] = 0.0;
-        if (n < D) {
-#pragma unroll 4
-            for (int q = 0; q < c.n; q++) {
-                const double x = X[(size_t)at[q] * D + n];
-#pragma unroll
-                for (int j = 0; j < MB_TRAIN_MAXH / 4; j++)
-                    if (kg + 4 * j < h1) acc[j] = fma(cf[q * h1 + kg + 4 * j], x, acc[j]);
-            }
-            if (c.force)
-                for (int q = 0; q < c.n; q++) {
-                    const double x = ft.Phi[(size_t)at[q] * D + n];
-#pragma unroll
-                    for (int j = 0; j < MB_TRAIN_MAXH / 4; j++)
-                        if (kg + 4 * j < h1) acc[j] = fma(-ft.AD1[(size_t)at[q] * h1 + kg + 4 * j], x, acc[j]);
+        const int lane = tid & 31, n0 = blockIdx.y * GR_N + 8 * (tid >> 5), r = lane >> 2, q = lane & 3;
+        for (int u0 = 0; u0 < h1; u0 += 16) {
+            double acc[4] = {0.0, 0.0, 0.0, 0.0};
+            for (int pass = 0; pass < (c.force ? 2 : 1); pass++) {
+                __syncthreads();
+                for (int e = tid; e < m4 * h1; e += 256) {
+                    const int k = e / h1;
+                    const size_t o = (size_t)at[k] * h1 + (e - k * h1);
+                    cf[e] = k >= c.n ? 0.0 : !c.force ? cc[k] * AD1[o] : pass ? -AD1[o] : -ft.Gam[o];
                 }
+                __syncthreads();
+                if (n0 < D) gr_product(cf, at, m4, h1, u0, D, n0, pass ? ft.Phi : X, lane, acc);
+            }
+            const int n = n0 + 2 * q;
 #pragma unroll
-            for (int j = 0; j < MB_TRAIN_MAXH / 4; j++)
-                if (kg + 4 * j < h1) out[off_W0(t) + (size_t)(kg + 4 * j) * D + n] = acc[j];
+            for (int h = 0; h < 2; h++) {
+                const int u = u0 + 8 * h + r;
+                double *o = out + off_W0(t) + (size_t)u * D + n;
+                if (u < h1 && n < D) o[0] = acc[2 * h];
+                if (u < h1 && n + 1 < D) o[1] = acc[2 * h + 1];
+            }
         }
         return;
     }
     /* the other parameters, one a thread */
+    if (!c.force) {
+        const double *W2 = V + (size_t)c.spc * t.P + off_W2(t);
+        for (int e = tid; e < c.n * h2; e += 256) {
+            const int k = e / h2, m = e - k * h2;
+            const double g = H2[(size_t)at[k] * h2 + m];
+            cf[e] = cc[k] * W2[m] * (1.0 - g * g);
+        }
+    }
+    __syncthreads();
     const int rest = t.P - h1 * D;
     for (int r = tid; r < rest; r += 256) {
         const int p = r < off_W0(t) ? r : r + h1 * D;
         double acc = 0.0;
         if (p < off_b1(t)) {
-            if (c.force)
+            if (c.force) {
+#pragma unroll 16
                 for (int q = 0; q < c.n; q++) acc -= ft.Gam[(size_t)at[q] * h1 + p];
-            else
-                for (int q = 0; q < c.n; q++) acc += d0[(size_t)at[q] * h1 + p];
+            } else {
+#pragma unroll 16
+                for (int q = 0; q < c.n; q++) acc = fma(cc[q], AD1[(size_t)at[q] * h1 + p], acc);
+            }
         } else if (p < off_b2(t)) {
-            const double *v = (c.force ? ft.fB1 : d1) + p - off_b1(t);
-            for (int q = 0; q < c.n; q++) acc += v[(size_t)at[q] * h2];
+            const int m = p - off_b1(t);
+            if (c.force) {
+#pragma unroll 16
+                for (int q = 0; q < c.n; q++) acc += ft.fB1[(size_t)at[q] * h2 + m];
+            } else {
+                for (int q = 0; q < c.n; q++) acc += cf[q * h2 + m];
+            }
         } else if (p < off_W0(t)) {
-            if (!c.force)
-                for (int q = 0; q < c.n; q++) acc += ca[at[q]];
+            for (int q = 0; q < c.n; q++) acc += cc[q];
         } else if (p < off_W2(t)) {
             const int m = (p - off_W1(t)) / h1, k = (p - off_W1(t)) % h1;
-            if (c.force)
+            if (c.force) {
+#pragma unroll 16
                 for (int q = 0; q < c.n; q++) acc += ft.fW1[((size_t)at[q] * h2 + m) * h1 + k];
-            else
-#pragma unroll 4
-                for (int q = 0; q < c.n; q++)
-                    acc = fma(d1[(size_t)at[q] * h2 + m], H1[(size_t)at[q] * h1 + k], acc);
+            } else {
+#pragma unroll 16
+                for (int q = 0; q < c.n; q++) acc = fma(cf[q * h2 + m], H1[(size_t)at[q] * h1 + k], acc);
+            }
         } else {
             const int m = p - off_W2(t);
-            if (c.force)
+            if (c.force) {
+#pragma unroll 16
                 for (int q = 0; q < c.n; q++) acc += ft.fW2[(size_t)at[q] * h2 + m];
-            else
-                for (int q = 0; q < c.n; q++) acc = fma(ca[at[q]], H2[(size_t)at[q] * h2 + m], acc);
+            } else {
+#pragma unroll 16
+                for (int q = 0; q < c.n; q++) acc = fma(cc[q], H2[(size_t)at[q] * h2 + m], acc);
+            }
         }
         out[p] = acc;
     }
@@ -470,7 +493,7 @@ struct mb_train {
     cudaStream_t st;
     TrainDims t;
     int NW;
-    double *X, *Eref, *wt, *V, *H1, *H2, *Eat, *Es, *cs, *ls, *d0, *d1, *ca, *grad;
+    double *X, *Eref, *wt, *V, *H1, *H2, *Eat, *Es, *cs, *ls, *AD1, *grad;
     int *spc, *sat, *soff, *satoms;
     /* chunks of the gradient sums (tr_chunks): coff[s] the first of species s */
     GradChunk *chunks;
@@ -483,7 +506,7 @@ struct mb_train {
     int NF, NB, Nown;
     double WF;
     int *fatom, *boff, *bown, *bmk, *owners, *ooff, *olist;
-    double *Fref, *Fn, *Pj, *AD1, *fpred, *dfq, *lf, *Phi, *Gam, *fB1, *fW1, *fW2, *h_lf;
+    double *Fref, *Fn, *Pj, *fpred, *dfq, *lf, *Phi, *Gam, *fB1, *fW1, *fW2, *h_lf;
 };
 
 static int tr_cuda(cudaError_t e, const char *what) {
@@ -498,7 +521,7 @@ extern "C" int mb_train_close(mb_train *tr) {
     cudaSetDevice(tr->device);
     if (tr->st) cudaStreamSynchronize(tr->st);
     cudaFree(tr->X); cudaFree(tr->Eref); cudaFree(tr->wt); cudaFree(tr->V); cudaFree(tr->grad);
-    cudaFree(tr->H1); cudaFree(tr->H2); cudaFree(tr->d0); cudaFree(tr->d1); cudaFree(tr->Eat); cudaFree(tr->ca);
+    cudaFree(tr->H1); cudaFree(tr->H2); cudaFree(tr->Eat);
     cudaFree(tr->Es); cudaFree(tr->cs); cudaFree(tr->ls); cudaFree(tr->spc); cudaFree(tr->sat); cudaFree(tr->soff);
     cudaFree(tr->satoms);
     cudaFree(tr->chunks); cudaFree(tr->coff); cudaFree(tr->sowners); cudaFree(tr->part);
@@ -613,10 +636,8 @@ extern "C" int mb_train_open(int device, int S, const int *nat, const int *atmn,
     TA(grad, tr->NW);
     TA(H1, (size_t)Na * h1);
     TA(H2, (size_t)Na * h2);
-    TA(d0, (size_t)Na * h1);
-    TA(d1, (size_t)Na * h2);
+    TA(AD1, (size_t)Na * h1);
     TA(Eat, Na);
-    TA(ca, Na);
     TA(Es, S);
     TA(cs, S);
     TA(ls, S);
@@ -739,7 +760,7 @@ extern "C" int mb_train_set_forces(mb_train *tr, int NF, const int *f_atom, cons
     if (!rc) rc = tr_cuda(cudaMemcpy(tr->dst, src, sizeof(*tr->dst) * (size_t)(n), cudaMemcpyHostToDevice), "H2D " #dst)
     TA(fatom, NF); TA(boff, NF + 1); TA(bown, NB); TA(bmk, NB); TA(owners, tr->Nown); TA(ooff, tr->Nown + 1);
     TA(olist, NB); TA(Fref, 3 * NF); TA(Fn, (size_t)NB * t.D * 3); TA(Pj, (size_t)NB * t.h1 * 3);
-    TA(AD1, (size_t)t.Na * t.h1); TA(fpred, 3 * NF); TA(dfq, 3 * NF); TA(lf, NF); TA(Phi, (size_t)t.Na * t.D);
+    TA(fpred, 3 * NF); TA(dfq, 3 * NF); TA(lf, NF); TA(Phi, (size_t)t.Na * t.D);
     TA(Gam, (size_t)t.Na * t.h1); TA(fB1, (size_t)t.Na * t.h2); TA(fW1, (size_t)t.Na * t.h2 * t.h1);
     TA(fW2, (size_t)t.Na * t.h2); TA(sowners, tr->Nown);
     TC(fatom, f_atom, NF); TC(boff, blk_off, NF + 1); TC(bown, blk_atom, NB); TC(bmk, bmk, NB);
@@ -768,27 +789,31 @@ static int tr_run(mb_train *tr, const double *V, double *grad) {
     if (!rc) rc = tr_cuda(cudaMemcpyAsync(tr->V, V, sizeof(double) * tr->NW, cudaMemcpyHostToDevice, st), "H2D V");
     if (rc) return rc;
     const bool F = tr->NF > 0;
-    k_tr_fwd<<<(t.Na + 3) / 4, 128, 0, st>>>(t, tr->X, tr->spc, tr->V, tr->H1, tr->H2, tr->Eat);
+    SpeciesOff so = {{0, 0, 0, 0}};
+    int tiles = 0;
+    for (int s = 0; s < t.nspc; s++) {
+        so.o[s + 1] = tr->hsoffs[s + 1];
+        tiles += (so.o[s + 1] - so.o[s] + 7) / 8;
+    }
+    k_tr_fwd<<<(tiles + FW_WARPS - 1) / FW_WARPS, FW_WARPS * 32, 0, st>>>(t, so, tr->satoms, tr->X, tr->V, tr->H1,
+                                                                          tr->H2, tr->Eat, tr->AD1);
     k_tr_struct<<<(t.S + 127) / 128, 128, 0, st>>>(t, tr->soff, tr->Eat, tr->Eref, tr->wt, tr->Es, tr->cs, tr->ls);
     if (F) {
-        k_tr_ad1<<<(t.Na + 127) / 128, 128, 0, st>>>(t, tr->spc, tr->V, tr->H1, tr->H2, tr->AD1);
         k_tr_fproj<<<tr->NB, 128, 0, st>>>(t, tr->NB, tr->bown, tr->spc, tr->V, tr->Fn, tr->Pj);
         k_tr_frc<<<(tr->NF + 3) / 4, 128, 0, st>>>(t, tr->NF, tr->fatom, tr->boff, tr->bown, tr->sat, tr->wt,
                                                    tr->Fref, tr->AD1, tr->Pj, tr->WF, tr->fpred, tr->dfq, tr->lf);
     }
     if (grad) {
-        k_tr_delta<<<(t.Na + 127) / 128, 128, 0, st>>>(t, tr->spc, tr->sat, tr->V, tr->H1, tr->H2, tr->cs, tr->d0,
-                                                       tr->d1, tr->ca);
-        ForceTerms ft = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+        ForceTerms ft = {nullptr, nullptr, nullptr, nullptr, nullptr};
         if (F) {
             k_tr_fown<<<tr->Nown, 128, sizeof(double) * t.D, st>>>(t, tr->owners, tr->ooff, tr->olist, tr->bmk,
                                                                    tr->spc, tr->V, tr->H1, tr->H2, tr->Fn, tr->Pj,
                                                                    tr->dfq, tr->Phi, tr->Gam, tr->fB1, tr->fW1,
                                                                    tr->fW2);
-            ft = {tr->AD1, tr->Phi, tr->Gam, tr->fB1, tr->fW1, tr->fW2};
+            ft = {tr->Phi, tr->Gam, tr->fB1, tr->fW1, tr->fW2};
         }
         k_tr_gpart<<<dim3(tr->nchunk, (t.D + GR_N - 1) / GR_N + 1), 256, 0, st>>>(
-            t, tr->chunks, tr->satoms, tr->sowners, tr->X, tr->H1, tr->H2, tr->d0, tr->d1, tr->ca, ft, tr->part);
+            t, tr->chunks, tr->satoms, tr->sowners, tr->sat, tr->cs, tr->V, tr->X, tr->H1, tr->H2, tr->AD1, ft, tr->part);
         k_tr_gsum<<<(tr->NW + 127) / 128, 128, 0, st>>>(t, tr->coff, tr->part, tr->V, tr->grad);
     }
     rc = tr_cuda(cudaGetLastError(), "training kernels");
