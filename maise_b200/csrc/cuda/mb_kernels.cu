@@ -2758,6 +2758,7 @@ static int tune_family(mb_dev *d, const mb_model *m, int N, int mode, const TriA
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         cudaGetLastError();
+        d->f_clear = 0; /* the trials added to F */
     }
     if (d->tune_n < MB_TUNE_SLOTS) {
         d->tune_key[d->tune_n] = key;
@@ -2857,8 +2858,7 @@ extern "C" int mbk_descriptor_pass(mb_dev *d, const mb_model *m, int N, int mode
         la.smem_group = 0;
         la.P = m->P;
         la.T = m->T;
-        const int tuned = d->tune_n, v = tune_family(d, m, N, mode, la, a, st);
-        if (d->tune_n != tuned) d->f_clear = 0; /* trial launches added to F */
+        const int v = tune_family(d, m, N, mode, la, a, st);
         if (v >= 16) {
             d->last_shape = v;
             cudaEvent_t e0 = 0, e1 = 0;
