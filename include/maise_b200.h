@@ -291,7 +291,7 @@ int mb_graphs(mb_potential *p, int enable);
 /* Start (enable=1) or stop timing of the fused descriptor/force kernel: every
  * launch is bracketed by CUDA events on the handle's stream (up to
  * `capacity` launches), and the kernel's pair/triplet counters are reset. */
-/* The autotuner's decisions so far: *count (at most cap) entries; entry k
+/* The autotuner's decisions so far (the latest 128): *count (at most cap) entries; entry k
  * holds the pass mode (0 descriptors, 1 energy, 2 E/F/S, 3 VJP), whether the
  * fused triplet kernel of the reference bases ran (legs) or the general one,
  * the size bucket (N <= 2^bucket), the neighbour capacity, the chosen shape

@@ -240,7 +240,7 @@ class Potential:
         capacity, wpa, apb, layout), modes 'descriptors', 'energy', 'efs',
         'vjp'; legs tells the fused triplet kernel (reference bases) from the
         general one, layout its reverse pass ('rounds') from that one's ('runs')."""
-        cap = 32
+        cap = 128  # the table's size
         cols = [np.zeros(cap, np.int32) for _ in range(7)]
         cnt = ctypes.c_int()
         self._check(self.lib.mb_tune_read(self.h, cap, ctypes.byref(cnt), *(c.ctypes.data_as(_I) for c in cols)))

@@ -27,6 +27,7 @@
 #include <math_constants.h>
 #include <stdint.h>
 #include <stdlib.h>
+#include <string.h>
 
 #include "../mb_internal.h"
 
@@ -2713,6 +2714,20 @@ static int tune_key(const mb_dev *d, int N, int mode) {
     return (mode << 28) | ((d->tri_on ? 1 : 0) << 26) | (bucket << 20) | (d->capNB & 0xfffff);
 }
 
+/* Record a decision; a full table gives up its oldest one, so that a key is
+ * not timed again on every call.  The capacity of a handle only grows, and at
+ * one capacity there are 4 modes of at most 31 size buckets: the keys in use
+ * always fit. */
+static void tune_store(mb_dev *d, int key, int val) {
+    if (d->tune_n == MB_TUNE_SLOTS) {
+        memmove(d->tune_key, d->tune_key + 1, sizeof(int) * (MB_TUNE_SLOTS - 1));
+        memmove(d->tune_val, d->tune_val + 1, sizeof(int) * (MB_TUNE_SLOTS - 1));
+        d->tune_n--;
+    }
+    d->tune_key[d->tune_n] = key;
+    d->tune_val[d->tune_n++] = val;
+}
+
 /* Decision for a pass that may run on k_efs_tri: its shapes are each timed
  * once (after an untimed launch) and the fastest kept, as 16 + shape.  k_efs,
  * slower at every size measured (32 atoms: 73 us against 40; 487: 199 against
@@ -2760,11 +2775,7 @@ static int tune_family(mb_dev *d, const mb_model *m, int N, int mode, const TriA
         cudaGetLastError();
         d->f_clear = 0; /* the trials added to F */
     }
-    if (d->tune_n < MB_TUNE_SLOTS) {
-        d->tune_key[d->tune_n] = key;
-        d->tune_val[d->tune_n] = best;
-        d->tune_n++;
-    }
+    tune_store(d, key, best);
     return best;
 }
 
@@ -2775,10 +2786,7 @@ static int tune_shape(mb_dev *d, const mb_model *m, int N, int mode, const EfsAr
         if (d->tune_key[k] == key) return d->tune_val[k];
     if (d->tune_fixed >= 0) {
         const int v = d->tune_fixed < MB_NSHAPES ? d->tune_fixed : 0;
-        if (d->tune_n < MB_TUNE_SLOTS) {
-            d->tune_key[d->tune_n] = key;
-            d->tune_val[d->tune_n++] = v;
-        }
+        tune_store(d, key, v);
         return v;
     }
     EfsArgs t = a;
@@ -2804,11 +2812,7 @@ static int tune_shape(mb_dev *d, const mb_model *m, int N, int mode, const EfsAr
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     cudaGetLastError();
-    if (d->tune_n < MB_TUNE_SLOTS) {
-        d->tune_key[d->tune_n] = key;
-        d->tune_val[d->tune_n] = best;
-        d->tune_n++;
-    }
+    tune_store(d, key, best);
     return best;
 }
 

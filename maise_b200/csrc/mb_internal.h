@@ -177,7 +177,7 @@ typedef struct {
     void *flush;
     size_t flush_bytes;
     /* kernel-shape autotuner cache (see mb_kernels.cu) */
-#define MB_TUNE_SLOTS 32
+#define MB_TUNE_SLOTS 128
     int tune_n, tune_fixed, last_shape;
     int tune_key[MB_TUNE_SLOTS], tune_val[MB_TUNE_SLOTS];
 } mb_dev;

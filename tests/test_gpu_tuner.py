@@ -69,3 +69,13 @@ def test_forces_after_many_keys(model, worn):
     np.testing.assert_allclose(U, wantU, atol=tol)
     # seven steps of 1 fs: forces that agree to 1e-9 eV/A move an atom by less than 1e-12 A
     np.testing.assert_allclose(md["X"], wmd["X"], atol=1e-10)
+
+
+def test_new_key_is_recorded(model, worn):
+    """A key met after the table is full is kept, so its shapes are not timed
+    again on the next call (which then runs as a graph)."""
+    _, w = model
+    args = (w["X"], w["LAT"], w["atmn"])
+    for mode, call in (("efs", worn.efs), ("energy", worn.energy), ("descriptors", worn.descriptors)):
+        call(*args, ND=3)
+        assert [e for e in worn.tune_table() if (e["mode"], e["size_bucket"], e["capacity"]) == (mode, 5, 104)], mode
