@@ -361,9 +361,10 @@ static long double fn_h(long double v, const long double *a) {
 /* The fused triplet kernel applies when every forward and derivative
  * function shares the list cutoff, the pair-mixed G4 exponents equal the
  * species-0 ones to rounding (so that one factor serves the energy and the
- * derivative terms), the basis has the reference's shape (<= 8 G4 exponents,
- * <= 4 integer zeta, <= 2 lambda) and no exponent is so large that the
- * polynomial would need more than MB_TRI_MAXSQ squarings. */
+ * derivative terms) and the basis has the reference's shape (<= 8 G4 exponents,
+ * <= 4 integer zeta, <= 2 lambda).  Exponents so large that the polynomial
+ * would need more than MB_TRI_MAXSQ squarings, each of which doubles its
+ * relative error, are left to exp(). */
 static void tri_tables(mb_model *m) {
     const mb_params *P = &m->P;
     mb_tri *T = &m->T;
@@ -379,26 +380,25 @@ static void tri_tables(mb_model *m) {
             const int p = s * s + t * t;
             if (P->f_rc2[p] != m->rc_list || P->f_rc4[p] != m->rc_list) return;
             for (e = 0; e < P->ne; e++)
-                if (fabs(P->f_eta4[p][e] - P->d_eta4[e]) > 1e-12 * fabs(P->d_eta4[e])) return;
+                if (!(fabs(P->f_eta4[p][e] - P->d_eta4[e]) <= 1e-12 * fabs(P->d_eta4[e]))) return;
         }
     for (e = 0; e < P->ne; e++) {
-        if (!(P->d_eta4[e] >= 0.0)) return;
+        T->tab.eta[e] = P->d_eta4[e];
+        if (!(P->d_eta4[e] >= 0.0)) top = INFINITY;
         if (P->d_eta4[e] > top) top = P->d_eta4[e];
     }
     top *= 1.5L * rc * rc; /* the largest eta rho at the middle of rho's range */
-    if (!(top <= 0.42L * (1 << MB_TRI_MAXSQ))) return;
-    /* two squarings always (the kernel's straight-line form), more where needed */
-    top *= 0.25L;
-    T->nsq = 2;
-    while (top > 0.42L) {
-        top *= 0.5L;
-        T->nsq++;
-    }
-    if (!(top > 1e-6L)) top = 1e-6L;
-    poly_fit(fn_exp, &top, MB_TRI_DEG, T->tab.ex);
-    for (e = 0; e < P->ne; e++) {
-        T->tab.kw[e] = (double)(P->d_eta4[e] / (top * (1 << T->nsq)));
-        T->tab.eta[e] = P->d_eta4[e];
+    if (top <= 0.42L * (1 << MB_TRI_MAXSQ)) {
+        /* two squarings always (the kernel's straight-line form), more where needed */
+        top *= 0.25L;
+        T->nsq = 2;
+        while (top > 0.42L) {
+            top *= 0.5L;
+            T->nsq++;
+        }
+        if (!(top > 1e-6L)) top = 1e-6L;
+        poly_fit(fn_exp, &top, MB_TRI_DEG, T->tab.ex);
+        for (e = 0; e < P->ne; e++) T->tab.kw[e] = (double)(P->d_eta4[e] / (top * (1 << T->nsq)));
     }
     poly_fit(fn_fc, &rc, MB_TRI_FDEG, T->tab.f);
     poly_fit(fn_h, &rc, MB_TRI_FDEG, h);
@@ -426,7 +426,7 @@ static void tri_tables(mb_model *m) {
             r[P->h1] = off[t];
         }
     }
-    T->std = T->nsq == 2 && P->zeta_std && P->nlam == 2 && P->lam[0] == -1.0 && P->lam[1] == 1.0;
+    T->std = P->zeta_std && P->nlam == 2 && P->lam[0] == -1.0 && P->lam[1] == 1.0;
     for (e = 0; e < MB_TRI_LOW && e < MB_TRI_MAXE; e++)
         for (s = 4; s < 8; s++)
             if (T->cell_fn[8 * e + s] >= 0) T->std = 0;

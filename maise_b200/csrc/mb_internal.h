@@ -84,9 +84,11 @@ typedef struct {
 } mb_tri_tab;
 typedef struct {
     mb_tri_tab tab;
-    int ok, nsq;                  /* the basis qualifies for k_efs_tri; squarings (at least 2) */
+    /* the basis qualifies for k_efs_tri; squarings (at least 2), or 0: an
+     * exponent is too steep for the polynomial (or negative), exp() is called */
+    int ok, nsq;
     /* the reference's function table: zeta = 1, 2, 4, 16, lambda = -1, 1,
-     * nsq = 2, and the first MB_TRI_LOW exponents used with zeta = 1, 2 only */
+     * and the first MB_TRI_LOW exponents used with zeta = 1, 2 only */
     int std;
     double sv;                    /* 2 / Rc^2 */
     /* (eta, zeta, lambda) cell -> its first G4 function (-1: none), and the
