@@ -2610,18 +2610,20 @@ template <int NE, int NZ, int NLAM, int WPA, int APB>
 static int launch_shape(const EfsArgs &a, cudaStream_t st, cudaEvent_t e0, cudaEvent_t e1) {
     auto kern = k_efs<NE, NZ, NLAM, WPA, APB>;
     size_t smem = a.smem_group * APB;
-    /* the shared-memory opt-in is a per-device attribute of the function:
-     * remembered per device */
-    static size_t configured[MB_MAX_DEVICES_K] = {0};
+    /* the shared-memory opt-in is a per-device attribute of the function: set
+     * once per device, to the most there is, since a limit of one handle's own
+     * size could fall between another thread's limit and its launch */
+    static bool configured[MB_MAX_DEVICES_K] = {false};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MB_MAX_DEVICES_K) return (int)cudaErrorInvalidDevice;
     /* the 48 KB default and the 227 KB opt-in limit both count the kernel's
      * static shared block (the staged mb_params) as well as the dynamic part */
     if (smem + EFS_STATIC_SMEM > 227 * 1024) return (int)cudaErrorInvalidConfiguration;
-    if (smem + EFS_STATIC_SMEM > 48 * 1024 && smem > configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem + EFS_STATIC_SMEM > 48 * 1024 && !configured[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             227 * 1024 - (int)EFS_STATIC_SMEM);
         if (e != cudaSuccess) return (int)e;
-        configured[dev] = smem;
+        configured[dev] = true;
     }
     if (e0) mbk_record(e0, st);
     kern<<<(a.N + APB - 1) / APB, WPA * 32 * APB, smem, st>>>(a);
@@ -2668,14 +2670,15 @@ template <int NE, int WPA, int APB, bool STD, bool EXP>
 static int launch_tri(const TriArgs &a, cudaStream_t st) {
     auto kern = k_efs_tri<NE, WPA, APB, STD, EXP>;
     const size_t smem = a.smem_group * APB;
-    static size_t configured[MB_MAX_DEVICES_K] = {0};
+    static bool configured[MB_MAX_DEVICES_K] = {false}; /* as in launch_shape */
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MB_MAX_DEVICES_K) return (int)cudaErrorInvalidDevice;
     if (smem + TRI_STATIC_SMEM > 227 * 1024) return (int)cudaErrorInvalidConfiguration;
-    if (smem + TRI_STATIC_SMEM > 48 * 1024 && smem > configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem + TRI_STATIC_SMEM > 48 * 1024 && !configured[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             227 * 1024 - (int)TRI_STATIC_SMEM);
         if (e != cudaSuccess) return (int)e;
-        configured[dev] = smem;
+        configured[dev] = true;
     }
     kern<<<(a.N + APB - 1) / APB, WPA * 32 * APB, smem, st>>>(a);
     return (int)cudaGetLastError();
@@ -2929,7 +2932,7 @@ extern "C" int mbk_jvp(mb_dev *d, const mb_model *m, int N, const double *dx, co
                         sizeof(int) * d->capNB;
     if (smem > 227 * 1024) return (int)cudaErrorInvalidConfiguration;
     if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k_jvp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(k_jvp, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         if (e != cudaSuccess) return (int)e;
     }
     k_jvp<<<N, 32, smem, (cudaStream_t)stream>>>(a);

@@ -27,6 +27,7 @@
 namespace {
 
 constexpr int RDF_THREADS = 512;
+constexpr int RDF_MAX_HIST = 200 * 1024; /* bytes of a structure's histograms */
 constexpr int RDF_SHIFTS = 128; /* image shifts kept in shared memory (more are formed again per pair) */
 
 /* squared distance of j's image from i in LIST's operation order
@@ -272,7 +273,7 @@ extern "C" int mb_rdf(int device, int S, const int *nat, const int *atmn, const 
         return mb_handle_fail(MB_ERR_ARG, "bad arguments");
     const int npair = nspc * (nspc + 1) / 2;
     const size_t smem = sizeof(double) * (size_t)npair * nbins;
-    if (smem > 200 * 1024) return mb_handle_fail(MB_ERR_ARG, "nbins x species pairs exceed the shared histogram");
+    if (smem > RDF_MAX_HIST) return mb_handle_fail(MB_ERR_ARG, "nbins x species pairs exceed the shared histogram");
     int *off = (int *)malloc(sizeof(int) * (S + 1));
     off[0] = 0;
     for (int s = 0; s < S; s++) {
@@ -302,8 +303,8 @@ extern "C" int mb_rdf(int device, int S, const int *nat, const int *atmn, const 
     if (!rc) rc = rdf_cuda(cudaMemcpy(d_lat, lat, sizeof(double) * 9 * S, cudaMemcpyHostToDevice), "H2D");
     if (!rc) rc = rdf_cuda(cudaMemcpy(d_x, x, sizeof(double) * 3 * off[S], cudaMemcpyHostToDevice), "H2D");
     if (!rc && smem + 4096 > 48 * 1024) /* (k_rdf_ref's static arrays count too) */
-        rc = rdf_cuda(cudaFuncSetAttribute(k_rdf_ref, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                      "shared-memory opt-in");
+        rc = rdf_cuda(cudaFuncSetAttribute(k_rdf_ref, cudaFuncAttributeMaxDynamicSharedMemorySize, RDF_MAX_HIST),
+                      "shared-memory opt-in"); /* one limit for every call: other threads may be launching */
     if (!rc) {
         RdfArgs a;
         a.S = S; a.nspc = nspc; a.nbins = nbins; a.ND = ND; a.normalise = normalise ? 1 : 0;

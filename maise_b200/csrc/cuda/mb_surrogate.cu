@@ -393,7 +393,9 @@ extern "C" int surk_rdf(int S, const int *off, const int *spc, const double *lat
     const size_t hist = sizeof(float) * P * nbins, smem = hist + sizeof(double) * nbins;
     if (nspc < 1 || nspc > SUR_MAX_SPC || nbins < 1 || hist > 48 * 1024) return (int)cudaErrorInvalidValue;
     if (smem > 16 * 1024) { /* with the static arrays (26 KB) past the default limit */
-        const cudaError_t e = cudaFuncSetAttribute(k_rdf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        /* the largest size any call has (one species): a limit of a call's own
+         * size could fall between another thread's limit and its launch */
+        const cudaError_t e = cudaFuncSetAttribute(k_rdf, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * 48 * 1024);
         if (e != cudaSuccess) return (int)e;
     }
     k_rdf<<<S, 256, smem, (cudaStream_t)stream>>>(S, off, spc, lat, x, nspc, nbins, rmax, sigma, feat, status);
