@@ -117,21 +117,30 @@ static int cuda_fail(cudaError_t e, const char *what) {
         if (e_ != cudaSuccess) return cuda_fail(e_, what); \
     } while (0)
 
+/* a size to allocate for `need` bytes where there were `had`: at least half as
+ * much again, so that a run of slowly growing calls allocates a few times only */
+static size_t grown(size_t need, size_t had) {
+    const size_t more = had + had / 2, unit = (size_t)1 << 16;
+    return ((need > more ? need : more) + unit - 1) / unit * unit;
+}
+
 int mb_ws_grow(mb_ws *w, size_t dev_bytes, size_t host_bytes) {
     cudaError_t e = cudaSuccess;
     if (dev_bytes > w->dev_len) {
+        const size_t n = grown(dev_bytes, w->dev_len);
         cudaFree(w->dev);
         w->dev = NULL;
         w->dev_len = 0;
-        e = cudaMalloc(&w->dev, dev_bytes);
-        if (!e) w->dev_len = dev_bytes;
+        e = cudaMalloc(&w->dev, n);
+        if (!e) w->dev_len = n;
     }
     if (!e && host_bytes > w->host_len) {
+        const size_t n = grown(host_bytes, w->host_len);
         cudaFreeHost(w->host);
         w->host = NULL;
         w->host_len = 0;
-        e = cudaMallocHost(&w->host, host_bytes);
-        if (!e) w->host_len = host_bytes;
+        e = cudaMallocHost(&w->host, n);
+        if (!e) w->host_len = n;
     }
     return (int)e;
 }
@@ -474,13 +483,15 @@ int mb_reserve(mb_potential *p, int max_atoms, int max_neighbours) {
     return ensure(p, max_atoms, max_neighbours, 1);
 }
 
-static int host_buf(mb_potential *p, size_t n) {
-    if (n <= p->h_buf_len) return MB_OK;
-    cudaFreeHost(p->h_buf);
-    p->h_buf = NULL;
-    p->h_buf_len = 0;
-    CK(cudaMallocHost((void **)&p->h_buf, sizeof(double) * n), "cudaMallocHost");
-    p->h_buf_len = n;
+/* room for n doubles in a pinned buffer of the handle; contents are lost on growth */
+static int pinned(double **buf, size_t *len, size_t n) {
+    if (n <= *len) return MB_OK;
+    n = grown(sizeof(double) * n, sizeof(double) * *len) / sizeof(double);
+    cudaFreeHost(*buf);
+    *buf = NULL;
+    *len = 0;
+    CK(cudaMallocHost((void **)buf, sizeof(double) * n), "cudaMallocHost");
+    *len = n;
     return MB_OK;
 }
 
@@ -579,7 +590,7 @@ static int stage(mb_potential *p, int N, int XT, const int *atmn, const double *
     double *hx;
     for (s = 0; s < N; s++)
         if (atmn[s] < 0 || atmn[s] >= p->m.nspc) return fail(MB_ERR_ARG, "atom %d has species %d (model has %d)", s, atmn[s], p->m.nspc);
-    if ((r = host_buf(p, 3 * (size_t)N + N))) return r;
+    if ((r = pinned(&p->h_buf, &p->h_buf_len, 3 * (size_t)N + N))) return r;
     hx = p->h_buf;
     if (XT == 0)
         frac_to_cart(N, x, lat9, hx);
@@ -721,13 +732,7 @@ static int run_pass(mb_potential *p, int N, int NM, int ND, const double *lat9, 
     ncell = c.M[0] ? c.M[0] * c.M[1] * c.M[2] : 1;
     if ((r = ensure(p, N, p->d.capNB ? p->d.capNB : (NM < 64 ? NM : 64), ncell))) return r;
     p->d.tri_on = p->tri_enabled && mbk_tri_usable(&p->d, &p->m);
-    if (7 * (size_t)N > p->h_res_len) {
-        cudaFreeHost(p->h_res);
-        p->h_res = NULL;
-        p->h_res_len = 0;
-        CK(cudaMallocHost((void **)&p->h_res, sizeof(double) * 7 * N), "cudaMallocHost");
-        p->h_res_len = 7 * (size_t)N;
-    }
+    if ((r = pinned(&p->h_res, &p->h_res_len, 7 * (size_t)N))) return r;
     r = MB_FALLBACK;
     if (p->use_graphs && !p->pbroken && !p->d.ev_on && mbk_shape_ready(&p->d, N, mode)) {
         r = graph_pass(p, N, NM, ND, &c, pV, mode, urep);

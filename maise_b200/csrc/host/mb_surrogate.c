@@ -29,8 +29,8 @@ struct mb_surrogate {
     double tmean, tstd;     /* target standardisation */
     long t;                 /* Adam steps taken */
     int bcap;               /* rows the work buffers hold */
-    float *x, *tt, *z[NL], *a[NL], *dz[NL];
-    int *idx;
+    mb_ws work;
+    float *x, *tt, *z[NL], *a[NL], *dz[NL]; /* in work */
     double *loss;
     int loss_cap;
     mb_ws io;   /* structures of a call, staged through pinned memory */
@@ -61,35 +61,32 @@ static double sm_normal(uint64_t *s) { /* Box-Muller */
     return sqrt(-2.0 * log(u)) * cos(2.0 * M_PI * w);
 }
 
-static void free_work(mb_surrogate *s) {
-    int l;
-    cudaFree(s->x);
-    cudaFree(s->tt);
-    cudaFree(s->idx);
-    for (l = 0; l < NL; l++) {
-        cudaFree(s->z[l]);
-        cudaFree(s->a[l]);
-        cudaFree(s->dz[l]);
-        s->z[l] = s->a[l] = s->dz[l] = NULL;
-    }
-    s->x = s->tt = NULL;
-    s->idx = NULL;
-    s->bcap = 0;
-}
-
-/* work buffers for B rows */
+/* work buffers for B rows, in one block: with an allocation each
+ * the first screen of 2048 structures on a handle took 9 ms, with one 7 */
 static int ensure_rows(mb_surrogate *s, int B) {
+    size_t at = 0, x, tt, z[NL], a[NL], dz[NL];
+    char *w;
     int l;
     if (B <= s->bcap) return MB_OK;
-    free_work(s);
-    CK(cudaMalloc((void **)&s->x, sizeof(float) * (size_t)B * s->nin));
-    CK(cudaMalloc((void **)&s->tt, sizeof(float) * B));
-    CK(cudaMalloc((void **)&s->idx, sizeof(int) * B));
+#define PUT(name, n) (name = at, at += (sizeof(float) * (size_t)(n) + 255) & ~(size_t)255)
+    PUT(x, (size_t)B * s->nin);
+    PUT(tt, B);
     for (l = 0; l < NL; l++) {
         const size_t n = (size_t)B * s->dims[l + 1];
-        CK(cudaMalloc((void **)&s->z[l], sizeof(float) * n));
-        CK(cudaMalloc((void **)&s->a[l], sizeof(float) * n));
-        CK(cudaMalloc((void **)&s->dz[l], sizeof(float) * n));
+        PUT(z[l], n);
+        PUT(a[l], n);
+        PUT(dz[l], n);
+    }
+#undef PUT
+    s->bcap = 0;
+    CK((cudaError_t)mb_ws_grow(&s->work, at, 0));
+    w = (char *)s->work.dev;
+    s->x = (float *)(w + x);
+    s->tt = (float *)(w + tt);
+    for (l = 0; l < NL; l++) {
+        s->z[l] = (float *)(w + z[l]);
+        s->a[l] = (float *)(w + a[l]);
+        s->dz[l] = (float *)(w + dz[l]);
     }
     s->bcap = B;
     return MB_OK;
@@ -186,7 +183,7 @@ static int init_state(mb_surrogate *s, unsigned seed) {
 void mb_sur_close(mb_surrogate *s) {
     if (!s) return;
     cudaSetDevice(s->device);
-    free_work(s);
+    mb_ws_free(&s->work);
     cudaFree(s->p);
     cudaFree(s->g);
     cudaFree(s->m);
@@ -337,7 +334,7 @@ int mb_sur_features(mb_surrogate *s, int S, const int *nat, const int *atmn, con
 static int predict_dev(mb_surrogate *s, int S, const float *d_feat, double *pred) {
     float *y;
     int c0, k, rc;
-    if ((rc = ensure_rows(s, S < PRED_CHUNK ? S : PRED_CHUNK))) return rc;
+    if ((rc = ensure_rows(s, PRED_CHUNK))) return rc;
     CK((cudaError_t)mb_ws_grow(&s->feat, 0, sizeof(float) * (size_t)S));
     y = (float *)s->feat.host;
     for (c0 = 0; c0 < S; c0 += PRED_CHUNK) {
