@@ -1920,20 +1920,29 @@ static double batch_sigma() {
 /* CTAs (SMs) per structure.  A launch lasts as long as its total work on all
  * units or as its longest BFGS chain on one, whichever is more; an evaluation
  * on a cluster of 2 or 4 CTAs takes 0.62 or 0.44 of one CTA's time (536, 330 and
- * 235 us for 64 atoms).  Structures stop after about 200 iterations on
- * average, the longest run to mitr.  256 Mg-Ca structures, one CTA, pairs and
- * clusters of 4: 6 iterations 6.4, 6.5 and 9.4 ms; 100 iterations 110, 131
- * and 188 ms; 1000 iterations 1.60, 0.93 and 0.88 s.  40 structures, 6
- * iterations: 4.6, 2.8 and 2.0 ms. */
-static int batch_clusters(int S, int mitr, int sms) {
+ * 235 us for 64 atoms).  How many iterations the structures take is not known
+ * beforehand; 80 on average and 300 for the longest, where mitr allows them,
+ * and one CTA from more than two structures an SM on, are the values at which
+ * none of 186 measured launches was slower than with the simple rule of 4 CTAs
+ * up to two structures an SM and one above (the worst 1.05 of its time, 0.81 on
+ * average; populations of 2 and 3 species, 8 to 64, 16 to 24 and 40 to 64
+ * atoms, 40 to 1000 structures, mitr 6 to 500).  ms on one CTA, pairs and
+ * clusters of 4, two and three species of 8 to 64 atoms:
+ *   256 structures, mitr 6    5.7   6.2   9.2     28   25   36
+ *   256             100       103   115   172    223  178  244
+ *   256             500       543   632   926    505  342  279
+ *   400             500       832   942  1442    717  587  822
+ *    40             6         4.7   2.7   2.0     21   11  7.6 */
+extern "C" int mbk_batch_clusters(int S, int mitr, int sms) {
     const double t[3] = {1.0, 0.62, 0.44};
-    const double it = mitr + 1.0, mean = it < 200.0 ? it : 200.0;
+    const double it = mitr + 1.0, mean = it < 80.0 ? it : 80.0, longest = it < 300.0 ? it : 300.0;
     int best = 1;
     double tb = 0.0;
+    if (S > 2 * sms) return 1;
     for (int k = 0; k < 3; k++) {
         const int c = 1 << k, units = sms / c;
         const double work = 0.7 * t[k] * mean * S / units; /* the mean structure costs 0.7 of the largest */
-        const double chain = t[k] * it;
+        const double chain = t[k] * longest;
         const double d = work > chain ? work : chain;
         if (k == 0 || d < tb) {
             tb = d;
@@ -1990,7 +1999,7 @@ extern "C" int mbk_relax_batch(const mb_model *m, mb_batch_ws *ws, int S, const 
     if (e != cudaSuccess) return (int)e;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int wide = 1, csize = batch_clusters(S, mitr, sms);
+    int wide = 1, csize = mbk_batch_clusters(S, mitr, sms);
     {
         /* MAISE_B200_BATCH_WARPS=4 selects the narrow CTA and
          * MAISE_B200_BATCH_CLUSTER=1|2|4 the CTAs per structure (A/B timing) */

@@ -17,6 +17,7 @@ int mbk_relax_batch(const mb_model *m, mb_batch_ws *ws, int S, const int *d_nat,
                     const int *d_order, double *d_lat, double *d_x, double p_ev, double urep, int rlxt, int mitr, double fmax, double *d_H, int *d_iters,
                     int *d_status, double *d_frc, double *d_str, long long *d_evals, void *stream);
 void mbk_batch_free(mb_batch_ws *ws);
+int mbk_batch_clusters(int S, int mitr, int sms); /* CTAs per structure */
 #ifdef __cplusplus
 }
 #endif
