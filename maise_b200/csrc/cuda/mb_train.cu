@@ -558,20 +558,30 @@ static int tr_chunks(mb_train *tr, const int *hfoffs) {
         }
     }
     for (int s = t.nspc; s < 4; s++) coff[s] = n;
+    /* the new layout takes the old one's place only when it is complete */
+    GradChunk *chunks = nullptr;
+    int *dcoff = nullptr;
+    double *part = nullptr;
+    rc = tr_cuda(cudaMalloc((void **)&chunks, sizeof(GradChunk) * (n ? n : 1)), "cudaMalloc chunks");
+    if (!rc) rc = tr_cuda(cudaMalloc((void **)&dcoff, sizeof(coff)), "cudaMalloc coff");
+    if (!rc) rc = tr_cuda(cudaMalloc((void **)&part, sizeof(double) * (size_t)(n ? n : 1) * t.P), "cudaMalloc part");
+    if (!rc) rc = tr_cuda(cudaMemcpy(chunks, h, sizeof(GradChunk) * n, cudaMemcpyHostToDevice), "H2D chunks");
+    if (!rc) rc = tr_cuda(cudaMemcpy(dcoff, coff, sizeof(coff), cudaMemcpyHostToDevice), "H2D coff");
+    free(h);
+    if (rc) {
+        cudaFree(chunks);
+        cudaFree(dcoff);
+        cudaFree(part);
+        return rc;
+    }
     cudaFree(tr->chunks);
     cudaFree(tr->coff);
     cudaFree(tr->part);
-    tr->chunks = nullptr;
-    tr->coff = nullptr;
-    tr->part = nullptr;
+    tr->chunks = chunks;
+    tr->coff = dcoff;
+    tr->part = part;
     tr->nchunk = n;
-    rc = tr_cuda(cudaMalloc((void **)&tr->chunks, sizeof(GradChunk) * (n ? n : 1)), "cudaMalloc chunks");
-    if (!rc) rc = tr_cuda(cudaMalloc((void **)&tr->coff, sizeof(coff)), "cudaMalloc coff");
-    if (!rc) rc = tr_cuda(cudaMalloc((void **)&tr->part, sizeof(double) * (size_t)(n ? n : 1) * t.P), "cudaMalloc part");
-    if (!rc) rc = tr_cuda(cudaMemcpy(tr->chunks, h, sizeof(GradChunk) * n, cudaMemcpyHostToDevice), "H2D chunks");
-    if (!rc) rc = tr_cuda(cudaMemcpy(tr->coff, coff, sizeof(coff), cudaMemcpyHostToDevice), "H2D coff");
-    free(h);
-    return rc;
+    return MB_OK;
 }
 
 extern "C" int mb_train_open(int device, int S, const int *nat, const int *atmn, int nspc, int D, int h1, int h2,
@@ -751,11 +761,12 @@ extern "C" int mb_train_set_forces(mb_train *tr, int NF, const int *f_atom, cons
                 hFn[k] = scale_blocks ? Fn[k] * dr[(size_t)so * t.D + l] : Fn[k];
             }
     }
-    tr->NF = NF;
-    tr->NB = NB;
-    tr->WF = WF;
 #define TA(ptr, n) \
-    if (!rc) rc = tr_cuda(cudaMalloc((void **)&tr->ptr, sizeof(*tr->ptr) * (size_t)(n)), "cudaMalloc " #ptr)
+    if (!rc) { \
+        cudaFree(tr->ptr); /* of an attempt that failed */ \
+        tr->ptr = nullptr; \
+        rc = tr_cuda(cudaMalloc((void **)&tr->ptr, sizeof(*tr->ptr) * (size_t)(n)), "cudaMalloc " #ptr); \
+    }
 #define TC(dst, src, n) \
     if (!rc) rc = tr_cuda(cudaMemcpy(tr->dst, src, sizeof(*tr->dst) * (size_t)(n), cudaMemcpyHostToDevice), "H2D " #dst)
     TA(fatom, NF); TA(boff, NF + 1); TA(bown, NB); TA(bmk, NB); TA(owners, tr->Nown); TA(ooff, tr->Nown + 1);
@@ -766,16 +777,18 @@ extern "C" int mb_train_set_forces(mb_train *tr, int NF, const int *f_atom, cons
     TC(fatom, f_atom, NF); TC(boff, blk_off, NF + 1); TC(bown, blk_atom, NB); TC(bmk, bmk, NB);
     TC(owners, owners, tr->Nown); TC(ooff, ooff, tr->Nown + 1); TC(olist, olist, NB); TC(Fref, F_ref, 3 * NF);
     TC(Fn, hFn, (size_t)NB * t.D * 3); TC(sowners, sown, tr->Nown);
+    cudaFreeHost(tr->h_lf);
+    tr->h_lf = nullptr;
+    if (!rc) rc = tr_cuda(cudaMallocHost((void **)&tr->h_lf, sizeof(double) * NF), "cudaMallocHost");
     if (!rc) rc = tr_chunks(tr, hfoffs);
 #undef TA
 #undef TC
-    /* atoms that own no block keep zero force terms */
-    if (!rc) rc = tr_cuda(cudaMemset(tr->Phi, 0, sizeof(double) * (size_t)t.Na * t.D), "memset");
-    if (!rc) rc = tr_cuda(cudaMemset(tr->Gam, 0, sizeof(double) * (size_t)t.Na * t.h1), "memset");
-    if (!rc) rc = tr_cuda(cudaMemset(tr->fB1, 0, sizeof(double) * (size_t)t.Na * t.h2), "memset");
-    if (!rc) rc = tr_cuda(cudaMemset(tr->fW1, 0, sizeof(double) * (size_t)t.Na * t.h2 * t.h1), "memset");
-    if (!rc) rc = tr_cuda(cudaMemset(tr->fW2, 0, sizeof(double) * (size_t)t.Na * t.h2), "memset");
-    if (!rc) rc = tr_cuda(cudaMallocHost((void **)&tr->h_lf, sizeof(double) * NF), "cudaMallocHost");
+    /* with everything in place, evaluations include the forces */
+    if (!rc) {
+        tr->NF = NF;
+        tr->NB = NB;
+        tr->WF = WF;
+    }
 out:
     free(sat); free(atmn); free(cnt); free(bmk); free(ooff); free(olist); free(owners); free(sown); free(hFn);
     return rc;
