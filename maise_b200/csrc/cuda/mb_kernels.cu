@@ -2662,6 +2662,12 @@ extern "C" int mbk_tri_usable(const mb_dev *d, const mb_model *m) {
 static const EfsShape kTriShapes[] = {{1, 4}, {1, 2}, {2, 1}, {4, 1}, {8, 1}};
 #define MB_NTRISHAPES 5
 
+/* list entries of a warp and shared memory of an atom, for capacity cap */
+extern "C" int mbk_tri_list(int cap, int warps) { return tri_list(cap, warps); }
+extern "C" size_t mbk_tri_smem(int cap, int D, int ns, int ng2, int warps) {
+    return tri_smem_bytes(cap, D, ns, ng2, warps);
+}
+
 static size_t tri_group_bytes(const mb_model *m, int capNB, int wpa) {
     return tri_smem_bytes(capNB, m->P.D, m->P.nspc, m->P.ng2, wpa);
 }
@@ -2721,9 +2727,10 @@ extern "C" int mbk_shape_dims(int tri, int shape, int *wpa, int *apb) {
     return 0;
 }
 
-/* Autotuner: on the first pass of a (mode, size bucket, capacity) the three
- * shapes are each timed once (after an untimed launch) and the fastest is
- * kept for later passes of that key. */
+/* Autotuner: on the first pass of a (mode, size bucket, capacity) the shapes of
+ * the kernel it runs on, k_efs_tri's five or k_efs's three, are each timed once
+ * (after an untimed launch) and the fastest is kept for later passes of that
+ * key. */
 static int tune_key(const mb_dev *d, int N, int mode) {
     int bucket = 0;
     while ((1 << bucket) < N) bucket++;
@@ -2744,46 +2751,38 @@ static void tune_store(mb_dev *d, int key, int val) {
     d->tune_val[d->tune_n++] = val;
 }
 
-/* Decision for a pass that may run on k_efs_tri: its shapes are each timed
- * once (after an untimed launch) and the fastest kept, as 16 + shape.  k_efs,
- * slower at every size measured (32 atoms: 73 us against 40; 487: 199 against
- * 64; 4000: 890 against 375), stands by for shapes that do not fit. */
-static int tune_family(mb_dev *d, const mb_model *m, int N, int mode, const TriArgs &la, const EfsArgs &a,
-                       cudaStream_t st) {
+/* The shape of k_efs_tri for a pass: each is timed once (after an untimed
+ * launch) and the fastest kept, recorded as 16 + shape (k_efs, slower at every
+ * size measured -- 32 atoms: 73 us against 40; 487: 199 against 64; 4000: 890
+ * against 375 -- is not among them; a shape that does not fit is passed over,
+ * and up to MB_TRI_MAX_CAP neighbours one warp an atom always does). */
+static int tune_tri(mb_dev *d, const mb_model *m, int N, int mode, const TriArgs &a, cudaStream_t st) {
     const int key = tune_key(d, N, mode);
     for (int k = 0; k < d->tune_n; k++)
-        if (d->tune_key[k] == key) return d->tune_val[k];
-    int best = 16;
+        if (d->tune_key[k] == key) return d->tune_val[k] - 16;
+    int best = 0;
     if (d->tune_fixed >= 0) {
-        /* a forced shape (of k_efs_tri) is recorded as the decision for this key */
-        best = 16 + (d->tune_fixed < MB_NTRISHAPES ? d->tune_fixed : 0);
+        /* a forced shape is recorded as the decision for this key */
+        best = d->tune_fixed < MB_NTRISHAPES ? d->tune_fixed : 0;
     } else {
-        TriArgs tl = la;
-        EfsArgs te = a;
-        tl.counters = nullptr;
-        te.counters = nullptr;
+        TriArgs t = a;
+        t.counters = nullptr;
         cudaEvent_t e0, e1;
         cudaEventCreate(&e0);
         cudaEventCreate(&e1);
         float best_ms = 1e30f;
-        for (int c = 0; c < MB_NTRISHAPES + MB_NSHAPES; c++) {
-            const bool tri = c < MB_NTRISHAPES;
-            if (!tri && best_ms < 1e30f) break;
-            const int sh = tri ? c : c - MB_NTRISHAPES;
-            const size_t need = tri ? tri_group_bytes(m, la.cap, kTriShapes[sh].wpa) * kTriShapes[sh].apb + TRI_STATIC_SMEM
-                                    : group_bytes(m, a.cap, kShapes[sh].wpa) * kShapes[sh].apb + EFS_STATIC_SMEM;
-            if (need > 227 * 1024) continue;
+        for (int sh = 0; sh < MB_NTRISHAPES; sh++) {
+            if (tri_group_bytes(m, a.cap, kTriShapes[sh].wpa) * kTriShapes[sh].apb + TRI_STATIC_SMEM > 227 * 1024) continue;
             float ms = 1e30f;
             int bad = 0;
             for (int rep = 0; rep < 2 && !bad; rep++) {
                 if (mode == MB_MODE_EFS || mode == MB_MODE_VJP) cudaMemsetAsync(d->F, 0, sizeof(double) * 3 * N, st);
-                bad = tri ? launch_tri_pass(m, sh, tl, st, rep ? e0 : nullptr, rep ? e1 : nullptr)
-                          : launch_any(m, sh, te, st, rep ? e0 : nullptr, rep ? e1 : nullptr);
+                bad = launch_tri_pass(m, sh, t, st, rep ? e0 : nullptr, rep ? e1 : nullptr);
             }
             if (!bad && cudaEventSynchronize(e1) == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
             if (ms < best_ms) {
                 best_ms = ms;
-                best = tri ? 16 + sh : sh;
+                best = sh;
             }
         }
         cudaEventDestroy(e0);
@@ -2791,7 +2790,7 @@ static int tune_family(mb_dev *d, const mb_model *m, int N, int mode, const TriA
         cudaGetLastError();
         d->f_clear = 0; /* the trials added to F */
     }
-    tune_store(d, key, best);
+    tune_store(d, key, 16 + best);
     return best;
 }
 
@@ -2855,7 +2854,6 @@ extern "C" int mbk_descriptor_pass(mb_dev *d, const mb_model *m, int N, int mode
     a.vir = d->vir;
     a.counters = d->counters;
     a.smem_group = 0;
-    int fam = -1; /* k_efs shape chosen against k_efs_tri */
     if (d->tri_on) {
         TriArgs la;
         la.N = N;
@@ -2878,27 +2876,24 @@ extern "C" int mbk_descriptor_pass(mb_dev *d, const mb_model *m, int N, int mode
         la.smem_group = 0;
         la.P = m->P;
         la.T = m->T;
-        const int v = tune_family(d, m, N, mode, la, a, st);
-        if (v >= 16) {
-            d->last_shape = v;
-            cudaEvent_t e0 = 0, e1 = 0;
-            if (d->ev_on && d->ev_n < d->ev_cap) {
-                e0 = ((cudaEvent_t *)d->ev_pool)[2 * d->ev_n];
-                e1 = ((cudaEvent_t *)d->ev_pool)[2 * d->ev_n + 1];
-                d->ev_n++;
-            }
-            if ((mode == MB_MODE_EFS || mode == MB_MODE_VJP) && !d->f_clear)
-                cudaMemsetAsync(d->F, 0, sizeof(double) * 3 * N, st);
-            d->f_clear = 0;
-            const int rc = launch_tri_pass(m, v - 16, la, st, e0, e1);
-            (*launches)++;
-            return rc;
+        const int sh = tune_tri(d, m, N, mode, la, st);
+        d->last_shape = 16 + sh;
+        cudaEvent_t e0 = 0, e1 = 0;
+        if (d->ev_on && d->ev_n < d->ev_cap) {
+            e0 = ((cudaEvent_t *)d->ev_pool)[2 * d->ev_n];
+            e1 = ((cudaEvent_t *)d->ev_pool)[2 * d->ev_n + 1];
+            d->ev_n++;
         }
-        fam = v;
+        if ((mode == MB_MODE_EFS || mode == MB_MODE_VJP) && !d->f_clear)
+            cudaMemsetAsync(d->F, 0, sizeof(double) * 3 * N, st);
+        d->f_clear = 0;
+        const int rc = launch_tri_pass(m, sh, la, st, e0, e1);
+        (*launches)++;
+        return rc;
     }
     d->f_clear = 0;
     cudaMemsetAsync(d->EU, 0, sizeof(double) * N, st);
-    int shape = fam >= 0 ? fam : tune_shape(d, m, N, mode, a, st);
+    int shape = tune_shape(d, m, N, mode, a, st);
     d->last_shape = shape;
     cudaEvent_t e0 = 0, e1 = 0;
     if (d->ev_on && d->ev_n < d->ev_cap) {

@@ -308,7 +308,10 @@ __global__ void __launch_bounds__(256) k_gemm(int M, int N, int K, const float *
 
 extern "C" int surk_gemm(int ta, int tb, int ep, int M, int N, int K, const float *A, int lda, const float *B, int ldb,
                          float *C, int ldc, const float *bias, float *Z, const float *Zp, void *stream) {
-    const bool small = (long)((N + 63) / 64) * ((M + 63) / 64) < 148;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const bool small = (long)((N + 63) / 64) * ((M + 63) / 64) < sms;
     const int gb = small ? 32 : 64;
     dim3 grid((N + gb - 1) / gb, (M + gb - 1) / gb);
     cudaStream_t st = (cudaStream_t)stream;

@@ -373,8 +373,7 @@ __device__ __forceinline__ void gr_product(const double *cf, const int *at, int 
 /* The energy part's coefficients are c_s AD1 for the first layer (c_s of the
  * atom's structure) and c_s W2 (1 - e2^2) for the second: formed here as they
  * are staged.  The outer products run on the FP64 tensor cores, 8 inputs and 16
- * units a warp, so that an input is read once and 8 loads are in flight
- * (GPART_NOTE). */
+ * units a warp, so that an input is read once and 8 loads are in flight. */
 __global__ void __launch_bounds__(256) k_tr_gpart(TrainDims t, const GradChunk *__restrict__ chunks,
                                                   const int *__restrict__ satoms, const int *__restrict__ sowners,
                                                   const int *__restrict__ sat, const double *__restrict__ cs,

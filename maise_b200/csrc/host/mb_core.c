@@ -307,9 +307,8 @@ int mb_tune_read(const mb_potential *p, int cap, int *count, int *mode, int *leg
     n = p->d.tune_n < cap ? p->d.tune_n : cap;
     *count = n;
     for (k = 0; k < n; k++) {
-        /* a key with the fused triplet kernel usable holds 16 + shape when it
-         * won and a k_efs shape otherwise */
-        const int key = p->d.tune_key[k], v = p->d.tune_val[k], lg = ((key >> 26) & 1) && v >= 16;
+        /* a key of the fused triplet kernel holds 16 + shape, one of k_efs its shape */
+        const int key = p->d.tune_key[k], v = p->d.tune_val[k], lg = (key >> 26) & 1;
         mode[k] = key >> 28;
         legs[k] = lg;
         size_bucket[k] = (key >> 20) & 0x3f;

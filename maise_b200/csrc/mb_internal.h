@@ -218,6 +218,8 @@ void mbk_record(void *event, void *stream);
 int mbk_shape_ready(const mb_dev *d, int N, int mode);
 int mbk_tri_usable(const mb_dev *d, const mb_model *m);
 int mbk_shape_dims(int tri, int shape, int *wpa, int *apb);
+int mbk_tri_list(int cap, int warps);
+size_t mbk_tri_smem(int cap, int D, int ns, int ng2, int warps);
 int mbk_graph_cell_nodes(void *graph, void **nodes, int *rows, int cap);
 int mbk_graph_set_cell(void *exec, void *const *nodes, const int *rows, int count, const mb_cell *c, double pV);
 size_t mbk_efs_smem(const mb_model *m, int capNB, int shape);
