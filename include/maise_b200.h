@@ -154,7 +154,7 @@ int mb_relax_fmax(mb_potential *pot, int N, int NM, int ND, const int *atmn, dou
  * reductions.  A structure stops when max |F| < fmax (eV/A) and
  * max |U_ab - pV delta_ab| / N < fmax (eV), or after mitr iterations.
  * The handle keeps the launch's scratch between calls (inverse Hessians and
- * neighbour lists of the resident CTAs, at most 100 MB on a B200, and the
+ * neighbour lists of the resident CTAs, at most 140 MB on a B200, and the
  * call's arrays) and frees it in mb_close.
  * x (Cartesian) and lat are updated in place; H[s] gets the enthalpy,
  * iters[s] the iterations and status[s] 0 (converged), 1 (iteration limit),

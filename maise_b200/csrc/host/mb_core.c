@@ -117,11 +117,11 @@ static int cuda_fail(cudaError_t e, const char *what) {
         if (e_ != cudaSuccess) return cuda_fail(e_, what); \
     } while (0)
 
-/* a size to allocate for `need` bytes where there were `had`: at least half as
- * much again, so that a run of slowly growing calls allocates a few times only */
+/* a size to allocate for `need` bytes where there were `had`: at least twice as
+ * much, so that a run of slowly growing calls allocates a few times only */
 static size_t grown(size_t need, size_t had) {
-    const size_t more = had + had / 2, unit = (size_t)1 << 16;
-    return ((need > more ? need : more) + unit - 1) / unit * unit;
+    const size_t unit = (size_t)1 << 16;
+    return ((need > 2 * had ? need : 2 * had) + unit - 1) / unit * unit;
 }
 
 int mb_ws_grow(mb_ws *w, size_t dev_bytes, size_t host_bytes) {

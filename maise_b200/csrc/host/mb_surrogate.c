@@ -61,34 +61,30 @@ static double sm_normal(uint64_t *s) { /* Box-Muller */
     return sqrt(-2.0 * log(u)) * cos(2.0 * M_PI * w);
 }
 
-/* work buffers for B rows, in one block: with an allocation each
- * the first screen of 2048 structures on a handle took 9 ms, with one 7 */
+/* work buffers for B rows at least, in one block: with an allocation each the
+ * first screen of 2048 structures on a handle took 9 ms, with one 7 */
 static int ensure_rows(mb_surrogate *s, int B) {
-    size_t at = 0, x, tt, z[NL], a[NL], dz[NL];
+    const size_t pad = (2 + 3 * NL) * 256; /* every buffer starts on 256 bytes */
+    size_t row = (size_t)s->nin + 1, at = 0;
     char *w;
-    int l;
+    int l, rows;
     if (B <= s->bcap) return MB_OK;
-#define PUT(name, n) (name = at, at += (sizeof(float) * (size_t)(n) + 255) & ~(size_t)255)
-    PUT(x, (size_t)B * s->nin);
-    PUT(tt, B);
-    for (l = 0; l < NL; l++) {
-        const size_t n = (size_t)B * s->dims[l + 1];
-        PUT(z[l], n);
-        PUT(a[l], n);
-        PUT(dz[l], n);
-    }
-#undef PUT
+    for (l = 0; l < NL; l++) row += 3 * (size_t)s->dims[l + 1];
+    row *= sizeof(float);
     s->bcap = 0;
-    CK((cudaError_t)mb_ws_grow(&s->work, at, 0));
+    CK((cudaError_t)mb_ws_grow(&s->work, B * row + pad, 0));
+    rows = (int)((s->work.dev_len - pad) / row); /* as many as fit */
     w = (char *)s->work.dev;
-    s->x = (float *)(w + x);
-    s->tt = (float *)(w + tt);
+#define TAKE(ptr, n) (ptr = (float *)(w + at), at += (sizeof(float) * (size_t)rows * (n) + 255) & ~(size_t)255)
+    TAKE(s->x, s->nin);
+    TAKE(s->tt, 1);
     for (l = 0; l < NL; l++) {
-        s->z[l] = (float *)(w + z[l]);
-        s->a[l] = (float *)(w + a[l]);
-        s->dz[l] = (float *)(w + dz[l]);
+        TAKE(s->z[l], s->dims[l + 1]);
+        TAKE(s->a[l], s->dims[l + 1]);
+        TAKE(s->dz[l], s->dims[l + 1]);
     }
-    s->bcap = B;
+#undef TAKE
+    s->bcap = rows;
     return MB_OK;
 }
 
@@ -334,7 +330,7 @@ int mb_sur_features(mb_surrogate *s, int S, const int *nat, const int *atmn, con
 static int predict_dev(mb_surrogate *s, int S, const float *d_feat, double *pred) {
     float *y;
     int c0, k, rc;
-    if ((rc = ensure_rows(s, PRED_CHUNK))) return rc;
+    if ((rc = ensure_rows(s, S < PRED_CHUNK ? S : PRED_CHUNK))) return rc;
     CK((cudaError_t)mb_ws_grow(&s->feat, 0, sizeof(float) * (size_t)S));
     y = (float *)s->feat.host;
     for (c0 = 0; c0 < S; c0 += PRED_CHUNK) {

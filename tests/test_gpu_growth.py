@@ -34,7 +34,7 @@ def test_workspace_growth():
     assert lib.mb_ws_grow(ctypes.byref(ws), need // 3, need // 3) == 0  # never shrinks
     assert (ws.dev_len, ws.host_len) == (dev, host)
     lib.mb_ws_free(ctypes.byref(ws))
-    # each block grows by half or more: at most 1 + log(7.2) / log(1.5) = 5.9 sizes
+    # a block at least doubles: at most 1 + log2(7.2) = 3.8 sizes of each, so 12 is generous
     assert len(seen) <= 12
     assert dev <= 2 * need and host <= need
 
@@ -54,5 +54,6 @@ def test_generations_of_growing_size():
         sur.screen(pop[:S])
         free.append(torch.cuda.mem_get_info()[0])
     sur.close()
-    # 13 calls: their features and inputs grow from 200 to 2000 structures in at most 1 + log(10) / log(1.5) steps
+    # 13 calls from 200 to 2000 structures: inputs, features and rows at least double, 1 + log2(10) = 4.3 sizes each,
+    # mostly at the same calls
     assert len(set(free)) <= 7
