@@ -213,7 +213,7 @@ def measured_peaks():
 def profile_traffic():
     """DRAM bytes of one descriptor pass (one ncu capture) from the committed
     summary."""
-    path = os.path.join(ROOT, "profiles", "descriptor_pass_md4000.md")
+    path = os.path.join(ROOT, "profiles", "descriptor_pass_tri_md4000.md")
     try:
         for line in open(path):
             if line.startswith("traffic_bytes_per_pass:"):
