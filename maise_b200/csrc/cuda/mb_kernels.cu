@@ -1775,7 +1775,7 @@ __global__ void __launch_bounds__(WPA * 32 * APB, 512 / (WPA * 32 * APB)) k_efs_
     int *bnd = s.bnd + 8 * warp;
     int pos = 0;
     {
-        int blkid = 0;
+        int blkid = 0, pad = 0;
         const unsigned below = (1u << lane) - 1u;
         for (int al = 0; al < ns; al++)
             for (int be = al; be < ns; be++, blkid++) {
@@ -1808,9 +1808,11 @@ __global__ void __launch_bounds__(WPA * 32 * APB, 512 / (WPA * 32 * APB)) k_efs_
                     }
                 }
                 if (lane < (-pos & 3)) tl[pos + lane] = (unsigned short)TRI_NONE;
+                pad += -pos & 3;
                 pos = (pos + 3) & ~3;
             }
         if (lane == 0) bnd[blkid] = pos;
+        if (A.counters && lane == 0) atomicAdd(&A.counters[1], (unsigned long long)(pos - pad));
     }
     __syncwarp();
 
@@ -1823,11 +1825,10 @@ __global__ void __launch_bounds__(WPA * 32 * APB, 512 / (WPA * 32 * APB)) k_efs_
         double *stw = s.stage + warp * 16 * TRI_STG + lane;
         const double *str = s.stage + warp * 16 * TRI_STG + (lane >> 2) * TRI_STG + (lane & 3);
         double2 *red = reinterpret_cast<double2 *>(s.red + (size_t)warp * nblk * 64) + lane;
-        int blk = 0, nb = bnd[1], nacc = 0;
+        int blk = 0, nb = bnd[1];
         for (int base = 0; base < pos; base += 32) {
             const unsigned ent = base + lane < pos ? tl[base + lane] : TRI_NONE;
             const bool valid = ent != TRI_NONE;
-            nacc += __popc(__ballot_sync(FULL, valid));
             /* padding lanes evaluate entry (0, 0) with weight 0 */
             const unsigned ab = valid ? ent : 0u;
             const double2 *pa = reinterpret_cast<const double2 *>(s.row + TRI_ROW * (ab & 0xffu));
@@ -1867,7 +1868,6 @@ __global__ void __launch_bounds__(WPA * 32 * APB, 512 / (WPA * 32 * APB)) k_efs_
             red[32 * blk] = make_double2(c0, c1);
             c0 = c1 = 0.0;
         }
-        if (A.counters && lane == 0) atomicAdd(&A.counters[1], (unsigned long long)nacc);
         group_sync<WPA>();
         /* descriptors: the warps' sums in warp order; the cells carry the zeta
          * normalisation left out of the angular terms (a power of two) */
