@@ -1899,7 +1899,7 @@ static cudaError_t batch_run(int wide, int csize, int units, cudaStream_t st, co
  * iterations of a population: 1.6% of the iteration counts and status words
  * changed, positions by up to 0.05 A), where results are expected to repeat. */
 static bool batch_tri(const mb_model *m, int mitr) {
-    return mitr == 0 && m->T.ok && m->T.std && m->T.nsq == 2 && m->P.ne <= BNE;
+    return mitr == 0 && m->T.ok && m->T.std && !m->T.steep && m->P.ne <= BNE;
 }
 
 /* Curvature constant of the line search's strong Wolfe test.  The

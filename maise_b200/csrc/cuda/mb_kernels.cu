@@ -1540,13 +1540,12 @@ __device__ inline TriSmem tri_carve(char *p, int cap, int D, int ns, int ng2, in
     return s;
 }
 
-/* exp(-eta_e rho) for e < NE.  NSQ > 0 squarings, or nsq of them (NSQ < 0):
- * the polynomial, whose chains run side by side over one coefficient at a time
- * (two per 16-byte shared load).  NSQ = 0: exp() for the ne exponents there are
- * (steep bases). */
-template <int NE, int NSQ>
-__device__ __forceinline__ void tri_exp(const mb_tri_tab &tab, int nsq, int ne, double rho, double *E) {
-    if constexpr (NSQ == 0) {
+/* exp(-eta_e rho) for e < NE: the polynomial and its two squarings, the chains
+ * side by side over one coefficient at a time (two per 16-byte shared load), or
+ * exp() for the ne exponents there are (EXP, steep bases). */
+template <int NE, bool EXP>
+__device__ __forceinline__ void tri_exp(const mb_tri_tab &tab, int ne, double rho, double *E) {
+    if constexpr (EXP) {
 #pragma unroll
         for (int e = 0; e < NE; e++) E[e] = e < ne ? exp(-tab.eta[e] * rho) : 0.0;
         return;
@@ -1567,16 +1566,10 @@ __device__ __forceinline__ void tri_exp(const mb_tri_tab &tab, int nsq, int ne, 
 #pragma unroll
         for (int e = 0; e < NE; e++) E[e] = fma(E[e], w[e], ck.y);
     }
-    if constexpr (NSQ > 0) {
 #pragma unroll
-        for (int q = 0; q < NSQ; q++)
+    for (int q = 0; q < MB_TRI_SQ; q++)
 #pragma unroll
-            for (int e = 0; e < NE; e++) E[e] *= E[e];
-    } else {
-        for (int q = 0; q < nsq; q++)
-#pragma unroll
-            for (int e = 0; e < NE; e++) E[e] *= E[e];
-    }
+        for (int e = 0; e < NE; e++) E[e] *= E[e];
 }
 
 __device__ __forceinline__ double tri_f(const mb_tri_tab &tab, double v) {
@@ -1637,17 +1630,17 @@ __device__ __forceinline__ int abs_species(int s0, int v, int ns) {
 }
 
 /* NE: exponents evaluated (ne <= NE); WPA: warps per atom; APB: atoms per
- * CTA; STD: the reference's function table (mb_tri), whose powers and
- * squarings are straight-line code (the general form is 20% slower: the
- * branches keep the compiler from interleaving the chains); EXP: exponents too
- * steep for the polynomial, exp() in its place (E/F/S calls of 32, 500 and 4000
- * atoms with exponents up to 1 / A^2: 125, 248 and 972 us on k_efs, 82, 131 and
- * 578 here; up to 8 exponents and all function cells 367, 940 and 6700 against
- * 92, 147 and 677).  All shapes are compiled for 16 resident warps per SM (128
- * registers a thread). */
+ * CTA; STD: the reference's function table (mb_tri), whose powers are
+ * straight-line code (the general form is 20% slower: the branches keep the
+ * compiler from interleaving the chains); EXP: exponents too steep for the
+ * polynomial, exp() in its place (E/F/S calls of 32, 500 and 4000 atoms with
+ * exponents up to 1 / A^2: 120, 245 and 967 us on k_efs, 79, 129 and 574 here;
+ * up to 8 exponents and all function cells 364, 940 and 6727 against 89, 143 and
+ * 676).  All shapes are compiled for 16 resident warps per SM (128 registers a
+ * thread). */
 template <int NE, int WPA, int APB, bool STD, bool EXP>
 __global__ void __launch_bounds__(WPA * 32 * APB, 512 / (WPA * 32 * APB)) k_efs_tri(const __grid_constant__ TriArgs A) {
-    constexpr int NZL = 8, NSQ = EXP ? 0 : STD ? 2 : -1;
+    constexpr int NZL = 8;
     extern __shared__ __align__(16) char smem_raw[];
     __shared__ __align__(16) mb_tri_tab tab; /* polynomial coefficients: 16-byte broadcast loads */
     const mb_params &P = A.P;
@@ -1841,7 +1834,7 @@ __global__ void __launch_bounds__(WPA * 32 * APB, 512 / (WPA * 32 * APB)) k_efs_
             if (!valid) A3 = 0.0;
             double ex[8], lz[NZL];
             ex[7] = 0.0;
-            tri_exp<NE, NSQ>(tab, T.nsq, ne, a2.x + b2.x + s3, ex);
+            tri_exp<NE, EXP>(tab, ne, a2.x + b2.x + s3, ex);
             tri_angular<STD>(P, c, lz, nullptr);
 #pragma unroll
             for (int q = 0; q < 8; q++) {
@@ -2089,7 +2082,7 @@ __global__ void __launch_bounds__(WPA * 32 * APB, 512 / (WPA * 32 * APB)) k_efs_
             const double ir12 = a1.y * q1.y;
             const double c = (a0.x * q0.x + a0.y * q0.y + a1.x * q1.x) * ir12;
             double E[8], lz[NZL], lzp[NZL];
-            tri_exp<NE, NSQ>(tab, T.nsq, ne, a2.x + q2.x + s3, E);
+            tri_exp<NE, EXP>(tab, ne, a2.x + q2.x + s3, E);
             tri_angular<STD>(P, c, lz, lzp);
             double Q = 0.0, Qe = 0.0, Qc = 0.0, eta[8];
 #pragma unroll
@@ -2707,9 +2700,9 @@ static int launch_tri_pass(const mb_model *m, int shape, TriArgs &a, cudaStream_
     a.tlw = tri_list(a.cap, kTriShapes[shape].wpa);
     if (e0) mbk_record(e0, st);
     int rc;
-    if (m->T.nsq == 0)
+    if (m->T.steep)
         rc = m->T.std ? launch_tri_shape<8, true, true>(shape, a, st) : launch_tri_shape<8, false, true>(shape, a, st);
-    else if (m->T.std && m->T.nsq == 2)
+    else if (m->T.std)
         rc = m->P.ne <= 7 ? launch_tri_shape<7, true, false>(shape, a, st) : launch_tri_shape<8, true, false>(shape, a, st);
     else
         rc = launch_tri_shape<8, false, false>(shape, a, st);

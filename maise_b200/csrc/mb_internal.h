@@ -66,14 +66,14 @@ typedef struct {
 /* Tables of the fused triplet kernel (k_efs_tri).  The sum of a triplet's
  * squared legs is rho = r_ij^2 + r_ik^2 + r_jk^2 < 3 Rc^2, so the factor
  * exp(-eta_e rho) of G4 is a smooth function on a known interval: one
- * polynomial of exp(-z) serves every exponent, at z = eta_e rho / 2^nsq, and
- * the result is squared nsq times.  The cutoff f = (1 + cos(pi r / Rc)) / 2
+ * polynomial of exp(-z) serves every exponent, at z = eta_e rho / 4, and the
+ * result is squared twice.  The cutoff f = (1 + cos(pi r / Rc)) / 2
  * and h = f'(r) / r are entire functions of r^2: polynomials in
  * 2 r^2 / Rc^2 - 1.  Coefficients are stored highest degree first. */
 #define MB_TRI_MAXE 8
 #define MB_TRI_DEG 11  /* exp: truncation below 2e-17 for z within +-0.42 of its middle */
 #define MB_TRI_FDEG 11 /* f and h: truncation below 1e-18 */
-#define MB_TRI_MAXSQ 4
+#define MB_TRI_SQ 2    /* squarings */
 #define MB_TRI_LOW 3
 typedef struct {
     double ex[MB_TRI_DEG + 1];    /* exp(-z), z = zmid (1 + w) */
@@ -84,9 +84,9 @@ typedef struct {
 } mb_tri_tab;
 typedef struct {
     mb_tri_tab tab;
-    /* the basis qualifies for k_efs_tri; squarings (at least 2), or 0: an
-     * exponent is too steep for the polynomial (or negative), exp() is called */
-    int ok, nsq;
+    /* the basis qualifies for k_efs_tri; an exponent is too steep for the
+     * polynomial, or negative: exp() is called */
+    int ok, steep;
     /* the reference's function table: zeta = 1, 2, 4, 16, lambda = -1, 1,
      * and the first MB_TRI_LOW exponents used with zeta = 1, 2 only */
     int std;
