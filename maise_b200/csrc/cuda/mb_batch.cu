@@ -792,25 +792,32 @@ __device__ __forceinline__ float ex2f(float x) {
 
 /* The cutoff in w = 1 - r^2 / Rc^2: f = cos^2(pi r / 2 Rc) has a double zero
  * at w = 0, so f = w^2 q(w) and f'(r) / r = -(2 / Rc^2) w g(w) with q and g
- * smooth and positive on [0, 1]: interpolated at 6 Chebyshev nodes, relative
- * errors 1.4e-9 and 5.7e-9.  No square root, division or trigonometry, and
- * accurate relative to f up to the cutoff. */
+ * smooth and positive on [0, 1]: polynomials of degree 5, relative errors below
+ * 6e-9 before rounding.  No square root, division or trigonometry, and accurate
+ * relative to f up to the cutoff.  The leading coefficient of q rounds to 2.9e-8
+ * below its value; the others are fitted one after the other to the rounded
+ * ones before them, for q 0.5e-8 and g 0.2e-8 high from w = 0.15 on: with three
+ * cutoffs a triplet that offsets the rounding of the products and the mean of
+ * ex2.approx, which is 2e-8 to 5e-8 below 2^x.  With every coefficient rounded
+ * to nearest each term was 1.5e-7 low, and the energy of 2-species populations
+ * off by a median 5.3e-7 eV/atom (now 1.2e-7, atom_pass 1.3e-7), forces by
+ * 5.9e-7 of the largest (4.9e-7, 4.7e-7). */
 __device__ __forceinline__ float cut_f(float w) {
-    float q = 4.25195744e-05f;
-    q = fmaf(q, w, 6.47454464e-04f);
-    q = fmaf(q, w, 8.10431821e-03f);
-    q = fmaf(q, w, 6.59302329e-02f);
-    q = fmaf(q, w, 3.08425200e-01f);
-    q = fmaf(q, w, 6.16850274e-01f);
+    float q = 4.33553760e-05f;
+    q = fmaf(q, w, 6.44999440e-04f);
+    q = fmaf(q, w, 8.10699258e-03f);
+    q = fmaf(q, w, 6.59289137e-02f);
+    q = fmaf(q, w, 3.08425486e-01f);
+    q = fmaf(q, w, 6.16850257e-01f);
     return w * w * q;
 }
 __device__ __forceinline__ float cut_g(float w) {
-    float g = 3.03081031e-04f;
-    g = fmaf(g, w, 3.87248896e-03f);
-    g = fmaf(g, w, 4.05310985e-02f);
-    g = fmaf(g, w, 2.63717965e-01f);
-    g = fmaf(g, w, 9.25275916e-01f);
-    g = fmaf(g, w, 1.23370054e+00f);
+    float g = 3.08439427e-04f;
+    g = fmaf(g, w, 3.85633856e-03f);
+    g = fmaf(g, w, 4.05491404e-02f);
+    g = fmaf(g, w, 2.63708830e-01f);
+    g = fmaf(g, w, 9.25277948e-01f);
+    g = fmaf(g, w, 1.23370039e+00f);
     return w * g;
 }
 
